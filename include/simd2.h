@@ -148,9 +148,10 @@ int simd2_closure_batched(simd2_op op, int count, float* const* X, const int* n,
                           simd2_conv conv, int* iters_out, cudaStream_t stream);
 
 /* Kernel configurations of the CUDA-core path (min/max semirings):
- * config = s | (skip << 2), split-K factor 1 << s (s in 0..3) over a
- * thread-block cluster whose CTAs fold their partial tiles through
- * distributed shared memory, and skip = 1 to drop k-blocks whose A or B block
+ * config = s | (skip << 2), split-K factor 1 << s (s in 0..3; s = 0 leaves the
+ * split to the persistent kernel, s > 0 forces a thread-block cluster whose
+ * CTAs fold their partial tiles through distributed shared memory), and
+ * skip = 1 to drop k-blocks whose A or B block
  * holds only the (x)-annihilator (block occupancy computed per call; applies
  * to min_plus, max_plus, max_min, min_max).  All configurations give the same
  * bits.  No reference counterpart: the autotuner and the learned dispatch
@@ -161,8 +162,8 @@ int simd2_srgemm_tuned(simd2_op op, int M, int N, int K,
                        int do_epilogue, int config, cudaStream_t stream);
 
 typedef enum simd2_dispatch {
-  SIMD2_DISPATCH_DENSE = 0,   /* no block skipping; split-K chosen from the tile count
-                                 (the plain autotuned dense path) */
+  SIMD2_DISPATCH_DENSE = 0,   /* no block skipping: the persistent kernel, which spreads each
+                                 step over the SMs by k-tile units (the plain dense path) */
   SIMD2_DISPATCH_FIXED = 1,   /* `fixed_config` every step (8: sparse steps, see below) */
   SIMD2_DISPATCH_LEARNED = 2, /* the MLP cost model picks each step's config, sparse or dense */
   SIMD2_DISPATCH_RULES = 3    /* the hand-written policy: sparse steps under fixed
@@ -204,7 +205,9 @@ int simd2_closure_ex(simd2_op op, int n, float* X, int ldx, int max_iter, simd2_
  * below n_min[0] the dense path keeps its rule (the largest split with
  * tiles * split <= SMs, at most 4).  count = 0 clears the table.  Applies to
  * simd2_closure and to SIMD2_DISPATCH_DENSE of simd2_closure_ex in this
- * process; same bits whatever the split. */
+ * process; same bits whatever the split.  The factor is what step_configs
+ * reports; the persistent kernel that runs these steps spreads each one over
+ * the SMs by itself, whatever the factor. */
 int simd2_set_dense_configs(const int* n_min, const int* config, int count);
 
 /* Cost-model MLP (15-32-32-1, ReLU) kernels.  X: [batch][15] features+config,

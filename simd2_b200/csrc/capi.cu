@@ -11,6 +11,7 @@
 #include <tuple>
 #include <mutex>
 #include <atomic>
+#include <cmath>
 #include <type_traits>
 #include <utility>
 #include <vector>
@@ -18,6 +19,7 @@
 #include "common.cuh"
 #include "prep.cuh"
 #include "srgemm_simt.cuh"
+#include "srgemm_sk.cuh"
 #include "tc_gemm.cuh"
 #include "tc_gemm2.cuh"
 #include "closure_batched.cuh"
@@ -198,20 +200,83 @@ float add_identity(int op) {
 // Padding value for out-of-range k: NaN products vanish under min/max.
 float pad_value(int op) { return is_sum_op(op) ? 0.0f : __builtin_nanf(""); }
 
+// SM count of the current device (asked once per device).
+int device_sms() {
+  static std::atomic<int> cached[64];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
+  int n = cached[dev].load(std::memory_order_relaxed);
+  if (n == 0) {
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n < 1) n = 148;
+    n = std::min(n, kSkMaxCounters / 2);  // a split leaves fewer than 2 n tiles to count
+    cached[dev].store(n, std::memory_order_relaxed);
+  }
+  return n;
+}
+
 // ---------------------------------------------------------------------------
 // srgemm plan: workspace layout for one call
 // ---------------------------------------------------------------------------
+// How srgemm_sk_kernel spreads a product: tile size, CTAs, and the tiles each
+// CTA computes alone before the rest is split by k-tile units.
+struct SkShape {
+  int tile, tiles_m, tiles_n, grid, whole;
+};
+
+// Tile size.  The 128 x 128 tile runs the inner loop at 117 (x)(+) pairs per
+// clock and SM (min_plus 4096^3, codes), the 64 x 64 one, which meets its k-tile
+// barriers four times as often, at 100; but the small tile cuts a small product
+// into four times as many pieces.  Measured (min_plus, us, 128 / 64): 36 big
+// tiles (700^3) 33 / 31, 64 (1024^3) 53 / 59, 256 (2048^3) 283 / 326: the line
+// lies at a third of a big tile per SM.
+//
+// Split.  With at least as many tiles as SMs, every CTA takes the same number
+// of whole tiles and the rest is split evenly by units, so no wave is partly
+// empty (2048^3: 256 tiles on 148 SMs, 381 us in two waves, 283 split).  With
+// fewer tiles, an equal number of CTAs per tile where that occupies at least
+// three quarters of the SMs -- few contributors per tile keep the fold short
+// (512^3 on 64 x 64 tiles: 2 CTAs per tile 17.6 us, an even split of all units
+// over 148 CTAs 21.5) -- else the even split.  More CTAs per tile than
+// sqrt(4 * k-tiles) lose more in the fold than they gain (30 x 30 x 3000:
+// 12 CTAs 20.0 us, 23 22.6, 46 30).
+SkShape sk_shape(int M, int N, int K, bool code16) {
+  const int sms = device_sms();
+  SkShape p{};
+  const long long big = (long long)((M + 127) / 128) * ((N + 127) / 128);
+  p.tile = 3 * big >= sms ? 128 : 64;
+  p.tiles_m = (M + p.tile - 1) / p.tile;
+  p.tiles_n = (N + p.tile - 1) / p.tile;
+  const int bk = code16 ? kSkBK16 : kBK;
+  const long long tiles = (long long)p.tiles_m * p.tiles_n, kt = (K + bk - 1) / bk;
+  if (tiles >= sms) {
+    p.grid = sms;
+    p.whole = (int)(tiles / sms - (tiles % sms ? 1 : 0));
+    return p;
+  }
+  const long long fold_max = std::max(1LL, (long long)std::sqrt(4.0 * (double)kt));
+  const long long per_tile = std::min({(long long)sms / tiles, fold_max, kt});
+  if (per_tile < fold_max && per_tile < kt && 4 * tiles * per_tile < 3 * sms) p.grid = (int)std::min<long long>(sms, tiles * kt);
+  else p.grid = (int)(tiles * per_tile);
+  p.whole = p.grid == tiles ? 1 : 0;
+  return p;
+}
+
 struct Plan {
   int Kp, Np;
   size_t bp_off, bp_bytes;  // interleaved B'
   size_t ap_off, ap_bytes;  // packed A (0 when TMA reads A in place)
-  int Kh;                   // FP16 selection path: K padded to 64 (0 = path off)
-  size_t ah_off, bh_off, flag_off;
+  bool full;                // the parts below exist
+  bool code16;              // 16-bit copies exist
+  int Kh;                   // K padded to 64
+  size_t a16_off, b16_off, note_off, cnt_off, part_off;
+  SkShape shape;
   size_t total;
 };
 
-// `half` reserves the FP16 selection path's operands (max_min / min_max).
-Plan make_plan(int M, int N, int K, bool pack_a, bool half = false) {
+// full: the parts srgemm_sk_kernel needs to split tiles between CTAs and, for
+// an op with 16-bit codes, the coded operands; without it the kernel runs
+// whole tiles on FP32 operands from B' (and packed A) alone.
+Plan make_plan(int M, int N, int K, bool pack_a, bool full = false, int op = SIMD2_MAX_MUL) {
   Plan p{};
   p.Kp = round_up(std::max(K, 1), kBK);
   p.Np = round_up(std::max(N, 1), kBN);
@@ -220,12 +285,20 @@ Plan make_plan(int M, int N, int K, bool pack_a, bool half = false) {
   p.ap_off = p.bp_bytes;
   p.ap_bytes = pack_a ? align_up((size_t)M * p.Kp * 4, kAlign) : 0;
   p.total = p.ap_off + p.ap_bytes;
-  if (half) {
-    p.Kh = round_up(std::max(K, 1), kH2BK);
-    p.ah_off = p.total;
-    p.bh_off = p.ah_off + align_up((size_t)M * p.Kh * 2, kAlign);
-    p.flag_off = p.bh_off + align_up((size_t)(p.Kh / 2) * p.Np * 4, kAlign);
-    p.total = p.flag_off + kAlign;
+  p.full = full;
+  p.code16 = full && has_code16(op);
+  p.shape = sk_shape(std::max(M, 1), std::max(N, 1), std::max(K, 1), p.code16);
+  if (full) {
+    p.Kh = round_up(std::max(K, 1), kSkBK16);
+    p.a16_off = p.total;
+    p.b16_off = p.a16_off + (p.code16 ? align_up((size_t)M * p.Kh * 2, kAlign) : 0);
+    p.note_off = p.b16_off + (p.code16 ? align_up((size_t)(p.Kh / 2) * p.Np * 4, kAlign) : 0);
+    p.cnt_off = p.note_off + align_up(kSkMaxPrepBlocks * 4, kAlign);
+    p.part_off = p.cnt_off + align_up(kSkMaxCounters * 4, kAlign);
+    // two slots per CTA when tiles are split
+    const long long tiles = (long long)p.shape.tiles_m * p.shape.tiles_n;
+    const bool split = tiles > (long long)p.shape.whole * p.shape.grid;
+    p.total = p.part_off + (split ? (size_t)2 * p.shape.grid * p.shape.tile * p.shape.tile * 4 : 0);
   }
   return p;
 }
@@ -243,7 +316,6 @@ struct SimtConfig {
   bool skip = false;
   const uint8_t* occA = nullptr;
   const uint8_t* occB = nullptr;
-  bool count_ops = true;  // false when an alternative kernel of the same call already counts them
 };
 
 // The (x)-annihilator whose products equal the (+)-identity: blocks made only
@@ -268,31 +340,26 @@ int launch_simt_cfg(int M, int N, int K, const CUtensorMap& mA, const CUtensorMa
   if (dev < 0 || dev >= 64) return SIMD2_ERR_NO_DEVICE;
   if (!configured[dev]) {
     SIMD2_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    if (SPLIT > 1) SIMD2_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    SIMD2_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     configured[dev] = true;
   }
   const int tiles_m = (M + kBM - 1) / kBM;
   const int tiles_n = (N + kBN - 1) / kBN;
-  auto* ev = prof_slot(cfg.count_ops ? 2LL * M * N * K : 0LL);
+  auto* ev = prof_slot(2LL * M * N * K);
   if (ev) cudaEventRecord(ev->first, stream);
-  if constexpr (SPLIT == 1) {
-    kern<<<tiles_m * tiles_n, kSimtThreads, smem, stream>>>(mA, mB, M, N, K, ep, tiles_m, tiles_n, cfg.occA,
-                                                            cfg.occB);
-  } else {
-    cudaLaunchConfig_t lc = {};
-    lc.gridDim = dim3(tiles_m * tiles_n * SPLIT);
-    lc.blockDim = dim3(kSimtThreads);
-    lc.dynamicSmemBytes = smem;
-    lc.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = SPLIT;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    lc.attrs = attr;
-    lc.numAttrs = 1;
-    SIMD2_CUDA_TRY(cudaLaunchKernelEx(&lc, kern, mA, mB, M, N, K, ep, tiles_m, tiles_n, cfg.occA, cfg.occB));
-  }
+  cudaLaunchConfig_t lc = {};
+  lc.gridDim = dim3(tiles_m * tiles_n * SPLIT);
+  lc.blockDim = dim3(kSimtThreads);
+  lc.dynamicSmemBytes = smem;
+  lc.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = SPLIT;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  lc.attrs = attr;
+  lc.numAttrs = 1;
+  SIMD2_CUDA_TRY(cudaLaunchKernelEx(&lc, kern, mA, mB, M, N, K, ep, tiles_m, tiles_n, cfg.occA, cfg.occB));
   count_launch();
   if (ev) cudaEventRecord(ev->second, stream);
   SIMD2_CUDA_TRY(cudaGetLastError());
@@ -303,7 +370,6 @@ template <int OP, bool SKIP>
 int launch_simt_split(int M, int N, int K, const CUtensorMap& mA, const CUtensorMap& mB, const EpilogueArgs& ep,
                       const SimtConfig& cfg, cudaStream_t stream) {
   switch (cfg.split) {
-    case 1: return launch_simt_cfg<OP, 1, SKIP>(M, N, K, mA, mB, ep, cfg, stream);
     case 2: return launch_simt_cfg<OP, 2, SKIP>(M, N, K, mA, mB, ep, cfg, stream);
     case 4: return launch_simt_cfg<OP, 4, SKIP>(M, N, K, mA, mB, ep, cfg, stream);
     case 8: return launch_simt_cfg<OP, 8, SKIP>(M, N, K, mA, mB, ep, cfg, stream);
@@ -416,99 +482,173 @@ int compute_step_stats(int op, int n, const float* X, long long ldx, uint8_t* ba
   return SIMD2_OK;
 }
 
-// FP16 selection path (max_min / min_max): on the device, check that A and B
-// hold only FP16 values; if so the packed-half kernel runs, else the FP32
-// kernel (both are enqueued, each gated by one of the two flags, so the call
-// stays asynchronous).  Same bits either way.
-int enqueue_half_path(int op, int M, int N, int K, const float* A, long long lda, const float* B, long long ldb,
-                      const EpilogueArgs& ep, uint8_t* ws, const Plan& plan, cudaStream_t stream) {
-  int* flags = reinterpret_cast<int*>(ws + plan.flag_off);
-  auto* Ah = reinterpret_cast<__half*>(ws + plan.ah_off);
-  auto* Bh = reinterpret_cast<__half2*>(ws + plan.bh_off);
-  // the FP16 copies are made unconditionally and clear flags[0] when an entry
-  // is not exactly an FP16 value; then flags[1] = !flags[0] gates the FP32 path
-  fp16_flags_init_kernel<<<1, 1, 0, stream>>>(flags);
-  pack_half_rows_kernel<<<grid_for((long long)M * plan.Kh / 8), 256, 0, stream>>>(A, lda, M, K, Ah, plan.Kh, ep.gate,
-                                                                              flags);
-  interleave_half_kernel<<<grid_for((long long)(plan.Kh / 2) * plan.Np / 4), 256, 0, stream>>>(B, ldb, K, N, Bh, plan.Kh,
-                                                                                            plan.Np, ep.gate, flags);
-  fp16_flags_finish_kernel<<<1, 1, 0, stream>>>(flags);
-  for (int i = 0; i < 4; i++) count_launch();
-  SIMD2_CUDA_TRY(cudaGetLastError());
-  CUtensorMap mA, mB;
-  int rc = make_map_2d(&mA, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, Ah, M, plan.Kh, plan.Kh, kH2BK, kBM,
-                       CU_TENSOR_MAP_SWIZZLE_128B);
-  if (rc) return rc;
-  rc = make_map_2d(&mB, CU_TENSOR_MAP_DATA_TYPE_UINT32, 4, Bh, plan.Kh / 2, plan.Np, plan.Np, kBN, kH2BK / 2,
-                   CU_TENSOR_MAP_SWIZZLE_NONE);
-  if (rc) return rc;
-  EpilogueArgs eh = ep;
-  eh.gate2 = flags;
-  const int tiles_m = (M + kBM - 1) / kBM;
-  const int tiles_n = (N + kBN - 1) / kBN;
-  const size_t smem = simt_smem_bytes(kSimtStages);
+template <int OP, int TILE>
+int launch_sk_tile(const CUtensorMap& a16, const CUtensorMap& b16, const CUtensorMap& a32, const CUtensorMap& b32,
+                   const SkArgs& args, int grid, const EpilogueArgs& ep, cudaStream_t stream) {
+  auto kern = srgemm_sk_kernel<OP, TILE>;
+  static bool configured[64] = {};
   int dev = 0;
   SIMD2_CUDA_TRY(cudaGetDevice(&dev));
-  static bool configured[2][64] = {};
-  const int which = op == SIMD2_MAX_MIN ? 0 : 1;
-  auto kern = op == SIMD2_MAX_MIN ? srgemm_h2_kernel<SIMD2_MAX_MIN> : srgemm_h2_kernel<SIMD2_MIN_MAX>;
   if (dev < 0 || dev >= 64) return SIMD2_ERR_NO_DEVICE;
-  if (!configured[which][dev]) {
-    SIMD2_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    configured[which][dev] = true;
+  if (!configured[dev]) {
+    SIMD2_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SkCfg<TILE>::kSmem));
+    configured[dev] = true;
   }
-  auto* ev = prof_slot(2LL * M * N * K);
+  auto* ev = prof_slot(2LL * args.M * args.N * args.K);
   if (ev) cudaEventRecord(ev->first, stream);
-  kern<<<tiles_m * tiles_n, kSimtThreads, smem, stream>>>(mA, mB, M, N, K, eh, tiles_m, tiles_n);
+  kern<<<grid, kSimtThreads, SkCfg<TILE>::kSmem, stream>>>(a16, b16, a32, b32, args, ep);
   count_launch();
   if (ev) cudaEventRecord(ev->second, stream);
   SIMD2_CUDA_TRY(cudaGetLastError());
   return SIMD2_OK;
 }
 
-// Core float srgemm with an explicit workspace.  T/MODE describe how A and B
-// are read (float as-is, or any type normalised to {0,1}).
-template <typename T, int MODE>
-int srgemm_core(int op, int M, int N, int K, const T* A, long long lda, const T* B, long long ldb,
+template <int OP>
+int launch_sk_skip(const CUtensorMap& a16, const CUtensorMap& b16, const CUtensorMap& a32, const CUtensorMap& b32,
+                   const SkSkipArgs& args, const EpilogueArgs& ep, cudaStream_t stream) {
+  auto kern = srgemm_sk_skip_kernel<OP>;
+  static bool configured[64] = {};
+  int dev = 0;
+  SIMD2_CUDA_TRY(cudaGetDevice(&dev));
+  if (dev < 0 || dev >= 64) return SIMD2_ERR_NO_DEVICE;
+  if (!configured[dev]) {
+    SIMD2_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SkCfg<128>::kSmem));
+    configured[dev] = true;
+  }
+  const int grid = (int)std::min<long long>((long long)args.tiles_m * args.tiles_n, device_sms());
+  auto* ev = prof_slot(2LL * args.M * args.N * args.K);
+  if (ev) cudaEventRecord(ev->first, stream);
+  kern<<<grid, kSimtThreads, SkCfg<128>::kSmem, stream>>>(a16, b16, a32, b32, args, ep);
+  count_launch();
+  if (ev) cudaEventRecord(ev->second, stream);
+  SIMD2_CUDA_TRY(cudaGetLastError());
+  return SIMD2_OK;
+}
+
+// One product on srgemm_sk_kernel (with cfg.skip or change maps to write, on
+// srgemm_sk_skip_kernel): the operand preparation, then the kernel.
+template <int OP>
+int launch_sk(int M, int N, int K, const float* A, long long lda, const float* B, long long ldb,
+              const EpilogueArgs& ep, uint8_t* ws, const Plan& plan, bool pack_a, const SimtConfig& cfg,
+              cudaStream_t stream) {
+  const bool skip = cfg.skip || ep.chgA;
+  SkShape sh = plan.shape;
+  if (skip) sh = {128, (M + 127) / 128, (N + 127) / 128, 0, 0};
+  const long long tiles = (long long)sh.tiles_m * sh.tiles_n;
+  const bool split = !skip && plan.full && tiles > (long long)sh.whole * sh.grid;
+  SkPrepArgs pa{};
+  pa.A = A, pa.lda = lda, pa.B = B, pa.ldb = ldb, pa.M = M, pa.N = N, pa.K = K;
+  pa.Kh = plan.Kh, pa.Kp = plan.Kp, pa.Np = plan.Np;
+  pa.B32 = reinterpret_cast<float*>(ws + plan.bp_off);
+  pa.A32 = pack_a ? reinterpret_cast<float*>(ws + plan.ap_off) : nullptr;
+  pa.pad = pad_value(OP);
+  pa.gate = ep.gate;
+  long long items = (long long)(plan.Kp / 2) * plan.Np / 4;
+  if (plan.code16) {
+    pa.A16 = reinterpret_cast<uint16_t*>(ws + plan.a16_off);
+    pa.B16 = reinterpret_cast<uint32_t*>(ws + plan.b16_off);
+    pa.notes = reinterpret_cast<unsigned*>(ws + plan.note_off);
+    items = std::max(items, (long long)M * plan.Kh / 8);
+  }
+  if (pack_a) items = std::max(items, (long long)M * plan.Kp / 4);
+  if (split || skip) {
+    pa.counters = reinterpret_cast<int*>(ws + plan.cnt_off);
+    pa.ncounters = skip ? 1 : (int)(tiles - (long long)sh.whole * sh.grid);
+  }
+  const int prep_grid = (int)std::max(1LL, std::min<long long>((items + 255) / 256, kSkMaxPrepBlocks));
+  sk_prep_kernel<OP><<<prep_grid, 256, 0, stream>>>(pa);
+  count_launch();
+  SIMD2_CUDA_TRY(cudaGetLastError());
+  const int t = sh.tile;
+  CUtensorMap a16{}, b16{}, a32, b32;
+  int rc;
+  if (plan.code16) {
+    if ((rc = make_map_2d(&a16, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, pa.A16, M, plan.Kh, plan.Kh, kSkBK16, t,
+                          CU_TENSOR_MAP_SWIZZLE_128B)))
+      return rc;
+    if ((rc = make_map_2d(&b16, CU_TENSOR_MAP_DATA_TYPE_UINT32, 4, pa.B16, plan.Kh / 2, plan.Np, plan.Np, t,
+                          kSkBK16 / 2, CU_TENSOR_MAP_SWIZZLE_NONE)))
+      return rc;
+  }
+  if ((rc = make_map_f32(&a32, pack_a ? pa.A32 : A, M, pack_a ? plan.Kp : K, pack_a ? plan.Kp : lda, kBK, t,
+                         CU_TENSOR_MAP_SWIZZLE_128B, true)))
+    return rc;
+  if ((rc = make_map_f32(&b32, pa.B32, plan.Kp / 2, 2LL * plan.Np, 2LL * plan.Np, 2 * t, kBK / 2,
+                         CU_TENSOR_MAP_SWIZZLE_NONE, false)))
+    return rc;
+  if (skip) {
+    if constexpr (has_code16(OP)) {
+      SkSkipArgs sa{};
+      sa.M = M, sa.N = N, sa.K = K;
+      sa.tiles_m = sh.tiles_m, sa.tiles_n = sh.tiles_n;
+      sa.notes = pa.notes;
+      sa.nnotes = prep_grid;
+      sa.queue = pa.counters;
+      sa.occA = cfg.skip ? cfg.occA : nullptr;
+      sa.occB = cfg.skip ? cfg.occB : nullptr;
+      return launch_sk_skip<OP>(a16, b16, a32, b32, sa, ep, stream);
+    }
+    return SIMD2_ERR_UNSUPPORTED;  // every op that skips blocks has codes
+  }
+  SkArgs ga{};
+  ga.M = M, ga.N = N, ga.K = K;
+  ga.tiles_m = sh.tiles_m, ga.tiles_n = sh.tiles_n;
+  ga.whole = sh.whole;
+  ga.notes = pa.notes;
+  ga.nnotes = prep_grid;
+  ga.counters = pa.counters;
+  ga.part = split ? reinterpret_cast<float*>(ws + plan.part_off) : nullptr;
+  const int grid = split ? sh.grid : (int)std::min<long long>(tiles, device_sms());
+  return t == 128 ? launch_sk_tile<OP, 128>(a16, b16, a32, b32, ga, grid, ep, stream)
+                  : launch_sk_tile<OP, 64>(a16, b16, a32, b32, ga, grid, ep, stream);
+}
+
+// Core float srgemm of the min/max semirings with an explicit workspace (a full
+// plan for anything but the plain configuration).  A forced split-K factor runs
+// on srgemm_simt_kernel, everything else on the persistent kernels.
+int srgemm_core(int op, int M, int N, int K, const float* A, long long lda, const float* B, long long ldb,
                 const EpilogueArgs& ep, uint8_t* ws, const Plan& plan, bool pack_a, cudaStream_t stream,
                 const SimtConfig& cfg = SimtConfig()) {
-  const float pad = pad_value(op);
-  float* Bp = reinterpret_cast<float*>(ws + plan.bp_off);
-  const int* path_gate = nullptr;  // gates the FP32 path when the FP16 path is enqueued too
-  if constexpr (MODE == 0 && std::is_same<T, float>::value) {
-    if (plan.Kh > 0 && selection_op(op) && cfg.split == 1 && !cfg.skip) {
-      int rc = enqueue_half_path(op, M, N, K, A, lda, B, ldb, ep, ws, plan, stream);
-      if (rc) return rc;
-      path_gate = reinterpret_cast<const int*>(ws + plan.flag_off) + 1;
+  SimtConfig c1 = cfg;
+  c1.skip = cfg.skip && cfg.occA && cfg.occB && skip_supported(op);
+  if (cfg.split == 1) {
+    switch (op) {
+#define SIMD2_SK_CASE(OPV) \
+  case OPV: return launch_sk<OPV>(M, N, K, A, lda, B, ldb, ep, ws, plan, pack_a, c1, stream);
+      SIMD2_SK_CASE(SIMD2_MIN_PLUS)
+      SIMD2_SK_CASE(SIMD2_MAX_PLUS)
+      SIMD2_SK_CASE(SIMD2_MAX_MIN)
+      SIMD2_SK_CASE(SIMD2_MAX_MUL)
+      SIMD2_SK_CASE(SIMD2_MIN_MUL)
+      SIMD2_SK_CASE(SIMD2_MIN_MAX)
+#undef SIMD2_SK_CASE
+      default: return SIMD2_ERR_UNSUPPORTED;
     }
   }
-  EpilogueArgs ep32 = ep;
-  ep32.gate2 = path_gate;
-  SimtConfig cfg32 = cfg;
-  if (path_gate) cfg32.count_ops = false;  // the FP16 kernel's slot carries the operation count
-  interleave_pairs_kernel<T, MODE><<<grid_for((long long)plan.Kp / 2 * plan.Np / 4), 256, 0, stream>>>(
-      B, ldb, K, N, Bp, plan.Kp, plan.Np, pad, ep.gate, path_gate);
+  const float pad = pad_value(op);
+  float* Bp = reinterpret_cast<float*>(ws + plan.bp_off);
+  interleave_pairs_kernel<float, 0><<<grid_for((long long)plan.Kp / 2 * plan.Np / 4), 256, 0, stream>>>(
+      B, ldb, K, N, Bp, plan.Kp, plan.Np, pad, ep.gate);
   count_launch();
   SIMD2_CUDA_TRY(cudaGetLastError());
   const void* a_base = A;
   long long a_pitch = lda;
   if (pack_a) {
     float* Ap = reinterpret_cast<float*>(ws + plan.ap_off);
-    pack_rows_kernel<T, MODE><<<grid_for((long long)M * plan.Kp), 256, 0, stream>>>(A, lda, M, K, Ap, plan.Kp, pad,
-                                                                                    ep.gate, path_gate);
+    pack_rows_kernel<float, 0><<<grid_for((long long)M * plan.Kp), 256, 0, stream>>>(A, lda, M, K, Ap, plan.Kp, pad,
+                                                                                    ep.gate);
     count_launch();
     SIMD2_CUDA_TRY(cudaGetLastError());
     a_base = Ap;
     a_pitch = plan.Kp;
   }
   CUtensorMap mA, mB;
-  int rc = make_map_f32(&mA, a_base, M, pack_a ? plan.Kp : K, a_pitch, kBK, kBM, CU_TENSOR_MAP_SWIZZLE_128B,
-                        !is_sum_op(op));
+  int rc = make_map_f32(&mA, a_base, M, pack_a ? plan.Kp : K, a_pitch, kBK, kBM, CU_TENSOR_MAP_SWIZZLE_128B, true);
   if (rc) return rc;
   rc = make_map_f32(&mB, Bp, plan.Kp / 2, 2LL * plan.Np, 2LL * plan.Np, 2 * kBN, kBK / 2, CU_TENSOR_MAP_SWIZZLE_NONE,
                     false);
   if (rc) return rc;
-  return dispatch_simt(op, M, N, K, mA, mB, ep32, cfg32, stream);
+  return dispatch_simt(op, M, N, K, mA, mB, ep, cfg, stream);
 }
 
 // ---------------------------------------------------------------------------
@@ -806,9 +946,8 @@ int srgemm_f32_ws(int op, int M, int N, int K, const float* A, long long lda, co
     return srgemm_tc_sum(op, M, N, K, A, lda, B, ldb, C, ldc, D, ldd, do_epilogue, ws, tp, stream);
   }
   const bool pack_a = !a_tma_ok(A, lda);
-  // the FP16 selection path needs workspace beyond the base plan, so it is
-  // only planned when the library provides the workspace itself
-  const Plan plan = make_plan(M, N, K, pack_a, ws_or_null == nullptr && selection_op(op));
+  // a caller's workspace holds the base plan only
+  const Plan plan = make_plan(M, N, K, pack_a, ws_or_null == nullptr, op);
   uint8_t* ws = ws_or_null;
   if (!ws) {
     void* p = nullptr;
@@ -817,7 +956,7 @@ int srgemm_f32_ws(int op, int M, int N, int K, const float* A, long long lda, co
     ws = static_cast<uint8_t*>(p);
   }
   const EpilogueArgs ep = make_epilogue(C, ldc, D, ldd, do_epilogue, changed, conv);
-  return srgemm_core<float, 0>(op, M, N, K, A, lda, B, ldb, ep, ws, plan, pack_a, stream);
+  return srgemm_core(op, M, N, K, A, lda, B, ldb, ep, ws, plan, pack_a, stream);
 }
 
 // or_and on the INT8 tensor cores (0/1 bytes, S32 counts), exact.
@@ -936,7 +1075,7 @@ int closure_gated(int op, int n, float* X, long long ldx, int max_iter, int conv
         cudaEventRecord(a, stream);
       }
       SimtConfig cfg;
-      cfg.split = fixed ? config_split(fixed_cfg) : auto_split;
+      cfg.split = fixed ? config_split(fixed_cfg) : 1;
       cfg.skip = fixed && config_skip(fixed_cfg) && can_skip && need_occ;
       if (cfg.skip) {
         // occupancy of a gated-off step is harmless work on an unchanged matrix
@@ -944,15 +1083,16 @@ int closure_gated(int op, int n, float* X, long long ldx, int max_iter, int conv
         cfg.occA = obase + occ.occA;
         cfg.occB = obase + occ.occB;
       }
-      if (step_cfg) step_cfg[t] = (cfg.skip ? 4 : 0) | (cfg.split == 1 ? 0 : cfg.split == 2 ? 1 : cfg.split == 4 ? 2 : 3);
+      const int rep_split = fixed ? cfg.split : auto_split;
+      if (step_cfg) step_cfg[t] = (cfg.skip ? 4 : 0) | (rep_split == 1 ? 0 : rep_split == 2 ? 1 : rep_split == 4 ? 2 : 3);
       // A operand: X_t (repeated squaring) or the fixed adjacency A0 (Bellman-Ford form)
       const float* Aop = A0 ? A0 : cur;
       const long long lda_op = A0 ? lda0 : ldcur;
       const bool pk = !a_tma_ok(Aop, lda_op);
-      const Plan pl = make_plan(n, n, n, pk, selection_op(op));
+      const Plan pl = make_plan(n, n, n, pk, true, op);
       EpilogueArgs ep = make_epilogue(cur, ldcur, nxt, ldnxt, 1, changed + t, conv);
       ep.gate = gate;
-      if ((rc = srgemm_core<float, 0>(op, n, n, n, Aop, lda_op, cur, ldcur, ep, ws, pl, pk, stream, cfg))) break;
+      if ((rc = srgemm_core(op, n, n, n, Aop, lda_op, cur, ldcur, ep, ws, pl, pk, stream, cfg))) break;
       if (step_ms) cudaEventRecord(evs.back(), stream);
     }
     if (rc) break;
@@ -1050,7 +1190,7 @@ int closure_f32_ex(int op, int n, float* X, long long ldx, int max_iter, int con
   const bool need_occ = dispatch == 2 || step_feat != nullptr || (fixed_skip && can_skip);
   // Workspace: [srgemm plan][Xnew n x n][flag + decision][occupancy]
   const bool pack_a = !a_tma_ok(X, ldx) || (n % 4 != 0);
-  const Plan plan = make_plan(n, n, n, pack_a, selection_op(op));
+  const Plan plan = make_plan(n, n, n, pack_a, true, op);
   const OccPlan occ = make_occ_plan(n, n, n, true);
   const size_t x_off = align_up(plan.total, kAlign);
   const size_t f_off = x_off + align_up((size_t)n * n * 4, kAlign);
@@ -1206,14 +1346,16 @@ int closure_f32_ex(int op, int n, float* X, long long ldx, int max_iter, int con
   }
   while (changed && it < max_iter) {
     SimtConfig cfg;
-    cfg.split = config_split(cfg_id);
+    // the persistent kernel spreads a step over the SMs by itself; only a fixed
+    // configuration forces its split factor
+    cfg.split = dispatch == 1 ? config_split(cfg_id) : 1;
     const bool delta = use_delta && prev_chg && (occ_fresh || occ_full);
     cfg.skip = can_skip && ((config_skip(cfg_id) && occ_on) || delta);
     if (cfg.skip) {
       cfg.occA = obase + occ.occA;
       cfg.occB = obase + occ.occB;
     }
-    if (step_cfg) step_cfg[it] = (cfg.skip ? 4 : 0) | (cfg.split == 1 ? 0 : cfg.split == 2 ? 1 : cfg.split == 4 ? 2 : 3);
+    if (step_cfg) step_cfg[it] = (cfg.skip ? 4 : 0) | (cfg_id & 3);
     const float step_occ_ms = (occ_on && cfg.skip) ? occ_ms : 0.f;  // a skip step pays for its occupancy pass
     if (cudaMemsetAsync(flag, 0, sizeof(int), stream) != cudaSuccess) {
       rc = SIMD2_ERR_CUDA;
@@ -1221,7 +1363,7 @@ int closure_f32_ex(int op, int n, float* X, long long ldx, int max_iter, int con
     }
     if (step_ms) cudaEventRecord(ev[0], stream);
     const bool pk = !a_tma_ok(cur, ldcur);
-    const Plan pl = make_plan(n, n, n, pk, selection_op(op));
+    const Plan pl = make_plan(n, n, n, pk, true, op);
     EpilogueArgs ep = make_epilogue(cur, ldcur, nxt, ldnxt, 1, flag, conv);
     if (use_delta) {
       if (cudaMemsetAsync(chg[par][0], 0, cmA + cmB, stream) != cudaSuccess) {
@@ -1235,7 +1377,7 @@ int closure_f32_ex(int op, int n, float* X, long long ldx, int max_iter, int con
         ep.dB = chg[par ^ 1][1];
       }
     }
-    rc = srgemm_core<float, 0>(op, n, n, n, cur, ldcur, cur, ldcur, ep, ws, pl, pk, stream, cfg);
+    rc = srgemm_core(op, n, n, n, cur, ldcur, cur, ldcur, ep, ws, pl, pk, stream, cfg);
     if (rc) break;
     if (step_ms) cudaEventRecord(ev[1], stream);
     it++;
@@ -2269,8 +2411,10 @@ int simd2_mst(int n, const float* W, int ldw, int* edges, float* weights, int* c
 
 int simd2_reserve_workspace(simd2_op op, int M, int N, int K, cudaStream_t stream, size_t* bytes_out) {
   if (M < 0 || N < 0 || K < 0 || (int)op < 0 || (int)op > 8) return SIMD2_ERR_INVALID_ARG;
-  const Plan plan = make_plan(M, N, K, true);
-  size_t total = plan.total + 2 * align_up((size_t)M * N * 4, kAlign) + kAlign;
+  const Plan plan = make_plan(M, N, K, true, true, op);
+  // a smaller product may be cut into larger partial tiles than this one
+  const size_t part = (size_t)2 * device_sms() * kBM * kBN * 4;
+  size_t total = plan.total + part + 2 * align_up((size_t)M * N * 4, kAlign) + kAlign;
   void* p = nullptr;
   int rc = get_workspace(stream, total, &p);
   if (bytes_out) *bytes_out = rc ? 0 : total;
@@ -2554,7 +2698,7 @@ int simd2_srgemm_tuned(simd2_op op, int M, int N, int K, const float* A, int lda
   if ((rc = check_device())) return rc;
   if (K == 0) return srgemm_k0(op, M, N, C, ldc, D, ldd, do_epilogue, stream);
   const bool pack_a = !a_tma_ok(A, lda);
-  const Plan plan = make_plan(M, N, K, pack_a);
+  const Plan plan = make_plan(M, N, K, pack_a, true, op);
   const bool skip = config_skip(config) && skip_supported(op) && (K + kBK - 1) / kBK <= kMaxSkipKtiles;
   const OccPlan occ = make_occ_plan(M, N, K, false);
   const size_t o_off = align_up(plan.total, kAlign);
@@ -2570,7 +2714,7 @@ int simd2_srgemm_tuned(simd2_op op, int M, int N, int K, const float* A, int lda
     cfg.occB = ws + o_off + occ.occB;
   }
   const EpilogueArgs ep = make_epilogue(C, ldc, D, ldd, do_epilogue, nullptr, 0);
-  return srgemm_core<float, 0>(op, M, N, K, A, lda, B, ldb, ep, ws, plan, pack_a, stream, cfg);
+  return srgemm_core(op, M, N, K, A, lda, B, ldb, ep, ws, plan, pack_a, stream, cfg);
 }
 
 int simd2_closure_ex(simd2_op op, int n, float* X, int ldx, int max_iter, simd2_conv conv, simd2_dispatch dispatch,
@@ -3075,7 +3219,7 @@ extern "C" int simd2_closure_bf(simd2_op op, int n, const float* A0, int lda0, f
   int dev = 0, sms = 148;
   SIMD2_CUDA_TRY(cudaGetDevice(&dev));
   SIMD2_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  const Plan plan = make_plan(n, n, n, true, selection_op(op));
+  const Plan plan = make_plan(n, n, n, true, true, op);
   const OccPlan occ = make_occ_plan(n, n, n, true);
   const size_t x_off = align_up(plan.total, kAlign);
   const size_t f_off = x_off + align_up((size_t)n * n * 4, kAlign);

@@ -86,13 +86,13 @@ struct EpilogueArgs {
   int conv_mode;  // simd2_conv, used with `changed`
   const int* gate;  // nullable: when *gate == 0 the kernel does nothing (closure
                     // step enqueued after the fixed point was reached)
-  const int* gate2;  // nullable second gate (the FP16 / FP32 path choice)
-  // Closure delta steps (square M = N = K, srgemm_simt_kernel only): chgA /
+  // Closure delta steps (square M = N = K, srgemm_sk_skip_kernel only): chgA /
   // chgB, when set, receive a 1 for every 32 x 32 block of D that differs from
-  // C, in the layouts of the occupancy maps (chgA[tile row][k-tile] for the
-  // block's rows as an A block, chgB[k-tile][tile column] as a B block); dA /
-  // dB, when set, are the previous step's maps, and a SKIP kernel keeps only
-  // the k-tiles whose A or B block changed in that step.
+  // C, in the layouts of the occupancy maps (chgA[tile row][k block] for the
+  // block's rows as an A block, chgB[k block][tile column] as a B block); dA /
+  // dB, when set, are the maps of the step that made C = X_t: every product of
+  // two blocks unchanged in it was a product of that step too and is already
+  // folded into X_t, so with a min / max (+) the next step may leave it out.
   uint8_t* chgA;
   uint8_t* chgB;
   const uint8_t* dA;
@@ -133,8 +133,9 @@ __device__ __forceinline__ float ld_dsmem_f32(const float* local_ptr, uint32_t r
   return v;
 }
 
-// One CTA (or one CTA of a SPLIT-wide cluster) per 128 x 128 output tile.
-//   SPLIT > 1 : the cluster's CTAs take every SPLIT-th k-tile of the tile's
+// SPLIT = 2, 4 or 8 CTAs of a cluster per 128 x 128 output tile (the forced
+// split-K configurations; srgemm_sk.cuh runs everything else).
+//   SPLIT     : the cluster's CTAs take every SPLIT-th k-tile of the tile's
 //               k list, park their partial tile in shared memory, and each
 //               CTA then folds 128/SPLIT rows of all partials (read through
 //               distributed shared memory) with (+) and runs the epilogue on
@@ -142,12 +143,7 @@ __device__ __forceinline__ float ld_dsmem_f32(const float* local_ptr, uint32_t r
 //   SKIP      : the k list holds only the k-tiles whose A block (128 rows x
 //               32 k) and B block (32 k x 128 columns) both contain an entry
 //               other than the (x)-annihilator (occupancy maps occA, occB);
-//               a skipped block can only produce identity products.  With
-//               ep.dA / ep.dB (a closure step X_{t+1} = X_t (+) X_t (x) X_t
-//               whose C is X_t) it also needs the A or the B block to have
-//               changed in step t: every product of unchanged blocks was a
-//               product of step t too and is already folded into X_t, so with
-//               a min / max (+) it cannot change the result.
+//               a skipped block can only produce identity products.
 template <int OP, int STAGES, int SPLIT, bool SKIP>
 __global__ void __launch_bounds__(kSimtThreads, 1)
     srgemm_simt_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, int M,
@@ -155,7 +151,7 @@ __global__ void __launch_bounds__(kSimtThreads, 1)
                        const uint8_t* __restrict__ occB) {
   // A closure step enqueued after the previous step reported no change does
   // nothing; every CTA (every cluster member) sees the same word.
-  if ((ep.gate && *ep.gate == 0) || (ep.gate2 && *ep.gate2 == 0)) return;
+  if (ep.gate && *ep.gate == 0) return;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + STAGES * kStageBytes);
@@ -165,7 +161,7 @@ __global__ void __launch_bounds__(kSimtThreads, 1)
 
   // Grouped raster: 8 consecutive tile rows share each B' column panel in L2.
   const int tile = blockIdx.x / SPLIT;
-  const int rank = SPLIT > 1 ? (int)cluster_ctarank() : 0;
+  const int rank = (int)cluster_ctarank();
   const int group = 8;
   const int per_group = group * tiles_n;
   const int g = tile / per_group;
@@ -195,8 +191,7 @@ __global__ void __launch_bounds__(kSimtThreads, 1)
     int running = 0;
     for (int base = 0; base < ktiles; base += kSimtThreads) {
       const int kt = base + threadIdx.x;
-      const bool f = kt < ktiles && occA[(long long)tm * ktiles + kt] && occB[(long long)kt * tiles_n + tn] &&
-                     (!ep.dA || ep.dA[(long long)tm * ktiles + kt] || ep.dB[(long long)kt * tiles_n + tn]);
+      const bool f = kt < ktiles && occA[(long long)tm * ktiles + kt] && occB[(long long)kt * tiles_n + tn];
       const unsigned ballot = __ballot_sync(0xffffffffu, f);
       if (lane == 0) s_warp_cnt[warp] = __popc(ballot);
       __syncthreads();
@@ -301,7 +296,6 @@ __global__ void __launch_bounds__(kSimtThreads, 1)
     // Every issued copy must land before this CTA's shared memory is released.
     if (threadIdx.x == 0)
       for (int i = max(0, issued - STAGES); i < issued; i++) mbar_wait(&full[i % STAGES], (i / STAGES) & 1);
-    if constexpr (SPLIT == 1) return;
   }
 
   // ---------------- epilogue ----------------
@@ -312,280 +306,43 @@ __global__ void __launch_bounds__(kSimtThreads, 1)
   float* Dbase = ep.D;
   const long long ldc = ep.ldc, ldd = ep.ldd;
   int changed = 0;
-  // bit 4 g + c: an element of the tile's 32 x 32 block (row group g, column
-  // group c) changed (used only when ep.chgA is set)
-  uint32_t bmask = 0;
 
-  if constexpr (SPLIT == 1) {
-    const int vec2 = ep.vec2;
-    // The thread's C pairs are loaded first, all in flight together (each
-    // load-then-use pair in turn would wait out the memory latency 16 times).
-    float2 cpre[8][WN];
-#pragma unroll
-    for (int i = 0; i < 8; i++) {
-      const int row = m0 + ty + 16 * i;
-#pragma unroll
-      for (int c = 0; c < WN; c++) {
-        const int col = n0 + cbase + 32 * c + 2 * tx;
-        cpre[i][c] = (do_epi && vec2 && row < M && col + 1 < N)
-                         ? *reinterpret_cast<const float2*>(Cbase + (long long)row * ldc + col)
-                         : make_float2(0.f, 0.f);
-      }
-    }
-#pragma unroll
-    for (int i = 0; i < 8; i++) {
-      const int row = m0 + ty + 16 * i;
-      if (row < M) {
-        const float* crow = Cbase + (long long)row * ldc;
-        float* drow = Dbase + (long long)row * ldd;
-#pragma unroll
-        for (int c = 0; c < WN; c++) {
-          const int col = n0 + cbase + 32 * c + 2 * tx;
-          int ch = 0;
-          if (vec2 && col + 1 < N) {
-            const float2 cv = cpre[i][c];
-            float2 v;
-            v.x = epilogue_value<OP>(do_epi, conv_mode, track, acc[i][2 * c], cv.x, ch);
-            v.y = epilogue_value<OP>(do_epi, conv_mode, track, acc[i][2 * c + 1], cv.y, ch);
-            *reinterpret_cast<float2*>(drow + col) = v;
-          } else {
-#pragma unroll
-            for (int e = 0; e < 2; e++) {
-              if (col + e < N) {
-                const float cv = do_epi ? crow[col + e] : 0.0f;
-                drow[col + e] = epilogue_value<OP>(do_epi, conv_mode, track, acc[i][2 * c + e], cv, ch);
-              }
-            }
-          }
-          if (ch) {
-            changed = 1;
-            bmask |= 1u << (((i >> 1) << 2) | ((cbase >> 5) + c));  // row ty + 16 i lies in group i / 2
-          }
-        }
-      }
-    }
-  } else {
-    // Park the partial tile (row-major 128 x 128, padded rows) in the now idle stage memory.
-    constexpr int kPitch = kBN + 4;
-    float* part = reinterpret_cast<float*>(smem);
-    __syncthreads();
-#pragma unroll
-    for (int i = 0; i < 8; i++)
-#pragma unroll
-      for (int c = 0; c < WN; c++) {
-        const int r = ty + 16 * i, col = cbase + 32 * c + 2 * tx;
-        part[r * kPitch + col] = acc[i][2 * c];
-        part[r * kPitch + col + 1] = acc[i][2 * c + 1];
-      }
-    cluster_sync_all();  // every partial is in place
-    constexpr int kRows = kBM / SPLIT;
-    for (int e = threadIdx.x; e < kRows * kBN; e += kSimtThreads) {
-      const int r = rank * kRows + e / kBN;
-      const int col = e % kBN;
-      float v = part[r * kPitch + col];
-#pragma unroll
-      for (int peer = 0; peer < SPLIT; peer++)
-        if (peer != rank) v = Mac<OP>::add(v, ld_dsmem_f32(part + r * kPitch + col, (uint32_t)peer));
-      const int row = m0 + r, gcol = n0 + col;
-      if (ok && row < M && gcol < N) {
-        const float cv = do_epi ? Cbase[(long long)row * ldc + gcol] : 0.0f;
-        int ch = 0;
-        Dbase[(long long)row * ldd + gcol] = epilogue_value<OP>(do_epi, conv_mode, track, v, cv, ch);
-        if (ch) {
-          changed = 1;
-          bmask |= 1u << (((r >> 5) << 2) | (col >> 5));
-        }
-      }
-    }
-    cluster_sync_all();  // peers stay resident until every CTA has read their partials
-  }
-  if (track) {
-    if (__any_sync(0xffffffffu, changed) && lane == 0) atomicOr(ep.changed, 1);
-  }
-  if (ep.chgA) {
-    // every writer stores 1, so no atomics; a set bit implies an element
-    // inside the matrix, so both indices are in range
-    const uint32_t m = __reduce_or_sync(0xffffffffu, bmask);
-    if (lane == 0 && m) {
-#pragma unroll
-      for (int q = 0; q < 4; q++) {
-        if (m & (0x1111u << q)) ep.chgA[(long long)tm * ktiles + 4 * tn + q] = 1;  // column group q
-        if (m & (0xfu << (4 * q))) ep.chgB[(long long)(4 * tm + q) * tiles_n + tn] = 1;  // row group q
-      }
-    }
-  }
-}
-
-// ---------------------------------------------------------------------------
-// FP16 selection kernel for max_min / min_max.  Used when every entry of A and
-// B is exactly an FP16 value: (x) and (+) only select, so every product and
-// every accumulator value is one of those FP16 values and the result is
-// bit-identical to the FP32 computation.  Packed min/max.f16x2 handle two k
-// values per lane per instruction (2 ALU instructions per 2 pairs instead of
-// 3).  A is half [M][Kp] (128-byte swizzled TMA tiles of 128 rows x 64 k),
-// B is k-pair words [Kp/2][Np] (tiles of 32 pair-rows x 128 words); the
-// two halves of each accumulator hold the even- and odd-k partial results.
-// ---------------------------------------------------------------------------
-constexpr int kH2BK = 64;  // k per stage
-
-__device__ __forceinline__ uint32_t hmin2u(uint32_t a, uint32_t b) {
-  uint32_t r;
-  asm("min.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
-  return r;
-}
-__device__ __forceinline__ uint32_t hmax2u(uint32_t a, uint32_t b) {
-  uint32_t r;
-  asm("max.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
-  return r;
-}
-
-template <int OP>
-__global__ void __launch_bounds__(kSimtThreads, 1)
-    srgemm_h2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, int M, int N,
-                     int K, EpilogueArgs ep, int tiles_m, int tiles_n) {
-  static_assert(OP == SIMD2_MAX_MIN || OP == SIMD2_MIN_MAX, "selection semirings only");
-  constexpr int STAGES = kSimtStages;
-  if ((ep.gate && *ep.gate == 0) || (ep.gate2 && *ep.gate2 == 0)) return;
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint64_t* full = reinterpret_cast<uint64_t*>(smem + STAGES * kStageBytes);
-  uint64_t* empty = full + STAGES;
-
-  const int group = 8;
-  const int per_group = group * tiles_n;
-  const int g = blockIdx.x / per_group;
-  const int first_m = g * group;
-  const int gsize = min(tiles_m - first_m, group);
-  const int local = blockIdx.x - g * per_group;
-  const int m0 = (first_m + local % gsize) * kBM;
-  const int n0 = (local / gsize) * kBN;
-  const int ktiles = (K + kH2BK - 1) / kH2BK;
-  const int warp = threadIdx.x >> 5;
-  const int lane = threadIdx.x & 31;
-
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < STAGES; s++) {
-      mbar_init(&full[s], 1);
-      mbar_init(&empty[s], kSimtWarps);
-    }
-    fence_mbar_init();
-  }
+  // Park the partial tile (row-major 128 x 128, padded rows) in the now idle stage memory.
+  constexpr int kPitch = kBN + 4;
+  float* part = reinterpret_cast<float*>(smem);
   __syncthreads();
-  if (threadIdx.x == 0) {
-    prefetch_tensormap(&tmA);
-    prefetch_tensormap(&tmB);
-    for (int kt = 0; kt < min(STAGES, ktiles); kt++) {
-      uint8_t* sa = smem + kt * kStageBytes;
-      mbar_arrive_expect_tx(&full[kt], kStageBytes);
-      tma_load_2d(sa, &tmA, &full[kt], kt * kH2BK, m0);
-      tma_load_2d(sa + kATileBytes, &tmB, &full[kt], n0, kt * (kH2BK / 2));
-    }
-  }
-
-  const int tx = lane & 15;
-  const int ty = (warp & 7) * 2 + (lane >> 4);
-  const int cbase = (warp >> 3) * 64;
-  const int swz = ty & 7;
-  // identity of (+) in both halves: -inf (max) or +inf (min)
-  const uint32_t ident = OP == SIMD2_MAX_MIN ? 0xfc00fc00u : 0x7c007c00u;
-  uint32_t acc[8][4];
 #pragma unroll
   for (int i = 0; i < 8; i++)
 #pragma unroll
-    for (int j = 0; j < 4; j++) acc[i][j] = ident;
-
-  bool ok = true;
-  int issued = min(STAGES, ktiles);
-  for (int kt = 0; kt < ktiles; kt++) {
-    const int s = kt % STAGES;
-    if (threadIdx.x == 0 && kt >= 1 && kt - 1 + STAGES < ktiles) {
-      const int r = kt - 1, rs = r % STAGES;
-      if (mbar_wait(&empty[rs], (r / STAGES) & 1)) {
-        uint8_t* sa = smem + rs * kStageBytes;
-        const int nk = r + STAGES;
-        mbar_arrive_expect_tx(&full[rs], kStageBytes);
-        tma_load_2d(sa, &tmA, &full[rs], nk * kH2BK, m0);
-        tma_load_2d(sa + kATileBytes, &tmB, &full[rs], n0, nk * (kH2BK / 2));
-        issued = nk + 1;
-      } else {
-        report_timeout(3);
-      }
+    for (int c = 0; c < WN; c++) {
+      const int r = ty + 16 * i, col = cbase + 32 * c + 2 * tx;
+      part[r * kPitch + col] = acc[i][2 * c];
+      part[r * kPitch + col + 1] = acc[i][2 * c + 1];
     }
-    if (!mbar_wait(&full[s], (kt / STAGES) & 1)) {
-      report_timeout(4);
-      ok = false;
-      break;
-    }
-    const uint8_t* As = smem + s * kStageBytes;                               // 128 rows x 128 bytes
-    const uint32_t* Bs = reinterpret_cast<const uint32_t*>(As + kATileBytes);  // 32 rows x 128 words
-#pragma unroll 2
-    for (int q = 0; q < 8; q++) {  // 16-byte chunk q = k pairs 4q .. 4q+3
-      uint4 a[8];
+  cluster_sync_all();  // every partial is in place
+  constexpr int kRows = kBM / SPLIT;
+  for (int e = threadIdx.x; e < kRows * kBN; e += kSimtThreads) {
+    const int r = rank * kRows + e / kBN;
+    const int col = e % kBN;
+    float v = part[r * kPitch + col];
 #pragma unroll
-      for (int i = 0; i < 8; i++)
-        a[i] = *reinterpret_cast<const uint4*>(As + (ty + 16 * i) * 128 + ((q ^ swz) << 4));
-#pragma unroll
-      for (int h = 0; h < 4; h++) {
-        const int pr = 4 * q + h;
-        uint2 b[2];
-#pragma unroll
-        for (int c = 0; c < 2; c++) b[c] = *reinterpret_cast<const uint2*>(Bs + pr * kBN + cbase + 32 * c + 2 * tx);
-#pragma unroll
-        for (int i = 0; i < 8; i++) {
-          const uint32_t ap = h == 0 ? a[i].x : h == 1 ? a[i].y : h == 2 ? a[i].z : a[i].w;
-#pragma unroll
-          for (int c = 0; c < 2; c++) {
-            if constexpr (OP == SIMD2_MAX_MIN) {
-              acc[i][2 * c] = hmax2u(acc[i][2 * c], hmin2u(ap, b[c].x));
-              acc[i][2 * c + 1] = hmax2u(acc[i][2 * c + 1], hmin2u(ap, b[c].y));
-            } else {
-              acc[i][2 * c] = hmin2u(acc[i][2 * c], hmax2u(ap, b[c].x));
-              acc[i][2 * c + 1] = hmin2u(acc[i][2 * c + 1], hmax2u(ap, b[c].y));
-            }
-          }
-        }
-      }
-    }
-    __syncwarp();
-    if (lane == 0) mbar_arrive(&empty[s]);
-  }
-  if (!ok) {
-    if (threadIdx.x == 0)
-      for (int kt = max(0, issued - STAGES); kt < issued; kt++) mbar_wait(&full[kt % STAGES], (kt / STAGES) & 1);
-    return;
-  }
-
-  const int do_epi = ep.do_epilogue;
-  const int conv_mode = ep.conv_mode;
-  const bool track = ep.changed != nullptr;
-  int changed = 0;
-#pragma unroll
-  for (int i = 0; i < 8; i++) {
-    const int row = m0 + ty + 16 * i;
-    if (row < M) {
-      const float* crow = ep.C + (long long)row * ep.ldc;
-      float* drow = ep.D + (long long)row * ep.ldd;
-#pragma unroll
-      for (int c = 0; c < 2; c++) {
-#pragma unroll
-        for (int e = 0; e < 2; e++) {
-          const int col = n0 + cbase + 32 * c + 2 * tx + e;
-          if (col < N) {
-            const uint32_t w = acc[i][2 * c + e];
-            const float lo = __half2float(__ushort_as_half((unsigned short)(w & 0xffffu)));
-            const float hi = __half2float(__ushort_as_half((unsigned short)(w >> 16)));
-            const float v = Semiring<OP>::add(lo, hi);
-            const float cv = do_epi ? crow[col] : 0.0f;
-            drow[col] = epilogue_value<OP>(do_epi, conv_mode, track, v, cv, changed);
-          }
-        }
-      }
+    for (int peer = 0; peer < SPLIT; peer++)
+      if (peer != rank) v = Mac<OP>::add(v, ld_dsmem_f32(part + r * kPitch + col, (uint32_t)peer));
+    const int row = m0 + r, gcol = n0 + col;
+    if (ok && row < M && gcol < N) {
+      const float cv = do_epi ? Cbase[(long long)row * ldc + gcol] : 0.0f;
+      int ch = 0;
+      Dbase[(long long)row * ldd + gcol] = epilogue_value<OP>(do_epi, conv_mode, track, v, cv, ch);
+      changed |= ch;
     }
   }
+  cluster_sync_all();  // peers stay resident until every CTA has read their partials
   if (track) {
     if (__any_sync(0xffffffffu, changed) && lane == 0) atomicOr(ep.changed, 1);
   }
 }
+
+constexpr int kH2BK = 64;  // k per stage of the batched FP16 kernel
 
 // Block occupancy of X (rows x cols) in wide strips, optionally with entry
 // counts.  A CTA of 256 threads covers 128 rows x 512 columns: warp w reads
