@@ -303,8 +303,6 @@ Plan make_plan(int M, int N, int K, bool pack_a, bool full = false, int op = SIM
   return p;
 }
 
-bool selection_op(int op) { return op == SIMD2_MAX_MIN || op == SIMD2_MIN_MAX; }
-
 bool a_tma_ok(const void* A, long long lda) {
   return (reinterpret_cast<uintptr_t>(A) % 16 == 0) && ((lda * 4) % 16 == 0);
 }
@@ -1427,71 +1425,48 @@ struct BatchedPlan {
   int op;
   int count;
   int max_iter;
-  int conv;
-  void* mem;            // one device allocation: descriptors, maps, order, queue, buffers
-  BatchGraph* d_graphs;
-  BatchMaps* d_maps;
-  int* d_order;
-  int* d_queue;
-  bool fp16;            // FP16 copies exist (max_min / min_max, change test other than APLP)
-  int* d_fp16_bad;      // set by the FP16 prep when an entry is not an FP16 value
+  void* mem;            // one device allocation: descriptors, maps, order, state, entries, buffers
+  BatchArgs args;
+  void* cleared;        // state and control words, zeroed before every run
+  size_t cleared_bytes;
+  size_t slot_bytes;    // slots past the first steps'
+  int grid;             // CTAs of the closure kernel
+  int prep_x;           // blocks per graph of the prep and finish kernels
   std::vector<BatchGraph> host;
 };
 
-template <int OP, bool H2>
-int launch_batched(BatchedPlan* p, cudaStream_t stream) {
-  auto kern = H2 ? closure_batched_h2_kernel<(OP == SIMD2_MIN_MAX ? SIMD2_MIN_MAX : SIMD2_MAX_MIN)>
-                 : closure_batched_kernel<OP>;
-  const size_t smem = simt_smem_bytes(kSimtStages);
+template <int OP>
+int batched_run_op(BatchedPlan* p, cudaStream_t stream) {
+  auto kern = closure_batched_kernel<OP>;
+  constexpr size_t smem = SkCfg<128>::kSmem;
   static bool configured[64] = {};
+  if (p->dev < 0 || p->dev >= 64) return SIMD2_ERR_NO_DEVICE;
   if (!configured[p->dev]) {
     SIMD2_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     configured[p->dev] = true;
   }
-  int sms = 0;
-  SIMD2_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p->dev));
-  const int grid = std::max(1, std::min(sms, p->count));
-  kern<<<grid, kSimtThreads, smem, stream>>>(p->d_graphs, p->d_maps, p->d_order, p->count, p->d_queue, p->max_iter,
-                                             p->conv, p->fp16 ? p->d_fp16_bad : nullptr);
-  count_launch();
+  const dim3 pg(p->prep_x, std::min(p->count, 65535));
+  batched_prep_kernel<OP><<<pg, 256, 0, stream>>>(p->args);
+  kern<<<p->grid, kSimtThreads, smem, stream>>>(p->args);
+  batched_finish_kernel<OP><<<pg, 256, 0, stream>>>(p->args);
+  for (int i = 0; i < 3; i++) count_launch();
   SIMD2_CUDA_TRY(cudaGetLastError());
   return SIMD2_OK;
 }
 
 int batched_run(BatchedPlan* p, cudaStream_t stream) {
-  SIMD2_CUDA_TRY(cudaMemsetAsync(p->d_queue, 0, sizeof(int), stream));
-  dim3 pg(64, std::min(p->count, 65535));
-  const int* bad = p->fp16 ? p->d_fp16_bad : nullptr;
-  if (p->fp16) {
-    // FP16 copies first; they flag an entry that is not an FP16 value, and the
-    // FP32 prep and kernel below run only then (the FP16 kernel otherwise)
-    SIMD2_CUDA_TRY(cudaMemsetAsync(p->d_fp16_bad, 0, sizeof(int), stream));
-    batched_prep_h_kernel<<<pg, 256, 0, stream>>>(p->d_graphs, p->count, p->d_fp16_bad);
-    count_launch();
-  }
-  batched_prep_kernel<<<pg, 256, 0, stream>>>(p->d_graphs, p->count, bad);
-  count_launch();
-  SIMD2_CUDA_TRY(cudaGetLastError());
-  int rc;
+  SIMD2_CUDA_TRY(cudaMemsetAsync(p->cleared, 0, p->cleared_bytes, stream));
+  if (p->slot_bytes)
+    SIMD2_CUDA_TRY(cudaMemsetAsync(p->args.slots + p->args.nfirst, 0, p->slot_bytes, stream));
   switch (p->op) {
-    case SIMD2_MIN_PLUS: rc = launch_batched<SIMD2_MIN_PLUS, false>(p, stream); break;
-    case SIMD2_MAX_PLUS: rc = launch_batched<SIMD2_MAX_PLUS, false>(p, stream); break;
-    case SIMD2_MAX_MIN: rc = launch_batched<SIMD2_MAX_MIN, false>(p, stream); break;
-    case SIMD2_MAX_MUL: rc = launch_batched<SIMD2_MAX_MUL, false>(p, stream); break;
-    case SIMD2_MIN_MUL: rc = launch_batched<SIMD2_MIN_MUL, false>(p, stream); break;
-    case SIMD2_MIN_MAX: rc = launch_batched<SIMD2_MIN_MAX, false>(p, stream); break;
+    case SIMD2_MIN_PLUS: return batched_run_op<SIMD2_MIN_PLUS>(p, stream);
+    case SIMD2_MAX_PLUS: return batched_run_op<SIMD2_MAX_PLUS>(p, stream);
+    case SIMD2_MAX_MIN: return batched_run_op<SIMD2_MAX_MIN>(p, stream);
+    case SIMD2_MAX_MUL: return batched_run_op<SIMD2_MAX_MUL>(p, stream);
+    case SIMD2_MIN_MUL: return batched_run_op<SIMD2_MIN_MUL>(p, stream);
+    case SIMD2_MIN_MAX: return batched_run_op<SIMD2_MIN_MAX>(p, stream);
     default: return SIMD2_ERR_UNSUPPORTED;
   }
-  if (rc) return rc;
-  if (p->fp16) {
-    rc = p->op == SIMD2_MAX_MIN ? launch_batched<SIMD2_MAX_MIN, true>(p, stream)
-                                : launch_batched<SIMD2_MIN_MAX, true>(p, stream);
-    if (rc) return rc;
-  }
-  batched_finish_kernel<<<pg, 256, 0, stream>>>(p->d_graphs, p->count, bad);
-  count_launch();
-  SIMD2_CUDA_TRY(cudaGetLastError());
-  return SIMD2_OK;
 }
 
 }  // namespace
@@ -2527,38 +2502,59 @@ int simd2_batched_plan_create(simd2_op op, int count, float* const* X, const int
   p->op = op;
   p->count = count;
   p->max_iter = max_iter;
-  p->conv = conv;
   p->host.resize(count);
-  // the FP16 path of the selection semirings (the APLP change test writes
-  // -FLT_MAX, which is no FP16 value)
-  p->fp16 = selection_op(op) && conv != SIMD2_CONV_APLP;
-  // layout: [graphs][order][queue][FP16 flag] then per-graph buffers
+  // the APLP change test writes -FLT_MAX, which has no code
+  const bool codes = has_code16(op) && conv != SIMD2_CONV_APLP;
+  // Graphs by descending size, the shared ones first: all of more than one
+  // tile.  Closing the smaller of them by one CTA each instead gained nothing
+  // (296 graphs of 256 vertices 1.29 ms for 1.30) and cost the mixed batches
+  // their tail (512 graphs of up to 1024 vertices: 10.5 ms, and 11.4 with the
+  // graphs under 15 % of the batch's time per SM left whole).
+  std::vector<int> order(count);
+  for (int g = 0; g < count; g++) order[g] = g;
+  std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return n[a] > n[b]; });
+  int nbig = 0;
+  long long tasks = 0;
+  while (nbig < count && n[order[nbig]] > kBM && count <= kBatchSlotMax && n[order[nbig]] <= 1000 * kBM) nbig++;
+  // room for kBatchSlotSteps steps of every shared graph; when the slots are
+  // used up a graph is finished by the CTA that had its last tile
+  std::vector<unsigned long long> first;
+  for (int q = 0; q < nbig; q++) {
+    const int t = (n[order[q]] + kBM - 1) / kBM;
+    for (int i = 0; i < t * t; i++) first.push_back(batch_slot(0, 0, i, order[q]));
+  }
+  const unsigned cap =
+      (unsigned)std::min<unsigned long long>(1u << 30, first.size() * (std::min(max_iter, kBatchSlotSteps) + 3ull));
   size_t off = 0;
   auto take = [&](size_t bytes) { size_t o = off; off += align_up(bytes, kAlign); return o; };
   const size_t g_off = take(sizeof(BatchGraph) * std::max(count, 1));
   const size_t m_off = take(sizeof(BatchMaps) * std::max(count, 1));
   const size_t o_off = take(sizeof(int) * std::max(count, 1));
-  const size_t q_off = take(sizeof(int));
-  const size_t f_off = take(sizeof(int));
-  std::vector<size_t> buf_off(count);
-  auto half_bytes = [&](const BatchGraph& G, size_t* xh, size_t* ph) {
-    *xh = p->fp16 ? (size_t)G.Mp * G.Kh * 2 : 0;
-    *ph = p->fp16 ? (size_t)(G.Kh / 2) * G.Np * 4 : 0;
+  const size_t s_off = take(sizeof(BatchState) * std::max(count, 1));
+  const size_t c_off = take(sizeof(BatchCtl));
+  const size_t sl_off = off;
+  take(sizeof(unsigned long long) * std::max(cap, 1u));
+  p->cleared_bytes = sl_off - s_off;
+  p->slot_bytes = (cap - first.size()) * sizeof(unsigned long long);
+  struct Sizes { size_t x, p, xc, pc; };
+  auto sizes = [&](const BatchGraph& G) {
+    return Sizes{(size_t)G.Mp * G.Kp * 4, (size_t)G.Kp * G.Np * 4, codes ? (size_t)G.Mp * G.Kh * 2 : 0,
+                 codes ? (size_t)G.Kh * G.Np * 2 : 0};
   };
+  std::vector<size_t> buf_off(count);
   for (int g = 0; g < count; g++) {
     BatchGraph& G = p->host[g];
+    G = BatchGraph{};
     G.n = n[g];
     G.Mp = round_up(std::max(n[g], 1), kBM);
     G.Kp = round_up(std::max(n[g], 1), kBK);
+    G.Kh = round_up(std::max(n[g], 1), kSkBK16);
     G.Np = round_up(std::max(n[g], 1), kBN);
-    G.Kh = round_up(std::max(n[g], 1), kH2BK);
     G.user = X[g];
     G.ldu = ldx[g];
-    const size_t xb = (size_t)G.Mp * G.Kp * 4, pb = (size_t)(G.Kp / 2) * 2 * G.Np * 4;
-    size_t xh, ph;
-    half_bytes(G, &xh, &ph);
-    buf_off[g] = take(2 * xb + 2 * pb);
-    if (p->fp16) take(2 * xh + 2 * ph);
+    tasks += (long long)(G.Mp / kBM) * (G.Np / kBN);
+    const Sizes z = sizes(G);
+    buf_off[g] = take(2 * (z.x + z.p + z.xc + z.pc));
   }
   void* mem = nullptr;
   if (cudaMalloc(&mem, std::max(off, (size_t)kAlign)) != cudaSuccess) {
@@ -2568,69 +2564,61 @@ int simd2_batched_plan_create(simd2_op op, int count, float* const* X, const int
   }
   p->mem = mem;
   uint8_t* base = static_cast<uint8_t*>(mem);
-  p->d_graphs = reinterpret_cast<BatchGraph*>(base + g_off);
-  p->d_maps = reinterpret_cast<BatchMaps*>(base + m_off);
-  p->d_order = reinterpret_cast<int*>(base + o_off);
-  p->d_queue = reinterpret_cast<int*>(base + q_off);
-  p->d_fp16_bad = reinterpret_cast<int*>(base + f_off);
-  for (int g = 0; g < count; g++) {
-    BatchGraph& G = p->host[g];
-    const size_t xb = (size_t)G.Mp * G.Kp * 4, pb = (size_t)(G.Kp / 2) * 2 * G.Np * 4;
-    uint8_t* b = base + buf_off[g];
-    G.X[0] = reinterpret_cast<float*>(b);
-    G.X[1] = reinterpret_cast<float*>(b + xb);
-    G.P[0] = reinterpret_cast<float*>(b + 2 * xb);
-    G.P[1] = reinterpret_cast<float*>(b + 2 * xb + pb);
-    G.Xh[0] = G.Xh[1] = nullptr;
-    G.Ph[0] = G.Ph[1] = nullptr;
-    if (p->fp16) {
-      size_t xh, ph;
-      half_bytes(G, &xh, &ph);
-      uint8_t* h = b + align_up(2 * xb + 2 * pb, kAlign);
-      G.Xh[0] = reinterpret_cast<__half*>(h);
-      G.Xh[1] = reinterpret_cast<__half*>(h + xh);
-      G.Ph[0] = reinterpret_cast<uint32_t*>(h + 2 * xh);
-      G.Ph[1] = reinterpret_cast<uint32_t*>(h + 2 * xh + ph);
-    }
-    G.iters = 0;
-    G.changed = 0;
-  }
-  // tensor maps: A role = X[b] [Mp][Kp], B role = P[b] [Kp/2][2Np] (all padded, never out of bounds)
+  BatchArgs& A = p->args;
+  A = BatchArgs{};
+  A.graphs = reinterpret_cast<BatchGraph*>(base + g_off);
+  auto* d_maps = reinterpret_cast<BatchMaps*>(base + m_off);
+  A.maps = d_maps;
+  auto* d_order = reinterpret_cast<int*>(base + o_off);
+  A.order = d_order;
+  A.nbig = nbig;
+  A.count = count;
+  A.state = reinterpret_cast<BatchState*>(base + s_off);
+  A.ctl = reinterpret_cast<BatchCtl*>(base + c_off);
+  A.slots = reinterpret_cast<unsigned long long*>(base + sl_off);
+  A.nfirst = (unsigned)first.size();
+  A.cap = cap;
+  A.max_iter = max_iter;
+  A.conv_mode = conv;
+  A.use_codes = codes ? 1 : 0;
+  p->cleared = base + s_off;
+  p->grid = (int)std::max(1LL, std::min<long long>(device_sms(), tasks));
+  const int nmax = count > 0 ? n[order[0]] : 1;
+  p->prep_x = (int)std::max(1LL, std::min<long long>(16, ((long long)nmax * nmax / 8 + 255) / 256));
   std::vector<BatchMaps> hmaps(count);
   for (int g = 0; g < count; g++) {
     BatchGraph& G = p->host[g];
-    for (int b = 0; b < 2 && rc == SIMD2_OK; b++) {
-      rc = make_map_f32(&hmaps[g].a[b], G.X[b], G.Mp, G.Kp, G.Kp, kBK, kBM, CU_TENSOR_MAP_SWIZZLE_128B, false);
+    const Sizes z = sizes(G);
+    uint8_t* b = base + buf_off[g];
+    for (int q = 0; q < 2 && rc == SIMD2_OK; q++) {
+      G.X[q] = reinterpret_cast<float*>(b + q * z.x);
+      G.P[q] = reinterpret_cast<float*>(b + 2 * z.x + q * z.p);
+      // all padded to the boxes, never out of bounds
+      rc = make_map_f32(&hmaps[g].a[q], G.X[q], G.Mp, G.Kp, G.Kp, kBK, kBM, CU_TENSOR_MAP_SWIZZLE_128B, false);
       if (rc == SIMD2_OK)
-        rc = make_map_f32(&hmaps[g].b[b], G.P[b], G.Kp / 2, 2LL * G.Np, 2LL * G.Np, 2 * kBN, kBK / 2,
+        rc = make_map_f32(&hmaps[g].b[q], G.P[q], G.Kp / 2, 2LL * G.Np, 2LL * G.Np, 2 * kBN, kBK / 2,
                           CU_TENSOR_MAP_SWIZZLE_NONE, false);
-      if (p->fp16 && rc == SIMD2_OK)
-        rc = make_map_2d(&hmaps[g].ah[b], CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, G.Xh[b], G.Mp, G.Kh, G.Kh, kH2BK, kBM,
-                         CU_TENSOR_MAP_SWIZZLE_128B);
-      if (p->fp16 && rc == SIMD2_OK)
-        rc = make_map_2d(&hmaps[g].bh[b], CU_TENSOR_MAP_DATA_TYPE_UINT32, 4, G.Ph[b], G.Kh / 2, G.Np, G.Np, kBN,
-                         kH2BK / 2, CU_TENSOR_MAP_SWIZZLE_NONE);
+      if (!codes || rc != SIMD2_OK) continue;
+      G.Xc[q] = reinterpret_cast<uint16_t*>(b + 2 * (z.x + z.p) + q * z.xc);
+      G.Pc[q] = reinterpret_cast<uint32_t*>(b + 2 * (z.x + z.p + z.xc) + q * z.pc);
+      rc = make_map_2d(&hmaps[g].ac[q], CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, G.Xc[q], G.Mp, G.Kh, G.Kh, kSkBK16, kBM,
+                       CU_TENSOR_MAP_SWIZZLE_128B);
+      if (rc == SIMD2_OK)
+        rc = make_map_2d(&hmaps[g].bc[q], CU_TENSOR_MAP_DATA_TYPE_UINT32, 4, G.Pc[q], G.Kh / 2, G.Np, G.Np, kBN,
+                         kSkBK16 / 2, CU_TENSOR_MAP_SWIZZLE_NONE);
     }
   }
   if (rc == SIMD2_OK && count > 0 &&
-      cudaMemcpy(p->d_maps, hmaps.data(), sizeof(BatchMaps) * count, cudaMemcpyHostToDevice) != cudaSuccess)
+      (cudaMemcpy(d_maps, hmaps.data(), sizeof(BatchMaps) * count, cudaMemcpyHostToDevice) != cudaSuccess ||
+       cudaMemcpy(A.graphs, p->host.data(), sizeof(BatchGraph) * count, cudaMemcpyHostToDevice) != cudaSuccess ||
+       cudaMemcpy(d_order, order.data(), sizeof(int) * count, cudaMemcpyHostToDevice) != cudaSuccess ||
+       (!first.empty() && cudaMemcpy(A.slots, first.data(), sizeof(first[0]) * first.size(),
+                                     cudaMemcpyHostToDevice) != cudaSuccess)))
     rc = SIMD2_ERR_CUDA;
   if (rc) {
     cudaFree(mem);
     delete p;
     return rc;
-  }
-  // longest-processing-time order: largest graphs first
-  std::vector<int> order(count);
-  for (int g = 0; g < count; g++) order[g] = g;
-  std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return n[a] > n[b]; });
-  if (count > 0) {
-    if (cudaMemcpy(p->d_graphs, p->host.data(), sizeof(BatchGraph) * count, cudaMemcpyHostToDevice) != cudaSuccess ||
-        cudaMemcpy(p->d_order, order.data(), sizeof(int) * count, cudaMemcpyHostToDevice) != cudaSuccess) {
-      cudaFree(mem);
-      delete p;
-      return SIMD2_ERR_CUDA;
-    }
   }
   *out = reinterpret_cast<simd2_batched_plan>(p);
   return SIMD2_OK;
@@ -2651,7 +2639,7 @@ int simd2_batched_plan_iters(simd2_batched_plan plan, int* iters_out, int* not_c
     return SIMD2_OK;
   }
   std::vector<BatchGraph> h(p->count);
-  SIMD2_CUDA_TRY(cudaMemcpy(h.data(), p->d_graphs, sizeof(BatchGraph) * p->count, cudaMemcpyDeviceToHost));
+  SIMD2_CUDA_TRY(cudaMemcpy(h.data(), p->args.graphs, sizeof(BatchGraph) * p->count, cudaMemcpyDeviceToHost));
   int nc = 0;
   for (int g = 0; g < p->count; g++) {
     if (iters_out) iters_out[g] = h[g].iters;

@@ -342,8 +342,6 @@ __global__ void __launch_bounds__(kSimtThreads, 1)
   }
 }
 
-constexpr int kH2BK = 64;  // k per stage of the batched FP16 kernel
-
 // Block occupancy of X (rows x cols) in wide strips, optionally with entry
 // counts.  A CTA of 256 threads covers 128 rows x 512 columns: warp w reads
 // rows w, w + 8, ..., w + 120 and, per 128-column segment, each lane four

@@ -48,6 +48,7 @@ struct Code16<SIMD2_MIN_PLUS> {
   static constexpr bool kHas = true;
   static constexpr uint32_t kPad = 0x7fffu;
   static constexpr uint32_t kIdent = 0xffffffffu;
+  __device__ static float entry(uint32_t c) { return c >= 0x7fffu ? __int_as_float(0x7f800000) : (float)c; }
   __device__ static uint32_t encode(float x, bool& bad) {
     if (__float_as_uint(x) == 0x7f800000u) return 0x7fffu;
     uint32_t v;
@@ -57,6 +58,14 @@ struct Code16<SIMD2_MIN_PLUS> {
   __device__ static float decode(uint32_t acc) {
     const uint32_t m = min(acc & 0xffffu, acc >> 16);
     return m >= 0x7fffu ? __int_as_float(0x7f800000) : (float)m;
+  }
+  // The codes of two neighbouring columns' accumulators combined with the
+  // codes `old`; over gets a bit where a result is finite and has no code.
+  __device__ static uint32_t fold2(uint32_t a0, uint32_t a1, uint32_t old, uint32_t& over) {
+    const uint32_t m = __vminu2(__byte_perm(a0, a1, 0x5410), __byte_perm(a0, a1, 0x7632));
+    const uint32_t r = __vminu2(__vminu2(m, 0x7fff7fffu), old);
+    over |= r & 0x40004000u & ~((r + 0x00010001u) >> 1);  // bit 14 set, but not 0x7fff
+    return r;
   }
   // Folds the pairs (x, y) and (x2, y2) into acc.  Odd columns use the fused
   // add-min, even ones two adds (no carry leaves a half) and a three-operand
@@ -74,6 +83,7 @@ struct Code16<SIMD2_MAX_PLUS> {
   static constexpr bool kHas = true;
   static constexpr uint32_t kPad = 0u;
   static constexpr uint32_t kIdent = 0u;
+  __device__ static float entry(uint32_t c) { return c < 0x4000u ? __int_as_float(0xff800000) : (float)(c - 0x4000u); }
   __device__ static uint32_t encode(float x, bool& bad) {
     if (__float_as_uint(x) == 0xff800000u) return 0u;
     uint32_t v;
@@ -83,6 +93,12 @@ struct Code16<SIMD2_MAX_PLUS> {
   __device__ static float decode(uint32_t acc) {
     const uint32_t m = max(acc & 0xffffu, acc >> 16);
     return m < 0x8000u ? __int_as_float(0xff800000) : (float)(m - 0x8000u);
+  }
+  __device__ static uint32_t fold2(uint32_t a0, uint32_t a1, uint32_t old, uint32_t& over) {
+    const uint32_t m = __vmaxu2(__byte_perm(a0, a1, 0x5410), __byte_perm(a0, a1, 0x7632));
+    const uint32_t finite = ((m >> 15) & 0x00010001u) * 0xffffu;  // halves that hold a finite sum
+    over |= m & finite & 0x40004000u;                             // past 16383
+    return __vmaxu2(((m & 0x3fff3fffu) | 0x40004000u) & finite, old);
   }
   __device__ static uint32_t mac(uint32_t acc, uint32_t x, uint32_t y, uint32_t x2, uint32_t y2, bool odd) {
     if (odd) return __viaddmax_u16x2(x2, y2, __viaddmax_u16x2(x, y, acc));
@@ -100,6 +116,7 @@ struct SelectCode16 {
     return code(__half_as_ushort(h));
   }
   __device__ static uint32_t code(uint32_t u) { return u ^ ((u & 0x8000u) ? 0x7fffu : 0u); }
+  __device__ static float entry(uint32_t c) { return value((int)c); }
   __device__ static float value(int s) { return __half2float(__ushort_as_half((unsigned short)code((uint32_t)s & 0xffffu))); }
 };
 template <>
@@ -107,6 +124,9 @@ struct Code16<SIMD2_MAX_MIN> : SelectCode16 {
   static constexpr uint32_t kPad = 0x83ffu;  // -inf
   static constexpr uint32_t kIdent = 0x83ff83ffu;
   __device__ static float decode(uint32_t acc) { return value(max((int)(int16_t)(acc & 0xffffu), (int)acc >> 16)); }
+  __device__ static uint32_t fold2(uint32_t a0, uint32_t a1, uint32_t old, uint32_t&) {
+    return __vmaxs2(__vmaxs2(__byte_perm(a0, a1, 0x5410), __byte_perm(a0, a1, 0x7632)), old);
+  }
   __device__ static uint32_t mac(uint32_t acc, uint32_t x, uint32_t y, uint32_t x2, uint32_t y2, bool) {
     return __vimax3_s16x2(acc, __vmins2(x, y), __vmins2(x2, y2));
   }
@@ -116,6 +136,9 @@ struct Code16<SIMD2_MIN_MAX> : SelectCode16 {
   static constexpr uint32_t kPad = 0x7c00u;  // +inf
   static constexpr uint32_t kIdent = 0x7c007c00u;
   __device__ static float decode(uint32_t acc) { return value(min((int)(int16_t)(acc & 0xffffu), (int)acc >> 16)); }
+  __device__ static uint32_t fold2(uint32_t a0, uint32_t a1, uint32_t old, uint32_t&) {
+    return __vmins2(__vmins2(__byte_perm(a0, a1, 0x5410), __byte_perm(a0, a1, 0x7632)), old);
+  }
   __device__ static uint32_t mac(uint32_t acc, uint32_t x, uint32_t y, uint32_t x2, uint32_t y2, bool) {
     return __vimin3_s16x2(acc, __vmaxs2(x, y), __vmaxs2(x2, y2));
   }
@@ -282,7 +305,8 @@ struct SkArgs {
 // One k-tile of a warp's register tile on 16-bit codes: chunk q of an A row
 // (8 k, 16 bytes) lies at chunk q ^ (row & 7); B pair row pr holds TILE words.
 // A warp group takes chunks kg, kg + kGroups, ... below nq (FULL: all 8).
-template <int OP, int TILE, bool FULL>
+// ROWS < 8 leaves out the rows kRows * i, i >= ROWS.
+template <int OP, int TILE, bool FULL, int ROWS = 8>
 __device__ __forceinline__ void sk_ktile16(uint32_t (&acc)[8][4], const uint8_t* As, const uint8_t* Bs, int ty, int tx,
                                            int cbase, int kg, int nq) {
   constexpr int KG = SkCfg<TILE>::kGroups;
@@ -290,9 +314,9 @@ __device__ __forceinline__ void sk_ktile16(uint32_t (&acc)[8][4], const uint8_t*
   const uint8_t* bp = Bs + (cbase + 4 * tx) * 4;
 #pragma unroll(FULL ? 2 : 1)
   for (int q = kg; q < (FULL ? 8 : nq); q += KG) {
-    uint4 a[8];
+    uint4 a[ROWS];
 #pragma unroll
-    for (int i = 0; i < 8; i++)
+    for (int i = 0; i < ROWS; i++)
       a[i] = *reinterpret_cast<const uint4*>(As + (ty + SkCfg<TILE>::kRows * i) * 128 + ((q ^ swz) << 4));
 #pragma unroll
     for (int h = 0; h < 2; h++) {
@@ -300,7 +324,7 @@ __device__ __forceinline__ void sk_ktile16(uint32_t (&acc)[8][4], const uint8_t*
       const uint4 v = *reinterpret_cast<const uint4*>(bp + (4 * q + 2 * h + 1) * (TILE * 4));
       const uint32_t b0[4] = {u.x, u.y, u.z, u.w}, b1[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-      for (int i = 0; i < 8; i++) {
+      for (int i = 0; i < ROWS; i++) {
         const uint32_t x = h ? a[i].z : a[i].x, x2 = h ? a[i].w : a[i].y;
 #pragma unroll
         for (int j = 0; j < 4; j++) acc[i][j] = Code16<OP>::mac(acc[i][j], x, b0[j], x2, b1[j], j & 1);
@@ -311,16 +335,16 @@ __device__ __forceinline__ void sk_ktile16(uint32_t (&acc)[8][4], const uint8_t*
 
 // The same on FP32 operands: chunk q = 4 k of an A row; B' pair row p holds
 // 2 TILE floats (see srgemm_simt.cuh).  Columns 32c + 2tx + e of the warp's 64.
-template <int OP, int TILE, bool FULL>
+template <int OP, int TILE, bool FULL, int ROWS = 8>
 __device__ __forceinline__ void sk_ktile32(float (&acc)[8][4], const uint8_t* As, const uint8_t* Bs, int ty, int tx,
                                            int cbase, int kg, int nq) {
   constexpr int KG = SkCfg<TILE>::kGroups;
   const int swz = ty & 7;
 #pragma unroll(FULL ? 2 : 1)
   for (int q = kg; q < (FULL ? 8 : nq); q += KG) {
-    float4 a[8];
+    float4 a[ROWS];
 #pragma unroll
-    for (int i = 0; i < 8; i++)
+    for (int i = 0; i < ROWS; i++)
       a[i] = *reinterpret_cast<const float4*>(As + (ty + SkCfg<TILE>::kRows * i) * 128 + ((q ^ swz) << 4));
 #pragma unroll
     for (int h = 0; h < 2; h++) {
@@ -329,7 +353,7 @@ __device__ __forceinline__ void sk_ktile32(float (&acc)[8][4], const uint8_t* As
       for (int c = 0; c < 2; c++)
         b[c] = *reinterpret_cast<const float4*>(Bs + ((2 * q + h) * (2 * TILE) + (cbase + 32 * c + 2 * tx) * 2) * 4);
 #pragma unroll
-      for (int i = 0; i < 8; i++) {
+      for (int i = 0; i < ROWS; i++) {
         const float2 ap = h == 0 ? make_float2(a[i].x, a[i].y) : make_float2(a[i].z, a[i].w);
 #pragma unroll
         for (int c = 0; c < 2; c++) {

@@ -1,0 +1,90 @@
+"""The batched closure's tile scheduling, code range and restarts against the
+oracle, bit for bit: graphs of one and of several tiles in one batch, few large
+graphs among many small ones, results that outgrow the 16-bit codes in the
+middle of a closure, and more steps than the entry list holds."""
+import numpy as np
+import pytest
+import torch
+
+import oracle
+import simd2_b200 as s2
+from simd2_b200 import datagen
+
+pytestmark = pytest.mark.gpu
+
+
+def same(got, want, msg=""):
+    np.testing.assert_array_equal(got.cpu().numpy().view(np.uint32), np.ascontiguousarray(want).view(np.uint32),
+                                  err_msg=msg)
+
+
+def check(op, graphs, **kw):
+    mats = [torch.from_numpy(g.copy()).cuda() for g in graphs]
+    iters = s2.closure_batched(op, mats, **kw)
+    for g, m, it in zip(graphs, mats, iters):
+        want, want_it = oracle.closure(op, g)
+        assert it == want_it, (op, g.shape, it, want_it)
+        same(m, want, f"{op} n={g.shape[0]}")
+    assert s2.device_status() == 0
+
+
+@pytest.mark.parametrize("op", ["min_plus", "max_plus", "max_min", "min_mul"])
+def test_mixed_sizes(cuda, op):
+    """One large graph, some of a few tiles, many of one."""
+    rng = np.random.default_rng(3)
+    sizes = [640, 300, 257, 256, 129, 130, 191, 193] + [int(v) for v in rng.integers(1, 129, 30)]
+    graphs = []
+    for i, n in enumerate(sizes):
+        x = datagen.closure_graph("min_plus" if op in ("min_plus", "min_mul") else "max_min", n, 0.05, seed=i)
+        if op == "max_plus":  # a DAG, so longest paths exist
+            x = np.where(np.triu(np.ones((n, n), bool), 1), x, np.float32(-np.inf)).astype(np.float32)
+        if op == "min_mul":
+            x = np.where(np.isinf(x), x, 1.0 + x / 128.0).astype(np.float32)
+            np.fill_diagonal(x, 1.0)
+        graphs.append(x)
+    check(op, graphs)
+
+
+@pytest.mark.parametrize("n", [100, 300])
+def test_outgrows_codes(cuda, n):
+    """A path of heavy edges: distances pass 16383 in the second squaring, so the
+    graph starts again on FP32; its neighbours in the batch stay coded."""
+    chain = np.full((n, n), np.inf, np.float32)
+    np.fill_diagonal(chain, 0.0)
+    for i in range(n - 1):
+        chain[i, i + 1] = 6000.0 + i
+    big = datagen.er_graph(n, 0.1, seed=1)
+    big[3, 5] = 16384.0  # no code from the start
+    frac = datagen.er_graph(n, 0.1, seed=2) + np.float32(0.25)
+    check("min_plus", [chain, datagen.er_graph(n, 0.1, seed=3), big, frac, datagen.er_graph(40, 0.1, seed=4)])
+
+
+def test_more_steps_than_entries(cuda):
+    """Longest paths around a cycle never settle: every step changes X, past the
+    codes' range and past the steps the entry list has room for."""
+    n, steps = 150, 90
+    rng = np.random.default_rng(8)
+    x = np.full((n, n), -np.inf, np.float32)
+    x[rng.random((n, n)) < 0.03] = 1.0
+    x[np.arange(n), (np.arange(n) + 1) % n] = 1.0
+    graphs = [x, np.roll(x, 1, 0), datagen.closure_graph("max_min", 200, 0.1, seed=2)]
+    mats = [torch.from_numpy(g.copy()).cuda() for g in graphs]
+    plan = s2.BatchedClosure("max_plus", mats, max_iter=steps)
+    plan.run()
+    torch.cuda.synchronize()
+    its, not_converged = plan.iters()
+    for g, m, it in zip(graphs, mats, its):
+        want, cur = g, g
+        done = 0
+        while done < steps:
+            cur = oracle.srgemm("max_plus", want, want, want, do_epilogue=True, threads=8)
+            done += 1
+            stop = np.array_equal(cur.view(np.uint32), want.view(np.uint32))
+            want = cur
+            if stop:
+                break
+        assert it == done
+        same(m, want)
+    assert not_converged >= 2
+    plan.close()
+    assert s2.device_status() == 0
