@@ -121,7 +121,7 @@ int simd2_closure_bf(simd2_op op, int n, const float* A0, int lda0, float* X, in
 /* or_and transitive closure on uint8 0/1 (apps/gtc/cuASR), synchronous.
  * From n = 8192 a sparse X is first squared as CSR SpGEMM steps (while X
  * holds at most n^2/32 entries and a step forms at most n^3/16384 products),
- * then on the INT8 tensor cores; same result and step count either way. */
+ * then on the FP4 tensor cores; same result and step count either way. */
 int simd2_closure_orand_u8(int n, uint8_t* X, int ldx, int max_iter,
                            int* iters_out, cudaStream_t stream);
 

@@ -674,7 +674,7 @@ int launch_tc(int M, int N, int K, const CUtensorMap& a0, const CUtensorMap& a1,
     configured[dev] = true;
   }
   const int tiles_m = (M + kTcBM - 1) / kTcBM;
-  const int tiles_n = (N + kTcBN - 1) / kTcBN;
+  const int tiles_n = (N + tc_bn<KIND>() - 1) / tc_bn<KIND>();
   auto* ev = prof_slot(2LL * M * N * K, kProfTensor);
   if (ev) cudaEventRecord(ev->first, stream);
   // persistent: at most one CTA per SM (shared memory and TMEM hold one)
@@ -726,7 +726,7 @@ int launch_tc2(int M, int N, int K, const CUtensorMap& a0, const CUtensorMap& a1
     max_pairs[dev] = std::max(1, clusters);
   }
   const int tiles_m = (M + kTc2BM - 1) / kTc2BM;
-  const int tiles_n = (N + kTcBN - 1) / kTcBN;
+  const int tiles_n = (N + tc_bn<KIND>() - 1) / tc_bn<KIND>();
   const int pairs = std::min(tiles_m * tiles_n, max_pairs[dev]);
   lc.gridDim = dim3(2 * pairs);
   auto* ev = prof_slot(2LL * M * N * K, kProfTensor);
@@ -760,14 +760,14 @@ TcPlan tc_plan_bf16(int M, int N, int K) {
   return p;
 }
 
-// 0/1 byte operands (or_and)
-TcPlan tc_plan_u8(int M, int N, int K) {
+// 0/1 operands as FP4, two a byte (or_and)
+TcPlan tc_plan_fp4(int M, int N, int K) {
   TcPlan p{};
-  p.Kp = round_up(std::max(K, 1), 16);
+  p.Kp = round_up(std::max(K, 1), 32);
   size_t off = 0;
   auto take = [&](size_t bytes) { size_t o = off; off += align_up(bytes, kAlign); return o; };
-  p.a0 = take((size_t)M * p.Kp);
-  p.b0 = take((size_t)N * p.Kp);
+  p.a0 = take((size_t)M * p.Kp / 2);
+  p.b0 = take((size_t)N * p.Kp / 2);
   p.a1 = p.a0;
   p.b1 = p.b0;
   p.na = p.nb = p.nb64 = 0;
@@ -791,7 +791,7 @@ int srgemm_tc_sum(int op, int M, int N, int K, const float* A, long long lda, co
   double* nb64 = op == SIMD2_MINUS_SQUARE ? reinterpret_cast<double*>(ws + plan.nb64) : nullptr;
   if (nb64) SIMD2_CUDA_TRY(cudaMemsetAsync(nb64, 0, sizeof(double) * N, stream));
   dim3 tgrid((N + 31) / 32, (Kp + 31) / 32), tblock(32, 8);
-  transpose_prep_kernel<float, 0><<<tgrid, tblock, 0, stream>>>(B, ldb, K, N, ws + plan.b0, ws + plan.b1, Kp, nb64);
+  transpose_prep_kernel<<<tgrid, tblock, 0, stream>>>(B, ldb, K, N, ws + plan.b0, ws + plan.b1, Kp, nb64);
   count_launch();
   if (op == SIMD2_MINUS_SQUARE) {
     row_norms_kernel<<<grid_for((long long)M * 32), 256, 0, stream>>>(A, lda, M, K, na);
@@ -850,27 +850,23 @@ int srgemm_tc_orand(int M, int N, int K, const T* A, long long lda, const T* B, 
                     long long ldc, T* D, long long ldd, int do_epilogue, int* changed, uint8_t* ws,
                     const TcPlan& plan, cudaStream_t stream, const TcDelta& delta = TcDelta()) {
   const int Kp = plan.Kp;
-  uint8_t* a8 = ws + plan.a0;
-  uint8_t* b8 = ws + plan.b0;
-  bool_rows_u8_kernel<T><<<grid_for((long long)M * Kp / 16), 256, 0, stream>>>(A, lda, M, K, a8, Kp);
+  uint8_t* a4 = ws + plan.a0;
+  uint8_t* b4 = ws + plan.b0;
+  bool_rows_fp4_kernel<T><<<grid_for((long long)M * Kp / 16), 256, 0, stream>>>(A, lda, M, K, a4, Kp);
+  transpose_fp4_kernel<T><<<dim3((N + 63) / 64, (Kp + 127) / 128), 256, 0, stream>>>(B, ldb, K, N, b4, Kp);
   count_launch();
-  if constexpr (std::is_same_v<T, uint8_t>) {
-    transpose_bool_u8_kernel<<<dim3((N + 63) / 64, (Kp + 63) / 64), 256, 0, stream>>>(B, ldb, K, N, b8, Kp);
-  } else {
-    dim3 tgrid((N + 31) / 32, (Kp + 31) / 32), tblock(32, 8);
-    transpose_prep_kernel<T, 1><<<tgrid, tblock, 0, stream>>>(B, ldb, K, N, b8, nullptr, Kp);
-  }
   count_launch();
   SIMD2_CUDA_TRY(cudaGetLastError());
   CUtensorMap ma, mb;
   const auto U8 = CU_TENSOR_MAP_DATA_TYPE_UINT8;
   const auto SW = CU_TENSOR_MAP_SWIZZLE_128B;
+  constexpr int BN = tc_bn<1>();
   int rc;
   const bool pair = use_tc2(M, N);
-  if ((rc = make_map_2d(&ma, U8, 1, a8, M, Kp, Kp, 128, kTcBM, SW))) return rc;
-  if ((rc = make_map_2d(&mb, U8, 1, b8, N, Kp, Kp, 128, pair ? 128 : kTcBN, SW))) return rc;
+  if ((rc = make_map_2d(&ma, U8, 1, a4, M, Kp / 2, Kp / 2, 128, kTcBM, SW))) return rc;
+  if ((rc = make_map_2d(&mb, U8, 1, b4, N, Kp / 2, Kp / 2, 128, pair ? BN / 2 : BN, SW))) return rc;
   CUtensorMap mbh = mb;  // the pair kernel's half tiles stage 64 rows of B^T per CTA
-  if (pair && (rc = make_map_2d(&mbh, U8, 1, b8, N, Kp, Kp, 128, 64, SW))) return rc;
+  if (pair && (rc = make_map_2d(&mbh, U8, 1, b4, N, Kp / 2, Kp / 2, 128, 64, SW))) return rc;
   TcEpilogue ep{};
   ep.op = SIMD2_OR_AND;
   ep.do_epilogue = do_epilogue;
@@ -878,7 +874,7 @@ int srgemm_tc_orand(int M, int N, int K, const T* A, long long lda, const T* B, 
   ep.ldc = do_epilogue ? ldc : ldd;
   ep.D = D;
   ep.ldd = ldd;
-  ep.out_u8 = sizeof(T) == 1;
+  ep.out_type = sizeof(T) == 1 ? kOrU8 : kOrI32;
   ep.changed = changed;
   if (pair) {
     ep.chg_row = delta.chg_row;
@@ -957,7 +953,7 @@ int srgemm_f32_ws(int op, int M, int N, int K, const float* A, long long lda, co
   return srgemm_core(op, M, N, K, A, lda, B, ldb, ep, ws, plan, pack_a, stream);
 }
 
-// or_and on the INT8 tensor cores (0/1 bytes, S32 counts), exact.
+// or_and on the FP4 tensor cores (0 / 1.0 values, FP32 sums), exact.
 template <typename T>
 int srgemm_orand(int M, int N, int K, const T* A, long long lda, const T* B, long long ldb, const T* C, long long ldc,
                  T* D, long long ldd, int do_epilogue, cudaStream_t stream) {
@@ -976,7 +972,7 @@ int srgemm_orand(int M, int N, int K, const T* A, long long lda, const T* B, lon
     SIMD2_CUDA_TRY(cudaGetLastError());
     return SIMD2_OK;
   }
-  const TcPlan plan = tc_plan_u8(M, N, K);
+  const TcPlan plan = tc_plan_fp4(M, N, K);
   void* p = nullptr;
   if ((rc = get_workspace(stream, plan.total, &p))) return rc;
   return srgemm_tc_orand<T>(M, N, K, A, lda, B, ldb, C, ldc, D, ldd, do_epilogue, nullptr,
@@ -1524,7 +1520,7 @@ int simd2_closure_orand_u8(int n, uint8_t* X, int ldx, int max_iter, int* iters_
   if (n == 0 || max_iter == 0) return SIMD2_OK;
   int rc = check_device();
   if (rc) return rc;
-  // From n = 8192 a dense INT8 step takes ~0.4 ms or more, so a sparse X is
+  // From n = 8192 a dense step takes ~0.2 ms or more, so a sparse X is
   // first squared as CSR SpGEMM steps (see closure_sparse_opening_t); smaller
   // closures would spend more on the opening's host round trips than it saves.
   int it0 = 0;
@@ -1538,7 +1534,7 @@ int simd2_closure_orand_u8(int n, uint8_t* X, int ldx, int max_iter, int* iters_
     max_iter -= it0;
   }
   // Workspace: [tensor-core operands][Xnew n x n bytes, without delta steps][change flag][delta maps]
-  const TcPlan plan = tc_plan_u8(n, n, n);
+  const TcPlan plan = tc_plan_fp4(n, n, n);
   const bool delta = use_tc2(n, n);
   const size_t x_off = align_up(plan.total, kAlign);
   const size_t f_off = x_off + (delta ? 0 : align_up((size_t)n * n, kAlign));
@@ -1549,7 +1545,7 @@ int simd2_closure_orand_u8(int n, uint8_t* X, int ldx, int max_iter, int* iters_
   // skipped and keeps its bytes (step t's products of unchanged rows and
   // columns are all in X already).  Ping-pong maps of changed tile rows and
   // columns carry that from step to step.
-  const int trows = (n + kTc2BM - 1) / kTc2BM, tcols = (n + kTcBN - 1) / kTcBN;
+  const int trows = (n + kTc2BM - 1) / kTc2BM, tcols = (n + tc_bn<1>() - 1) / tc_bn<1>();
   const size_t d_off = f_off + kAlign;
   const size_t dmap = align_up((size_t)trows + tcols, kAlign);
   void* p = nullptr;
@@ -1606,7 +1602,7 @@ int simd2_closure_panel_step(simd2_op op, int rows, int n, const void* panel, in
   int rc = check_device();
   if (rc) return rc;
   if (op == SIMD2_OR_AND) {
-    const TcPlan plan = tc_plan_u8(rows, n, n);
+    const TcPlan plan = tc_plan_fp4(rows, n, n);
     void* p = nullptr;
     if ((rc = get_workspace(stream, plan.total, &p))) return rc;
     const auto* P = static_cast<const uint8_t*>(panel);
@@ -2113,8 +2109,8 @@ int closure_sparse_opening(int op, int n, float* X, long long ldx, int max_iter,
   return closure_sparse_opening_t<float>(op, n, X, ldx, max_iter, pol, steps, changed, step_cfg, step_ms, stream);
 }
 
-// The or_and closure's opening: the dense step runs on the INT8 tensor cores
-// (about 1.3 P MAC/s), so a sparse step must stay under n^3/16384 products.
+// The or_and closure's opening: the dense step runs on the FP4 tensor cores
+// (about 3 P MAC/s), so a sparse step must stay under n^3/16384 products.
 int closure_sparse_opening_u8(int n, uint8_t* X, long long ldx, int max_iter, int* steps, bool* changed,
                               cudaStream_t stream) {
   const unsigned long long nn2 = (unsigned long long)n * (unsigned long long)n;

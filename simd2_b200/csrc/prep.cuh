@@ -202,54 +202,114 @@ __global__ void split_rows_bf16_kernel(const float* __restrict__ A, long long ld
   }
 }
 
-// A [M][K] of T -> bytes {0,1} [M][Kp].  Kp is a multiple of 16: a thread
-// writes 16 bytes of a row; byte inputs with 16-byte aligned rows are read
-// with one 16-byte load and normalised four bytes at a time.
+// True as the FP4 (E2M1) value 1.0 in each nibble of 8 bytes of 0 / 1 (two words
+// of four): byte j of the result holds elements 2j (low nibble) and 2j + 1.
+__device__ __forceinline__ uint32_t nibbles_fp4(uint32_t w0, uint32_t w1) {
+  // byte pairs (b0, b1) -> b0 | b1 << 4 at the even bytes
+  const uint32_t p0 = (w0 | w0 >> 4) & 0x00ff00ffu, p1 = (w1 | w1 >> 4) & 0x00ff00ffu;
+  return __byte_perm(p0, p1, 0x6420) << 1;
+}
+
 template <typename T>
-__global__ void bool_rows_u8_kernel(const T* __restrict__ A, long long lda, int M, int K, uint8_t* __restrict__ out,
-                                    int Kp) {
+__device__ __forceinline__ bool is_true(T x) {
+  if constexpr (std::is_same<T, __half>::value) return (__half_as_ushort(x) & 0x7fffu) != 0;  // -0 is false
+  else return x != T(0);
+}
+
+// 16 elements from p, of which `left` exist, as 0 / 1 bytes (16 / sizeof(T)
+// elements a load where p is aligned and all exist).
+template <typename T>
+__device__ __forceinline__ void load_bool16(const T* p, int left, uint32_t (&w)[4]) {
+  constexpr int PER = 16 / (int)sizeof(T);
+  if (left >= 16 && (reinterpret_cast<uintptr_t>(p) & 15) == 0) {
+#pragma unroll
+    for (int q = 0; q < 16 / PER; q++) {
+      const uint4 u = __ldg(reinterpret_cast<const uint4*>(p) + q);
+      const uint32_t in[4] = {u.x, u.y, u.z, u.w};
+      if constexpr (sizeof(T) == 1) {
+#pragma unroll
+        for (int e = 0; e < 4; e++) w[e] = bytes_nonzero_01(in[e]);
+      } else if constexpr (sizeof(T) == 4) {
+        w[q] = (in[0] != 0u) | (in[1] != 0u) << 8 | (in[2] != 0u) << 16 | (uint32_t)(in[3] != 0u) << 24;
+      } else {
+#pragma unroll
+        for (int e = 0; e < 2; e++)
+          w[2 * q + e] = ((in[2 * e] & 0x7fffu) != 0u) | ((in[2 * e] & 0x7fff0000u) != 0u) << 8 |
+                         ((in[2 * e + 1] & 0x7fffu) != 0u) << 16 |
+                         (uint32_t)((in[2 * e + 1] & 0x7fff0000u) != 0u) << 24;
+      }
+    }
+  } else {
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      uint32_t v = 0;
+#pragma unroll
+      for (int e = 0; e < 4; e++)
+        v |= (uint32_t)(4 * q + e < left && is_true(p[4 * q + e])) << (8 * e);
+      w[q] = v;
+    }
+  }
+}
+
+// or_and's A: A [M][K] of T -> FP4 [M][Kp / 2 bytes], zeros for k >= K.  Kp is a
+// multiple of 32: a thread packs 16 elements of a row into 8 bytes.
+template <typename T>
+__global__ void __launch_bounds__(256) bool_rows_fp4_kernel(const T* __restrict__ A, long long lda, int M, int K,
+                                                            uint8_t* __restrict__ out, int Kp) {
   const int groups = Kp >> 4;
   const long long total = (long long)M * groups;
-  constexpr bool kBytes = sizeof(T) == 1;
-  const bool vec = kBytes && (lda % 16 == 0) && (reinterpret_cast<uintptr_t>(A) % 16 == 0);
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
        t += (long long)gridDim.x * blockDim.x) {
     const int i = (int)(t / groups);
     const int k0 = (int)(t - (long long)i * groups) * 16;
-    const T* row = A + (long long)i * lda;
     uint32_t w[4];
-    if (kBytes && vec && k0 + 16 <= K) {
-      const uint4 u = __ldg(reinterpret_cast<const uint4*>(row + k0));
-      const uint32_t in[4] = {u.x, u.y, u.z, u.w};
+    load_bool16(A + (long long)i * lda + k0, K - k0, w);
+    reinterpret_cast<uint2*>(out)[t] = make_uint2(nibbles_fp4(w[0], w[1]), nibbles_fp4(w[2], w[3]));
+  }
+}
+
+// or_and's B: B [K][N] of T (pitch ldb) -> FP4 [N][Kp / 2 bytes], zeros for k >= K.
+// One tile of 128 k x 64 columns per block of 256 threads: a thread reads 16
+// elements of two rows of B and writes 16 bytes (32 k) of a row of out.  The shared tile's
+// 68-byte rows keep both phases at most 2-way bank conflicted.
+template <typename T>
+__global__ void __launch_bounds__(256) transpose_fp4_kernel(const T* __restrict__ B, long long ldb, int K, int N,
+                                                            uint8_t* __restrict__ out, int Kp) {
+  __shared__ uint32_t tile[128][17];
+  const int t = threadIdx.x;
+  const int k0 = blockIdx.y * 128, j0 = blockIdx.x * 64;
 #pragma unroll
-      for (int q = 0; q < 4; q++) {
-        // 0x01 in every byte that is nonzero, carry-free
-        const uint32_t b = in[q];
-        w[q] = bytes_nonzero_01(b);
-      }
-    } else {
+  for (int h = 0; h < 2; h++) {
+    const int r = (t >> 2) + 64 * h, c0 = (t & 3) * 16;
+    const int k = k0 + r, j = j0 + c0;
+    uint32_t w[4] = {0u, 0u, 0u, 0u};
+    if (k < K && j < N) load_bool16(B + (long long)k * ldb + j, N - j, w);
 #pragma unroll
-      for (int q = 0; q < 4; q++) {
-        uint32_t v = 0;
+    for (int q = 0; q < 4; q++) tile[r][(c0 >> 2) + q] = w[q];
+  }
+  __syncthreads();
+  const int jj = t >> 2, kc = (t & 3) * 32;
+  const int jo = j0 + jj, ko = k0 + kc;
+  if (jo < N && ko < Kp) {
+    const int sh = 8 * (jj & 3);
+    uint32_t o[4];
 #pragma unroll
-        for (int e = 0; e < 4; e++) {
-          const int k = k0 + 4 * q + e;
-          v |= (uint32_t)(k < K && row[k] != T(0)) << (8 * e);
-        }
-        w[q] = v;
-      }
+    for (int q = 0; q < 4; q++) {
+      uint32_t x = 0u;
+#pragma unroll
+      for (int b = 0; b < 8; b++) x |= ((tile[kc + 8 * q + b][jj >> 2] >> sh) & 1u) << (4 * b + 1);
+      o[q] = x;
     }
-    reinterpret_cast<uint4*>(out)[t] = make_uint4(w[0], w[1], w[2], w[3]);
+    *reinterpret_cast<uint4*>(out + ((long long)jo * Kp + ko) / 2) = make_uint4(o[0], o[1], o[2], o[3]);
   }
 }
 
 // B [K][N] (pitch ldb) -> transposed K-major [N][Kp] through a 32 x 32 shared
 // tile (coalesced reads along n, coalesced writes along k).
-// MODE 0: BF16 hi/lo split (out0 = hi, out1 = lo); MODE 1: bytes {0,1} (out0).
+// BF16 hi/lo split: out0 = hi, out1 = lo.
 // colsq (nullable): sum over k of B[k][j]^2 accumulated in FP64 (atomicAdd per
 // 32-row tile; the caller zeroes it and rounds it to float afterwards).
-template <typename T, int MODE>
-__global__ void transpose_prep_kernel(const T* __restrict__ B, long long ldb, int K, int N, void* __restrict__ out0,
+__global__ void transpose_prep_kernel(const float* __restrict__ B, long long ldb, int K, int N, void* __restrict__ out0,
                                       void* __restrict__ out1, int Kp, double* __restrict__ colsq = nullptr) {
   __shared__ float tile[32][33];
   const int k0 = blockIdx.y * 32;
@@ -258,9 +318,7 @@ __global__ void transpose_prep_kernel(const T* __restrict__ B, long long ldb, in
     const int k = k0 + i, j = j0 + threadIdx.x;
     float v = 0.f;
     if (k < K && j < N) {
-      const T x = B[(long long)k * ldb + j];
-      if constexpr (MODE == 1) v = (x != T(0)) ? 1.f : 0.f;
-      else v = static_cast<float>(x);
+      v = B[(long long)k * ldb + j];
     }
     tile[i][threadIdx.x] = v;
   }
@@ -278,60 +336,11 @@ __global__ void transpose_prep_kernel(const T* __restrict__ B, long long ldb, in
     if (j < N && k < Kp) {
       const float v = tile[threadIdx.x][i];
       const long long o = (long long)j * Kp + k;
-      if constexpr (MODE == 1) {
-        static_cast<uint8_t*>(out0)[o] = (uint8_t)(v != 0.f);
-      } else {
-        __nv_bfloat16 h, l;
-        split_bf16(v, h, l);
-        static_cast<__nv_bfloat16*>(out0)[o] = h;
-        static_cast<__nv_bfloat16*>(out1)[o] = l;
-      }
+      __nv_bfloat16 h, l;
+      split_bf16(v, h, l);
+      static_cast<__nv_bfloat16*>(out0)[o] = h;
+      static_cast<__nv_bfloat16*>(out1)[o] = l;
     }
-  }
-}
-
-// or_and's B operand for bytes: B [K][N] (pitch ldb) -> out [N][Kp], 1 where
-// B is nonzero, zeros for K <= k < Kp (transpose_prep_kernel<T, 1>'s result).
-// One 64 x 64 tile per block of 256 threads: a thread reads 16 bytes of a row
-// of B (one 16-byte load where B allows) and writes 16 bytes of a row of out;
-// the shared tile's 68-byte rows keep both phases at most 2-way bank
-// conflicted.  Kp is a multiple of 16, out 16-byte aligned; the grid covers
-// ceil(N / 64) x ceil(Kp / 64) tiles.
-__global__ void __launch_bounds__(256) transpose_bool_u8_kernel(const uint8_t* __restrict__ B, long long ldb, int K,
-                                                                int N, uint8_t* __restrict__ out, int Kp) {
-  __shared__ uint32_t tile[64][17];
-  const int t = threadIdx.x;
-  const int k0 = blockIdx.y * 64, j0 = blockIdx.x * 64;
-  {
-    const int r = t >> 2, c0 = (t & 3) * 16;
-    const int k = k0 + r, j = j0 + c0;
-    uint32_t w[4] = {0u, 0u, 0u, 0u};
-    if (k < K && j < N) {
-      const uint8_t* src = B + (long long)k * ldb + j;
-      if (j + 16 <= N && (reinterpret_cast<uintptr_t>(src) & 15) == 0) {
-        const uint4 v = __ldg(reinterpret_cast<const uint4*>(src));
-        w[0] = v.x, w[1] = v.y, w[2] = v.z, w[3] = v.w;
-      } else {
-        for (int e = 0; e < 16 && j + e < N; e++) w[e >> 2] |= (uint32_t)src[e] << (8 * (e & 3));
-      }
-    }
-#pragma unroll
-    for (int q = 0; q < 4; q++) tile[r][(c0 >> 2) + q] = bytes_nonzero_01(w[q]);
-  }
-  __syncthreads();
-  const int jj = t >> 2, kc = (t & 3) * 16;
-  const int jo = j0 + jj, ko = k0 + kc;
-  if (jo < N && ko < Kp) {
-    const int sh = 8 * (jj & 3);
-    uint32_t o[4];
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-      uint32_t x = 0u;
-#pragma unroll
-      for (int b = 0; b < 4; b++) x |= ((tile[kc + 4 * q + b][jj >> 2] >> sh) & 0xffu) << (8 * b);
-      o[q] = x;
-    }
-    *reinterpret_cast<uint4*>(out + (long long)jo * Kp + ko) = make_uint4(o[0], o[1], o[2], o[3]);
   }
 }
 

@@ -1,7 +1,15 @@
 // tc_gemm.cuh -- tensor-core (tcgen05 / TMEM) srgemm paths for sm_100a.
 //
 // Used for the semirings that are dense contractions:
-//   * or_and       : kind::i8, unsigned 0/1 bytes, S32 counts; D = (count > 0) | C.
+//   * or_and       : kind::mxf4, true as the FP4 value 1.0 with every block scale
+//                    1.0, FP32 accumulate; D = (sum > 0) | C.  Exact: the products
+//                    are 0 or 1, a sum of them is exact up to 2^24 and never
+//                    shrinks, so it is positive just when a product was 1.  Twice
+//                    the rate of kind::i8 on half the operand bytes; what bounds it
+//                    is the shared memory's bandwidth (operand reads and TMA writes
+//                    of a 256 x 224 pair tile: 165 of 128 bytes a clock at full
+//                    rate).  16384^3 step, kernel: kind::i8 2240 us, now 1400;
+//                    3000 x 2500 x 2000 int32 call 117 us, now 56.
 //   * plus_mul     : kind::f16 with BF16 hi/lo operands, FP32 accumulate:
 //                    a*b ~= a_hi*b_hi + a_hi*b_lo + a_lo*b_hi  (three MMAs per k step).
 //   * minus_square : the same BF16 hi/lo product gives a.b; the epilogue forms
@@ -12,10 +20,10 @@
 // Persistent: one CTA per SM walks the 128 x 256 tiles of D (grouped raster)
 // with 6 warps:
 //   warp 0 lane 0  -- TMA producer (2D tiled loads, no multicast; 64-byte
-//                     swizzled rows for BF16, 128-byte for INT8) over every
+//                     swizzled rows for BF16, 128-byte for FP4) over every
 //                     k-tile of every tile, one ring of stages,
-//   warp 1 lane 0  -- MMA issuer (tcgen05.mma, cta_group::1, M=128 N=256) into
-//                     one of two 256-column TMEM accumulators, so the next
+//   warp 1 lane 0  -- MMA issuer (tcgen05.mma, cta_group::1, M=128, N=256 or
+//                     224) into one of two TMEM accumulators, so the next
 //                     tile's MMAs run while the previous tile is written out,
 //   warps 2..5     -- epilogue: tcgen05.ld of the accumulator (warp w reads
 //                     TMEM lanes 32(w%4)..+31 = tile rows), fused (+) C, stores.
@@ -23,11 +31,18 @@
 // stored transposed ([N][K]) by the operand-prep kernel.
 #pragma once
 #include "common.cuh"
+#include "prep.cuh"
 
 namespace simd2 {
 
 constexpr int kTcBM = 128;
 constexpr int kTcBN = 256;
+// Columns of a tile.  or_and takes 224: two accumulators of 224 columns leave
+// the 512 TMEM columns room for the block scales.
+template <int KIND>
+__host__ __device__ constexpr int tc_bn() { return KIND == 1 ? 224 : kTcBN; }
+constexpr int kTcScaleCol = 448;  // first TMEM column of the block scales
+constexpr int kTcScaleCols = 32;  // 4 columns of A's and 8 of B's, all the same byte
 constexpr int kTcEpiWarps = 4;
 constexpr int kTcThreads = (2 + kTcEpiWarps) * 32;  // TMA warp, MMA warp, 4 epilogue warps
 template <int KIND>
@@ -48,24 +63,28 @@ struct TcCfg<0> {
   static constexpr uint32_t kIdesc =
       (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kTcBN >> 3) << 17) | ((uint32_t)(kTcBM >> 4) << 24);
 };
-// INT8 0/1: BK = 128 elements, one A and one B tile per stage.
+// FP4 0/1, two per byte: BK = 256 elements, one A and one B tile per stage.
 template <>
 struct TcCfg<1> {
-  static constexpr int kBK = 128;
+  static constexpr int kBK = 256;
   static constexpr int kRowBytes = 128;
   static constexpr int kNumA = 1;
   static constexpr int kNumB = 1;
   static constexpr int kStages = 4;
-  static constexpr int kKStep = 32;  // K per tcgen05.mma kind::i8
-  // c_format S32 (2), a/b format unsigned 8-bit (0), K-major, N=256, M=128
-  static constexpr uint32_t kIdesc = (2u << 4) | ((uint32_t)(kTcBN >> 3) << 17) | ((uint32_t)(kTcBM >> 4) << 24);
+  static constexpr int kKStep = 64;  // K per tcgen05.mma kind::mxf4
+  // a/b format E2M1 (1), scale format UE8M0 (bit 23), scale ids 0, K-major, N=224, M=128 (bits 27-28: M / 128)
+  static constexpr uint32_t kIdesc = (1u << 7) | (1u << 10) | ((uint32_t)(224 >> 3) << 17) | (1u << 23) |
+                                     ((uint32_t)(kTcBM >> 7) << 27);
 };
 
 template <int KIND>
 __host__ __device__ constexpr int tc_a_tile() { return kTcBM * TcCfg<KIND>::kRowBytes; }
 template <int KIND>
-__host__ __device__ constexpr int tc_b_tile() { return kTcBN * TcCfg<KIND>::kRowBytes; }
+__host__ __device__ constexpr int tc_b_tile() { return tc_bn<KIND>() * TcCfg<KIND>::kRowBytes; }
 
+// k-tile step in tensor-map elements: BF16 values, or bytes of two FP4 values.
+template <int KIND>
+__host__ __device__ constexpr int tc_box_x() { return KIND == 1 ? TcCfg<1>::kRowBytes : TcCfg<0>::kBK; }
 template <int KIND>
 __host__ __device__ constexpr int tc_stage_bytes() {
   return TcCfg<KIND>::kNumA * tc_a_tile<KIND>() + TcCfg<KIND>::kNumB * tc_b_tile<KIND>();
@@ -98,8 +117,10 @@ __device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t smem_addr) {
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 
+// `scales`: TMEM address of the block scales (KIND 1; both operands read the same columns).
 template <int KIND>
-__device__ __forceinline__ void tc_mma(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t accumulate) {
+__device__ __forceinline__ void tc_mma(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t accumulate,
+                                       uint32_t scales = 0) {
   if constexpr (KIND == 0) {
     asm volatile(
         "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
@@ -108,9 +129,21 @@ __device__ __forceinline__ void tc_mma(uint32_t tmem_d, uint64_t adesc, uint64_t
   } else {
     asm volatile(
         "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}\n" ::"r"(tmem_d),
-        "l"(adesc), "l"(bdesc), "r"(TcCfg<1>::kIdesc), "r"(accumulate), "r"(0), "r"(0), "r"(0), "r"(0));
+        "tcgen05.mma.cta_group::1.kind::mxf4.block_scale.scale_vec::2X [%0], %1, %2, %3, [%5], [%5], p;\n\t}\n" ::"r"(
+            tmem_d),
+        "l"(adesc), "l"(bdesc), "r"(TcCfg<1>::kIdesc), "r"(accumulate), "r"(scales));
   }
+}
+
+// Sets this warp's 32 TMEM lanes of the scale columns to 1.0 (UE8M0 127): with
+// every scale the same, their layout does not matter.
+__device__ __forceinline__ void tc_fill_scales(uint32_t taddr) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
+      "{%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1};" ::"r"(taddr),
+      "r"(0x7f7f7f7fu)
+      : "memory");
+  asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
 
 // Arrive on `bar` once every tcgen05 operation issued so far by this thread completes.
@@ -153,15 +186,17 @@ __device__ __forceinline__ void tmem_ld64(uint32_t taddr, uint32_t (&r)[64]) {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
+enum TcOrType { kOrU8 = 0, kOrI32 = 1, kOrF32 = 2 };
+
 // Epilogue arguments of the tensor-core paths.
 struct TcEpilogue {
   int op;               // SIMD2_PLUS_MUL, SIMD2_MINUS_SQUARE or SIMD2_OR_AND
   int do_epilogue;
-  const void* C;        // float (sums) or int32 / uint8 (or_and)
+  const void* C;        // float (sums) or out_type (or_and)
   long long ldc;
   void* D;
   long long ldd;
-  int out_u8;           // or_and: 1 = uint8 C/D, 0 = int32 C/D
+  int out_type;         // or_and: type of C and D (kOrU8, kOrI32, kOrF32)
   // minus_square: row norms of A (M), column norms of B (N), and the FP32
   // operands for the exact recompute inside the cancellation band.
   const float* norm_a;
@@ -205,95 +240,117 @@ __device__ __forceinline__ float exact_minus_square(const float* a, const float*
   return s;
 }
 
-// Epilogue of one 128 x ncols tile (ncols = 256, or 128 for a split tail
-// tile) for the 32 rows of one warp: lane l holds row row0 + l of the
-// accumulator in TMEM at trow (lane quadrant and column base included).  Sets
-// changed when an or_and output differs from C.
-template <int KIND>
-__device__ __forceinline__ void tc_tile_epilogue(const TcEpilogue& ep, int M, int N, int n0, int row0, uint32_t trow,
-                                                 uint32_t* epi_tile, int lane, int& changed, int ncols = kTcBN) {
-  if constexpr (KIND == 1) {
-    // or_and: 32 flags of one row are 32 contiguous bytes (u8) or 128 bytes
-    // (i32), so each lane writes its own row with 16-byte vector stores.
-    const int row = row0 + lane;
-    const bool u8 = ep.out_u8 != 0;
-    const int esz = u8 ? 1 : 4;
-    const bool vec_ok = ((ep.ldd * esz) % 16 == 0) && ((reinterpret_cast<uintptr_t>(ep.D) & 15) == 0) &&
-                        (!ep.do_epilogue ||
-                         (((ep.ldc * esz) % 16 == 0) && ((reinterpret_cast<uintptr_t>(ep.C) & 15) == 0)));
+// or_and: the (sum > 0) flags of one warp's 32 rows x ncols columns, taken out of
+// TMEM as bits (lane l: row l, word c: columns 32c..) and parked in the warp's
+// shared buffer, row pitch kOrPitch words.  The accumulator is free after this.
+constexpr int kOrPitch = 9;
+__device__ __forceinline__ void tc_or_bits(uint32_t trow, uint32_t* buf, int lane, int ncols) {
+  __syncwarp();  // the previous tile's bits have been read
 #pragma unroll 1
-    for (int c0 = 0; c0 < ncols; c0 += 32) {
-      uint32_t r[32];
-      tmem_ld32(trow + c0, r);  // all lanes take part (sync.aligned)
-      if (row >= M) continue;
-      const int colb = n0 + c0;
-      if (u8) {
-        const uint8_t* crow = static_cast<const uint8_t*>(ep.C) + (long long)row * ep.ldc;
-        uint8_t* drow = static_cast<uint8_t*>(ep.D) + (long long)row * ep.ldd;
-        if (vec_ok && colb + 32 <= N) {
-          uint32_t w[8];
+  for (int c0 = 0; c0 < ncols; c0 += 32) {
+    uint32_t r[32];
+    tmem_ld32(trow + c0, r);
+    uint32_t w = 0;
 #pragma unroll
-          for (int q = 0; q < 8; q++)
-            w[q] = (r[4 * q] != 0u) | ((r[4 * q + 1] != 0u) << 8) | ((r[4 * q + 2] != 0u) << 16) |
-                   ((uint32_t)(r[4 * q + 3] != 0u) << 24);
-          if (ep.do_epilogue) {
-            const uint4 c0v = *reinterpret_cast<const uint4*>(crow + colb);
-            const uint4 c1v = *reinterpret_cast<const uint4*>(crow + colb + 16);
-            const uint32_t cw[8] = {c0v.x, c0v.y, c0v.z, c0v.w, c1v.x, c1v.y, c1v.z, c1v.w};
+    for (int j = 0; j < 32; j++) w |= (uint32_t)(r[j] != 0u) << j;
+    buf[lane * kOrPitch + (c0 >> 5)] = w;
+  }
+  __syncwarp();
+}
+
+// Writes the parked flags | C.  A row's columns go to the warp's lanes in order,
+// four to a lane where D's (and C's) rows allow a word of bytes or an int4 --
+// each instruction then covers 128 columns of one row -- else one to a lane;
+// C is loaded for 4 rows before any of it is used.  (With a lane per row, every
+// store of unaligned rows touched 32 rows: the 3000^3 kernel on bytes 184 us, now 39.)
+template <typename T>
+__device__ __forceinline__ void tc_or_store(const TcEpilogue& ep, int M, int N, int n0, int row0, const uint32_t* buf,
+                                            int lane, int& changed, int ncols) {
+  T* D = static_cast<T*>(ep.D);
+  const T* C = static_cast<const T*>(ep.C);
+  const bool epi = ep.do_epilogue != 0;
+  const int rows = min(32, M - row0);
+  constexpr int kVec = sizeof(T) == 1 ? 4 : 16;  // bytes of 4 elements
+  const bool vec = (n0 + ncols <= N) && ((ep.ldd * (long long)sizeof(T)) % kVec == 0) &&
+                   ((reinterpret_cast<uintptr_t>(D) + (size_t)n0 * sizeof(T)) % kVec == 0) &&
+                   (!epi || (((ep.ldc * (long long)sizeof(T)) % kVec == 0) &&
+                             ((reinterpret_cast<uintptr_t>(C) + (size_t)n0 * sizeof(T)) % kVec == 0)));
+  if (vec) {
+    using V = typename std::conditional<sizeof(T) == 1, uint32_t, int4>::type;
+#pragma unroll 1
+    for (int c = lane * 4; c < ncols; c += 128) {
+#pragma unroll 1
+      for (int r0 = 0; r0 < rows; r0 += 4) {
+        V old[4];
 #pragma unroll
-            for (int q = 0; q < 8; q++) {
-              const uint32_t cb = bytes_nonzero_01(cw[q]);  // C's bytes as 0/1 before the OR
-              const uint32_t v = w[q] | cb;
-              if (ep.changed && v != cb) changed = 1;
-              w[q] = v;
+        for (int q = 0; q < 4; q++)
+          if (epi && r0 + q < rows) old[q] = *reinterpret_cast<const V*>(C + (row0 + r0 + q) * ep.ldc + n0 + c);
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+          if (r0 + q >= rows) break;
+          const uint32_t nib = (buf[(r0 + q) * kOrPitch + (c >> 5)] >> (c & 31)) & 15u;
+          V* dst = reinterpret_cast<V*>(D + (row0 + r0 + q) * ep.ldd + n0 + c);
+          if constexpr (sizeof(T) == 1) {
+            uint32_t v = (nib * 0x00204081u) & 0x01010101u;  // bit i to byte i
+            if (epi) {
+              const uint32_t o = bytes_nonzero_01(old[q]);
+              v |= o;
+              if (v != o) changed = 1;
             }
-          }
-          *reinterpret_cast<uint4*>(drow + colb) = make_uint4(w[0], w[1], w[2], w[3]);
-          *reinterpret_cast<uint4*>(drow + colb + 16) = make_uint4(w[4], w[5], w[6], w[7]);
-        } else {
-#pragma unroll
-          for (int j = 0; j < 32; j++) {
-            const int col = colb + j;
-            if (col < N) {
-              uint8_t v = r[j] != 0u;
-              if (ep.do_epilogue) {
-                const uint8_t cv = crow[col] != 0;
-                v |= cv;
-                if (ep.changed && v != cv) changed = 1;
-              }
-              drow[col] = v;
+            *dst = v;
+          } else {
+            int4 v = make_int4(nib & 1, nib >> 1 & 1, nib >> 2 & 1, nib >> 3);
+            if (epi) {
+              v.x |= old[q].x != 0;
+              v.y |= old[q].y != 0;
+              v.z |= old[q].z != 0;
+              v.w |= old[q].w != 0;
             }
-          }
-        }
-      } else {
-        const int32_t* crow = static_cast<const int32_t*>(ep.C) + (long long)row * ep.ldc;
-        int32_t* drow = static_cast<int32_t*>(ep.D) + (long long)row * ep.ldd;
-        if (vec_ok && colb + 32 <= N) {
-#pragma unroll
-          for (int q = 0; q < 8; q++) {
-            int4 v = make_int4(r[4 * q] != 0u, r[4 * q + 1] != 0u, r[4 * q + 2] != 0u, r[4 * q + 3] != 0u);
-            if (ep.do_epilogue) {
-              const int4 c = *reinterpret_cast<const int4*>(crow + colb + 4 * q);
-              v.x |= c.x != 0;
-              v.y |= c.y != 0;
-              v.z |= c.z != 0;
-              v.w |= c.w != 0;
-            }
-            *reinterpret_cast<int4*>(drow + colb + 4 * q) = v;
-          }
-        } else {
-#pragma unroll
-          for (int j = 0; j < 32; j++) {
-            const int col = colb + j;
-            if (col < N) {
-              int32_t v = r[j] != 0u;
-              if (ep.do_epilogue) v |= (crow[col] != 0);
-              drow[col] = v;
-            }
+            *dst = v;
           }
         }
       }
     }
+  } else {
+#pragma unroll 1
+    for (int c = lane; c < ncols && n0 + c < N; c += 32) {
+#pragma unroll 1
+      for (int r0 = 0; r0 < rows; r0 += 4) {
+        T old[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+          if (epi && r0 + q < rows) old[q] = C[(row0 + r0 + q) * ep.ldc + n0 + c];
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+          if (r0 + q >= rows) break;
+          uint32_t v = (buf[(r0 + q) * kOrPitch + (c >> 5)] >> (c & 31)) & 1u;
+          if (epi) {
+            const uint32_t o = is_true(old[q]);
+            v |= o;
+            if (v != o) changed = 1;
+          }
+          D[(row0 + r0 + q) * ep.ldd + n0 + c] = static_cast<T>(static_cast<float>(v));
+        }
+      }
+    }
+  }
+}
+
+// Epilogue of one 128 x ncols tile (ncols a multiple of 32: tc_bn, or less for
+// a split tail tile) for the 32 rows of one warp: lane l holds row row0 + l of the
+// accumulator in TMEM at trow (lane quadrant and column base included).  release()
+// hands the accumulator back.  Sets changed when an or_and output differs from C.
+template <int KIND, typename F>
+__device__ __forceinline__ void tc_tile_epilogue(const TcEpilogue& ep, int M, int N, int n0, int row0, uint32_t trow,
+                                                 uint32_t* epi_tile, int lane, int& changed, F release,
+                                                 int ncols = tc_bn<KIND>()) {
+  if constexpr (KIND == 1) {
+    ncols = min(ncols, (N - n0 + 31) & ~31);
+    tc_or_bits(trow, epi_tile, lane, ncols);
+    release();
+    if (ep.out_type == kOrU8) tc_or_store<uint8_t>(ep, M, N, n0, row0, epi_tile, lane, changed, ncols);
+    else if (ep.out_type == kOrI32) tc_or_store<int32_t>(ep, M, N, n0, row0, epi_tile, lane, changed, ncols);
+    else tc_or_store<float>(ep, M, N, n0, row0, epi_tile, lane, changed, ncols);
   } else {
     // Sums: a 32 x 32 chunk is transposed through shared memory (the stage
     // ring is idle now) and written row by row: lane l handles column l, so
@@ -354,6 +411,7 @@ __device__ __forceinline__ void tc_tile_epilogue(const TcEpilogue& ep, int M, in
       }
       __syncwarp();
     }
+    release();
   }
 }
 template <int KIND>
@@ -387,7 +445,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     const int gsize = min(tiles_m - first_m, group);
     const int local = t - g * per_group;
     m0 = (first_m + local % gsize) * kTcBM;
-    n0 = (local / gsize) * kTcBN;
+    n0 = (local / gsize) * tc_bn<KIND>();
   };
 
   if (threadIdx.x == 0) {
@@ -403,7 +461,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     fence_mbar_init();
   }
   if (warp == 0) {
-    // 512 TMEM columns: two 128 x 256 FP32/S32 accumulators.
+    // 512 TMEM columns: two FP32 accumulators (and or_and's scales).
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
                  "r"(512)
                  : "memory");
@@ -413,6 +471,12 @@ __global__ void __launch_bounds__(kTcThreads, 1)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  if constexpr (KIND == 1) {
+    if (warp >= 2) tc_fill_scales(tmem + kTcScaleCol + ((uint32_t)((warp & 3) * 32) << 16));
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+  }
 
   if (warp == 0) {
     if (lane == 0) {
@@ -433,7 +497,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
           }
           uint8_t* st = smem + s * kStage;
           mbar_arrive_expect_tx(&full[s], kStage);
-          const int kx = kt * Cfg::kBK;
+          const int kx = kt * tc_box_x<KIND>();
           tma_load_2d(st, &tmA0, &full[s], kx, m0);
           if constexpr (Cfg::kNumA == 2) tma_load_2d(st + tc_a_tile<KIND>(), &tmA1, &full[s], kx, m0);
           uint8_t* sb = st + Cfg::kNumA * tc_a_tile<KIND>();
@@ -456,7 +520,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
           break;
         }
         tc_fence_after();
-        const uint32_t d = tmem + acc * kTcBN;
+        const uint32_t d = tmem + acc * tc_bn<KIND>();
         for (int kt = 0; kt < ktiles; kt++, j++) {
           const int s = j % S;
           if (!mbar_wait(&full[s], (j / S) & 1)) {
@@ -471,7 +535,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
           constexpr int RB = Cfg::kRowBytes;
 #pragma unroll
           for (int ks = 0; ks < Cfg::kBK / Cfg::kKStep; ks++) {
-            const uint32_t koff = ks * Cfg::kKStep * (KIND == 0 ? 2 : 1);  // bytes along the swizzled row
+            const uint32_t koff = ks * 32;  // bytes along the swizzled row
             const uint32_t acc0 = (kt > 0 || ks > 0) ? 1u : 0u;
             if constexpr (KIND == 0) {
               // hi*hi, hi*lo, lo*hi
@@ -479,7 +543,8 @@ __global__ void __launch_bounds__(kTcThreads, 1)
               tc_mma<0>(d, umma_desc_swizzled(a0 + koff, RB), umma_desc_swizzled(b1 + koff, RB), 1u);
               tc_mma<0>(d, umma_desc_swizzled(a1 + koff, RB), umma_desc_swizzled(b0 + koff, RB), 1u);
             } else {
-              tc_mma<1>(d, umma_desc_swizzled(a0 + koff, RB), umma_desc_swizzled(b0 + koff, RB), acc0);
+              tc_mma<1>(d, umma_desc_swizzled(a0 + koff, RB), umma_desc_swizzled(b0 + koff, RB), acc0,
+                        tmem + kTcScaleCol);
             }
           }
           tc_commit(&empty[s]);  // stage s is free once these MMAs have read it
@@ -506,17 +571,19 @@ __global__ void __launch_bounds__(kTcThreads, 1)
       tc_fence_after();
       int m0, n0;
       tile_origin(t, m0, n0);
-      const uint32_t trow = tmem + acc * kTcBN + ((uint32_t)(quad * 32) << 16);
+      const uint32_t trow = tmem + acc * tc_bn<KIND>() + ((uint32_t)(quad * 32) << 16);
       const int row0 = m0 + quad * 32;
       int changed = 0;
-      tc_tile_epilogue<KIND>(ep, M, N, n0, row0, trow, epi_tile, lane, changed);
+      // the accumulator half is read out: the MMA warp may reuse it
+      auto release = [&] {
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&acc_empty[acc]);
+      };
+      tc_tile_epilogue<KIND>(ep, M, N, n0, row0, trow, epi_tile, lane, changed, release);
       if (ep.changed && KIND == 1) {
         if (__any_sync(0xffffffffu, changed) && lane == 0) atomicOr(ep.changed, 1);
       }
-      // the accumulator half is read out: the MMA warp may reuse it
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&acc_empty[acc]);
     }
   }
 

@@ -46,9 +46,10 @@ template <int KIND>
 constexpr size_t tc2_smem_bytes() {
   return (size_t)kTc2Stages * tc2_stage_bytes<KIND>() + (size_t)kTcEpiWarps * 32 * 33 * 4 + 1024 + 256;
 }
-// instruction descriptor: TcCfg's with M = 256 and N = n
+// instruction descriptor: TcCfg's with M = 256 and N = n (M / 16 at bit 24 is
+// mxf4's M / 128 at bit 27)
 template <int KIND>
-__host__ __device__ constexpr uint32_t tc2_idesc(int n = kTcBN) {
+__host__ __device__ constexpr uint32_t tc2_idesc(int n = tc_bn<KIND>()) {
   return (TcCfg<KIND>::kIdesc & ~(0x1Fu << 24) & ~(0x3Fu << 17)) | ((uint32_t)(kTc2BM >> 4) << 24) |
          ((uint32_t)(n >> 3) << 17);
 }
@@ -82,7 +83,7 @@ __device__ __forceinline__ void tma_load_2d_pair(void* dst, const CUtensorMap* m
 }
 template <int KIND>
 __device__ __forceinline__ void tc2_mma(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t accumulate,
-                                        uint32_t idesc) {
+                                        uint32_t idesc, uint32_t scales = 0) {
   if constexpr (KIND == 0) {
     asm volatile(
         "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
@@ -93,10 +94,9 @@ __device__ __forceinline__ void tc2_mma(uint32_t tmem_d, uint64_t adesc, uint64_
   } else {
     asm volatile(
         "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::2.kind::i8 [%0], %1, %2, %3, {%5, %6, %7, %8, %9, %10, %11, %12}, p;\n\t}\n" ::"r"(
+        "tcgen05.mma.cta_group::2.kind::mxf4.block_scale.scale_vec::2X [%0], %1, %2, %3, [%5], [%5], p;\n\t}\n" ::"r"(
             tmem_d),
-        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(0), "r"(0), "r"(0), "r"(0), "r"(0), "r"(0), "r"(0),
-        "r"(0));
+        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(scales));
   }
 }
 // arrive on `bar` (same offset) in both CTAs of the pair once the issued MMAs complete
@@ -116,6 +116,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                     int K, TcEpilogue ep, int tiles_m, int tiles_n) {
   using Cfg = TcCfg<KIND>;
   constexpr int S = kTc2Stages;
+  constexpr int BN = tc_bn<KIND>();
   constexpr int kStage = tc2_stage_bytes<KIND>();
   constexpr int kHalf = tc2_half_tile<KIND>();
   extern __shared__ uint8_t smem_raw[];
@@ -142,7 +143,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     const int gsize = min(tiles_m - first_m, group);
     const int local = t - g * per_group;
     m0 = (first_m + local % gsize) * kTc2BM;
-    n0 = (local / gsize) * kTcBN;
+    n0 = (local / gsize) * BN;
   };
   // work items: the first `whole` tiles, then the tail's tiles as half tiles
   const int rem = tiles % pairs;
@@ -152,12 +153,12 @@ __global__ void __launch_bounds__(kTcThreads, 1)
   auto item_origin = [&](int w, int& m0, int& n0, int& ncols) {
     if (w < whole) {
       tile_origin(w, m0, n0);
-      ncols = kTcBN;
+      ncols = BN;
     } else {
       const int h = w - whole;
       tile_origin(whole + (h >> 1), m0, n0);
-      n0 += (h & 1) * (kTcBN / 2);
-      ncols = kTcBN / 2;
+      n0 += (h & 1) * 128;
+      ncols = (h & 1) ? BN - 128 : 128;
     }
   };
 
@@ -167,7 +168,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     if (!ep.need_row) return false;
     int m0, n0, ncols;
     item_origin(w, m0, n0, ncols);
-    return !ep.need_row[m0 / kTc2BM] && !ep.need_col[n0 / kTcBN];
+    return !ep.need_row[m0 / kTc2BM] && !ep.need_col[n0 / BN];
   };
 
   if (threadIdx.x == 0) {
@@ -192,6 +193,12 @@ __global__ void __launch_bounds__(kTcThreads, 1)
   cluster_barrier();  // barriers initialised in both CTAs before any cross-CTA signal
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  if constexpr (KIND == 1) {  // the block scales, in both CTAs before the even one issues an MMA
+    if (warp >= 2) tc_fill_scales(tmem + kTcScaleCol + ((uint32_t)((warp & 3) * 32) << 16));
+    tc_fence_before();
+    cluster_barrier();
+    tc_fence_after();
+  }
 
   if (warp == 0) {
     if (lane == 0) {
@@ -205,11 +212,13 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         if (skip_item(t)) continue;
         int m0, n0, ncols;
         item_origin(t, m0, n0, ncols);
-        // this CTA's ncols/2 rows of B^T: a 128-row box, or 64 rows for a half tile
-        const bool half = ncols != kTcBN;
+        // this CTA's ncols/2 rows of B^T: a BN/2-row box, or 64 rows for a half
+        // tile (the or_and tail's second half reads 48 of them)
+        const bool half = ncols != BN;
         const CUtensorMap* mb0 = half ? &tmBh0 : &tmB0;
         const CUtensorMap* mb1 = half ? &tmBh1 : &tmB1;
-        const uint32_t bytes = 2 * (Cfg::kNumA * kHalf + Cfg::kNumB * (half ? kHalf / 2 : kHalf));
+        const uint32_t bytes =
+            2 * (Cfg::kNumA * kHalf + Cfg::kNumB * (half ? 64 : BN / 2) * Cfg::kRowBytes);
         const int ma = m0 + (int)rank * 128, nb = n0 + (int)rank * (ncols / 2);
         for (int kt = 0; kt < ktiles; kt++, j++) {
           const int s = j % S;
@@ -221,7 +230,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
           if (rank == 0) mbar_arrive_expect_tx(&full[s], bytes);
           const uint32_t bar0 = map_to_rank(&full[s], 0);
           uint8_t* st = smem + s * kStage;
-          const int kx = kt * Cfg::kBK;
+          const int kx = kt * tc_box_x<KIND>();
           tma_load_2d_pair(st, &tmA0, bar0, kx, ma);
           if constexpr (Cfg::kNumA == 2) tma_load_2d_pair(st + kHalf, &tmA1, bar0, kx, ma);
           uint8_t* sb = st + Cfg::kNumA * kHalf;
@@ -242,13 +251,13 @@ __global__ void __launch_bounds__(kTcThreads, 1)
       for (int t = pair; t < items && ok; t += pairs) {
         if (skip_item(t)) continue;
         const int acc = lt & 1;
-        const uint32_t idesc = t < whole ? tc2_idesc<KIND>() : tc2_idesc<KIND>(kTcBN / 2);
+        const uint32_t idesc = t < whole ? tc2_idesc<KIND>() : tc2_idesc<KIND>(((t - whole) & 1) ? BN - 128 : 128);
         if (!mbar_wait(&acc_empty[acc], ((lt >> 1) & 1) ^ 1)) {
           report_timeout(124);
           break;
         }
         tc_fence_after();
-        const uint32_t d = tmem + acc * kTcBN;
+        const uint32_t d = tmem + acc * BN;
         for (int kt = 0; kt < ktiles; kt++, j++) {
           const int s = j % S;
           if (!mbar_wait(&full[s], (j / S) & 1)) {
@@ -263,14 +272,15 @@ __global__ void __launch_bounds__(kTcThreads, 1)
           constexpr int RB = Cfg::kRowBytes;
 #pragma unroll
           for (int ks = 0; ks < Cfg::kBK / Cfg::kKStep; ks++) {
-            const uint32_t koff = ks * Cfg::kKStep * (KIND == 0 ? 2 : 1);
+            const uint32_t koff = ks * 32;  // bytes along the swizzled row
             const uint32_t acc0 = (kt > 0 || ks > 0) ? 1u : 0u;
             if constexpr (KIND == 0) {
               tc2_mma<0>(d, umma_desc_swizzled(a0 + koff, RB), umma_desc_swizzled(b0 + koff, RB), acc0, idesc);
               tc2_mma<0>(d, umma_desc_swizzled(a0 + koff, RB), umma_desc_swizzled(b1 + koff, RB), 1u, idesc);
               tc2_mma<0>(d, umma_desc_swizzled(a1 + koff, RB), umma_desc_swizzled(b0 + koff, RB), 1u, idesc);
             } else {
-              tc2_mma<1>(d, umma_desc_swizzled(a0 + koff, RB), umma_desc_swizzled(b0 + koff, RB), acc0, idesc);
+              tc2_mma<1>(d, umma_desc_swizzled(a0 + koff, RB), umma_desc_swizzled(b0 + koff, RB), acc0, idesc,
+                         tmem + kTcScaleCol);
             }
           }
           tc2_commit_both(&empty[s]);  // stage s free in both CTAs once these MMAs have read it
@@ -299,23 +309,25 @@ __global__ void __launch_bounds__(kTcThreads, 1)
       tc_fence_after();
       int m0, n0, ncols;
       item_origin(t, m0, n0, ncols);
-      const uint32_t trow = tmem + acc * kTcBN + ((uint32_t)(quad * 32) << 16);
+      const uint32_t trow = tmem + acc * BN + ((uint32_t)(quad * 32) << 16);
       const int row0 = m0 + (int)rank * 128 + quad * 32;
       int changed = 0;
-      tc_tile_epilogue<KIND>(ep, M, N, n0, row0, trow, epi_tile, lane, changed, ncols);
+      auto release = [&] {
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(map_to_rank(&acc_empty[acc], 0));
+      };
+      tc_tile_epilogue<KIND>(ep, M, N, n0, row0, trow, epi_tile, lane, changed, release, ncols);
       if (ep.changed && KIND == 1) {
         const bool any = __any_sync(0xffffffffu, changed);
         if (any && lane == 0) {
           atomicOr(ep.changed, 1);
           if (ep.chg_row) {  // every writer stores 1
             ep.chg_row[m0 / kTc2BM] = 1;
-            ep.chg_col[n0 / kTcBN] = 1;
+            ep.chg_col[n0 / BN] = 1;
           }
         }
       }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive_cluster(map_to_rank(&acc_empty[acc], 0));
       lt++;
     }
   }
