@@ -525,16 +525,16 @@ int launch_sk_skip(const CUtensorMap& a16, const CUtensorMap& b16, const CUtenso
 
 // One product on srgemm_sk_kernel (with cfg.skip or change maps to write, on
 // srgemm_sk_skip_kernel): the operand preparation, then the kernel.
-template <int OP>
-int launch_sk(int M, int N, int K, const float* A, long long lda, const float* B, long long ldb,
-              const EpilogueArgs& ep, uint8_t* ws, const Plan& plan, bool pack_a, const SimtConfig& cfg,
+// T: float, or __half (pack_a then: TMA reads the FP32 copy of A).
+template <int OP, typename T>
+int launch_sk(int M, int N, int K, const T* A, long long lda, const T* B, long long ldb, const EpilogueArgs& ep, uint8_t* ws, const Plan& plan, bool pack_a, const SimtConfig& cfg,
               cudaStream_t stream) {
   const bool skip = cfg.skip || ep.chgA;
   SkShape sh = plan.shape;
   if (skip) sh = {128, (M + 127) / 128, (N + 127) / 128, 0, 0};
   const long long tiles = (long long)sh.tiles_m * sh.tiles_n;
   const bool split = !skip && plan.full && tiles > (long long)sh.whole * sh.grid;
-  SkPrepArgs pa{};
+  SkPrepArgs<T> pa{};
   pa.A = A, pa.lda = lda, pa.B = B, pa.ldb = ldb, pa.M = M, pa.N = N, pa.K = K;
   pa.Kh = plan.Kh, pa.Kp = plan.Kp, pa.Np = plan.Np;
   pa.B32 = reinterpret_cast<float*>(ws + plan.bp_off);
@@ -554,7 +554,7 @@ int launch_sk(int M, int N, int K, const float* A, long long lda, const float* B
     pa.ncounters = skip ? 1 : (int)(tiles - (long long)sh.whole * sh.grid);
   }
   const int prep_grid = (int)std::max(1LL, std::min<long long>((items + 255) / 256, kSkMaxPrepBlocks));
-  sk_prep_kernel<OP><<<prep_grid, 256, 0, stream>>>(pa);
+  sk_prep_kernel<OP, T><<<prep_grid, 256, 0, stream>>>(pa);
   count_launch();
   SIMD2_CUDA_TRY(cudaGetLastError());
   const int t = sh.tile;
@@ -568,7 +568,7 @@ int launch_sk(int M, int N, int K, const float* A, long long lda, const float* B
                           kSkBK16 / 2, CU_TENSOR_MAP_SWIZZLE_NONE)))
       return rc;
   }
-  if ((rc = make_map_f32(&a32, pack_a ? pa.A32 : A, M, pack_a ? plan.Kp : K, pack_a ? plan.Kp : lda, kBK, t,
+  if ((rc = make_map_f32(&a32, pack_a ? (const void*)pa.A32 : (const void*)A, M, pack_a ? plan.Kp : K, pack_a ? plan.Kp : lda, kBK, t,
                          CU_TENSOR_MAP_SWIZZLE_128B, true)))
     return rc;
   if ((rc = make_map_f32(&b32, pa.B32, plan.Kp / 2, 2LL * plan.Np, 2LL * plan.Np, 2 * t, kBK / 2,
@@ -601,6 +601,24 @@ int launch_sk(int M, int N, int K, const float* A, long long lda, const float* B
                   : launch_sk_tile<OP, 64>(a16, b16, a32, b32, ga, grid, ep, stream);
 }
 
+template <typename T>
+int launch_sk_op(int op, int M, int N, int K, const T* A, long long lda, const T* B, long long ldb,
+                 const EpilogueArgs& ep, uint8_t* ws, const Plan& plan, bool pack_a, const SimtConfig& cfg,
+                 cudaStream_t stream) {
+  switch (op) {
+#define SIMD2_SK_CASE(OPV) \
+  case OPV: return launch_sk<OPV, T>(M, N, K, A, lda, B, ldb, ep, ws, plan, pack_a, cfg, stream);
+    SIMD2_SK_CASE(SIMD2_MIN_PLUS)
+    SIMD2_SK_CASE(SIMD2_MAX_PLUS)
+    SIMD2_SK_CASE(SIMD2_MAX_MIN)
+    SIMD2_SK_CASE(SIMD2_MAX_MUL)
+    SIMD2_SK_CASE(SIMD2_MIN_MUL)
+    SIMD2_SK_CASE(SIMD2_MIN_MAX)
+#undef SIMD2_SK_CASE
+    default: return SIMD2_ERR_UNSUPPORTED;
+  }
+}
+
 // Core float srgemm of the min/max semirings with an explicit workspace (a full
 // plan for anything but the plain configuration).  A forced split-K factor runs
 // on srgemm_simt_kernel, everything else on the persistent kernels.
@@ -609,20 +627,7 @@ int srgemm_core(int op, int M, int N, int K, const float* A, long long lda, cons
                 const SimtConfig& cfg = SimtConfig()) {
   SimtConfig c1 = cfg;
   c1.skip = cfg.skip && cfg.occA && cfg.occB && skip_supported(op);
-  if (cfg.split == 1) {
-    switch (op) {
-#define SIMD2_SK_CASE(OPV) \
-  case OPV: return launch_sk<OPV>(M, N, K, A, lda, B, ldb, ep, ws, plan, pack_a, c1, stream);
-      SIMD2_SK_CASE(SIMD2_MIN_PLUS)
-      SIMD2_SK_CASE(SIMD2_MAX_PLUS)
-      SIMD2_SK_CASE(SIMD2_MAX_MIN)
-      SIMD2_SK_CASE(SIMD2_MAX_MUL)
-      SIMD2_SK_CASE(SIMD2_MIN_MUL)
-      SIMD2_SK_CASE(SIMD2_MIN_MAX)
-#undef SIMD2_SK_CASE
-      default: return SIMD2_ERR_UNSUPPORTED;
-    }
-  }
+  if (cfg.split == 1) return launch_sk_op<float>(op, M, N, K, A, lda, B, ldb, ep, ws, plan, pack_a, c1, stream);
   const float pad = pad_value(op);
   float* Bp = reinterpret_cast<float*>(ws + plan.bp_off);
   interleave_pairs_kernel<float, 0><<<grid_for((long long)plan.Kp / 2 * plan.Np / 4), 256, 0, stream>>>(
@@ -660,10 +665,11 @@ constexpr CUtensorMapSwizzle tc_swizzle() {
   return TcCfg<KIND>::kRowBytes == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B;
 }
 
-template <int KIND>
+// bn: columns of a tile.  BT: B is N-major ([K][N]).
+template <int KIND, bool BT>
 int launch_tc(int M, int N, int K, const CUtensorMap& a0, const CUtensorMap& a1, const CUtensorMap& b0,
-              const CUtensorMap& b1, const TcEpilogue& ep, cudaStream_t stream) {
-  auto kern = tc_gemm_kernel<KIND>;
+              const CUtensorMap& b1, const TcEpilogue& ep, int bn, cudaStream_t stream) {
+  auto kern = tc_gemm_kernel<KIND, BT>;
   const size_t smem = tc_smem_bytes<KIND>();
   static bool configured[64] = {};
   int dev = 0;
@@ -674,14 +680,12 @@ int launch_tc(int M, int N, int K, const CUtensorMap& a0, const CUtensorMap& a1,
     configured[dev] = true;
   }
   const int tiles_m = (M + kTcBM - 1) / kTcBM;
-  const int tiles_n = (N + tc_bn<KIND>() - 1) / tc_bn<KIND>();
+  const int tiles_n = (N + bn - 1) / bn;
   auto* ev = prof_slot(2LL * M * N * K, kProfTensor);
   if (ev) cudaEventRecord(ev->first, stream);
   // persistent: at most one CTA per SM (shared memory and TMEM hold one)
-  int sms = 148;
-  SIMD2_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  const int grid = std::min(tiles_m * tiles_n, sms);
-  kern<<<grid, kTcThreads, smem, stream>>>(a0, a1, b0, b1, M, N, K, ep, tiles_m, tiles_n);
+  const int grid = std::min(tiles_m * tiles_n, device_sms());
+  kern<<<grid, kTcThreads, smem, stream>>>(a0, a1, b0, b1, M, N, K, ep, tiles_m, tiles_n, bn);
   count_launch();
   if (ev) cudaEventRecord(ev->second, stream);
   SIMD2_CUDA_TRY(cudaGetLastError());
@@ -699,8 +703,7 @@ inline bool use_tc2(int M, int N) {
 // SM-pair launch: clusters of 2 CTAs, one pair per pair of SMs at most.
 template <int KIND>
 int launch_tc2(int M, int N, int K, const CUtensorMap& a0, const CUtensorMap& a1, const CUtensorMap& b0,
-               const CUtensorMap& b1, const CUtensorMap& bh0, const CUtensorMap& bh1, const TcEpilogue& ep,
-               cudaStream_t stream) {
+               const CUtensorMap& b1, const CUtensorMap& bh, const TcEpilogue& ep, cudaStream_t stream) {
   auto kern = tc_gemm2_kernel<KIND>;
   const size_t smem = tc2_smem_bytes<KIND>();
   static int max_pairs[64] = {};
@@ -731,31 +734,52 @@ int launch_tc2(int M, int N, int K, const CUtensorMap& a0, const CUtensorMap& a1
   lc.gridDim = dim3(2 * pairs);
   auto* ev = prof_slot(2LL * M * N * K, kProfTensor);
   if (ev) cudaEventRecord(ev->first, stream);
-  SIMD2_CUDA_TRY(cudaLaunchKernelEx(&lc, kern, a0, a1, b0, b1, bh0, bh1, M, N, K, ep, tiles_m, tiles_n));
+  SIMD2_CUDA_TRY(cudaLaunchKernelEx(&lc, kern, a0, a1, b0, b1, bh, M, N, K, ep, tiles_m, tiles_n));
   count_launch();
   if (ev) cudaEventRecord(ev->second, stream);
   SIMD2_CUDA_TRY(cudaGetLastError());
   return SIMD2_OK;
 }
 
+// Columns of a tile of the single-SM kernel for the sums: the one whose tiles take
+// the fewest SM-times of arithmetic and epilogue.  A K step of 16 costs N / 2
+// cycles an MMA (three for the BF16 split), the epilogue about 20 cycles a
+// column, a tile about 3000 cycles by itself.  1500 x 2100 x 300 on 148 SMs: 108
+// tiles of 256 columns or 132 of 192; 1000 x 800 x 3000: 32 tiles of 256 or 104 of 64.
+int tc_tile_columns(int M, int N, int K, int mmas) {
+  const int sms = device_sms();
+  int best = kTcBN;
+  double best_cost = 1e300;
+  for (int bn : {256, 192, 128, 64}) {
+    const long long tiles = (long long)((M + kTcBM - 1) / kTcBM) * ((N + bn - 1) / bn);
+    const double cost = (double)((tiles + sms - 1) / sms) * (bn * ((K + 15) / 16 * mmas / 2.0 + 20.0) + 3000.0);
+    if (cost < best_cost) {
+      best_cost = cost;
+      best = bn;
+    }
+  }
+  return best;
+}
+
 struct TcPlan {
-  int Kp;
-  size_t a0, a1, b0, b1, na, nb, nb64, total;
+  int Kp, Np;
+  size_t a0, a1, b0, b1, na, nb, total;
 };
 
-// bf16 hi/lo operands (plus_mul, minus_square)
-TcPlan tc_plan_bf16(int M, int N, int K) {
+// Copies of the sums' operands (BF16 hi / lo, or halves: a1 and b1 unused), A
+// [M][Kp], B [K][Np].
+TcPlan tc_plan_sum(int M, int N, int K) {
   TcPlan p{};
   p.Kp = round_up(std::max(K, 1), 8);
+  p.Np = round_up(std::max(N, 1), 8);
   size_t off = 0;
   auto take = [&](size_t bytes) { size_t o = off; off += align_up(bytes, kAlign); return o; };
   p.a0 = take((size_t)M * p.Kp * 2);
   p.a1 = take((size_t)M * p.Kp * 2);
-  p.b0 = take((size_t)N * p.Kp * 2);
-  p.b1 = take((size_t)N * p.Kp * 2);
+  p.b0 = take((size_t)K * p.Np * 2);
+  p.b1 = take((size_t)K * p.Np * 2);
   p.na = take((size_t)M * 4);
   p.nb = take((size_t)N * 4);
-  p.nb64 = take((size_t)N * 8);
   p.total = off;
   return p;
 }
@@ -770,7 +794,7 @@ TcPlan tc_plan_fp4(int M, int N, int K) {
   p.b0 = take((size_t)N * p.Kp / 2);
   p.a1 = p.a0;
   p.b1 = p.b0;
-  p.na = p.nb = p.nb64 = 0;
+  p.na = p.nb = 0;
   p.total = off;
   return p;
 }
@@ -778,45 +802,55 @@ TcPlan tc_plan_fp4(int M, int N, int K) {
 // Band of the minus_square exact recompute: distances below 2^-6 of |a|^2+|b|^2.
 constexpr float kMinusSquareBand = 1.0f / 64.0f;
 
-int srgemm_tc_sum(int op, int M, int N, int K, const float* A, long long lda, const float* B, long long ldb,
-                  const float* C, long long ldc, float* D, long long ldd, int do_epilogue, uint8_t* ws,
-                  const TcPlan& plan, cudaStream_t stream) {
-  const int Kp = plan.Kp;
-  auto* ahi = reinterpret_cast<__nv_bfloat16*>(ws + plan.a0);
-  auto* alo = reinterpret_cast<__nv_bfloat16*>(ws + plan.a1);
-  split_rows_bf16_kernel<<<grid_for((long long)M * Kp / 8), 256, 0, stream>>>(A, lda, M, K, ahi, alo, Kp);
-  count_launch();
-  float* na = reinterpret_cast<float*>(ws + plan.na);
-  float* nb = reinterpret_cast<float*>(ws + plan.nb);
-  double* nb64 = op == SIMD2_MINUS_SQUARE ? reinterpret_cast<double*>(ws + plan.nb64) : nullptr;
-  if (nb64) SIMD2_CUDA_TRY(cudaMemsetAsync(nb64, 0, sizeof(double) * N, stream));
-  dim3 tgrid((N + 31) / 32, (Kp + 31) / 32), tblock(32, 8);
-  transpose_prep_kernel<<<tgrid, tblock, 0, stream>>>(B, ldb, K, N, ws + plan.b0, ws + plan.b1, Kp, nb64);
-  count_launch();
-  if (op == SIMD2_MINUS_SQUARE) {
-    row_norms_kernel<<<grid_for((long long)M * 32), 256, 0, stream>>>(A, lda, M, K, na);
-    count_launch();
-    round_norms_kernel<<<grid_for(N), 256, 0, stream>>>(nb64, N, nb);
-    count_launch();
+// plus_mul and minus_square on FP32 (BF16 hi / lo split, three MMAs a k step) or
+// float16 operands (one).
+template <typename T>
+int srgemm_tc_sum(int op, int M, int N, int K, const T* A, long long lda, const T* B, long long ldb, const float* C,
+                  long long ldc, float* D, long long ldd, int do_epilogue, uint8_t* ws, const TcPlan& plan,
+                  cudaStream_t stream) {
+  constexpr bool kHalf = std::is_same<T, __half>::value;
+  constexpr int KIND = kHalf ? 2 : 0;
+  const bool msq = op == SIMD2_MINUS_SQUARE;
+  // TMA reads float16 operands as they are where their rows lie on 16-byte boundaries
+  auto tma_ok = [](const T* p, long long ld) { return reinterpret_cast<uintptr_t>(p) % 16 == 0 && ld % 8 == 0; };
+  const bool copy_a = !kHalf || !tma_ok(A, lda), copy_b = !kHalf || !tma_ok(B, ldb);
+  SumPrepArgs pa{};
+  pa.A = A, pa.lda = lda, pa.B = B, pa.ldb = ldb;
+  pa.M = M, pa.N = N, pa.K = K, pa.Kp = plan.Kp, pa.Np = plan.Np;
+  if (copy_a) {
+    pa.a_hi = reinterpret_cast<uint16_t*>(ws + plan.a0);
+    pa.a_lo = reinterpret_cast<uint16_t*>(ws + plan.a1);
   }
-  SIMD2_CUDA_TRY(cudaGetLastError());
+  if (copy_b) {
+    pa.b_hi = reinterpret_cast<uint16_t*>(ws + plan.b0);
+    pa.b_lo = reinterpret_cast<uint16_t*>(ws + plan.b1);
+  }
+  if (msq) {
+    pa.na = reinterpret_cast<float*>(ws + plan.na);
+    pa.nb = reinterpret_cast<float*>(ws + plan.nb);
+  }
+  pa.a_blocks = copy_a || msq ? std::min((M + 7) / 8, 148 * 8) : 0;
+  pa.b_blocks = copy_b ? (int)std::min<long long>(((long long)K * plan.Np / 8 + 255) / 256, 148 * 8) : 0;
+  const int blocks = pa.a_blocks + pa.b_blocks + (msq ? (N + 15) / 16 : 0);
+  if (blocks > 0) {
+    sum_prep_kernel<T><<<blocks, 256, 0, stream>>>(pa);
+    count_launch();
+    SIMD2_CUDA_TRY(cudaGetLastError());
+  }
+  const auto DT = kHalf ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
+  constexpr int BX = tc_box_k<KIND>();
+  const void* am = copy_a ? (const void*)pa.a_hi : (const void*)A;
+  const void* bm = copy_b ? (const void*)pa.b_hi : (const void*)B;
+  const long long ap = copy_a ? plan.Kp : lda, bp = copy_b ? plan.Np : ldb;
   CUtensorMap ma0, ma1, mb0, mb1;
-  const auto BF = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
-  const auto SW = tc_swizzle<0>();
-  constexpr int BX = tc_box_k<0>();
   int rc;
-  // the SM-pair kernel stages B in halves of 128 rows
-  const bool pair = use_tc2(M, N);
-  const int brows = pair ? 128 : kTcBN;
-  if ((rc = make_map_2d(&ma0, BF, 2, ahi, M, Kp, Kp, BX, kTcBM, SW))) return rc;
-  if ((rc = make_map_2d(&ma1, BF, 2, alo, M, Kp, Kp, BX, kTcBM, SW))) return rc;
-  if ((rc = make_map_2d(&mb0, BF, 2, ws + plan.b0, N, Kp, Kp, BX, brows, SW))) return rc;
-  if ((rc = make_map_2d(&mb1, BF, 2, ws + plan.b1, N, Kp, Kp, BX, brows, SW))) return rc;
-  // the pair kernel's half tiles stage 64 rows of B^T per CTA
-  CUtensorMap mbh0 = mb0, mbh1 = mb1;
-  if (pair) {
-    if ((rc = make_map_2d(&mbh0, BF, 2, ws + plan.b0, N, Kp, Kp, BX, 64, SW))) return rc;
-    if ((rc = make_map_2d(&mbh1, BF, 2, ws + plan.b1, N, Kp, Kp, BX, 64, SW))) return rc;
+  if ((rc = make_map_2d(&ma0, DT, 2, am, M, copy_a ? plan.Kp : K, ap, BX, kTcBM, tc_swizzle<KIND>()))) return rc;
+  if ((rc = make_map_2d(&mb0, DT, 2, bm, K, copy_b ? plan.Np : N, bp, 64, BX, CU_TENSOR_MAP_SWIZZLE_128B))) return rc;
+  ma1 = ma0;
+  mb1 = mb0;
+  if (!kHalf) {
+    if ((rc = make_map_2d(&ma1, DT, 2, pa.a_lo, M, plan.Kp, ap, BX, kTcBM, tc_swizzle<KIND>()))) return rc;
+    if ((rc = make_map_2d(&mb1, DT, 2, pa.b_lo, K, plan.Np, bp, 64, BX, CU_TENSOR_MAP_SWIZZLE_128B))) return rc;
   }
   TcEpilogue ep{};
   ep.op = op;
@@ -825,16 +859,16 @@ int srgemm_tc_sum(int op, int M, int N, int K, const float* A, long long lda, co
   ep.ldc = do_epilogue ? ldc : ldd;
   ep.D = D;
   ep.ldd = ldd;
-  ep.norm_a = na;
-  ep.norm_b = nb;
+  ep.norm_a = pa.na;
+  ep.norm_b = pa.nb;
   ep.A32 = A;
   ep.lda32 = lda;
   ep.B32 = B;
   ep.ldb32 = ldb;
   ep.K = K;
   ep.band = kMinusSquareBand;
-  if (pair) return launch_tc2<0>(M, N, K, ma0, ma1, mb0, mb1, mbh0, mbh1, ep, stream);
-  return launch_tc<0>(M, N, K, ma0, ma1, mb0, mb1, ep, stream);
+  if (use_tc2(M, N)) return launch_tc2<KIND>(M, N, K, ma0, ma1, mb0, mb1, mb0, ep, stream);
+  return launch_tc<KIND, true>(M, N, K, ma0, ma1, mb0, mb1, ep, tc_tile_columns(M, N, K, kHalf ? 1 : 3), stream);
 }
 
 // delta (or_and closure, pair kernel only): the maps of TcEpilogue.
@@ -845,9 +879,10 @@ struct TcDelta {
   const uint8_t* need_col = nullptr;
 };
 
-template <typename T>
-int srgemm_tc_orand(int M, int N, int K, const T* A, long long lda, const T* B, long long ldb, const T* C,
-                    long long ldc, T* D, long long ldd, int do_epilogue, int* changed, uint8_t* ws,
+// T: A and B; U: C and D.
+template <typename T, typename U>
+int srgemm_tc_orand(int M, int N, int K, const T* A, long long lda, const T* B, long long ldb, const U* C,
+                    long long ldc, U* D, long long ldd, int do_epilogue, int* changed, uint8_t* ws,
                     const TcPlan& plan, cudaStream_t stream, const TcDelta& delta = TcDelta()) {
   const int Kp = plan.Kp;
   uint8_t* a4 = ws + plan.a0;
@@ -874,16 +909,16 @@ int srgemm_tc_orand(int M, int N, int K, const T* A, long long lda, const T* B, 
   ep.ldc = do_epilogue ? ldc : ldd;
   ep.D = D;
   ep.ldd = ldd;
-  ep.out_type = sizeof(T) == 1 ? kOrU8 : kOrI32;
+  ep.out_type = std::is_same<U, uint8_t>::value ? kOrU8 : std::is_same<U, int32_t>::value ? kOrI32 : kOrF32;
   ep.changed = changed;
   if (pair) {
     ep.chg_row = delta.chg_row;
     ep.chg_col = delta.chg_col;
     ep.need_row = delta.need_row;
     ep.need_col = delta.need_col;
-    return launch_tc2<1>(M, N, K, ma, ma, mb, mb, mbh, mbh, ep, stream);
+    return launch_tc2<1>(M, N, K, ma, ma, mb, mb, mbh, ep, stream);
   }
-  return launch_tc<1>(M, N, K, ma, ma, mb, mb, ep, stream);
+  return launch_tc<1, false>(M, N, K, ma, ma, mb, mb, ep, BN, stream);
 }
 
 int check_dims(int M, int N, int K, long long lda, long long ldb, long long ldc, long long ldd, const void* A,
@@ -929,7 +964,7 @@ int srgemm_f32_ws(int op, int M, int N, int K, const float* A, long long lda, co
                   uint8_t* ws_or_null, cudaStream_t stream) {
   if (K == 0) return srgemm_k0(op, M, N, C, ldc, D, ldd, do_epilogue, stream);
   if (is_sum_op(op)) {
-    const TcPlan tp = tc_plan_bf16(M, N, K);
+    const TcPlan tp = tc_plan_sum(M, N, K);
     uint8_t* ws = ws_or_null;
     if (!ws) {
       void* p = nullptr;
@@ -937,7 +972,7 @@ int srgemm_f32_ws(int op, int M, int N, int K, const float* A, long long lda, co
       if (rc) return rc;
       ws = static_cast<uint8_t*>(p);
     }
-    return srgemm_tc_sum(op, M, N, K, A, lda, B, ldb, C, ldc, D, ldd, do_epilogue, ws, tp, stream);
+    return srgemm_tc_sum<float>(op, M, N, K, A, lda, B, ldb, C, ldc, D, ldd, do_epilogue, ws, tp, stream);
   }
   const bool pack_a = !a_tma_ok(A, lda);
   // a caller's workspace holds the base plan only
@@ -975,7 +1010,7 @@ int srgemm_orand(int M, int N, int K, const T* A, long long lda, const T* B, lon
   const TcPlan plan = tc_plan_fp4(M, N, K);
   void* p = nullptr;
   if ((rc = get_workspace(stream, plan.total, &p))) return rc;
-  return srgemm_tc_orand<T>(M, N, K, A, lda, B, ldb, C, ldc, D, ldd, do_epilogue, nullptr,
+  return srgemm_tc_orand<T, T>(M, N, K, A, lda, B, ldb, C, ldc, D, ldd, do_epilogue, nullptr,
                             static_cast<uint8_t*>(p), plan, stream);
 }
 
@@ -1574,7 +1609,7 @@ int simd2_closure_orand_u8(int n, uint8_t* X, int ldx, int max_iter, int* iters_
       par ^= 1;
     }
     it++;
-    rc = srgemm_tc_orand<uint8_t>(n, n, n, cur, ldcur, cur, ldcur, cur, ldcur, nxt, ldnxt, 1, flag, ws, plan, stream,
+    rc = srgemm_tc_orand<uint8_t, uint8_t>(n, n, n, cur, ldcur, cur, ldcur, cur, ldcur, nxt, ldnxt, 1, flag, ws, plan, stream,
                                   dl);
     if (rc) return rc;
     int h = 0;
@@ -1606,7 +1641,7 @@ int simd2_closure_panel_step(simd2_op op, int rows, int n, const void* panel, in
     void* p = nullptr;
     if ((rc = get_workspace(stream, plan.total, &p))) return rc;
     const auto* P = static_cast<const uint8_t*>(panel);
-    return srgemm_tc_orand<uint8_t>(rows, n, n, P, ldp, static_cast<const uint8_t*>(full), ldf, P, ldp,
+    return srgemm_tc_orand<uint8_t, uint8_t>(rows, n, n, P, ldp, static_cast<const uint8_t*>(full), ldf, P, ldp,
                                     static_cast<uint8_t*>(out), ldo, 1, changed, static_cast<uint8_t*>(p), plan,
                                     stream);
   }
@@ -3074,7 +3109,7 @@ extern "C" int simd2_knn_ex(const float* query, int Q, int ldq, const float* ref
     ep.b_rows = 1;
     ep.K = D;
     ep.band = kMinusSquareBand;
-    if ((rc = launch_tc<0>(rows, R, D, ma0, ma1, mb0, mb1, ep, stream))) return rc;
+    if ((rc = launch_tc<0, false>(rows, R, D, ma0, ma1, mb0, mb1, ep, kTcBN, stream))) return rc;
     float* od = out_dist + (size_t)q0 * ldo;
     int32_t* oi = out_idx + (size_t)q0 * ldo;
     if (k <= 4) rc = knn_topk_launch<4>(dist, R, rows, R, od, oi, ldo, k, stream);
@@ -3098,55 +3133,35 @@ extern "C" int simd2_srgemm_f16(simd2_op op, int M, int N, int K, const void* A,
   int rc = check_dims(M, N, K, lda, ldb, ldc, ldd, A, B, C, D, do_epilogue);
   if (rc || M == 0 || N == 0) return rc;
   if ((rc = check_device())) return rc;
-  // or_and on {0,1}: the max_min semiring on booleans (AND = min, OR = max)
-  const bool boolean = op == SIMD2_OR_AND;
-  const int run_op = boolean ? SIMD2_MAX_MIN : op;
-  size_t off = 0;
-  auto take = [&](size_t bytes) { size_t o = off; off += align_up(std::max(bytes, (size_t)4), kAlign); return o; };
-  const size_t a_off = take((size_t)M * K * 4), b_off = take((size_t)K * N * 4);
-  const size_t c_off = take(boolean && do_epilogue ? (size_t)M * N * 4 : 4);
-  const size_t plan_off = off;
-  const size_t need = is_sum_op(run_op) ? tc_plan_bf16(M, N, K).total : make_plan(M, N, K, false).total;
+  const auto* a = static_cast<const __half*>(A);
+  const auto* b = static_cast<const __half*>(B);
+  if (K == 0) {
+    if (op != SIMD2_OR_AND) return srgemm_k0(op, M, N, C, ldc, D, ldd, do_epilogue, stream);
+    if (do_epilogue) bool_copy_kernel<float><<<grid_for((long long)M * N), 256, 0, stream>>>(C, ldc, D, ldd, M, N);
+    else fill_kernel<float><<<grid_for((long long)M * N), 256, 0, stream>>>(D, ldd, M, N, 0.0f);
+    count_launch();
+    SIMD2_CUDA_TRY(cudaGetLastError());
+    return SIMD2_OK;
+  }
   void* p = nullptr;
-  if ((rc = get_workspace(stream, plan_off + need, &p))) return rc;
-  uint8_t* ws = static_cast<uint8_t*>(p);
-  float* Af = reinterpret_cast<float*>(ws + a_off);
-  float* Bf = reinterpret_cast<float*>(ws + b_off);
-  const float* Cuse = C;
-  long long ldc_use = ldc;
-  if (K > 0) {
-    if (boolean) {
-      half_to_float_kernel<1><<<grid_for((long long)M * K), 256, 0, stream>>>(static_cast<const __half*>(A), lda, M, K,
-                                                                              Af);
-      half_to_float_kernel<1><<<grid_for((long long)K * N), 256, 0, stream>>>(static_cast<const __half*>(B), ldb, K, N,
-                                                                              Bf);
-    } else {
-      half_to_float_kernel<0><<<grid_for((long long)M * K), 256, 0, stream>>>(static_cast<const __half*>(A), lda, M, K,
-                                                                              Af);
-      half_to_float_kernel<0><<<grid_for((long long)K * N), 256, 0, stream>>>(static_cast<const __half*>(B), ldb, K, N,
-                                                                              Bf);
-    }
-    count_launch();
-    count_launch();
+  if (op == SIMD2_OR_AND) {
+    const TcPlan plan = tc_plan_fp4(M, N, K);
+    if ((rc = get_workspace(stream, plan.total, &p))) return rc;
+    return srgemm_tc_orand<__half, float>(M, N, K, a, lda, b, ldb, C, ldc, D, ldd, do_epilogue, nullptr,
+                                          static_cast<uint8_t*>(p), plan, stream);
   }
-  if (boolean && do_epilogue) {
-    float* Cb = reinterpret_cast<float*>(ws + c_off);
-    float_bool_kernel<<<grid_for((long long)M * N), 256, 0, stream>>>(C, ldc, M, N, Cb);
-    count_launch();
-    Cuse = Cb;
-    ldc_use = N;
+  if (is_sum_op(op)) {
+    const TcPlan plan = tc_plan_sum(M, N, K);
+    if ((rc = get_workspace(stream, plan.total, &p))) return rc;
+    return srgemm_tc_sum<__half>(op, M, N, K, a, lda, b, ldb, C, ldc, D, ldd, do_epilogue, static_cast<uint8_t*>(p),
+                                 plan, stream);
   }
-  SIMD2_CUDA_TRY(cudaGetLastError());
-  rc = srgemm_f32_ws(run_op, M, N, K, Af, K, Bf, N, Cuse, ldc_use, D, ldd, do_epilogue, nullptr, 0, ws + plan_off,
-                     stream);
-  if (rc) return rc;
-  if (boolean && K == 0 && !do_epilogue) {
-    // or_and identity is 0, not max_min's -inf
-    fill_kernel<float><<<grid_for((long long)M * N), 256, 0, stream>>>(D, ldd, M, N, 0.0f);
-    count_launch();
-  }
-  SIMD2_CUDA_TRY(cudaGetLastError());
-  return SIMD2_OK;
+  // the prep kernel reads the halves and writes the same copies as for FP32
+  const Plan plan = make_plan(M, N, K, true, true, op);
+  if ((rc = get_workspace(stream, plan.total, &p))) return rc;
+  const EpilogueArgs ep = make_epilogue(C, ldc, D, ldd, do_epilogue, nullptr, 0);
+  return launch_sk_op<__half>(op, M, N, K, a, lda, b, ldb, ep, static_cast<uint8_t*>(p), plan, true, SimtConfig(),
+                              stream);
 }
 
 namespace simd2 {

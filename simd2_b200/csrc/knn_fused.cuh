@@ -299,9 +299,9 @@ __global__ void __launch_bounds__(kKfThreads, 1)
 #pragma unroll
           for (int ks = 0; ks < 4; ks++) {
             const uint32_t ko = ks * 32;  // 16 BF16 along the 128-byte row
-            tc_mma<0>(d, umma_desc_sw128(ah + ko), umma_desc_sw128(bh + ko), (p > 0 || ks > 0) ? 1u : 0u);
-            tc_mma<0>(d, umma_desc_sw128(ah + ko), umma_desc_sw128(bl + ko), 1u);
-            tc_mma<0>(d, umma_desc_sw128(al + ko), umma_desc_sw128(bh + ko), 1u);
+            tc_mma<0>(d, umma_desc_sw128(ah + ko), umma_desc_sw128(bh + ko), (p > 0 || ks > 0) ? 1u : 0u, TcCfg<0>::kIdesc);
+            tc_mma<0>(d, umma_desc_sw128(ah + ko), umma_desc_sw128(bl + ko), 1u, TcCfg<0>::kIdesc);
+            tc_mma<0>(d, umma_desc_sw128(al + ko), umma_desc_sw128(bh + ko), 1u, TcCfg<0>::kIdesc);
           }
           tc_commit(&empty[sh]);
           tc_commit(&empty[sl]);

@@ -82,30 +82,6 @@ __global__ void fill_kernel(T* D, long long ldd, int M, int N, T value) {
   }
 }
 
-// half -> float (MODE 0) or half -> {0,1} float (MODE 1), [M][K] pitch lda -> dense [M][K].
-template <int MODE>
-__global__ void half_to_float_kernel(const __half* __restrict__ A, long long lda, int M, int K, float* __restrict__ out) {
-  const long long total = (long long)M * K;
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
-       t += (long long)gridDim.x * blockDim.x) {
-    const int i = (int)(t / K);
-    const int k = (int)(t - (long long)i * K);
-    const float v = __half2float(A[(long long)i * lda + k]);
-    out[t] = MODE == 1 ? (v != 0.f ? 1.f : 0.f) : v;
-  }
-}
-
-// float -> {0,1} float, [M][N] pitch ldc -> dense.
-__global__ void float_bool_kernel(const float* __restrict__ C, long long ldc, int M, int N, float* __restrict__ out) {
-  const long long total = (long long)M * N;
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
-       t += (long long)gridDim.x * blockDim.x) {
-    const int i = (int)(t / N);
-    const int j = (int)(t - (long long)i * N);
-    out[t] = C[(long long)i * ldc + j] != 0.f ? 1.f : 0.f;
-  }
-}
-
 // Change test + copy, the work of comp_update / comp_update2
 // (kernel/converge.cuh:6-84): mode 1 |prev-cur| > 1e-4, mode 2 maps cur values
 // in (-1,1) to -FLT_MAX first (in cur and prev) then tests inequality, mode 0
@@ -304,42 +280,120 @@ __global__ void __launch_bounds__(256) transpose_fp4_kernel(const T* __restrict_
   }
 }
 
-// B [K][N] (pitch ldb) -> transposed K-major [N][Kp] through a 32 x 32 shared
-// tile (coalesced reads along n, coalesced writes along k).
-// BF16 hi/lo split: out0 = hi, out1 = lo.
-// colsq (nullable): sum over k of B[k][j]^2 accumulated in FP64 (atomicAdd per
-// 32-row tile; the caller zeroes it and rounds it to float afterwards).
-__global__ void transpose_prep_kernel(const float* __restrict__ B, long long ldb, int K, int N, void* __restrict__ out0,
-                                      void* __restrict__ out1, int Kp, double* __restrict__ colsq = nullptr) {
-  __shared__ float tile[32][33];
-  const int k0 = blockIdx.y * 32;
-  const int j0 = blockIdx.x * 32;
-  for (int i = threadIdx.y; i < 32; i += blockDim.y) {
-    const int k = k0 + i, j = j0 + threadIdx.x;
-    float v = 0.f;
-    if (k < K && j < N) {
-      v = B[(long long)k * ldb + j];
+// Operand preparation of the sums, one launch: blocks [0, a_blocks) take rows of
+// A, a warp each, the next b_blocks rows of B, the last ones 16 columns of B each.  FP32 operands are split into BF16 hi / lo copies of the same layout
+// (A [M][Kp], B [K][Np], zeros past K and N); float16 ones are copied only where
+// TMA cannot read them as they are (a_hi / b_hi set).  minus_square (na / nb set):
+// the squared row norms of A and column norms of B, summed in FP64.
+struct SumPrepArgs {
+  const void* A;
+  long long lda;
+  const void* B;
+  long long ldb;
+  int M, N, K, Kp, Np;
+  uint16_t *a_hi, *a_lo, *b_hi, *b_lo;
+  float *na, *nb;
+  int a_blocks, b_blocks;
+};
+
+// 8 consecutive elements as floats, zeros past `left`.
+template <typename T>
+__device__ __forceinline__ void load8(const T* p, int left, float (&x)[8]) {
+  if (left >= 8 && (reinterpret_cast<uintptr_t>(p) & 15) == 0) {
+    if constexpr (sizeof(T) == 4) {
+      const float4 u = __ldg(reinterpret_cast<const float4*>(p)), w = __ldg(reinterpret_cast<const float4*>(p) + 1);
+      x[0] = u.x, x[1] = u.y, x[2] = u.z, x[3] = u.w, x[4] = w.x, x[5] = w.y, x[6] = w.z, x[7] = w.w;
+    } else {
+      const uint4 u = __ldg(reinterpret_cast<const uint4*>(p));
+      const uint32_t in[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+        x[2 * q] = __half2float(__ushort_as_half((unsigned short)(in[q] & 0xffffu)));
+        x[2 * q + 1] = __half2float(__ushort_as_half((unsigned short)(in[q] >> 16)));
+      }
     }
-    tile[i][threadIdx.x] = v;
+  } else {
+#pragma unroll
+    for (int e = 0; e < 8; e++) x[e] = e < left ? (float)p[e] : 0.f;
   }
-  __syncthreads();
-  if (colsq != nullptr && threadIdx.y == 0 && j0 + (int)threadIdx.x < N) {
-    double s = 0.0;
-    for (int i = 0; i < 32; i++) {
-      const double v = tile[i][threadIdx.x];
-      s += v * v;
+}
+
+// The copies of 8 elements: hi / lo of BF16, or (lo null) the halves.
+template <typename T>
+__device__ __forceinline__ void store8(const float (&x)[8], uint16_t* hi, uint16_t* lo) {
+  uint32_t hw[4], lw[4];
+#pragma unroll
+  for (int q = 0; q < 4; q++) {
+    if constexpr (sizeof(T) == 4) {
+      __nv_bfloat16 h0, l0, h1, l1;
+      split_bf16(x[2 * q], h0, l0);
+      split_bf16(x[2 * q + 1], h1, l1);
+      hw[q] = pack_bf16x2(h0, h1);
+      lw[q] = pack_bf16x2(l0, l1);
+    } else {
+      hw[q] = (uint32_t)__half_as_ushort(__float2half_rn(x[2 * q])) |
+              (uint32_t)__half_as_ushort(__float2half_rn(x[2 * q + 1])) << 16;
     }
-    atomicAdd(colsq + j0 + threadIdx.x, s);
   }
-  for (int i = threadIdx.y; i < 32; i += blockDim.y) {
-    const int j = j0 + i, k = k0 + threadIdx.x;
-    if (j < N && k < Kp) {
-      const float v = tile[threadIdx.x][i];
-      const long long o = (long long)j * Kp + k;
-      __nv_bfloat16 h, l;
-      split_bf16(v, h, l);
-      static_cast<__nv_bfloat16*>(out0)[o] = h;
-      static_cast<__nv_bfloat16*>(out1)[o] = l;
+  *reinterpret_cast<uint4*>(hi) = make_uint4(hw[0], hw[1], hw[2], hw[3]);
+  if constexpr (sizeof(T) == 4) *reinterpret_cast<uint4*>(lo) = make_uint4(lw[0], lw[1], lw[2], lw[3]);
+}
+
+template <typename T>
+__global__ void __launch_bounds__(256) sum_prep_kernel(SumPrepArgs g) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const T* A = static_cast<const T*>(g.A);
+  const T* B = static_cast<const T*>(g.B);
+  if ((int)blockIdx.x < g.a_blocks) {
+    for (int i = blockIdx.x * 8 + warp; i < g.M; i += g.a_blocks * 8) {
+      double sum = 0.0;
+      for (int k = lane * 8; k < g.Kp; k += 256) {
+        float x[8];
+        load8(A + (long long)i * g.lda + k, g.K - k, x);
+        if (g.a_hi) {
+          const long long o = (long long)i * g.Kp + k;
+          store8<T>(x, g.a_hi + o, g.a_lo + o);
+        }
+        if (g.na) {
+#pragma unroll
+          for (int e = 0; e < 8; e++) sum += (double)x[e] * (double)x[e];
+        }
+      }
+      if (g.na) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        if (lane == 0) g.na[i] = (float)sum;
+      }
+    }
+  } else if ((int)blockIdx.x < g.a_blocks + g.b_blocks) {
+    const int groups = g.Np >> 3;
+    const long long total = (long long)g.K * groups;
+    for (long long t = (blockIdx.x - g.a_blocks) * 256LL + threadIdx.x; t < total; t += g.b_blocks * 256LL) {
+      const int k = (int)(t / groups), j = (int)(t - (long long)k * groups) * 8;
+      float x[8];
+      load8(B + (long long)k * g.ldb + j, g.N - j, x);
+      store8<T>(x, g.b_hi + t * 8, g.b_lo + t * 8);
+    }
+  } else {
+    // thread: one of 16 columns, one of 16 runs of k; the partial sums meet in order
+    __shared__ double part[16][16];
+    const int c = threadIdx.x & 15, q = threadIdx.x >> 4;
+    const int j = (blockIdx.x - g.a_blocks - g.b_blocks) * 16 + c;
+    const int per = (g.K + 15) / 16, k1 = min(g.K, (q + 1) * per);
+    double sum = 0.0;
+    if (j < g.N) {
+#pragma unroll 16
+      for (int k = q * per; k < k1; k++) {
+        const double v = (double)(float)B[(long long)k * g.ldb + j];
+        sum += v * v;
+      }
+    }
+    part[q][c] = sum;
+    __syncthreads();
+    if (q == 0 && j < g.N) {
+#pragma unroll
+      for (int r = 1; r < 16; r++) sum += part[r][c];
+      g.nb[j] = (float)sum;
     }
   }
 }
@@ -356,11 +410,6 @@ __global__ void row_norms_kernel(const float* __restrict__ A, long long lda, int
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     if (threadIdx.x % 32 == 0) out[i] = (float)s;
   }
-}
-
-// double -> float (norms accumulated in FP64).
-__global__ void round_norms_kernel(const double* __restrict__ in, int n, float* __restrict__ out) {
-  for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) out[j] = (float)in[j];
 }
 
 }  // namespace simd2

@@ -155,10 +155,11 @@ constexpr int kSkBK16 = 64;         // k of a 16-bit k-tile (128-byte rows)
 constexpr int kSkMaxPrepBlocks = 1184;  // 8 blocks of 256 threads on each SM
 constexpr int kSkMaxCounters = 512;
 
+template <typename T>
 struct SkPrepArgs {
-  const float* A;
+  const T* A;
   long long lda;
-  const float* B;
+  const T* B;
   long long ldb;
   int M, N, K;
   int Kh, Kp, Np;    // K padded to 64 / 32, N padded to 128
@@ -173,16 +174,29 @@ struct SkPrepArgs {
   const int* gate;
 };
 
+// 4 elements, aligned to 4 * sizeof(T).
+__device__ __forceinline__ void load4(const float* p, float (&x)[4]) {
+  const float4 u = __ldg(reinterpret_cast<const float4*>(p));
+  x[0] = u.x, x[1] = u.y, x[2] = u.z, x[3] = u.w;
+}
+__device__ __forceinline__ void load4(const __half* p, float (&x)[4]) {
+  const uint2 u = __ldg(reinterpret_cast<const uint2*>(p));
+  x[0] = __half2float(__ushort_as_half((unsigned short)(u.x & 0xffffu)));
+  x[1] = __half2float(__ushort_as_half((unsigned short)(u.x >> 16)));
+  x[2] = __half2float(__ushort_as_half((unsigned short)(u.y & 0xffffu)));
+  x[3] = __half2float(__ushort_as_half((unsigned short)(u.y >> 16)));
+}
+
 // Rows of A to codes (8 per thread), 4 columns x 2 k of B to both B layouts,
 // rows of A to the packed FP32 copy (4 per thread) where TMA cannot read A.
-template <int OP>
-__global__ void __launch_bounds__(256) sk_prep_kernel(SkPrepArgs g) {
+template <int OP, typename T>
+__global__ void __launch_bounds__(256) sk_prep_kernel(SkPrepArgs<T> g) {
   if (g.gate && *g.gate == 0) return;
   bool bad = false;
   const long long tid = blockIdx.x * 256LL + threadIdx.x, step = gridDim.x * 256LL;
   for (long long t = tid; t < g.ncounters; t += step) g.counters[t] = 0;
-  const bool va = (g.lda % 4 == 0) && (reinterpret_cast<uintptr_t>(g.A) % 16 == 0);
-  const bool vb = (g.ldb % 4 == 0) && (reinterpret_cast<uintptr_t>(g.B) % 16 == 0);
+  // 4 elements of B at a time where its rows allow (16 bytes, or 8 of halves)
+  const bool vb = (g.ldb % 4 == 0) && (reinterpret_cast<uintptr_t>(g.B) % (4 * sizeof(T)) == 0);
   constexpr bool k16 = has_code16(OP);
   if constexpr (k16) {
     if (g.A16) {
@@ -191,17 +205,16 @@ __global__ void __launch_bounds__(256) sk_prep_kernel(SkPrepArgs g) {
       for (long long t = tid; t < total; t += step) {
         const int i = (int)(t / groups);
         const int k0 = (int)(t - (long long)i * groups) * 8;
-        const float* row = g.A + (long long)i * g.lda;
+        const int left = g.K - k0;
+        float x[8];
+        load8(g.A + (long long)i * g.lda + k0, left, x);
         uint32_t c[8];
-        if (va && k0 + 8 <= g.K) {
-          const float4 u = __ldg(reinterpret_cast<const float4*>(row + k0));
-          const float4 w = __ldg(reinterpret_cast<const float4*>(row + k0 + 4));
-          const float x[8] = {u.x, u.y, u.z, u.w, w.x, w.y, w.z, w.w};
+        if (left >= 8) {
 #pragma unroll
           for (int e = 0; e < 8; e++) c[e] = Code16<OP>::encode(x[e], bad);
         } else {
 #pragma unroll
-          for (int e = 0; e < 8; e++) c[e] = k0 + e < g.K ? Code16<OP>::encode(row[k0 + e], bad) : Code16<OP>::kPad;
+          for (int e = 0; e < 8; e++) c[e] = e < left ? Code16<OP>::encode(x[e], bad) : Code16<OP>::kPad;
         }
         reinterpret_cast<uint4*>(g.A16)[t] =
             make_uint4(c[0] | c[1] << 16, c[2] | c[3] << 16, c[4] | c[5] << 16, c[6] | c[7] << 16);
@@ -220,17 +233,16 @@ __global__ void __launch_bounds__(256) sk_prep_kernel(SkPrepArgs g) {
 #pragma unroll
       for (int r = 0; r < 2; r++) {
         const int k = 2 * p + r;
-        const float* row = g.B + (long long)k * g.ldb;
+        const T* row = g.B + (long long)k * g.ldb;
         if (vb && k < g.K && j + 4 <= g.N) {
-          const float4 u = __ldg(reinterpret_cast<const float4*>(row + j));
-          x[r][0] = u.x, x[r][1] = u.y, x[r][2] = u.z, x[r][3] = u.w;
+          load4(row + j, x[r]);
 #pragma unroll
           for (int e = 0; e < 4; e++) in[r][e] = true;
         } else {
 #pragma unroll
           for (int e = 0; e < 4; e++) {
             in[r][e] = k < g.K && j + e < g.N;
-            x[r][e] = in[r][e] ? row[j + e] : g.pad;
+            x[r][e] = in[r][e] ? (float)row[j + e] : g.pad;
           }
         }
       }
@@ -259,10 +271,10 @@ __global__ void __launch_bounds__(256) sk_prep_kernel(SkPrepArgs g) {
     for (long long t = tid; t < total; t += step) {
       const int i = (int)(t / quads);
       const int k = (int)(t - (long long)i * quads) * 4;
-      const float* row = g.A + (long long)i * g.lda + k;
+      const T* row = g.A + (long long)i * g.lda + k;
       float x[4];
 #pragma unroll
-      for (int e = 0; e < 4; e++) x[e] = k + e < g.K ? row[e] : g.pad;
+      for (int e = 0; e < 4; e++) x[e] = k + e < g.K ? (float)row[e] : g.pad;
       reinterpret_cast<float4*>(g.A32)[t] = make_float4(x[0], x[1], x[2], x[3]);
     }
   }

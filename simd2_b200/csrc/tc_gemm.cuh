@@ -12,6 +12,8 @@
 //                    3000 x 2500 x 2000 int32 call 117 us, now 56.
 //   * plus_mul     : kind::f16 with BF16 hi/lo operands, FP32 accumulate:
 //                    a*b ~= a_hi*b_hi + a_hi*b_lo + a_lo*b_hi  (three MMAs per k step).
+//   * float16 operands (KIND 2): one kind::f16 MMA per k step on the halves
+//                    themselves, whose products FP32 holds exactly.
 //   * minus_square : the same BF16 hi/lo product gives a.b; the epilogue forms
 //                    |a|^2 + |b|^2 - 2 a.b with FP64-accumulated norms and
 //                    recomputes sum_k (a-b)^2 exactly in FP32 inside the
@@ -19,16 +21,19 @@
 //
 // Persistent: one CTA per SM walks the 128 x 256 tiles of D (grouped raster)
 // with 6 warps:
-//   warp 0 lane 0  -- TMA producer (2D tiled loads, no multicast; 64-byte
-//                     swizzled rows for BF16, 128-byte for FP4) over every
-//                     k-tile of every tile, one ring of stages,
+//   warp 0 lane 0  -- TMA producer (2D tiled loads, no multicast, 128-byte
+//                     swizzled rows) over every k-tile of every tile, one ring
+//                     of stages,
 //   warp 1 lane 0  -- MMA issuer (tcgen05.mma, cta_group::1, M=128, N=256 or
 //                     224) into one of two TMEM accumulators, so the next
 //                     tile's MMAs run while the previous tile is written out,
-//   warps 2..5     -- epilogue: tcgen05.ld of the accumulator (warp w reads
-//                     TMEM lanes 32(w%4)..+31 = tile rows), fused (+) C, stores.
-// Both operands are K-major in shared memory: A is [M][K] as given, B is
-// stored transposed ([N][K]) by the operand-prep kernel.
+//   warps 2..9     -- epilogue: tcgen05.ld of the accumulator (warp w reads
+//                     TMEM lanes 32(w%4)..+31 = tile rows, the lower or the upper
+//                     half of the tile's columns), fused (+) C, stores.
+// A is K-major in shared memory, [M][K] as given.  B: or_and's FP4 copy and
+// k-NN's references are K-major ([N][K]); the sums read B [K][N] as it is, N-major
+// (BT), so that no transposed copy is made (plus_mul 8192^3: the transposing
+// BF16 split of B took 163 us, the plain one takes 85).
 #pragma once
 #include "common.cuh"
 #include "prep.cuh"
@@ -43,21 +48,20 @@ template <int KIND>
 __host__ __device__ constexpr int tc_bn() { return KIND == 1 ? 224 : kTcBN; }
 constexpr int kTcScaleCol = 448;  // first TMEM column of the block scales
 constexpr int kTcScaleCols = 32;  // 4 columns of A's and 8 of B's, all the same byte
-constexpr int kTcEpiWarps = 4;
-constexpr int kTcThreads = (2 + kTcEpiWarps) * 32;  // TMA warp, MMA warp, 4 epilogue warps
+constexpr int kTcEpiWarps = 8;
+constexpr int kTcThreads = (2 + kTcEpiWarps) * 32;  // TMA warp, MMA warp, 8 epilogue warps
 template <int KIND>
 struct TcCfg;
-// BF16 hi/lo: BK = 32 elements (64-byte swizzled rows), two A tiles and two B
-// tiles per stage, 4 stages of 48 KiB: three stages stay in flight while one
-// feeds the tensor cores (two 96 KiB stages of 128-byte rows left the TMA
-// latency exposed).
+// BF16 hi/lo: BK = 64 elements, two A tiles and two B tiles per stage.  128-byte
+// rows halve the rows TMA has to fetch for A against 64-byte ones (BK = 32, twice
+// the stages): 4096^3 320 us for 308, 1000 x 800 x 3000 50 for 42.
 template <>
 struct TcCfg<0> {
-  static constexpr int kBK = 32;
-  static constexpr int kRowBytes = 64;
+  static constexpr int kBK = 64;
+  static constexpr int kRowBytes = 128;
   static constexpr int kNumA = 2;
   static constexpr int kNumB = 2;
-  static constexpr int kStages = 4;
+  static constexpr int kStages = 2;
   static constexpr int kKStep = 16;  // K per tcgen05.mma kind::f16
   // c_format F32 (1), a/b format BF16 (1), K-major A and B, N=256, M=128
   static constexpr uint32_t kIdesc =
@@ -77,6 +81,26 @@ struct TcCfg<1> {
                                      ((uint32_t)(kTcBM >> 7) << 27);
 };
 
+// Float16: BK = 64 elements, one A and one B tile per stage.
+template <>
+struct TcCfg<2> {
+  static constexpr int kBK = 64;
+  static constexpr int kRowBytes = 128;
+  static constexpr int kNumA = 1;
+  static constexpr int kNumB = 1;
+  static constexpr int kStages = 4;
+  static constexpr int kKStep = 16;
+  // c_format F32 (1), a/b format F16 (0)
+  static constexpr uint32_t kIdesc =
+      (1u << 4) | ((uint32_t)(kTcBN >> 3) << 17) | ((uint32_t)(kTcBM >> 4) << 24);
+};
+
+// Instruction descriptor with N = n, B N-major when bt.
+template <int KIND>
+__host__ __device__ constexpr uint32_t tc_idesc(int n, bool bt) {
+  return (TcCfg<KIND>::kIdesc & ~(0x3Fu << 17)) | ((uint32_t)(n >> 3) << 17) | (bt ? 1u << 16 : 0u);
+}
+
 template <int KIND>
 __host__ __device__ constexpr int tc_a_tile() { return kTcBM * TcCfg<KIND>::kRowBytes; }
 template <int KIND>
@@ -84,7 +108,10 @@ __host__ __device__ constexpr int tc_b_tile() { return tc_bn<KIND>() * TcCfg<KIN
 
 // k-tile step in tensor-map elements: BF16 values, or bytes of two FP4 values.
 template <int KIND>
-__host__ __device__ constexpr int tc_box_x() { return KIND == 1 ? TcCfg<1>::kRowBytes : TcCfg<0>::kBK; }
+__host__ __device__ constexpr int tc_box_x() { return KIND == 1 ? TcCfg<1>::kRowBytes : TcCfg<KIND>::kBK; }
+// N-major B: one box holds kBK rows of 64 columns.
+template <int KIND>
+__host__ __device__ constexpr int tc_b_group() { return TcCfg<KIND>::kBK * 128; }
 template <int KIND>
 __host__ __device__ constexpr int tc_stage_bytes() {
   return TcCfg<KIND>::kNumA * tc_a_tile<KIND>() + TcCfg<KIND>::kNumB * tc_b_tile<KIND>();
@@ -109,6 +136,19 @@ __device__ __forceinline__ uint64_t umma_desc_swizzled(uint32_t smem_addr, int r
   return d;
 }
 
+// The descriptor of an N-major operand tile: groups of 64 columns (128 bytes,
+// 128-byte swizzle) `group_bytes` apart (leading byte offset), 8-k groups 1024
+// bytes apart (stride byte offset).  Advancing K by 16 moves the start by 2048.
+__device__ __forceinline__ uint64_t umma_desc_nmajor(uint32_t smem_addr, int group_bytes) {
+  uint64_t d = 0;
+  d |= (uint64_t)((smem_addr >> 4) & 0x3FFFu);
+  d |= (uint64_t)((uint32_t)group_bytes >> 4) << 16;
+  d |= (uint64_t)(1024u >> 4) << 32;
+  d |= (uint64_t)1u << 46;
+  d |= (uint64_t)2u << 61;
+  return d;
+}
+
 // The descriptor for 128-byte swizzled rows (8-row groups 1024 bytes apart).
 __device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t smem_addr) {
   return umma_desc_swizzled(smem_addr, 128);
@@ -120,18 +160,18 @@ __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence:
 // `scales`: TMEM address of the block scales (KIND 1; both operands read the same columns).
 template <int KIND>
 __device__ __forceinline__ void tc_mma(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t accumulate,
-                                       uint32_t scales = 0) {
-  if constexpr (KIND == 0) {
+                                       uint32_t idesc, uint32_t scales = 0) {
+  if constexpr (KIND != 1) {
     asm volatile(
         "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
         "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}\n" ::"r"(tmem_d),
-        "l"(adesc), "l"(bdesc), "r"(TcCfg<0>::kIdesc), "r"(accumulate), "r"(0), "r"(0), "r"(0), "r"(0));
+        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(0), "r"(0), "r"(0), "r"(0));
   } else {
     asm volatile(
         "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
         "tcgen05.mma.cta_group::1.kind::mxf4.block_scale.scale_vec::2X [%0], %1, %2, %3, [%5], [%5], p;\n\t}\n" ::"r"(
             tmem_d),
-        "l"(adesc), "l"(bdesc), "r"(TcCfg<1>::kIdesc), "r"(accumulate), "r"(scales));
+        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(scales));
   }
 }
 
@@ -197,13 +237,14 @@ struct TcEpilogue {
   void* D;
   long long ldd;
   int out_type;         // or_and: type of C and D (kOrU8, kOrI32, kOrF32)
-  // minus_square: row norms of A (M), column norms of B (N), and the FP32
-  // operands for the exact recompute inside the cancellation band.
+  // minus_square: row norms of A (M), column norms of B (N), and the operands
+  // as given (FP32, KIND 2: float16) for the exact recompute inside the
+  // cancellation band.
   const float* norm_a;
   const float* norm_b;
-  const float* A32;
+  const void* A32;
   long long lda32;
-  const float* B32;
+  const void* B32;
   long long ldb32;
   int K;
   float band;           // recompute when dist < band * (|a|^2 + |b|^2)
@@ -222,18 +263,19 @@ struct TcEpilogue {
 
 // sum_k (a[k] - B[k][col])^2 in FP32; B is [K][N] (pitch ldb) or, when
 // b_rows, stored transposed as [N][K].
-__device__ __forceinline__ float exact_minus_square(const float* a, const float* B, long long ldb, int col, int K,
+template <typename T>
+__device__ __forceinline__ float exact_minus_square(const T* a, const T* B, long long ldb, int col, int K,
                                                     int b_rows) {
   float s = 0.f;
   if (b_rows) {
-    const float* b = B + (long long)col * ldb;
+    const T* b = B + (long long)col * ldb;
     for (int k = 0; k < K; k++) {
-      const float d = __fsub_rn(a[k], b[k]);
+      const float d = __fsub_rn((float)a[k], (float)b[k]);
       s = __fmaf_rn(d, d, s);
     }
   } else {
     for (int k = 0; k < K; k++) {
-      const float d = __fsub_rn(a[k], B[(long long)k * ldb + col]);
+      const float d = __fsub_rn((float)a[k], (float)B[(long long)k * ldb + col]);
       s = __fmaf_rn(d, d, s);
     }
   }
@@ -299,14 +341,14 @@ __device__ __forceinline__ void tc_or_store(const TcEpilogue& ep, int M, int N, 
             }
             *dst = v;
           } else {
-            int4 v = make_int4(nib & 1, nib >> 1 & 1, nib >> 2 & 1, nib >> 3);
-            if (epi) {
-              v.x |= old[q].x != 0;
-              v.y |= old[q].y != 0;
-              v.z |= old[q].z != 0;
-              v.w |= old[q].w != 0;
-            }
-            *dst = v;
+            // a float 1.0 and 0.0 by their bits; -0.0 is false
+            constexpr bool kF32 = std::is_same<T, float>::value;
+            constexpr int one = kF32 ? 0x3f800000 : 1, mask = kF32 ? 0x7fffffff : -1;
+            uint32_t f = nib;
+            if (epi)
+              f |= (uint32_t)((old[q].x & mask) != 0) | (uint32_t)((old[q].y & mask) != 0) << 1 |
+                   (uint32_t)((old[q].z & mask) != 0) << 2 | (uint32_t)((old[q].w & mask) != 0) << 3;
+            *dst = make_int4(f & 1 ? one : 0, f & 2 ? one : 0, f & 4 ? one : 0, f & 8 ? one : 0);
           }
         }
       }
@@ -329,23 +371,21 @@ __device__ __forceinline__ void tc_or_store(const TcEpilogue& ep, int M, int N, 
             v |= o;
             if (v != o) changed = 1;
           }
-          D[(row0 + r0 + q) * ep.ldd + n0 + c] = static_cast<T>(static_cast<float>(v));
+          D[(row0 + r0 + q) * ep.ldd + n0 + c] = static_cast<T>(v);
         }
       }
     }
   }
 }
 
-// Epilogue of one 128 x ncols tile (ncols a multiple of 32: tc_bn, or less for
-// a split tail tile) for the 32 rows of one warp: lane l holds row row0 + l of the
-// accumulator in TMEM at trow (lane quadrant and column base included).  release()
-// hands the accumulator back.  Sets changed when an or_and output differs from C.
+// Epilogue of the 32 rows x ncols columns (a multiple of 32) of one warp: lane l
+// holds row row0 + l of the accumulator in TMEM at trow (lane quadrant and column
+// base included), columns n0...  release() hands the accumulator back.  Sets changed when an or_and output differs from C.
 template <int KIND, typename F>
 __device__ __forceinline__ void tc_tile_epilogue(const TcEpilogue& ep, int M, int N, int n0, int row0, uint32_t trow,
-                                                 uint32_t* epi_tile, int lane, int& changed, F release,
-                                                 int ncols = tc_bn<KIND>()) {
+                                                 uint32_t* epi_tile, int lane, int& changed, F release, int ncols) {
+  ncols = min(ncols, max(0, (N - n0 + 31) & ~31));
   if constexpr (KIND == 1) {
-    ncols = min(ncols, (N - n0 + 31) & ~31);
     tc_or_bits(trow, epi_tile, lane, ncols);
     release();
     if (ep.out_type == kOrU8) tc_or_store<uint8_t>(ep, M, N, n0, row0, epi_tile, lane, changed, ncols);
@@ -394,8 +434,10 @@ __device__ __forceinline__ void tc_tile_epilogue(const TcEpilogue& ep, int M, in
         while (band) {
           const int rr = __ffs(band) - 1;
           band &= band - 1;
-          tile[rr * 33 + lane] = __float_as_uint(exact_minus_square(
-              ep.A32 + (long long)(row0 + rr) * ep.lda32, ep.B32, ep.ldb32, col, ep.K, ep.b_rows));
+          using T = typename std::conditional<KIND == 2, __half, float>::type;
+          tile[rr * 33 + lane] = __float_as_uint(
+              exact_minus_square(static_cast<const T*>(ep.A32) + (long long)(row0 + rr) * ep.lda32,
+                                 static_cast<const T*>(ep.B32), ep.ldb32, col, ep.K, ep.b_rows));
         }
       }
       if (col_ok) {
@@ -414,25 +456,49 @@ __device__ __forceinline__ void tc_tile_epilogue(const TcEpilogue& ep, int M, in
     release();
   }
 }
-template <int KIND>
+// The columns of a tile's epilogue that fall to `half` (0, 1): whole 32s.
+__device__ __forceinline__ void tc_epi_columns(int ncols, int half, int& first, int& count) {
+  const int h = (ncols / 2 + 31) & ~31;
+  first = half ? h : 0;
+  count = half ? ncols - h : h;
+}
+
+// Ring of the single-SM kernel: a stage holds A and bn columns of B, and as many
+// stages as fit are used, at most kTcMaxStages: a narrow tile's k-tiles pass
+// faster, so more of them have to be on their way.
+constexpr int kTcMaxStages = 8;
+template <int KIND, bool BT>
+__host__ __device__ constexpr int tc_stage_of(int bn) {
+  return BT ? TcCfg<KIND>::kNumA * tc_a_tile<KIND>() + TcCfg<KIND>::kNumB * (bn >> 6) * tc_b_group<KIND>()
+            : tc_stage_bytes<KIND>();
+}
+template <int KIND, bool BT>
+__host__ __device__ constexpr int tc_stages_of(int bn) {
+  const int fit = TcCfg<KIND>::kStages * tc_stage_bytes<KIND>() / tc_stage_of<KIND, BT>(bn);
+  return fit < kTcMaxStages ? fit : kTcMaxStages;
+}
+
+// bn: columns of a tile (a multiple of 64, at most 256; 224 for or_and).
+template <int KIND, bool BT>
 __global__ void __launch_bounds__(kTcThreads, 1)
     tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__ CUtensorMap tmA1,
                    const __grid_constant__ CUtensorMap tmB0, const __grid_constant__ CUtensorMap tmB1, int M, int N,
-                   int K, TcEpilogue ep, int tiles_m, int tiles_n) {
+                   int K, TcEpilogue ep, int tiles_m, int tiles_n, int bn) {
   using Cfg = TcCfg<KIND>;
-  constexpr int S = Cfg::kStages;
-  constexpr int kStage = tc_stage_bytes<KIND>();
+  const int S = tc_stages_of<KIND, BT>(bn);
+  const int stage_bytes = tc_stage_of<KIND, BT>(bn);
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint32_t* epi_smem = reinterpret_cast<uint32_t*>(smem + S * kStage);  // 4 x 32 x 33 words
+  uint32_t* epi_smem = reinterpret_cast<uint32_t*>(smem + Cfg::kStages * tc_stage_bytes<KIND>());  // 32 x 33 words per epilogue warp
   uint64_t* full = reinterpret_cast<uint64_t*>(epi_smem + kTcEpiWarps * 32 * 33);
-  uint64_t* empty = full + S;
-  uint64_t* acc_full = empty + S;
+  uint64_t* empty = full + kTcMaxStages;
+  uint64_t* acc_full = empty + kTcMaxStages;
   uint64_t* acc_empty = acc_full + 2;
   uint64_t* fin = acc_empty + 2;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(fin + 1);
 
   const int tiles = tiles_m * tiles_n;
+  const uint32_t idesc = tc_idesc<KIND>(bn, BT);
   const int ktiles = (K + Cfg::kBK - 1) / Cfg::kBK;
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -445,7 +511,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     const int gsize = min(tiles_m - first_m, group);
     const int local = t - g * per_group;
     m0 = (first_m + local % gsize) * kTcBM;
-    n0 = (local / gsize) * tc_bn<KIND>();
+    n0 = (local / gsize) * bn;
   };
 
   if (threadIdx.x == 0) {
@@ -483,26 +549,38 @@ __global__ void __launch_bounds__(kTcThreads, 1)
       // ---------------- TMA producer: every k-tile of every tile of this CTA ----------------
       prefetch_tensormap(&tmA0);
       prefetch_tensormap(&tmB0);
-      int j = 0;  // running stage counter
+      int s = 0;  // ring position
+      uint32_t ph = 1;
       bool ok = true;
       for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
         int m0, n0;
         tile_origin(t, m0, n0);
-        for (int kt = 0; kt < ktiles; kt++, j++) {
-          const int s = j % S;
-          if (!mbar_wait(&empty[s], ((j / S) & 1) ^ 1)) {
+        for (int kt = 0; kt < ktiles; kt++) {
+          if (!mbar_wait(&empty[s], ph)) {
             report_timeout(101);
             ok = false;
             break;
           }
-          uint8_t* st = smem + s * kStage;
-          mbar_arrive_expect_tx(&full[s], kStage);
+          uint8_t* st = smem + s * stage_bytes;
+          mbar_arrive_expect_tx(&full[s], stage_bytes);
           const int kx = kt * tc_box_x<KIND>();
           tma_load_2d(st, &tmA0, &full[s], kx, m0);
           if constexpr (Cfg::kNumA == 2) tma_load_2d(st + tc_a_tile<KIND>(), &tmA1, &full[s], kx, m0);
           uint8_t* sb = st + Cfg::kNumA * tc_a_tile<KIND>();
-          tma_load_2d(sb, &tmB0, &full[s], kx, n0);
-          if constexpr (Cfg::kNumB == 2) tma_load_2d(sb + tc_b_tile<KIND>(), &tmB1, &full[s], kx, n0);
+          if constexpr (BT) {
+            for (int g = 0; g < (bn >> 6); g++) {
+              tma_load_2d(sb + g * tc_b_group<KIND>(), &tmB0, &full[s], n0 + 64 * g, kx);
+              if constexpr (Cfg::kNumB == 2)
+                tma_load_2d(sb + ((bn >> 6) + g) * tc_b_group<KIND>(), &tmB1, &full[s], n0 + 64 * g, kx);
+            }
+          } else {
+            tma_load_2d(sb, &tmB0, &full[s], kx, n0);
+            if constexpr (Cfg::kNumB == 2) tma_load_2d(sb + tc_b_tile<KIND>(), &tmB1, &full[s], kx, n0);
+          }
+          if (++s == S) {
+            s = 0;
+            ph ^= 1;
+          }
         }
       }
     }
@@ -510,7 +588,8 @@ __global__ void __launch_bounds__(kTcThreads, 1)
   } else if (warp == 1) {
     if (lane == 0) {
       // ---------------- MMA issuer: tile lt accumulates into TMEM half lt & 1 ----------------
-      int j = 0;
+      int s = 0;
+      uint32_t ph = 0;
       bool ok = true;
       int lt = 0;
       for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x, lt++) {
@@ -521,33 +600,39 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         }
         tc_fence_after();
         const uint32_t d = tmem + acc * tc_bn<KIND>();
-        for (int kt = 0; kt < ktiles; kt++, j++) {
-          const int s = j % S;
-          if (!mbar_wait(&full[s], (j / S) & 1)) {
+        for (int kt = 0; kt < ktiles; kt++) {
+          if (!mbar_wait(&full[s], ph)) {
             report_timeout(102);
             ok = false;
             break;
           }
           tc_fence_after();
-          const uint32_t st = smem_u32(smem + s * kStage);
+          const uint32_t st = smem_u32(smem + s * stage_bytes);
           const uint32_t a0 = st, a1 = st + tc_a_tile<KIND>();
-          const uint32_t b0 = st + Cfg::kNumA * tc_a_tile<KIND>(), b1 = b0 + tc_b_tile<KIND>();
+          const uint32_t b0 = st + Cfg::kNumA * tc_a_tile<KIND>();
+          const uint32_t b1 = b0 + (BT ? (bn >> 6) * tc_b_group<KIND>() : tc_b_tile<KIND>());
           constexpr int RB = Cfg::kRowBytes;
 #pragma unroll
           for (int ks = 0; ks < Cfg::kBK / Cfg::kKStep; ks++) {
             const uint32_t koff = ks * 32;  // bytes along the swizzled row
             const uint32_t acc0 = (kt > 0 || ks > 0) ? 1u : 0u;
+            auto bdesc = [&](uint32_t b) {
+              return BT ? umma_desc_nmajor(b + ks * 2048, tc_b_group<KIND>()) : umma_desc_swizzled(b + koff, RB);
+            };
             if constexpr (KIND == 0) {
               // hi*hi, hi*lo, lo*hi
-              tc_mma<0>(d, umma_desc_swizzled(a0 + koff, RB), umma_desc_swizzled(b0 + koff, RB), acc0);
-              tc_mma<0>(d, umma_desc_swizzled(a0 + koff, RB), umma_desc_swizzled(b1 + koff, RB), 1u);
-              tc_mma<0>(d, umma_desc_swizzled(a1 + koff, RB), umma_desc_swizzled(b0 + koff, RB), 1u);
+              tc_mma<0>(d, umma_desc_swizzled(a0 + koff, RB), bdesc(b0), acc0, idesc);
+              tc_mma<0>(d, umma_desc_swizzled(a0 + koff, RB), bdesc(b1), 1u, idesc);
+              tc_mma<0>(d, umma_desc_swizzled(a1 + koff, RB), bdesc(b0), 1u, idesc);
             } else {
-              tc_mma<1>(d, umma_desc_swizzled(a0 + koff, RB), umma_desc_swizzled(b0 + koff, RB), acc0,
-                        tmem + kTcScaleCol);
+              tc_mma<KIND>(d, umma_desc_swizzled(a0 + koff, RB), bdesc(b0), acc0, idesc, tmem + kTcScaleCol);
             }
           }
           tc_commit(&empty[s]);  // stage s is free once these MMAs have read it
+          if (++s == S) {
+            s = 0;
+            ph ^= 1;
+          }
         }
         if (ok) tc_commit(&acc_full[acc]);  // accumulator complete
       }
@@ -555,7 +640,9 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     }
     __syncwarp();
   } else {
-    // ---------------- epilogue warps 2..5: warp w reads TMEM lanes 32 (w % 4) .. ----------------
+    // ---------------- epilogue warps 2..9: warp w reads TMEM lanes 32 (w % 4) .. ----------------
+    int cfirst, ccount;
+    tc_epi_columns(bn, (warp - 2) >> 2, cfirst, ccount);
     const int quad = warp & 3;
     uint32_t* epi_tile = epi_smem + (warp - 2) * (32 * 33);
     bool ok = true;
@@ -571,7 +658,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
       tc_fence_after();
       int m0, n0;
       tile_origin(t, m0, n0);
-      const uint32_t trow = tmem + acc * tc_bn<KIND>() + ((uint32_t)(quad * 32) << 16);
+      const uint32_t trow = tmem + acc * tc_bn<KIND>() + cfirst + ((uint32_t)(quad * 32) << 16);
       const int row0 = m0 + quad * 32;
       int changed = 0;
       // the accumulator half is read out: the MMA warp may reuse it
@@ -580,7 +667,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         __syncwarp();
         if (lane == 0) mbar_arrive(&acc_empty[acc]);
       };
-      tc_tile_epilogue<KIND>(ep, M, N, n0, row0, trow, epi_tile, lane, changed, release);
+      tc_tile_epilogue<KIND>(ep, M, N, n0 + cfirst, row0, trow, epi_tile, lane, changed, release, ccount);
       if (ep.changed && KIND == 1) {
         if (__any_sync(0xffffffffu, changed) && lane == 0) atomicOr(ep.changed, 1);
       }

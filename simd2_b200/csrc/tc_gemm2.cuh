@@ -16,7 +16,7 @@
 //   warp 1 lane 0 -- (even CTA only) MMA issuer: tcgen05.mma.cta_group::2,
 //                    commits multicast to both CTAs' stage-free and
 //                    accumulator-full barriers,
-//   warps 2..5    -- epilogue of this CTA's 128 rows (the tc_gemm.cuh tile
+//   warps 2..9    -- epilogue of this CTA's 128 rows (the tc_gemm.cuh tile
 //                    epilogue), releasing the accumulator on the even CTA's
 //                    barrier (remote arrive from the odd CTA).
 // Every wait is bounded; every path ends at one cluster barrier, so neither
@@ -24,7 +24,7 @@
 //
 // Tail split: with T tiles on P pairs the last round holds r = T mod P tiles.
 // When 2r <= P those r tiles run as 2r half tiles of 256 x 128 (MMA N = 128;
-// each CTA loads a 64-row B box through the tmBh maps), so the last round
+// each CTA loads one 64-column group of B, or a 64-row box through the tmBh map), so the last round
 // takes about half a tile's time: 4096^2 on 74 pairs is 3.5 rounds of work
 // instead of 4.
 #pragma once
@@ -34,7 +34,9 @@
 namespace simd2 {
 
 constexpr int kTc2BM = 256;      // rows of D per pair tile
-constexpr int kTc2Stages = 6;
+// 6 stages of 32 KiB (the BF16 split: 3 of 64)
+template <int KIND>
+__host__ __device__ constexpr int tc2_stages() { return KIND == 0 ? 3 : 6; }
 
 template <int KIND>
 __host__ __device__ constexpr int tc2_half_tile() { return 128 * TcCfg<KIND>::kRowBytes; }
@@ -44,14 +46,13 @@ __host__ __device__ constexpr int tc2_stage_bytes() {
 }
 template <int KIND>
 constexpr size_t tc2_smem_bytes() {
-  return (size_t)kTc2Stages * tc2_stage_bytes<KIND>() + (size_t)kTcEpiWarps * 32 * 33 * 4 + 1024 + 256;
+  return (size_t)tc2_stages<KIND>() * tc2_stage_bytes<KIND>() + (size_t)kTcEpiWarps * 32 * 33 * 4 + 1024 + 256;
 }
 // instruction descriptor: TcCfg's with M = 256 and N = n (M / 16 at bit 24 is
 // mxf4's M / 128 at bit 27)
 template <int KIND>
-__host__ __device__ constexpr uint32_t tc2_idesc(int n = tc_bn<KIND>()) {
-  return (TcCfg<KIND>::kIdesc & ~(0x1Fu << 24) & ~(0x3Fu << 17)) | ((uint32_t)(kTc2BM >> 4) << 24) |
-         ((uint32_t)(n >> 3) << 17);
+__host__ __device__ constexpr uint32_t tc2_idesc(int n, bool bt) {
+  return (tc_idesc<KIND>(n, bt) & ~(0x1Fu << 24)) | ((uint32_t)(kTc2BM >> 4) << 24);
 }
 
 __device__ __forceinline__ uint32_t cluster_rank2() {
@@ -84,7 +85,7 @@ __device__ __forceinline__ void tma_load_2d_pair(void* dst, const CUtensorMap* m
 template <int KIND>
 __device__ __forceinline__ void tc2_mma(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t accumulate,
                                         uint32_t idesc, uint32_t scales = 0) {
-  if constexpr (KIND == 0) {
+  if constexpr (KIND != 1) {
     asm volatile(
         "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
         "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8, %9, %10, %11, %12}, p;\n\t}\n" ::"r"(
@@ -108,15 +109,17 @@ __device__ __forceinline__ void tc2_commit_both(uint64_t* bar) {
       : "memory");
 }
 
+// B is N-major for the sums (KIND 0, 2; see tc_gemm.cuh), K-major for or_and.
 template <int KIND>
 __global__ void __launch_bounds__(kTcThreads, 1)
     tc_gemm2_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__ CUtensorMap tmA1,
                     const __grid_constant__ CUtensorMap tmB0, const __grid_constant__ CUtensorMap tmB1,
-                    const __grid_constant__ CUtensorMap tmBh0, const __grid_constant__ CUtensorMap tmBh1, int M, int N,
-                    int K, TcEpilogue ep, int tiles_m, int tiles_n) {
+                    const __grid_constant__ CUtensorMap tmBh, int M, int N, int K, TcEpilogue ep, int tiles_m,
+                    int tiles_n) {
   using Cfg = TcCfg<KIND>;
-  constexpr int S = kTc2Stages;
+  constexpr int S = tc2_stages<KIND>();
   constexpr int BN = tc_bn<KIND>();
+  constexpr bool BT = KIND != 1;
   constexpr int kStage = tc2_stage_bytes<KIND>();
   constexpr int kHalf = tc2_half_tile<KIND>();
   extern __shared__ uint8_t smem_raw[];
@@ -205,7 +208,6 @@ __global__ void __launch_bounds__(kTcThreads, 1)
       // ---------------- TMA producer of this CTA's halves ----------------
       prefetch_tensormap(&tmA0);
       prefetch_tensormap(&tmB0);
-      prefetch_tensormap(&tmBh0);
       int j = 0;
       bool ok = true;
       for (int t = pair; t < items && ok; t += pairs) {
@@ -215,8 +217,6 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         // this CTA's ncols/2 rows of B^T: a BN/2-row box, or 64 rows for a half
         // tile (the or_and tail's second half reads 48 of them)
         const bool half = ncols != BN;
-        const CUtensorMap* mb0 = half ? &tmBh0 : &tmB0;
-        const CUtensorMap* mb1 = half ? &tmBh1 : &tmB1;
         const uint32_t bytes =
             2 * (Cfg::kNumA * kHalf + Cfg::kNumB * (half ? 64 : BN / 2) * Cfg::kRowBytes);
         const int ma = m0 + (int)rank * 128, nb = n0 + (int)rank * (ncols / 2);
@@ -234,8 +234,15 @@ __global__ void __launch_bounds__(kTcThreads, 1)
           tma_load_2d_pair(st, &tmA0, bar0, kx, ma);
           if constexpr (Cfg::kNumA == 2) tma_load_2d_pair(st + kHalf, &tmA1, bar0, kx, ma);
           uint8_t* sb = st + Cfg::kNumA * kHalf;
-          tma_load_2d_pair(sb, mb0, bar0, kx, nb);
-          if constexpr (Cfg::kNumB == 2) tma_load_2d_pair(sb + kHalf, mb1, bar0, kx, nb);
+          if constexpr (BT) {
+            for (int g = 0; g < (half ? 1 : 2); g++) {
+              tma_load_2d_pair(sb + g * tc_b_group<KIND>(), &tmB0, bar0, nb + 64 * g, kx);
+              if constexpr (Cfg::kNumB == 2)
+                tma_load_2d_pair(sb + kHalf + g * tc_b_group<KIND>(), &tmB1, bar0, nb + 64 * g, kx);
+            }
+          } else {
+            tma_load_2d_pair(sb, half ? &tmBh : &tmB0, bar0, kx, nb);
+          }
         }
       }
     }
@@ -251,7 +258,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
       for (int t = pair; t < items && ok; t += pairs) {
         if (skip_item(t)) continue;
         const int acc = lt & 1;
-        const uint32_t idesc = t < whole ? tc2_idesc<KIND>() : tc2_idesc<KIND>(((t - whole) & 1) ? BN - 128 : 128);
+        const uint32_t idesc = t < whole ? tc2_idesc<KIND>(BN, BT) : tc2_idesc<KIND>(((t - whole) & 1) ? BN - 128 : 128, BT);
         if (!mbar_wait(&acc_empty[acc], ((lt >> 1) & 1) ^ 1)) {
           report_timeout(124);
           break;
@@ -274,13 +281,15 @@ __global__ void __launch_bounds__(kTcThreads, 1)
           for (int ks = 0; ks < Cfg::kBK / Cfg::kKStep; ks++) {
             const uint32_t koff = ks * 32;  // bytes along the swizzled row
             const uint32_t acc0 = (kt > 0 || ks > 0) ? 1u : 0u;
+            auto bdesc = [&](uint32_t b) {
+              return BT ? umma_desc_nmajor(b + ks * 2048, tc_b_group<KIND>()) : umma_desc_swizzled(b + koff, RB);
+            };
             if constexpr (KIND == 0) {
-              tc2_mma<0>(d, umma_desc_swizzled(a0 + koff, RB), umma_desc_swizzled(b0 + koff, RB), acc0, idesc);
-              tc2_mma<0>(d, umma_desc_swizzled(a0 + koff, RB), umma_desc_swizzled(b1 + koff, RB), 1u, idesc);
-              tc2_mma<0>(d, umma_desc_swizzled(a1 + koff, RB), umma_desc_swizzled(b0 + koff, RB), 1u, idesc);
+              tc2_mma<0>(d, umma_desc_swizzled(a0 + koff, RB), bdesc(b0), acc0, idesc);
+              tc2_mma<0>(d, umma_desc_swizzled(a0 + koff, RB), bdesc(b1), 1u, idesc);
+              tc2_mma<0>(d, umma_desc_swizzled(a1 + koff, RB), bdesc(b0), 1u, idesc);
             } else {
-              tc2_mma<1>(d, umma_desc_swizzled(a0 + koff, RB), umma_desc_swizzled(b0 + koff, RB), acc0, idesc,
-                         tmem + kTcScaleCol);
+              tc2_mma<KIND>(d, umma_desc_swizzled(a0 + koff, RB), bdesc(b0), acc0, idesc, tmem + kTcScaleCol);
             }
           }
           tc2_commit_both(&empty[s]);  // stage s free in both CTAs once these MMAs have read it
@@ -309,7 +318,9 @@ __global__ void __launch_bounds__(kTcThreads, 1)
       tc_fence_after();
       int m0, n0, ncols;
       item_origin(t, m0, n0, ncols);
-      const uint32_t trow = tmem + acc * BN + ((uint32_t)(quad * 32) << 16);
+      int cfirst, ccount;
+      tc_epi_columns(ncols, (warp - 2) >> 2, cfirst, ccount);
+      const uint32_t trow = tmem + acc * BN + cfirst + ((uint32_t)(quad * 32) << 16);
       const int row0 = m0 + (int)rank * 128 + quad * 32;
       int changed = 0;
       auto release = [&] {
@@ -317,7 +328,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         __syncwarp();
         if (lane == 0) mbar_arrive_cluster(map_to_rank(&acc_empty[acc], 0));
       };
-      tc_tile_epilogue<KIND>(ep, M, N, n0, row0, trow, epi_tile, lane, changed, release, ncols);
+      tc_tile_epilogue<KIND>(ep, M, N, n0 + cfirst, row0, trow, epi_tile, lane, changed, release, ccount);
       if (ep.changed && KIND == 1) {
         const bool any = __any_sync(0xffffffffu, changed);
         if (any && lane == 0) {
