@@ -23,6 +23,7 @@
 #include "tc_gemm.cuh"
 #include "tc_gemm2.cuh"
 #include "closure_batched.cuh"
+#include "closure_coop.cuh"
 #include "mlp.cuh"
 #include "knn.cuh"
 #include "knn_fused.cuh"
@@ -135,6 +136,46 @@ int get_workspace_slot(cudaStream_t stream, int slot, size_t bytes, void** out) 
 }
 
 int get_workspace(cudaStream_t stream, size_t bytes, void** out) { return get_workspace_slot(stream, 0, bytes, out); }
+
+// Page-locked host words that a kernel writes its outcome to (a copy into
+// pageable memory costs a staging round trip, 5 us of a 100 us closure).  A call
+// borrows one block; at most kHostBlocks are kept, and simd2_release_workspaces
+// frees them.
+constexpr size_t kHostBlocks = 64;
+std::mutex g_host_mu;
+std::vector<void*> g_host_free;
+
+struct HostBlock {
+  void* p = nullptr;
+  HostBlock() {
+    {
+      std::lock_guard<std::mutex> lk(g_host_mu);
+      if (!g_host_free.empty()) {
+        p = g_host_free.back();
+        g_host_free.pop_back();
+        return;
+      }
+    }
+    if (cudaHostAlloc(&p, 256, cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
+      cudaGetLastError();
+      p = nullptr;
+    }
+  }
+  ~HostBlock() {
+    if (!p) return;
+    std::lock_guard<std::mutex> lk(g_host_mu);
+    if (g_host_free.size() < kHostBlocks) g_host_free.push_back(p);
+    else cudaFreeHost(p);
+  }
+  HostBlock(const HostBlock&) = delete;
+  HostBlock& operator=(const HostBlock&) = delete;
+};
+
+void release_host_blocks() {
+  std::lock_guard<std::mutex> lk(g_host_mu);
+  for (void* p : g_host_free) cudaFreeHost(p);
+  g_host_free.clear();
+}
 
 // ---------------------------------------------------------------------------
 // TMA descriptors
@@ -1163,6 +1204,109 @@ int closure_gated(int op, int n, float* X, long long ldx, int max_iter, int conv
   return done_at >= 0 ? SIMD2_OK : SIMD2_ERR_NOT_CONVERGED;
 }
 
+// Vertices up to which a closure on codes runs as one cooperative launch, by the
+// time of a whole call, a launch per step / one (us; min_plus, max_min, 5 to 7
+// steps): n = 32 158 / 63, 512 213 / 94, 228 / 123, 1024 403 / 274, 553 / 431, 1500
+// 780 / 690, 1400 / 1374; at 2000 the launched steps' larger tiles win (2957 / 3070).
+constexpr int kCoopMaxN = 1536;
+
+template <int OP>
+int launch_coop(const CUtensorMap (&m)[4], CoopArgs& args, int grid, cudaStream_t stream) {
+  auto kern = closure_coop_kernel<OP>;
+  static bool configured[64] = {};
+  int dev = 0;
+  SIMD2_CUDA_TRY(cudaGetDevice(&dev));
+  if (dev < 0 || dev >= 64) return SIMD2_ERR_NO_DEVICE;
+  if (!configured[dev]) {
+    SIMD2_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SkCfg<64>::kSmem));
+    configured[dev] = true;
+  }
+  cudaLaunchConfig_t lc = {};
+  lc.gridDim = dim3(grid);
+  lc.blockDim = dim3(kSimtThreads);
+  lc.dynamicSmemBytes = SkCfg<64>::kSmem;
+  lc.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  lc.attrs = attr;
+  lc.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&lc, kern, m[0], m[1], m[2], m[3], args);
+  if (e == cudaErrorCooperativeLaunchTooLarge) {  // fewer SMs than the device reports
+    cudaGetLastError();
+    return SIMD2_ERR_UNSUPPORTED;
+  }
+  SIMD2_CUDA_TRY(e);
+  count_launch();
+  return SIMD2_OK;
+}
+
+// The whole closure as one cooperative launch on 16-bit codes.  *done = false:
+// an entry or a result has no code; X is as it was.
+int closure_coop(int op, int n, float* X, long long ldx, int max_iter, int conv, int* iters_out, bool* done,
+                 cudaStream_t stream) {
+  *done = false;
+  const int tiles = (n + 63) / 64, Kh = round_up(n, kSkBK16), Np = round_up(n, kBN), rows = tiles * 64;
+  const int sms = device_sms();
+  // CTAs and whole tiles as for a product on 64 x 64 tiles
+  const long long nt = (long long)tiles * tiles, kt = Kh / kSkBK16;
+  int grid = sms, whole = 0;
+  if (nt >= sms) whole = (int)(nt / sms - (nt % sms ? 1 : 0));
+  else grid = (int)std::min<long long>(sms, nt * std::min<long long>(kt, std::max(1LL, sms / nt)));
+  if (nt == grid) whole = 1;
+  size_t off = 0;
+  auto take = [&](size_t bytes) { size_t o = off; off += align_up(bytes, kAlign); return o; };
+  const size_t x_off[2] = {take((size_t)rows * Kh * 2), take((size_t)rows * Kh * 2)};
+  const size_t p_off[2] = {take((size_t)Kh * Np * 2), take((size_t)Kh * Np * 2)};
+  const size_t part_off = take((size_t)2 * grid * kSimtThreads * 16);
+  const size_t ctl_off = take(sizeof(CoopCtl));
+  const size_t cnt_off = take(kSkMaxCounters * sizeof(int));
+  void* w = nullptr;
+  int rc = get_workspace(stream, off, &w);
+  if (rc) return rc;
+  uint8_t* ws = static_cast<uint8_t*>(w);
+  CoopArgs a{};
+  a.X = X;
+  a.ldx = ldx;
+  a.n = n, a.Kh = Kh, a.Np = Np, a.tiles = tiles, a.whole = whole;
+  a.max_iter = max_iter;
+  a.conv = conv;
+  CUtensorMap m[4];
+  for (int q = 0; q < 2; q++) {
+    a.Xc[q] = reinterpret_cast<uint16_t*>(ws + x_off[q]);
+    a.Pc[q] = reinterpret_cast<uint32_t*>(ws + p_off[q]);
+    if ((rc = make_map_2d(&m[q], CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, a.Xc[q], rows, Kh, Kh, kSkBK16, 64,
+                          CU_TENSOR_MAP_SWIZZLE_128B)))
+      return rc;
+    if ((rc = make_map_2d(&m[2 + q], CU_TENSOR_MAP_DATA_TYPE_UINT32, 4, a.Pc[q], Kh / 2, Np, Np, 64, kSkBK16 / 2,
+                          CU_TENSOR_MAP_SWIZZLE_NONE)))
+      return rc;
+  }
+  a.part = reinterpret_cast<uint4*>(ws + part_off);
+  a.ctl = reinterpret_cast<CoopCtl*>(ws + ctl_off);
+  a.counters = reinterpret_cast<int*>(ws + cnt_off);
+  HostBlock host;
+  if (!host.p) return SIMD2_ERR_ALLOC;
+  a.out = static_cast<volatile int*>(host.p);
+  a.out[0] = a.out[1] = 0;
+  SIMD2_CUDA_TRY(cudaMemsetAsync(ws + ctl_off, 0, off - ctl_off, stream));
+  switch (op) {
+    case SIMD2_MIN_PLUS: rc = launch_coop<SIMD2_MIN_PLUS>(m, a, grid, stream); break;
+    case SIMD2_MAX_PLUS: rc = launch_coop<SIMD2_MAX_PLUS>(m, a, grid, stream); break;
+    case SIMD2_MAX_MIN: rc = launch_coop<SIMD2_MAX_MIN>(m, a, grid, stream); break;
+    case SIMD2_MIN_MAX: rc = launch_coop<SIMD2_MIN_MAX>(m, a, grid, stream); break;
+    default: rc = SIMD2_ERR_UNSUPPORTED;
+  }
+  if (rc) return rc == SIMD2_ERR_UNSUPPORTED ? SIMD2_OK : rc;  // the launch-per-step path takes over
+  SIMD2_CUDA_TRY(cudaStreamSynchronize(stream));
+  const int iters = a.out[0], outcome = a.out[1];
+  if (outcome == 3) return SIMD2_OK;
+  if (outcome == 0) return SIMD2_ERR_TIMEOUT;  // a bounded wait ran out
+  *done = true;
+  if (iters_out) *iters_out = iters;
+  return outcome == 1 ? SIMD2_OK : SIMD2_ERR_NOT_CONVERGED;
+}
+
 // Closure by repeated squaring with a per-step kernel configuration:
 //   dispatch 0 (dense)  : no skip, split-K from the tile count (the plain path);
 //   dispatch 1 (fixed)  : `fixed_cfg` every step: a dense configuration
@@ -1212,6 +1356,14 @@ int closure_f32_ex(int op, int n, float* X, long long ldx, int max_iter, int con
     dispatch = 0;
     if (step_feat) std::fill(step_feat, step_feat + (size_t)max_iter * kMlpFeat, 0.f);
     step_feat = nullptr;
+  }
+  // A small closure on codes: one cooperative launch (recorded ones keep a launch
+  // per step, whose times and configurations they ask for).
+  if (dispatch == 0 && n <= kCoopMaxN && has_code16(op) && conv != SIMD2_CONV_APLP && !step_cfg && !step_ms &&
+      !step_feat) {
+    bool done = false;
+    rc = closure_coop(op, n, X, ldx, max_iter, conv, iters_out, &done, stream);
+    if (done || rc) return rc;
   }
   const bool can_skip = skip_supported(op) && (n + kBK - 1) / kBK <= kMaxSkipKtiles;
   const bool opening = (dispatch == 2 || dispatch == 3 || fixed_sparse) && conv == SIMD2_CONV_EXACT;
@@ -2430,6 +2582,7 @@ int simd2_reserve_workspace(simd2_op op, int M, int N, int K, cudaStream_t strea
 int simd2_release_workspaces(void) {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return SIMD2_ERR_CUDA;
+  release_host_blocks();
   std::lock_guard<std::mutex> lk(g_ws_mu);
   cudaDeviceSynchronize();
   for (auto it = g_ws.begin(); it != g_ws.end();) {

@@ -329,8 +329,8 @@ __device__ __forceinline__ void batch_tile(const BatchArgs& a, BatchCta& x, cons
       uint32_t c0 = kPad2, c1 = kPad2;
       if (row < n && colin) {
         uint32_t b0 = 0, b1 = 0;
-        c0 = Code16<OP>::fold2(acc[i][0], acc[i][1], old[i].x, b0);
-        c1 = Code16<OP>::fold2(acc[i][2], acc[i][3], old[i].y, b1);
+        c0 = Code16<OP>::finish(Code16<OP>::pair(acc[i][0], acc[i][1]), old[i].x, b0);
+        c1 = Code16<OP>::finish(Code16<OP>::pair(acc[i][2], acc[i][3]), old[i].y, b1);
         bad |= (b0 & keep0) | (b1 & keep1);
         c0 = (c0 & keep0) | (kPad2 & ~keep0);
         c1 = (c1 & keep1) | (kPad2 & ~keep1);

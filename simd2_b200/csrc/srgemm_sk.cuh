@@ -59,10 +59,14 @@ struct Code16<SIMD2_MIN_PLUS> {
     const uint32_t m = min(acc & 0xffffu, acc >> 16);
     return m >= 0x7fffu ? __int_as_float(0x7f800000) : (float)m;
   }
-  // The codes of two neighbouring columns' accumulators combined with the
-  // codes `old`; over gets a bit where a result is finite and has no code.
-  __device__ static uint32_t fold2(uint32_t a0, uint32_t a1, uint32_t old, uint32_t& over) {
-    const uint32_t m = __vminu2(__byte_perm(a0, a1, 0x5410), __byte_perm(a0, a1, 0x7632));
+  // Two neighbouring columns' accumulators, each over its two halves, as one word.
+  __device__ static uint32_t pair(uint32_t a0, uint32_t a1) {
+    return join(__byte_perm(a0, a1, 0x5410), __byte_perm(a0, a1, 0x7632));
+  }
+  __device__ static uint32_t join(uint32_t x, uint32_t y) { return __vminu2(x, y); }
+  // Such a word combined with the codes `old`; over gets a bit where a result is
+  // finite and has no code.
+  __device__ static uint32_t finish(uint32_t m, uint32_t old, uint32_t& over) {
     const uint32_t r = __vminu2(__vminu2(m, 0x7fff7fffu), old);
     over |= r & 0x40004000u & ~((r + 0x00010001u) >> 1);  // bit 14 set, but not 0x7fff
     return r;
@@ -94,8 +98,11 @@ struct Code16<SIMD2_MAX_PLUS> {
     const uint32_t m = max(acc & 0xffffu, acc >> 16);
     return m < 0x8000u ? __int_as_float(0xff800000) : (float)(m - 0x8000u);
   }
-  __device__ static uint32_t fold2(uint32_t a0, uint32_t a1, uint32_t old, uint32_t& over) {
-    const uint32_t m = __vmaxu2(__byte_perm(a0, a1, 0x5410), __byte_perm(a0, a1, 0x7632));
+  __device__ static uint32_t pair(uint32_t a0, uint32_t a1) {
+    return join(__byte_perm(a0, a1, 0x5410), __byte_perm(a0, a1, 0x7632));
+  }
+  __device__ static uint32_t join(uint32_t x, uint32_t y) { return __vmaxu2(x, y); }
+  __device__ static uint32_t finish(uint32_t m, uint32_t old, uint32_t& over) {
     const uint32_t finite = ((m >> 15) & 0x00010001u) * 0xffffu;  // halves that hold a finite sum
     over |= m & finite & 0x40004000u;                             // past 16383
     return __vmaxu2(((m & 0x3fff3fffu) | 0x40004000u) & finite, old);
@@ -124,9 +131,11 @@ struct Code16<SIMD2_MAX_MIN> : SelectCode16 {
   static constexpr uint32_t kPad = 0x83ffu;  // -inf
   static constexpr uint32_t kIdent = 0x83ff83ffu;
   __device__ static float decode(uint32_t acc) { return value(max((int)(int16_t)(acc & 0xffffu), (int)acc >> 16)); }
-  __device__ static uint32_t fold2(uint32_t a0, uint32_t a1, uint32_t old, uint32_t&) {
-    return __vmaxs2(__vmaxs2(__byte_perm(a0, a1, 0x5410), __byte_perm(a0, a1, 0x7632)), old);
+  __device__ static uint32_t pair(uint32_t a0, uint32_t a1) {
+    return join(__byte_perm(a0, a1, 0x5410), __byte_perm(a0, a1, 0x7632));
   }
+  __device__ static uint32_t join(uint32_t x, uint32_t y) { return __vmaxs2(x, y); }
+  __device__ static uint32_t finish(uint32_t m, uint32_t old, uint32_t&) { return join(m, old); }
   __device__ static uint32_t mac(uint32_t acc, uint32_t x, uint32_t y, uint32_t x2, uint32_t y2, bool) {
     return __vimax3_s16x2(acc, __vmins2(x, y), __vmins2(x2, y2));
   }
@@ -136,9 +145,11 @@ struct Code16<SIMD2_MIN_MAX> : SelectCode16 {
   static constexpr uint32_t kPad = 0x7c00u;  // +inf
   static constexpr uint32_t kIdent = 0x7c007c00u;
   __device__ static float decode(uint32_t acc) { return value(min((int)(int16_t)(acc & 0xffffu), (int)acc >> 16)); }
-  __device__ static uint32_t fold2(uint32_t a0, uint32_t a1, uint32_t old, uint32_t&) {
-    return __vmins2(__vmins2(__byte_perm(a0, a1, 0x5410), __byte_perm(a0, a1, 0x7632)), old);
+  __device__ static uint32_t pair(uint32_t a0, uint32_t a1) {
+    return join(__byte_perm(a0, a1, 0x5410), __byte_perm(a0, a1, 0x7632));
   }
+  __device__ static uint32_t join(uint32_t x, uint32_t y) { return __vmins2(x, y); }
+  __device__ static uint32_t finish(uint32_t m, uint32_t old, uint32_t&) { return join(m, old); }
   __device__ static uint32_t mac(uint32_t acc, uint32_t x, uint32_t y, uint32_t x2, uint32_t y2, bool) {
     return __vimin3_s16x2(acc, __vmaxs2(x, y), __vmaxs2(x2, y2));
   }
