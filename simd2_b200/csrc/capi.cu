@@ -20,6 +20,7 @@
 #include "prep.cuh"
 #include "srgemm_simt.cuh"
 #include "srgemm_sk.cuh"
+#include "srgemm_small.cuh"
 #include "tc_gemm.cuh"
 #include "tc_gemm2.cuh"
 #include "closure_batched.cuh"
@@ -642,13 +643,46 @@ int launch_sk(int M, int N, int K, const T* A, long long lda, const T* B, long l
                   : launch_sk_tile<OP, 64>(a16, b16, a32, b32, ga, grid, ep, stream);
 }
 
+// Whether srgemm_small_kernel is the faster one, by the time (us) both take: its
+// 32 x 32 tiles 0.0137 a k and 0.35 each for those on one SM, after 4; the
+// persistent kernel's tiles 4.5 (128) or 1.13 (64) a 64-wide k-tile (twice that on
+// FP32, for the ops without codes) and 3.5 or 0.8 each, spread over the SMs, after
+// 11.  Measured, small / persistent: 100^3 4.3 / 13.0, 384^3 9.6 / 15.0, 450^3
+// 20.2 / 18.4, 1000 x 1000 x 64 9.5 / 14.8, 2000 x 2000 x 40 29.5 / 20.4,
+// 4096 x 4096 x 16 62 / 45, 30 x 30 x 3000 64 / 21.
+bool small_product(int op, int M, int N, int K) {
+  const double sms = device_sms();
+  auto up = [](int v, int t) { return (double)((v + t - 1) / t); };
+  const double small = 4.0 + std::ceil(up(M, 32) * up(N, 32) / sms) * (K * 0.0137 + 0.35);
+  const double unit = has_code16(op) ? 1.0 : 2.0, big = up(M, 128) * up(N, 128), tiles = up(M, 64) * up(N, 64);
+  const double large = 3.0 * big >= sms ? 11.0 + big * (K / 64.0 * 4.5 * unit + 3.5) / sms
+                                        : 11.0 + tiles * (up(K, 64) * 1.13 * unit + 0.8) / sms;
+  return small < large && up(M, 32) < 65536.0;
+}
+
+template <int OP, typename T>
+int launch_small(int M, int N, int K, const T* A, long long lda, const T* B, long long ldb, const EpilogueArgs& ep,
+                 cudaStream_t stream) {
+  const dim3 grid((N + kSmallTile - 1) / kSmallTile, (M + kSmallTile - 1) / kSmallTile);
+  auto* ev = prof_slot(2LL * M * N * K);
+  if (ev) cudaEventRecord(ev->first, stream);
+  srgemm_small_kernel<OP, T><<<grid, 256, 0, stream>>>(A, lda, B, ldb, M, N, K, ep);
+  count_launch();
+  if (ev) cudaEventRecord(ev->second, stream);
+  SIMD2_CUDA_TRY(cudaGetLastError());
+  return SIMD2_OK;
+}
+
 template <typename T>
 int launch_sk_op(int op, int M, int N, int K, const T* A, long long lda, const T* B, long long ldb,
                  const EpilogueArgs& ep, uint8_t* ws, const Plan& plan, bool pack_a, const SimtConfig& cfg,
                  cudaStream_t stream) {
+  const bool small = !cfg.skip && !ep.chgA && small_product(op, M, N, K);
   switch (op) {
-#define SIMD2_SK_CASE(OPV) \
-  case OPV: return launch_sk<OPV, T>(M, N, K, A, lda, B, ldb, ep, ws, plan, pack_a, cfg, stream);
+#define SIMD2_SK_CASE(OPV)                                                                    \
+  case OPV:                                                                                   \
+    return small ? launch_small<OPV, T>(M, N, K, A, lda, B, ldb, ep, stream)                  \
+                 : launch_sk<OPV, T>(M, N, K, A, lda, B, ldb, ep, ws, plan, pack_a, cfg, stream);
     SIMD2_SK_CASE(SIMD2_MIN_PLUS)
     SIMD2_SK_CASE(SIMD2_MAX_PLUS)
     SIMD2_SK_CASE(SIMD2_MAX_MIN)

@@ -84,3 +84,25 @@ def test_strided_unaligned_and_in_place(cuda, op):
         s2.srgemm(op, A, B, C, do_epilogue=True, D=C)
         torch.cuda.synchronize()
         same(C.cpu().numpy(), want, f"{op} offset {off}")
+
+
+@pytest.mark.parametrize("op", ["min_plus", "max_plus", "max_min", "max_mul", "min_mul", "min_max"])
+@pytest.mark.parametrize("shape", [(1, 1, 1), (31, 33, 31), (32, 32, 32), (33, 32, 33), (5, 300, 65), (100, 100, 100),
+                                   (383, 130, 64), (1000, 900, 5)])
+def test_small_products(cuda, op, shape):
+    """Sizes of the one-launch kernel (srgemm_small.cuh), float32 and float16, rows on
+    and off the 16-byte grid, with and without C."""
+    m, n, k = shape
+    a, b, c = datagen.semiring_operands(op, m, n, k, seed=m + n + k)
+    for off in (0, 1):
+        def place(x, dt=torch.float32):
+            buf = torch.full((x.shape[0], x.shape[1] + 2 * off), float("nan"), device=cuda, dtype=dt)
+            view = buf[:, off:off + x.shape[1]]
+            view.copy_(torch.from_numpy(x))
+            return view
+        for epi in (False, True):
+            got = s2.srgemm(op, place(a), place(b), place(c) if epi else None, do_epilogue=epi)
+            same(got.cpu().numpy(), oracle.srgemm(op, a, b, c, do_epilogue=epi), f"{op} {shape} {off} {epi}")
+        ah, bh = (x.astype(np.float16) for x in (a, b))
+        got = s2.srgemm_f16(op, place(ah, torch.float16), place(bh, torch.float16))
+        same(got.cpu().numpy(), oracle.srgemm(op, ah.astype(np.float32), bh.astype(np.float32)), f"{op} {shape} f16")
