@@ -3062,12 +3062,31 @@ int knn_fused_pass(const CUtensorMap& mqh, const CUtensorMap& mql, const CUtenso
 // result bit for bit.  Lists of 4 for k = 5..8 are cut short in most blocks
 // of 128 random queries (one of the ~30 lists holding 4 of the top 8 is
 // common), so those k run one pass.
+// Whether lists of `len` over `lists` (chunk halves) are long enough for most query
+// blocks: the chance that one of them holds more than len of a query's k
+// neighbours, spread evenly, is a binomial tail; a block of 128 queries is redone
+// when it happens to any of them, and already a few redone blocks take about as long
+// as all (they run in one wave), so one block in a hundred is the line
+// (16384 x 1000 x 128, k = 16, 2 lists: 263 us in two passes, 140 in one;
+// 5000 x 2000 x 50, k = 12, 4 lists, one block in five: 108 and 74;
+// 300 x 700 x 30, k = 30, 6 lists, none: 57 and 75).
+bool knn_half_lists(int k, int lists, int len) {
+  if (lists < 2) return false;
+  const double p = 1.0 / lists;
+  double term = std::pow(1.0 - p, k), tail = 0.0;  // P(exactly i), from i = 0
+  for (int i = 0; i < k; i++) {
+    term *= (double)(k - i) / (i + 1) * p / (1.0 - p);
+    if (i + 1 > len) tail += term;
+  }
+  return 128.0 * lists * tail <= 0.01;
+}
+
 template <int KT>
 int knn_fused_launch(const CUtensorMap& mqh, const CUtensorMap& mql, const CUtensorMap& mrh, const CUtensorMap& mrl,
                      KnnFusedArgs a, int qblocks, float* od, int32_t* oi, long long ldo, int kout, float* pd2,
                      int32_t* pi2, unsigned* ready2, int* flags, cudaStream_t stream) {
   if constexpr (KT >= 16) {
-    if (kout > KT / 2) {
+    if (kout > KT / 2 && knn_half_lists(kout, 2 * a.chunks, KT / 2)) {
       int rc = knn_fused_pass<KT / 2, KT>(mqh, mql, mrh, mrl, a, qblocks, od, oi, ldo, kout, flags, stream);
       if (rc) return rc;
       KnnFusedArgs b = a;

@@ -13,8 +13,11 @@
 //   warp 0 lane 0  -- TMA producer: the unit's query panels (BF16 hi and lo,
 //                     64-element K panels, 128-byte swizzle) once, then per
 //                     reference tile and K panel its hi and lo parts through
-//                     a 5-deep ring of 32 KiB stages,
-//   warp 1 lane 0  -- MMA issuer: per reference tile q.r ~ qh.rh + qh.rl + ql.rh
+//                     a 4-deep ring of 32 KiB stages,
+//   warp 1 lane 0  -- MMA issuer, which also fetches each tile's reference norms
+//                     into shared memory (from L2 the selection warps waited for
+//                     them 32 columns at a time: 16384 x 65536 x 128, k = 16, 731 us
+//                     a call for 719): per reference tile q.r ~ qh.rh + qh.rl + ql.rh
 //                     (tcgen05.mma kind::f16, M=128, N=256, FP32 accumulate)
 //                     into one of two TMEM accumulators (2 x 256 columns), so
 //                     the MMAs of tile t+1 run while tile t is selected,
@@ -48,14 +51,15 @@ namespace simd2 {
 constexpr int kKfBM = 128;                     // queries per unit (TMEM lanes)
 constexpr int kKfBN = 256;                     // references per tile (MMA N)
 constexpr int kKfMaxPanels = 2;                // D <= 128: two 64-element K panels
-constexpr int kKfStages = 5;                   // B ring depth (2.5 K panels of hi + lo)
+constexpr int kKfStages = 4;                   // B ring depth (2 K panels of hi + lo)
 constexpr int kKfATile = kKfBM * 128;          // 16 KiB: one K panel of 128 query rows
 constexpr int kKfBTile = kKfBN * 128;          // 32 KiB: one K panel of 256 reference rows
 constexpr int kKfEpiWarps = 8;
 constexpr int kKfThreads = (2 + kKfEpiWarps) * 32;
 constexpr int kKfTmemCols = 512;               // two 128 x 256 FP32 accumulators
+constexpr int kKfNormSlots = 4;                // reference norms of a tile, 1 KiB each
 constexpr size_t kKfSmemBytes =
-    (size_t)kKfMaxPanels * 2 * kKfATile + (size_t)kKfStages * kKfBTile + 1024 /* align */ + 256 /* barriers */;
+    (size_t)kKfMaxPanels * 2 * kKfATile + (size_t)kKfStages * kKfBTile + kKfNormSlots * kKfBN * 4 + 1024 /* align */ + 256 /* barriers */;
 
 struct KnnFusedArgs {
   int Q, R, D;
@@ -96,6 +100,15 @@ __device__ __forceinline__ uint32_t pick32(const uint32_t (&r)[32], int j) {
 
 __device__ __forceinline__ void st_release_gpu(unsigned* p, unsigned v) {
   asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+
+// Untiled bulk copy to shared memory (16-byte aligned addresses, a multiple of 16
+// bytes); completion is signalled as transaction bytes on `bar`.
+__device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                   smem_u32(dst)),
+               "l"(src), "r"(bytes), "r"(smem_u32(bar))
+               : "memory");
 }
 
 // Reference tiles [t0, t0 + ntiles) of a chunk.  With a pilot, chunk 0 is
@@ -194,7 +207,8 @@ __global__ void __launch_bounds__(kKfThreads, 1)
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sA = smem;                                    // [panel][hi, lo] 16 KiB each
   uint8_t* sB = smem + kKfMaxPanels * 2 * kKfATile;      // [stage] 32 KiB each
-  uint64_t* a_full = reinterpret_cast<uint64_t*>(sB + kKfStages * kKfBTile);
+  float* sN = reinterpret_cast<float*>(sB + kKfStages * kKfBTile);
+  uint64_t* a_full = reinterpret_cast<uint64_t*>(sN + kKfNormSlots * kKfBN);
   uint64_t* full = a_full + 1;
   uint64_t* empty = full + kKfStages;
   uint64_t* acc_full = empty + kKfStages;
@@ -220,7 +234,7 @@ __global__ void __launch_bounds__(kKfThreads, 1)
       mbar_init(&empty[s], 1);
     }
     for (int s = 0; s < 2; s++) {
-      mbar_init(&acc_full[s], 1);
+      mbar_init(&acc_full[s], 2);
       mbar_init(&acc_empty[s], kKfEpiWarps);
     }
     mbar_init(fin, 1);
@@ -282,6 +296,11 @@ __global__ void __launch_bounds__(kKfThreads, 1)
           break;
         }
         tc_fence_after();
+        // The tile's reference norms, with the accumulator: the selection warps
+        // have released tile t - 2, so no one reads tile t - 4's slot any more.
+        mbar_arrive_expect_tx(&acc_full[acc], kKfBN * 4);
+        bulk_load(sN + (t & (kKfNormSlots - 1)) * kKfBN, a.norm_r + (long long)(t0 + t) * kKfBN, kKfBN * 4,
+                  &acc_full[acc]);
         const uint32_t d = tmem + acc * kKfBN;
         for (int p = 0; p < P; p++, j += 2) {
           // stages j (hi) and j+1 (lo) hold K panel p of the tile
@@ -385,7 +404,7 @@ __global__ void __launch_bounds__(kKfThreads, 1)
           // Packed FP32 pairs: each lane of __fadd2_rn / __ffma2_rn rounds
           // like the scalar na + |r|^2 and fma(-2, q.r, .), so v keeps the
           // materialised epilogue's bits.
-          const float4* nb4 = reinterpret_cast<const float4*>(a.norm_r + cbase + c * 32);
+          const float4* nb4 = reinterpret_cast<const float4*>(sN + (t & (kKfNormSlots - 1)) * kKfBN + half * 128 + c * 32);
           const float2 na2 = make_float2(na, na), m2 = make_float2(-2.0f, -2.0f);
           // The mask bits are formed as 1.0 / 0.0 and summed with packed FMAs
           // into four accumulators of 16 bit positions each (exact: every sum
@@ -395,7 +414,7 @@ __global__ void __launch_bounds__(kKfThreads, 1)
           float2 mlo = make_float2(0.f, 0.f), mhi = make_float2(0.f, 0.f);
 #pragma unroll
           for (int q4 = 0; q4 < 8; q4++) {
-            const float4 nb = __ldg(nb4 + q4);
+            const float4 nb = nb4[q4];
 #pragma unroll
             for (int e = 0; e < 4; e += 2) {
               const int jj = q4 * 4 + e;
@@ -508,6 +527,63 @@ __global__ void __launch_bounds__(256) knn_merge_kernel(const float* __restrict_
     if (gate && gate[r0 / kKfBM] == 0) continue;  // uniform across the warp
     const int r = r0 + lane / G;
     const bool live = r < rows;
+    if constexpr (G == 32) {
+      // A list per lane and a query per warp (`rows` bounds r0 = r): each round
+      // takes the smallest head by two warp reductions, of the distances as
+      // order-preserving integers and of the indices among equal ones; lane t
+      // keeps result t.  (Five shuffle steps on pairs and a shift of K entries a
+      // round took 35 us for 16384 queries and 18 lists, this 17.)
+      if (lists <= 32) {
+        float hd[KL];
+        int hi[KL];
+#pragma unroll
+        for (int u = 0; u < KL; u++) {
+          hd[u] = inf;
+          hi[u] = 0x7fffffff;
+        }
+        if (lane < lists) {
+          const float4* ld = reinterpret_cast<const float4*>(part_d + ((long long)r * lists + lane) * KL);
+          const int4* li = reinterpret_cast<const int4*>(part_i + ((long long)r * lists + lane) * KL);
+#pragma unroll
+          for (int u = 0; u < KL / 4; u++) {
+            const float4 v = ld[u];
+            const int4 w = li[u];
+            hd[4 * u] = v.x, hd[4 * u + 1] = v.y, hd[4 * u + 2] = v.z, hd[4 * u + 3] = v.w;
+            hi[4 * u] = w.x, hi[4 * u + 1] = w.y, hi[4 * u + 2] = w.z, hi[4 * u + 3] = w.w;
+          }
+        }
+        const float last = hd[KL - 1];
+        const int lasti = hi[KL - 1];
+        float keep = inf, v = inf;
+        int keepi = 0x7fffffff, ix = 0x7fffffff;
+        for (int t = 0; t < kout; t++) {
+          const uint32_t b = __float_as_uint(hd[0] + 0.0f);
+          const uint32_t key = b ^ ((uint32_t)((int32_t)b >> 31) | 0x80000000u);
+          const uint32_t m = __reduce_min_sync(0xffffffffu, key);
+          ix = (int)__reduce_min_sync(0xffffffffu, key == m ? (uint32_t)hi[0] : 0x7fffffffu);
+          v = __uint_as_float(m ^ ((m >> 31) ? 0x80000000u : 0xffffffffu));
+          if (key == m && hi[0] == ix) {
+#pragma unroll
+            for (int u = 0; u < KL - 1; u++) {
+              hd[u] = hd[u + 1];
+              hi[u] = hi[u + 1];
+            }
+            hd[KL - 1] = inf;
+            hi[KL - 1] = 0x7fffffff;
+          }
+          if (lane == t) {
+            keep = v;
+            keepi = ix;
+          }
+        }
+        if (lane < kout) {
+          out_d[(long long)r * ldo + lane] = sqrtf(fmaxf(keep, 0.f));
+          out_i[(long long)r * ldo + lane] = keepi == 0x7fffffff ? -1 : keepi;
+        }
+        if (flags && lasti != 0x7fffffff && lex_less(last, lasti, v, ix)) atomicOr(&flags[r / kKfBM], 1);
+        continue;
+      }
+    }
     float bd[K];
     int bi[K];
 #pragma unroll

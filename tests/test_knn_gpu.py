@@ -162,3 +162,19 @@ def test_knn_fused_half_lists_redo_flagged_blocks(cuda, k, Q):
         assert np.all((ii[lo:hi] >= 256) & (ii[lo:hi] < 384))
     check(q, r, k, d1.cpu().numpy(), ii)
     assert s2.device_status() == 0
+
+
+@pytest.mark.parametrize("shape", [(130, 300, 17, 12), (130, 700, 33, 30), (700, 1500, 64, 16), (129, 5000, 100, 9)])
+def test_knn_few_lists_one_pass(cuda, shape):
+    """Few lists per query take one pass with full lists, more of them two passes:
+    both as the materialised path, bit for bit, with every neighbour of some
+    queries in one cluster of consecutive references."""
+    Q, R, D, k = shape
+    g = torch.Generator(device=cuda).manual_seed(Q + R)
+    ref = torch.randn((R, D), generator=g, device=cuda)
+    query = torch.randn((Q, D), generator=g, device=cuda)
+    query[::7] = ref[R // 2] + 0.01 * torch.randn((query[::7].shape[0], D), generator=g, device=cuda)
+    ref[R // 2:R // 2 + 40] = ref[R // 2] + 0.01 * torch.randn((40, D), generator=g, device=cuda)
+    d1, i1 = s2.knn(query, ref, k, mode="fused")
+    d2, i2 = s2.knn(query, ref, k, mode="materialised")
+    assert torch.equal(d1.view(torch.int32), d2.view(torch.int32)) and torch.equal(i1, i2)
