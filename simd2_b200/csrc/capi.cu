@@ -946,7 +946,8 @@ int srgemm_tc_sum(int op, int M, int N, int K, const T* A, long long lda, const 
   return launch_tc<KIND, true>(M, N, K, ma0, ma1, mb0, mb1, ep, tc_tile_columns(M, N, K, kHalf ? 1 : 3), stream);
 }
 
-// delta (or_and closure, pair kernel only): the maps of TcEpilogue.
+// delta (or_and closure, pair kernel only): the maps of TcEpilogue.  With need_row /
+// need_col, ws holds the operands of the step before.
 struct TcDelta {
   uint8_t* chg_row = nullptr;
   uint8_t* chg_col = nullptr;
@@ -962,15 +963,21 @@ int srgemm_tc_orand(int M, int N, int K, const T* A, long long lda, const T* B, 
   const int Kp = plan.Kp;
   uint8_t* a4 = ws + plan.a0;
   uint8_t* b4 = ws + plan.b0;
-  bool_rows_fp4_kernel<T><<<grid_for((long long)M * Kp / 16), 256, 0, stream>>>(A, lda, M, K, a4, Kp);
-  transpose_fp4_kernel<T><<<dim3((N + 63) / 64, (Kp + 127) / 128), 256, 0, stream>>>(B, ldb, K, N, b4, Kp);
-  count_launch();
+  constexpr int BN = tc_bn<1>();
+  // A matrix times itself (a closure step) is read once for both operands, and a
+  // delta step packs again only what the previous step changed.
+  const bool square = A == B && lda == ldb && M == K && N == K;
+  if (!square) {
+    bool_rows_fp4_kernel<T><<<grid_for((long long)M * Kp / 16), 256, 0, stream>>>(A, lda, M, K, a4, Kp);
+    count_launch();
+  }
+  transpose_fp4_kernel<T><<<dim3((N + 127) / 128, (Kp + 255) / 256), 256, 0, stream>>>(
+      B, ldb, K, N, b4, Kp, square ? a4 : nullptr, Kp, delta.need_row, delta.need_col, BN);
   count_launch();
   SIMD2_CUDA_TRY(cudaGetLastError());
   CUtensorMap ma, mb;
   const auto U8 = CU_TENSOR_MAP_DATA_TYPE_UINT8;
   const auto SW = CU_TENSOR_MAP_SWIZZLE_128B;
-  constexpr int BN = tc_bn<1>();
   int rc;
   const bool pair = use_tc2(M, N);
   if ((rc = make_map_2d(&ma, U8, 1, a4, M, Kp / 2, Kp / 2, 128, kTcBM, SW))) return rc;

@@ -244,40 +244,67 @@ __global__ void __launch_bounds__(256) bool_rows_fp4_kernel(const T* __restrict_
   }
 }
 
-// or_and's B: B [K][N] of T (pitch ldb) -> FP4 [N][Kp / 2 bytes], zeros for k >= K.
-// One tile of 128 k x 64 columns per block of 256 threads: a thread reads 16
-// elements of two rows of B and writes 16 bytes (32 k) of a row of out.  The shared tile's
-// 68-byte rows keep both phases at most 2-way bank conflicted.
+// or_and's B: B [K][N] of T (pitch ldb) -> FP4 [N][Kp / 2 bytes], zeros for k >= K,
+// and, where a4 is set, B's rows as an A operand too ([K][Np / 2 bytes], zeros past
+// N: the closure's X is both, read once).  chg_row / chg_col (may be null: all): a
+// 256-row group of a4, and the columns of a BN-column group of b4, are written only
+// where their byte is set (they hold what they held otherwise).
+//
+// One tile of 256 k x 128 columns per block, bounded by DRAM: as bytes 0 / 1 in
+// shared memory, 16 bytes a store; then a thread takes 32 k of 4 columns, a word of
+// 4 bytes per k: two words shifted together hold the nibbles of two k, and four of
+// those, transposed as 4 x 4 bytes, 8 k of each column.  A warp covers 8 k groups x 4
+// words, so it writes whole 128-byte lines; 4 words of padding per 32 rows keep
+// its loads free of bank conflicts.  16384^2 bytes as both operands 115 us (DRAM
+// alone: 82).  (A thread that gathered single bytes for one
+// column took 169, and 75 more for a separate pass over the rows.)
 template <typename T>
 __global__ void __launch_bounds__(256) transpose_fp4_kernel(const T* __restrict__ B, long long ldb, int K, int N,
-                                                            uint8_t* __restrict__ out, int Kp) {
-  __shared__ uint32_t tile[128][17];
+                                                            uint8_t* __restrict__ b4, int Kp,
+                                                            uint8_t* __restrict__ a4, int Np,
+                                                            const uint8_t* __restrict__ chg_row,
+                                                            const uint8_t* __restrict__ chg_col, int BN) {
+  __shared__ __align__(16) uint32_t tile[256 * 32 + 8 * 4];
   const int t = threadIdx.x;
-  const int k0 = blockIdx.y * 128, j0 = blockIdx.x * 64;
-#pragma unroll
-  for (int h = 0; h < 2; h++) {
-    const int r = (t >> 2) + 64 * h, c0 = (t & 3) * 16;
+  const int k0 = blockIdx.y * 256, j0 = blockIdx.x * 128;
+  const bool rows = a4 && (!chg_row || chg_row[blockIdx.y]);
+  const bool cols = !chg_col || chg_col[j0 / BN] || chg_col[min(j0 + 127, N - 1) / BN];
+  if (!rows && !cols) return;
+#pragma unroll(sizeof(T) == 1 ? 8 : 2)
+  for (int h = 0; h < 8; h++) {
+    const int r = (t >> 3) + 32 * h, c0 = (t & 7) * 16;
     const int k = k0 + r, j = j0 + c0;
     uint32_t w[4] = {0u, 0u, 0u, 0u};
     if (k < K && j < N) load_bool16(B + (long long)k * ldb + j, N - j, w);
-#pragma unroll
-    for (int q = 0; q < 4; q++) tile[r][(c0 >> 2) + q] = w[q];
+    *reinterpret_cast<uint4*>(&tile[r * 32 + (r >> 5) * 4 + (c0 >> 2)]) = make_uint4(w[0], w[1], w[2], w[3]);
+    if (rows && k < K && j < Np)
+      *reinterpret_cast<uint2*>(a4 + ((long long)k * Np + j) / 2) =
+          make_uint2(nibbles_fp4(w[0], w[1]), nibbles_fp4(w[2], w[3]));
   }
+  if (!cols) return;
   __syncthreads();
-  const int jj = t >> 2, kc = (t & 3) * 32;
-  const int jo = j0 + jj, ko = k0 + kc;
-  if (jo < N && ko < Kp) {
-    const int sh = 8 * (jj & 3);
-    uint32_t o[4];
+  const int kg = (t & 31) >> 2, cw = (t >> 5) * 4 + (t & 3);
+  const int ko = k0 + 32 * kg, jo = j0 + 4 * cw;
+  if (ko >= Kp || jo >= N) return;
+  const uint32_t* src = &tile[32 * kg * 32 + kg * 4 + cw];
+  uint32_t o[4][4];
 #pragma unroll
-    for (int q = 0; q < 4; q++) {
-      uint32_t x = 0u;
+  for (int q = 0; q < 4; q++) {
+    uint32_t p[4];
 #pragma unroll
-      for (int b = 0; b < 8; b++) x |= ((tile[kc + 8 * q + b][jj >> 2] >> sh) & 1u) << (4 * b + 1);
-      o[q] = x;
-    }
-    *reinterpret_cast<uint4*>(out + ((long long)jo * Kp + ko) / 2) = make_uint4(o[0], o[1], o[2], o[3]);
+    for (int e = 0; e < 4; e++) p[e] = src[(8 * q + 2 * e) * 32] << 1 | src[(8 * q + 2 * e + 1) * 32] << 5;
+    const uint32_t a = __byte_perm(p[0], p[1], 0x5140), b = __byte_perm(p[2], p[3], 0x5140);
+    const uint32_t c = __byte_perm(p[0], p[1], 0x7362), d = __byte_perm(p[2], p[3], 0x7362);
+    o[0][q] = __byte_perm(a, b, 0x5410);
+    o[1][q] = __byte_perm(a, b, 0x7632);
+    o[2][q] = __byte_perm(c, d, 0x5410);
+    o[3][q] = __byte_perm(c, d, 0x7632);
   }
+#pragma unroll
+  for (int c = 0; c < 4; c++)
+    if (jo + c < N)
+      *reinterpret_cast<uint4*>(b4 + ((long long)(jo + c) * Kp + ko) / 2) =
+          make_uint4(o[c][0], o[c][1], o[c][2], o[c][3]);
 }
 
 // Operand preparation of the sums, one launch: blocks [0, a_blocks) take rows of

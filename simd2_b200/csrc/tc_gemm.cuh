@@ -9,7 +9,7 @@
 //                    is the shared memory's bandwidth (operand reads and TMA writes
 //                    of a 256 x 224 pair tile: 165 of 128 bytes a clock at full
 //                    rate).  16384^3 step, kernel: kind::i8 2240 us, now 1400;
-//                    3000 x 2500 x 2000 int32 call 117 us, now 56.
+//                    3000 x 2500 x 2000 int32 call 117 us, now 51.
 //   * plus_mul     : kind::f16 with BF16 hi/lo operands, FP32 accumulate:
 //                    a*b ~= a_hi*b_hi + a_hi*b_lo + a_lo*b_hi  (three MMAs per k step).
 //   * float16 operands (KIND 2): one kind::f16 MMA per k step on the halves
