@@ -816,21 +816,103 @@ int launch_tc2(int M, int N, int K, const CUtensorMap& a0, const CUtensorMap& a1
   return SIMD2_OK;
 }
 
-// Columns of a tile of the single-SM kernel for the sums: the one whose tiles take
-// the fewest SM-times of arithmetic and epilogue.  A K step of 16 costs N / 2
-// cycles an MMA (three for the BF16 split), the epilogue about 20 cycles a
-// column, a tile about 3000 cycles by itself.  1500 x 2100 x 300 on 148 SMs: 108
-// tiles of 256 columns or 132 of 192; 1000 x 800 x 3000: 32 tiles of 256 or 104 of 64.
-int tc_tile_columns(int M, int N, int K, int mmas) {
-  const int sms = device_sms();
-  int best = kTcBN;
+// Columns of a tile of the single-SM kernel for the sums, and the CTAs (a cluster)
+// that share its k.
+struct TcShape {
+  int bn, splits;
+};
+
+// Launch configuration of the split kernel (clusters of `splits` CTAs).
+template <int KIND>
+int tc_split_config(cudaLaunchConfig_t* lc, cudaLaunchAttribute* attr, int splits, int clusters) {
+  static bool configured[64] = {};
+  int dev = 0;
+  SIMD2_CUDA_TRY(cudaGetDevice(&dev));
+  if (dev < 0 || dev >= 64) return SIMD2_ERR_NO_DEVICE;
+  if (!configured[dev]) {
+    SIMD2_CUDA_TRY(cudaFuncSetAttribute(tc_gemm_kernel<KIND, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        (int)tc_smem_bytes<KIND>()));
+    configured[dev] = true;
+  }
+  lc->gridDim = dim3(clusters * splits);
+  lc->blockDim = dim3(kTcThreads);
+  lc->dynamicSmemBytes = tc_smem_bytes<KIND>();
+  attr->id = cudaLaunchAttributeClusterDimension;
+  attr->val.clusterDim.x = splits;
+  attr->val.clusterDim.y = attr->val.clusterDim.z = 1;
+  lc->attrs = attr;
+  lc->numAttrs = 1;
+  return SIMD2_OK;
+}
+
+template <int KIND>
+int launch_tc_split(int M, int N, int K, const CUtensorMap& a0, const CUtensorMap& a1, const CUtensorMap& b0,
+                    const CUtensorMap& b1, const TcEpilogue& ep, TcShape sh, cudaStream_t stream) {
+  const int tiles_m = (M + kTcBM - 1) / kTcBM;
+  const int tiles_n = (N + sh.bn - 1) / sh.bn;
+  cudaLaunchConfig_t lc = {};
+  cudaLaunchAttribute attr;
+  const int rc = tc_split_config<KIND>(&lc, &attr, sh.splits, tiles_m * tiles_n);
+  if (rc) return rc;
+  lc.stream = stream;
+  auto* ev = prof_slot(2LL * M * N * K, kProfTensor);
+  if (ev) cudaEventRecord(ev->first, stream);
+  SIMD2_CUDA_TRY(cudaLaunchKernelEx(&lc, tc_gemm_kernel<KIND, true, true>, a0, a1, b0, b1, M, N, K, ep, tiles_m,
+                                    tiles_n, sh.bn));
+  count_launch();
+  if (ev) cudaEventRecord(ev->second, stream);
+  SIMD2_CUDA_TRY(cudaGetLastError());
+  return SIMD2_OK;
+}
+
+// Clusters of `splits` CTAs of the split kernel that the GPU holds at once.
+template <int KIND>
+int tc_split_slots(int splits) {
+  static int slots[64][9] = {};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+  if (slots[dev][splits] == 0) {
+    int n = 0;
+    cudaLaunchConfig_t lc = {};
+    cudaLaunchAttribute attr;
+    if (tc_split_config<KIND>(&lc, &attr, splits, device_sms() / splits) != SIMD2_OK ||
+        cudaOccupancyMaxActiveClusters(&n, tc_gemm_kernel<KIND, true, true>, &lc) != cudaSuccess) {
+      cudaGetLastError();
+      n = 0;
+    }
+    slots[dev][splits] = n > 0 ? n : -1;
+  }
+  return std::max(0, slots[dev][splits]);
+}
+
+// The tile width and split that take the fewest SM cycles.  Fitted to products of 64
+// to 300 rows, k to 20000: a k-tile of 64 takes 1060 cycles (float16: 490) up to 128
+// columns, bound by the loads, and 6.3 (2.7) a column past that; the epilogue 20 a
+// column, a tile 3000 by itself, and parking and folding the parts 10 + 28 / splits
+// a column.  Split or not, us: 500^3 11.1 / 13.9, 500 x 500 x 2000 17.7 / 29.2,
+// 4000 x 64 x 4000 41.8 / 64.4, 64 x 64 x 20000 59 / 205, 1000 x 800 x 3000
+// 30.6 / 40.5; float16 512 x 512 x 4096 12.5 / 24.5.
+template <int KIND>
+TcShape tc_shape(int M, int N, int K) {
+  constexpr double kTile = KIND == 0 ? 1060.0 : 490.0, kColumn = KIND == 0 ? 6.3 : 2.7;
+  const int ktiles = (K + TcCfg<KIND>::kBK - 1) / TcCfg<KIND>::kBK;
+  TcShape best{kTcBN, 1};
   double best_cost = 1e300;
-  for (int bn : {256, 192, 128, 64}) {
-    const long long tiles = (long long)((M + kTcBM - 1) / kTcBM) * ((N + bn - 1) / bn);
-    const double cost = (double)((tiles + sms - 1) / sms) * (bn * ((K + 15) / 16 * mmas / 2.0 + 20.0) + 3000.0);
-    if (cost < best_cost) {
-      best_cost = cost;
-      best = bn;
+  for (int splits : {1, 2, 4, 8}) {
+    if (splits > std::max(1, ktiles)) break;
+    for (int bn : {256, 192, 128, 64}) {
+      const long long tiles = (long long)((M + kTcBM - 1) / kTcBM) * ((N + bn - 1) / bn);
+      if (splits > 1 && tiles * splits > device_sms()) continue;
+      const int slots = splits == 1 ? device_sms() : tc_split_slots<KIND>(splits);
+      if (slots == 0) continue;
+      const double tile = (ktiles + splits - 1) / splits * std::max(kTile, kColumn * bn) + 3000.0 +
+                          bn * (20.0 + (splits > 1 ? 10.0 + 28.0 / splits : 0.0));
+      const double cost = (double)((tiles + slots - 1) / slots) * tile;
+      if (cost < best_cost) {
+        best_cost = cost;
+        best.bn = bn;
+        best.splits = splits;
+      }
     }
   }
   return best;
@@ -943,7 +1025,9 @@ int srgemm_tc_sum(int op, int M, int N, int K, const T* A, long long lda, const 
   ep.K = K;
   ep.band = kMinusSquareBand;
   if (use_tc2(M, N)) return launch_tc2<KIND>(M, N, K, ma0, ma1, mb0, mb1, mb0, ep, stream);
-  return launch_tc<KIND, true>(M, N, K, ma0, ma1, mb0, mb1, ep, tc_tile_columns(M, N, K, kHalf ? 1 : 3), stream);
+  const TcShape sh = tc_shape<KIND>(M, N, K);
+  if (sh.splits > 1) return launch_tc_split<KIND>(M, N, K, ma0, ma1, mb0, mb1, ep, sh, stream);
+  return launch_tc<KIND, true>(M, N, K, ma0, ma1, mb0, mb1, ep, sh.bn, stream);
 }
 
 // delta (or_and closure, pair kernel only): the maps of TcEpilogue.  With need_row /

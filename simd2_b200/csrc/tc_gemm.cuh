@@ -478,8 +478,122 @@ __host__ __device__ constexpr int tc_stages_of(int bn) {
   return fit < kTcMaxStages ? fit : kTcMaxStages;
 }
 
+// SPLIT: the CTAs of a cluster share one tile, each a range of its k-tiles.  A warp
+// parks its 32 rows x ncols columns of the accumulator in its CTA's shared memory
+// (the ring, idle by then) ...
+__device__ __forceinline__ int tc_part_pitch(int bn) { return bn + 4; }
+__device__ __forceinline__ void tc_park(uint32_t trow, float* row, int ncols) {
+#pragma unroll 1
+  for (int c0 = 0; c0 < ncols; c0 += 32) {
+    uint32_t r[32];
+    tmem_ld32(trow + c0, r);
+#pragma unroll
+    for (int j = 0; j < 32; j += 4) *reinterpret_cast<uint4*>(row + c0 + j) = make_uint4(r[j], r[j + 1], r[j + 2], r[j + 3]);
+  }
+}
+
+// ... and every CTA adds up the parts of 128 / S of the rows, in the order of the
+// ranks, and writes them out.  A thread has the parts of 8 / S quads of columns on
+// their way at once: one at a time, the fold of a tile took 10 to 25 us of latency.
+template <int KIND, int S>
+__device__ __forceinline__ void tc_fold(const TcEpilogue& ep, int M, int N, int m0, int n0, const float* part, int bn,
+                                        int rank, int thread) {
+  constexpr int U = 8 / S, T = kTcEpiWarps * 32;
+  constexpr int per = kTcBM / S;
+  const int first = rank * per, quads = bn >> 2;
+  const int end = min(per, M - m0 - first) * quads;
+  const bool msq = ep.op == SIMD2_MINUS_SQUARE;
+  const float* C = ep.do_epilogue ? static_cast<const float*>(ep.C) : nullptr;
+  float* D = static_cast<float*>(ep.D);
+  const bool vec = (reinterpret_cast<uintptr_t>(D) & 15) == 0 && (ep.ldd & 3) == 0 &&
+                   (!C || ((reinterpret_cast<uintptr_t>(C) & 15) == 0 && (ep.ldc & 3) == 0));
+  for (int e0 = thread; e0 < end; e0 += U * T) {
+    float4 p[U][S];
+    float4 c[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const int e = e0 + u * T;
+      if (e >= end) break;
+      const int r = e / quads, j = (e - r * quads) * 4, left = N - n0 - j;
+      const uint32_t at = smem_u32(part + (first + r) * tc_part_pitch(bn) + j);
+#pragma unroll
+      for (int q = 0; q < S; q++) {
+        uint32_t remote;
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(at), "r"(q));
+        asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+                     : "=f"(p[u][q].x), "=f"(p[u][q].y), "=f"(p[u][q].z), "=f"(p[u][q].w)
+                     : "r"(remote)
+                     : "memory");
+      }
+      if (C) {
+        const float* cr = C + (long long)(m0 + first + r) * ep.ldc + n0 + j;
+        if (vec && left >= 4) c[u] = *reinterpret_cast<const float4*>(cr);
+        else c[u] = make_float4(left > 0 ? cr[0] : 0.f, left > 1 ? cr[1] : 0.f, left > 2 ? cr[2] : 0.f, left > 3 ? cr[3] : 0.f);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const int e = e0 + u * T;
+      if (e >= end) break;
+      const int r = e / quads, j = (e - r * quads) * 4, left = N - n0 - j;
+      const long long row = m0 + first + r;
+      float v[4] = {p[u][0].x, p[u][0].y, p[u][0].z, p[u][0].w};
+#pragma unroll
+      for (int q = 1; q < S; q++) {
+        v[0] = __fadd_rn(v[0], p[u][q].x);
+        v[1] = __fadd_rn(v[1], p[u][q].y);
+        v[2] = __fadd_rn(v[2], p[u][q].z);
+        v[3] = __fadd_rn(v[3], p[u][q].w);
+      }
+      if (msq) {
+        const float na = ep.norm_a[row];
+        uint32_t band = 0;
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+          const float nsum = na + (i < left ? ep.norm_b[n0 + j + i] : 0.f);
+          v[i] = __fmaf_rn(-2.0f, v[i], nsum);
+          band |= (i < left && v[i] < ep.band * nsum ? 1u : 0u) << i;
+        }
+        while (band) {  // rare: inside the cancellation band
+          const int i = __ffs(band) - 1;
+          band &= band - 1;
+          using A = typename std::conditional<KIND == 2, __half, float>::type;
+          const float d =
+              exact_minus_square(static_cast<const A*>(ep.A32) + row * ep.lda32, static_cast<const A*>(ep.B32),
+                                 ep.ldb32, n0 + j + i, ep.K, ep.b_rows);
+          if (i == 0) v[0] = d;
+          else if (i == 1) v[1] = d;
+          else if (i == 2) v[2] = d;
+          else v[3] = d;
+        }
+      }
+      if (C) {
+        v[0] = __fadd_rn(v[0], c[u].x);
+        v[1] = __fadd_rn(v[1], c[u].y);
+        v[2] = __fadd_rn(v[2], c[u].z);
+        v[3] = __fadd_rn(v[3], c[u].w);
+      }
+      float* dr = D + row * ep.ldd + n0 + j;
+      if (vec && left >= 4) *reinterpret_cast<float4*>(dr) = make_float4(v[0], v[1], v[2], v[3]);
+      else {
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+          if (i < left) dr[i] = v[i];
+      }
+    }
+  }
+}
+
+__device__ __forceinline__ void tc_cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
 // bn: columns of a tile (a multiple of 64, at most 256; 224 for or_and).
-template <int KIND, bool BT>
+// SPLIT (the sums): a cluster of 2, 4 or 8 CTAs per tile, one tile each.  A product of
+// few tiles leaves most SMs idle and walks its k alone (64 x 64 x 20000: 1 SM, 205 us;
+// now 8, 59 us, of which the operands' split takes about 28).  No scratch memory, and the
+// parts are added in one order.
+template <int KIND, bool BT, bool SPLIT = false>
 __global__ void __launch_bounds__(kTcThreads, 1)
     tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__ CUtensorMap tmA1,
                    const __grid_constant__ CUtensorMap tmB0, const __grid_constant__ CUtensorMap tmB1, int M, int N,
@@ -499,7 +613,15 @@ __global__ void __launch_bounds__(kTcThreads, 1)
 
   const int tiles = tiles_m * tiles_n;
   const uint32_t idesc = tc_idesc<KIND>(bn, BT);
-  const int ktiles = (K + Cfg::kBK - 1) / Cfg::kBK;
+  const int all_ktiles = (K + Cfg::kBK - 1) / Cfg::kBK;
+  int splits = 1, rank = 0;
+  if constexpr (SPLIT) {
+    asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(splits));
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+  }
+  const int kt0 = (int)((long long)all_ktiles * rank / splits);
+  const int ktiles = (int)((long long)all_ktiles * (rank + 1) / splits);  // of this CTA: [kt0, ktiles)
+  const int first_tile = SPLIT ? blockIdx.x / splits : blockIdx.x, tile_step = SPLIT ? tiles : gridDim.x;
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   // Grouped raster over (tile_m, tile_n): 8 tile rows per group.
@@ -552,10 +674,10 @@ __global__ void __launch_bounds__(kTcThreads, 1)
       int s = 0;  // ring position
       uint32_t ph = 1;
       bool ok = true;
-      for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
+      for (int t = first_tile; t < tiles && ok; t += tile_step) {
         int m0, n0;
         tile_origin(t, m0, n0);
-        for (int kt = 0; kt < ktiles; kt++) {
+        for (int kt = kt0; kt < ktiles; kt++) {
           if (!mbar_wait(&empty[s], ph)) {
             report_timeout(101);
             ok = false;
@@ -592,7 +714,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
       uint32_t ph = 0;
       bool ok = true;
       int lt = 0;
-      for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x, lt++) {
+      for (int t = first_tile; t < tiles && ok; t += tile_step, lt++) {
         const int acc = lt & 1;
         if (!mbar_wait(&acc_empty[acc], ((lt >> 1) & 1) ^ 1)) {
           report_timeout(104);
@@ -600,7 +722,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         }
         tc_fence_after();
         const uint32_t d = tmem + acc * tc_bn<KIND>();
-        for (int kt = 0; kt < ktiles; kt++) {
+        for (int kt = kt0; kt < ktiles; kt++) {
           if (!mbar_wait(&full[s], ph)) {
             report_timeout(102);
             ok = false;
@@ -615,7 +737,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
 #pragma unroll
           for (int ks = 0; ks < Cfg::kBK / Cfg::kKStep; ks++) {
             const uint32_t koff = ks * 32;  // bytes along the swizzled row
-            const uint32_t acc0 = (kt > 0 || ks > 0) ? 1u : 0u;
+            const uint32_t acc0 = (kt > kt0 || ks > 0) ? 1u : 0u;
             auto bdesc = [&](uint32_t b) {
               return BT ? umma_desc_nmajor(b + ks * 2048, tc_b_group<KIND>()) : umma_desc_swizzled(b + koff, RB);
             };
@@ -647,7 +769,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     uint32_t* epi_tile = epi_smem + (warp - 2) * (32 * 33);
     bool ok = true;
     int lt = 0;
-    for (int t = blockIdx.x; t < tiles; t += gridDim.x, lt++) {
+    for (int t = first_tile; t < tiles; t += tile_step, lt++) {
       const int acc = lt & 1;
       if (ok && !mbar_wait(&acc_full[acc], (lt >> 1) & 1)) {
         report_timeout(103);
@@ -659,6 +781,10 @@ __global__ void __launch_bounds__(kTcThreads, 1)
       int m0, n0;
       tile_origin(t, m0, n0);
       const uint32_t trow = tmem + acc * tc_bn<KIND>() + cfirst + ((uint32_t)(quad * 32) << 16);
+      if constexpr (SPLIT) {
+        tc_park(trow, reinterpret_cast<float*>(smem) + (quad * 32 + lane) * tc_part_pitch(bn) + cfirst, ccount);
+        break;
+      }
       const int row0 = m0 + quad * 32;
       int changed = 0;
       // the accumulator half is read out: the MMA warp may reuse it
@@ -672,6 +798,21 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         if (__any_sync(0xffffffffu, changed) && lane == 0) atomicOr(ep.changed, 1);
       }
     }
+  }
+
+  if constexpr (SPLIT) {
+    static_assert(kTcBM * (kTcBN + 4) * 4 <= Cfg::kStages * tc_stage_bytes<KIND>(), "parts fit the ring");
+    int m0, n0;
+    tile_origin(first_tile, m0, n0);
+    tc_cluster_sync();  // every part is in place
+    if (warp >= 2) {
+      const float* part = reinterpret_cast<const float*>(smem);
+      const int thread = threadIdx.x - 64;
+      if (splits == 2) tc_fold<KIND, 2>(ep, M, N, m0, n0, part, bn, rank, thread);
+      else if (splits == 4) tc_fold<KIND, 4>(ep, M, N, m0, n0, part, bn, rank, thread);
+      else tc_fold<KIND, 8>(ep, M, N, m0, n0, part, bn, rank, thread);
+    }
+    tc_cluster_sync();  // peers stay until every CTA has read their parts
   }
 
   // every MMA has completed before TMEM is released

@@ -100,3 +100,21 @@ def test_minmax_f16(cuda, op, offset):
         want = oracle.srgemm(op, a.float().cpu().numpy(), b.float().cpu().numpy(), c.contiguous().cpu().numpy(),
                              do_epilogue=True)
         np.testing.assert_array_equal(got.view(np.uint32), want.view(np.uint32))
+
+
+@pytest.mark.parametrize("op", ["plus_mul", "minus_square"])
+@pytest.mark.parametrize("shape", [(64, 64, 128), (65, 63, 129), (1, 1, 2500), (200, 201, 1000), (500, 500, 2000),
+                                   (1000, 131, 700), (63, 1030, 5000), (1000, 800, 900)])
+@pytest.mark.parametrize("half", [False, True])
+def test_split_k(cuda, op, shape, half):
+    """Few tiles: the CTAs of a cluster share a tile's k.  Some rows of A are columns
+    of B, whose distances lie in the cancellation band."""
+    m, n, k = shape
+    for offset in (0, 1):
+        a, b, c = operands(m, n, k, torch.float16 if half else torch.float32, m + n + k, offset)
+        a[::9] = b[:, : len(a[::9])].T[: len(a[::9])] if n >= len(a[::9]) else b[:, :1].T
+        f = s2.srgemm_f16 if half else s2.srgemm
+        check(op, a, b, c, f(op, a, b, c, do_epilogue=True), half)
+        if not offset:
+            assert torch.equal(f(op, a, b, c, do_epilogue=True), f(op, a, b, c, do_epilogue=True))
+    assert s2.device_status() == 0
