@@ -238,9 +238,9 @@ int simd2_knn(const float* query, int Q, int ldq, const float* ref, int R, int l
 
 /* Execution strategy of simd2_knn_ex.  Both give bit-identical results. */
 typedef enum {
-  SIMD2_KNN_AUTO = 0,         /* FUSED when D <= 128, else MATERIALISED */
+  SIMD2_KNN_AUTO = 0,         /* FUSED, at any D (above 128 the queries are streamed as well) */
   SIMD2_KNN_FUSED = 1,        /* selection inside the distance MMA's epilogue; D <= 128
-                                 (SIMD2_ERR_UNSUPPORTED otherwise) */
+                                 (SIMD2_ERR_UNSUPPORTED otherwise; AUTO takes any D) */
   SIMD2_KNN_MATERIALISED = 2  /* distance blocks of ~1 GiB written, then selected */
 } simd2_knn_mode;
 

@@ -529,8 +529,8 @@ def knn(query: torch.Tensor, ref: torch.Tensor, k: int, stream=None, mode: str =
     Mirrors the PLD path of the reference (minus_square srgemm, insertion-sort
     top-k, sqrt); outputs are query-major.  ``mode``: "fused" selects inside
     the distance kernel (D <= 128), "materialised" writes distance blocks and
-    selects from them, "auto" picks fused when it applies; results are
-    bit-identical.
+    selects from them, "auto" selects inside the distance kernel at any D;
+    results are bit-identical.
     """
     Q, D = query.shape
     R, D2 = ref.shape

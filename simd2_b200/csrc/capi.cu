@@ -3108,10 +3108,10 @@ int knn_fused_chunks(int qblocks, int tiles, int sms, long long max_lists) {
   return best;
 }
 
-// One fused pass: knn_fused_kernel<KL> over every (query block, chunk) unit,
+// One fused pass: knn_fused_kernel<KL, WIDE> over every (query block, chunk) unit,
 // then the per-query merge of its lists of KL into kout results (lane lists
 // of KT).  flags / gate: see knn_merge_kernel.
-template <int KL, int KT>
+template <int KL, int KT, bool WIDE>
 int knn_fused_pass(const CUtensorMap& mqh, const CUtensorMap& mql, const CUtensorMap& mrh, const CUtensorMap& mrl,
                    const KnnFusedArgs& args, int qblocks, float* od, int32_t* oi, long long ldo, int kout, int* flags,
                    cudaStream_t stream) {
@@ -3121,13 +3121,13 @@ int knn_fused_pass(const CUtensorMap& mqh, const CUtensorMap& mql, const CUtenso
   if (dev < 0 || dev >= 64) return SIMD2_ERR_NO_DEVICE;
   if (!configured[dev]) {
     SIMD2_CUDA_TRY(
-        cudaFuncSetAttribute(knn_fused_kernel<KL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kKfSmemBytes));
+        cudaFuncSetAttribute(knn_fused_kernel<KL, WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kKfSmemBytes));
     configured[dev] = true;
   }
   // the second pass's time counts, its operations were counted by the first
   auto* ev = prof_slot(args.gate ? 0LL : 2LL * args.Q * args.R * args.D, kProfTensor);
   if (ev) cudaEventRecord(ev->first, stream);
-  knn_fused_kernel<KL><<<qblocks * args.chunks, kKfThreads, kKfSmemBytes, stream>>>(mqh, mql, mrh, mrl, args);
+  knn_fused_kernel<KL, WIDE><<<qblocks * args.chunks, kKfThreads, kKfSmemBytes, stream>>>(mqh, mql, mrh, mrl, args);
   count_launch();
   if (ev) cudaEventRecord(ev->second, stream);
   SIMD2_CUDA_TRY(cudaGetLastError());
@@ -3172,23 +3172,23 @@ bool knn_half_lists(int k, int lists, int len) {
   return 128.0 * lists * tail <= 0.01;
 }
 
-template <int KT>
+template <int KT, bool WIDE>
 int knn_fused_launch(const CUtensorMap& mqh, const CUtensorMap& mql, const CUtensorMap& mrh, const CUtensorMap& mrl,
                      KnnFusedArgs a, int qblocks, float* od, int32_t* oi, long long ldo, int kout, float* pd2,
                      int32_t* pi2, unsigned* ready2, int* flags, cudaStream_t stream) {
   if constexpr (KT >= 16) {
     if (kout > KT / 2 && knn_half_lists(kout, 2 * a.chunks, KT / 2)) {
-      int rc = knn_fused_pass<KT / 2, KT>(mqh, mql, mrh, mrl, a, qblocks, od, oi, ldo, kout, flags, stream);
+      int rc = knn_fused_pass<KT / 2, KT, WIDE>(mqh, mql, mrh, mrl, a, qblocks, od, oi, ldo, kout, flags, stream);
       if (rc) return rc;
       KnnFusedArgs b = a;
       b.part_d = pd2;
       b.part_i = pi2;
       b.ready = ready2;
       b.gate = flags;
-      return knn_fused_pass<KT, KT>(mqh, mql, mrh, mrl, b, qblocks, od, oi, ldo, kout, nullptr, stream);
+      return knn_fused_pass<KT, KT, WIDE>(mqh, mql, mrh, mrl, b, qblocks, od, oi, ldo, kout, nullptr, stream);
     }
   }
-  return knn_fused_pass<KT, KT>(mqh, mql, mrh, mrl, a, qblocks, od, oi, ldo, kout, nullptr, stream);
+  return knn_fused_pass<KT, KT, WIDE>(mqh, mql, mrh, mrl, a, qblocks, od, oi, ldo, kout, nullptr, stream);
 }
 
 // Query rows per chunk so that one chunk's distance block stays near 1 GiB.
@@ -3274,7 +3274,9 @@ int knn_fused(const float* query, int Q, int ldq, const float* ref, int R, int l
   pa.r_tiles = tiles;
   pa.clear = reinterpret_cast<unsigned*>(ws + rf);
   pa.clear_words = (long long)(qf + (size_t)qblocks * 4 - rf) / 4;
-  knn_prep_kernel<<<tiles + (Q + kKfBN - 1) / kKfBN, kKnnPrepThreads, 0, stream>>>(pa);
+  const bool wide = Dp > 64 * kKfMaxPanels;
+  (wide ? knn_prep_kernel<true> : knn_prep_kernel<false>)<<<tiles + (Q + kKfBN - 1) / kKfBN, kKnnPrepThreads, 0,
+                                                            stream>>>(pa);
   count_launch();
   SIMD2_CUDA_TRY(cudaGetLastError());
   const auto BF = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
@@ -3310,17 +3312,16 @@ int knn_fused(const float* query, int Q, int ldq, const float* ref, int R, int l
   int32_t* p_i2 = reinterpret_cast<int32_t*>(ws + pi2);
   unsigned* r2 = reinterpret_cast<unsigned*>(ws + rf2);
   int* flags = reinterpret_cast<int*>(ws + qf);
+  auto launch = [&](auto kt) {
+    constexpr int kKt = decltype(kt)::value;
+    return (wide ? knn_fused_launch<kKt, true> : knn_fused_launch<kKt, false>)(
+        mqh, mql, mrh, mrl, a, qblocks, out_dist, out_idx, ldo, k, p_d2, p_i2, r2, flags, stream);
+  };
   switch (KT) {
-    case 4:
-      return knn_fused_launch<4>(mqh, mql, mrh, mrl, a, qblocks, out_dist, out_idx, ldo, k, p_d2, p_i2, r2, flags, stream);
-    case 8:
-      return knn_fused_launch<8>(mqh, mql, mrh, mrl, a, qblocks, out_dist, out_idx, ldo, k, p_d2, p_i2, r2, flags, stream);
-    case 16:
-      return knn_fused_launch<16>(mqh, mql, mrh, mrl, a, qblocks, out_dist, out_idx, ldo, k, p_d2, p_i2, r2, flags,
-                                  stream);
-    default:
-      return knn_fused_launch<32>(mqh, mql, mrh, mrl, a, qblocks, out_dist, out_idx, ldo, k, p_d2, p_i2, r2, flags,
-                                  stream);
+    case 4: return launch(std::integral_constant<int, 4>());
+    case 8: return launch(std::integral_constant<int, 8>());
+    case 16: return launch(std::integral_constant<int, 16>());
+    default: return launch(std::integral_constant<int, 32>());
   }
 }
 
@@ -3353,9 +3354,10 @@ extern "C" int simd2_knn_ex(const float* query, int Q, int ldq, const float* ref
     return SIMD2_OK;
   }
   const int Dp = round_up(D, 8);
-  const bool fused = mode == SIMD2_KNN_FUSED || (mode == SIMD2_KNN_AUTO && Dp <= 64 * kKfMaxPanels);
-  if (fused && Dp > 64 * kKfMaxPanels) return SIMD2_ERR_UNSUPPORTED;
-  if (fused) return knn_fused(query, Q, ldq, ref, R, ldr, D, k, out_dist, out_idx, ldo, stream);
+  // Writing the distances out is slower at every D (64 x 256 x 150, k = 1: 54 us
+  // against 49; 16384 x 65536 x 136, k = 8: 4916 against 1025), so AUTO never does.
+  if (mode == SIMD2_KNN_FUSED && Dp > 64 * kKfMaxPanels) return SIMD2_ERR_UNSUPPORTED;
+  if (mode != SIMD2_KNN_MATERIALISED) return knn_fused(query, Q, ldq, ref, R, ldr, D, k, out_dist, out_idx, ldo, stream);
   const int Qc = knn_chunk_rows(Q, R);
   size_t off = 0;
   auto take = [&](size_t bytes) { size_t o = off; off += align_up(bytes, kAlign); return o; };

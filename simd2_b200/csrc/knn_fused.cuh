@@ -36,6 +36,13 @@
 // and a compare.
 //
 // Each unit writes, per query, two sorted lists of k (one per column half);
+// WIDE (D > 128): the query panels no longer fit beside the ring, so they come
+// through it as well, one stage (hi and lo, 16 KiB each) before the two of the
+// reference panel, again for every tile: 96 KiB a K panel for its 1536 cycles of
+// MMA, half as much again as the queries at rest.  A call, through a distance
+// block and this way (us): 2000 x 20000 x 300, k = 20, 652 / 183; 16384 x 65536 x
+// 136, k = 8, 4916 / 1025; 1000 x 4000 x 200, k = 8, 77 / 69.
+//
 // knn_merge_kernel merges the 2 x chunks lists of a query by (distance,
 // index) and writes the k results with their square roots.  Ties keep the
 // lower reference index first, the order of apps/pld/emulation/knncuda.cu:
@@ -52,6 +59,7 @@ constexpr int kKfBM = 128;                     // queries per unit (TMEM lanes)
 constexpr int kKfBN = 256;                     // references per tile (MMA N)
 constexpr int kKfMaxPanels = 2;                // D <= 128: two 64-element K panels
 constexpr int kKfStages = 4;                   // B ring depth (2 K panels of hi + lo)
+constexpr int kKfWideStages = 6;               // WIDE ring: 2 K panels of queries, hi, lo
 constexpr int kKfATile = kKfBM * 128;          // 16 KiB: one K panel of 128 query rows
 constexpr int kKfBTile = kKfBN * 128;          // 32 KiB: one K panel of 256 reference rows
 constexpr int kKfEpiWarps = 8;
@@ -60,10 +68,12 @@ constexpr int kKfTmemCols = 512;               // two 128 x 256 FP32 accumulator
 constexpr int kKfNormSlots = 4;                // reference norms of a tile, 1 KiB each
 constexpr size_t kKfSmemBytes =
     (size_t)kKfMaxPanels * 2 * kKfATile + (size_t)kKfStages * kKfBTile + kKfNormSlots * kKfBN * 4 + 1024 /* align */ + 256 /* barriers */;
+static_assert(kKfWideStages * kKfBTile == kKfMaxPanels * 2 * kKfATile + kKfStages * kKfBTile && 2 * kKfATile == kKfBTile,
+              "the WIDE ring takes the place of the query panels and the ring");
 
 struct KnnFusedArgs {
   int Q, R, D;
-  int panels;             // ceil(round_up(D, 8) / 64), 1 or 2
+  int panels;             // ceil(round_up(D, 8) / 64), 1 or 2 (WIDE: any)
   int chunks;             // reference chunks (units per 128 queries), the pilot included
   int tiles_per_chunk;    // reference tiles of 256 per chunk (after the pilot)
   int pilot_tiles;        // > 0: chunk 0 is a short pilot of this many tiles (see knn_unit_tiles)
@@ -198,20 +208,21 @@ __device__ __forceinline__ float knn_prior_fold(const KnnFusedArgs& a, int chunk
   return T;
 }
 
-template <int K>
+template <int K, bool WIDE>
 __global__ void __launch_bounds__(kKfThreads, 1)
     knn_fused_kernel(const __grid_constant__ CUtensorMap tmQh, const __grid_constant__ CUtensorMap tmQl,
                      const __grid_constant__ CUtensorMap tmRh, const __grid_constant__ CUtensorMap tmRl,
                      KnnFusedArgs a) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* sA = smem;                                    // [panel][hi, lo] 16 KiB each
-  uint8_t* sB = smem + kKfMaxPanels * 2 * kKfATile;      // [stage] 32 KiB each
-  float* sN = reinterpret_cast<float*>(sB + kKfStages * kKfBTile);
+  constexpr int S = WIDE ? kKfWideStages : kKfStages;
+  uint8_t* sA = smem;                                             // [panel][hi, lo] 16 KiB each
+  uint8_t* sB = smem + (WIDE ? 0 : kKfMaxPanels * 2 * kKfATile);  // [stage] 32 KiB each
+  float* sN = reinterpret_cast<float*>(sB + S * kKfBTile);
   uint64_t* a_full = reinterpret_cast<uint64_t*>(sN + kKfNormSlots * kKfBN);
   uint64_t* full = a_full + 1;
-  uint64_t* empty = full + kKfStages;
-  uint64_t* acc_full = empty + kKfStages;
+  uint64_t* empty = full + S;
+  uint64_t* acc_full = empty + S;
   uint64_t* acc_empty = acc_full + 2;
   uint64_t* fin = acc_empty + 2;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(fin + 1);
@@ -229,7 +240,7 @@ __global__ void __launch_bounds__(kKfThreads, 1)
 
   if (threadIdx.x == 0) {
     mbar_init(a_full, 1);
-    for (int s = 0; s < kKfStages; s++) {
+    for (int s = 0; s < S; s++) {
       mbar_init(&full[s], 1);
       mbar_init(&empty[s], 1);
     }
@@ -256,25 +267,32 @@ __global__ void __launch_bounds__(kKfThreads, 1)
       // ---------------- TMA producer ----------------
       prefetch_tensormap(&tmQh);
       prefetch_tensormap(&tmRh);
-      mbar_arrive_expect_tx(a_full, 2 * P * kKfATile);
-      for (int p = 0; p < P; p++) {
-        tma_load_2d(sA + (2 * p) * kKfATile, &tmQh, a_full, p * 64, m0);
-        tma_load_2d(sA + (2 * p + 1) * kKfATile, &tmQl, a_full, p * 64, m0);
+      if (!WIDE) {
+        mbar_arrive_expect_tx(a_full, 2 * P * kKfATile);
+        for (int p = 0; p < P; p++) {
+          tma_load_2d(sA + (2 * p) * kKfATile, &tmQh, a_full, p * 64, m0);
+          tma_load_2d(sA + (2 * p + 1) * kKfATile, &tmQl, a_full, p * 64, m0);
+        }
       }
       int j = 0;
       bool ok = true;
       for (int t = 0; t < ntiles && ok; t++) {
         const int n0 = (t0 + t) * kKfBN;
         for (int p = 0; p < P && ok; p++) {
-          for (int h = 0; h < 2; h++, j++) {  // panel p: hi stage, then lo stage
-            const int s = j % kKfStages;
-            if (!mbar_wait(&empty[s], ((j / kKfStages) & 1) ^ 1)) {
+          for (int h = WIDE ? -1 : 0; h < 2; h++, j++) {  // panel p: (queries,) hi stage, then lo stage
+            const int s = j % S;
+            if (!mbar_wait(&empty[s], ((j / S) & 1) ^ 1)) {
               report_timeout(111);
               ok = false;
               break;
             }
             mbar_arrive_expect_tx(&full[s], kKfBTile);
-            tma_load_2d(sB + s * kKfBTile, h == 0 ? &tmRh : &tmRl, &full[s], p * 64, n0);
+            if (h < 0) {
+              tma_load_2d(sB + s * kKfBTile, &tmQh, &full[s], p * 64, m0);
+              tma_load_2d(sB + s * kKfBTile + kKfATile, &tmQl, &full[s], p * 64, m0);
+            } else {
+              tma_load_2d(sB + s * kKfBTile, h == 0 ? &tmRh : &tmRl, &full[s], p * 64, n0);
+            }
           }
         }
       }
@@ -283,7 +301,7 @@ __global__ void __launch_bounds__(kKfThreads, 1)
   } else if (warp == 1) {
     if (lane == 0) {
       // ---------------- MMA issuer ----------------
-      bool ok = mbar_wait(a_full, 0);
+      bool ok = WIDE || mbar_wait(a_full, 0);
       if (!ok) report_timeout(112);
       tc_fence_after();
       const uint32_t a_base = smem_u32(sA), b_base = smem_u32(sB);
@@ -303,25 +321,37 @@ __global__ void __launch_bounds__(kKfThreads, 1)
                   &acc_full[acc]);
         const uint32_t d = tmem + acc * kKfBN;
         for (int p = 0; p < P; p++, j += 2) {
-          // stages j (hi) and j+1 (lo) hold K panel p of the tile
-          const int sh = j % kKfStages, sl = (j + 1) % kKfStages;
-          if (!mbar_wait(&full[sh], (j / kKfStages) & 1) || !mbar_wait(&full[sl], ((j + 1) / kKfStages) & 1)) {
+          // stages j (hi) and j+1 (lo) hold K panel p of the tile (WIDE: the queries' stage before them)
+          const int sq = j % S;
+          if (WIDE) {
+            if (!mbar_wait(&full[sq], (j / S) & 1)) {
+              report_timeout(117);
+              ok = false;
+              break;
+            }
+            j++;
+          }
+          const int sh = j % S, sl = (j + 1) % S;
+          if (!mbar_wait(&full[sh], (j / S) & 1) || !mbar_wait(&full[sl], ((j + 1) / S) & 1)) {
             report_timeout(114);
             ok = false;
             break;
           }
           tc_fence_after();
           const uint32_t bh = b_base + sh * kKfBTile, bl = b_base + sl * kKfBTile;
-          const uint32_t ah = a_base + (2 * p) * kKfATile, al = ah + kKfATile;
+          const uint32_t ah = WIDE ? b_base + sq * kKfBTile : a_base + (2 * p) * kKfATile, al = ah + kKfATile;
+          const int left = a.D - p * 64;  // elements of the panel; zeros past them
           // per 16-element K step: qh.rh, qh.rl, ql.rh -- the order of the
           // materialised minus_square kernel, so the FP32 sums are identical
 #pragma unroll
           for (int ks = 0; ks < 4; ks++) {
+            if (WIDE && ks * 16 >= left) break;
             const uint32_t ko = ks * 32;  // 16 BF16 along the 128-byte row
             tc_mma<0>(d, umma_desc_sw128(ah + ko), umma_desc_sw128(bh + ko), (p > 0 || ks > 0) ? 1u : 0u, TcCfg<0>::kIdesc);
             tc_mma<0>(d, umma_desc_sw128(ah + ko), umma_desc_sw128(bl + ko), 1u, TcCfg<0>::kIdesc);
             tc_mma<0>(d, umma_desc_sw128(al + ko), umma_desc_sw128(bh + ko), 1u, TcCfg<0>::kIdesc);
           }
+          if (WIDE) tc_commit(&empty[sq]);
           tc_commit(&empty[sh]);
           tc_commit(&empty[sl]);
         }
@@ -671,7 +701,8 @@ __global__ void __launch_bounds__(256) knn_merge_kernel(const float* __restrict_
 // queries each.  The grid also clears `clear_words` words at `clear` (the
 // passes' ready and block flags).  32 warps per block, 8 rows per warp: a
 // warp issues all its loads at once (lane l holds elements l, l+32, ... of
-// each row) and splits from the same registers.
+// each row) and splits from the same registers.  WIDE (D > 128): two rows at a
+// time, 128 elements after 128.
 struct KnnPrepArgs {
   const float* q;
   long long ldq;
@@ -679,7 +710,7 @@ struct KnnPrepArgs {
   const float* r;
   long long ldr;
   int R;
-  int D, Dp;  // D <= 32 * kKnnPrepMaxJ, Dp = D rounded up to 8
+  int D, Dp;  // Dp = D rounded up to 8; not WIDE: D <= 32 * kKnnPrepMaxJ
   __nv_bfloat16 *q_hi, *q_lo, *r_hi, *r_lo;
   float *n_q, *n_r, *t_max;
   int r_tiles;
@@ -692,6 +723,7 @@ constexpr int kKnnPrepRows = 8;                 // rows per warp
 constexpr int kKnnPrepThreads = 1024;           // 32 warps x 8 rows = 256 rows per block
 static_assert(kKnnPrepThreads / 32 * kKnnPrepRows == kKfBN, "one reference tile per block");
 
+template <bool WIDE>
 __global__ void __launch_bounds__(kKnnPrepThreads) knn_prep_kernel(KnnPrepArgs a) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   for (long long w = blockIdx.x * (long long)kKnnPrepThreads + threadIdx.x; w < a.clear_words;
@@ -708,50 +740,58 @@ __global__ void __launch_bounds__(kKnnPrepThreads) knn_prep_kernel(KnnPrepArgs a
   const int row0 = (ref ? blockIdx.x : blockIdx.x - a.r_tiles) * kKfBN + warp * kKnnPrepRows;
   const float inf = __int_as_float(0x7f800000);
   float mx = -inf;  // the warp's largest norm over valid rows (reference tiles)
-  {
-    float v[kKnnPrepRows][kKnnPrepMaxJ];
+  constexpr int RU = WIDE ? 2 : kKnnPrepRows;
+#pragma unroll 1
+  for (int ub = 0; ub < kKnnPrepRows; ub += RU) {
+    double s[RU] = {};
+#pragma unroll 1
+    for (int k0 = 0; k0 < (WIDE ? a.Dp : 1); k0 += 32 * kKnnPrepMaxJ) {
+      float v[RU][kKnnPrepMaxJ];
 #pragma unroll
-    for (int u = 0; u < kKnnPrepRows; u++) {
-      const int i = row0 + u;
+      for (int u = 0; u < RU; u++) {
+        const int i = row0 + ub + u;
 #pragma unroll
-      for (int j = 0; j < kKnnPrepMaxJ; j++) {
-        const int k = lane + 32 * j;
-        v[u][j] = (i < M && k < a.D) ? __ldg(A + (long long)i * lda + k) : 0.f;
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < kKnnPrepRows; u++) {
-      const int i = row0 + u;
-      double s = 0.0;
-#pragma unroll
-      for (int j = 0; j < kKnnPrepMaxJ; j++) {
-        if (lane + 32 * j < a.D) {
-          const double x = v[u][j];
-          s += x * x;
+        for (int j = 0; j < kKnnPrepMaxJ; j++) {
+          const int k = k0 + lane + 32 * j;
+          v[u][j] = (i < M && k < a.D) ? __ldg(A + (long long)i * lda + k) : 0.f;
         }
       }
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-      const float n = i < M ? (float)s : inf;
+      for (int u = 0; u < RU; u++) {
+#pragma unroll
+        for (int j = 0; j < kKnnPrepMaxJ; j++) {
+          if (k0 + lane + 32 * j < a.D) {
+            const double x = v[u][j];
+            s[u] += x * x;
+          }
+        }
+      }
+      // the BF16 split from the same registers: lane l writes elements l,
+      // l+32, ... of each row (zeros for D <= k < Dp)
+#pragma unroll
+      for (int u = 0; u < RU; u++) {
+        const int i = row0 + ub + u;
+        if (i >= M) continue;
+#pragma unroll
+        for (int j = 0; j < kKnnPrepMaxJ; j++) {
+          const int k = k0 + lane + 32 * j;
+          if (k < a.Dp) {
+            __nv_bfloat16 h, l;
+            split_bf16(v[u][j], h, l);
+            hi[(long long)i * a.Dp + k] = h;
+            lo[(long long)i * a.Dp + k] = l;
+          }
+        }
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < RU; u++) {
+      const int i = row0 + ub + u;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) s[u] += __shfl_xor_sync(0xffffffffu, s[u], o);
+      const float n = i < M ? (float)s[u] : inf;
       if (i < M) mx = fmaxf(mx, n);
       if (lane == 0 && i < rows) nrm[i] = n;
-    }
-    // the BF16 split from the same registers: lane l writes elements l,
-    // l+32, ... of each row (zeros for D <= k < Dp)
-#pragma unroll
-    for (int u = 0; u < kKnnPrepRows; u++) {
-      const int i = row0 + u;
-      if (i >= M) continue;
-#pragma unroll
-      for (int j = 0; j < kKnnPrepMaxJ; j++) {
-        const int k = lane + 32 * j;
-        if (k < a.Dp) {
-          __nv_bfloat16 h, l;
-          split_bf16(v[u][j], h, l);
-          hi[(long long)i * a.Dp + k] = h;
-          lo[(long long)i * a.Dp + k] = l;
-        }
-      }
     }
   }
   if (!ref) return;  // uniform across the block

@@ -125,6 +125,26 @@ def test_knn_fused_strided_and_unaligned_rows(cuda, D, pad, shift):
     assert s2.device_status() == 0
 
 
+@pytest.mark.parametrize("Q,R,D,k,pad", [(300, 1000, 129, 16, 0), (129, 257, 136, 5, 3), (64, 4096, 300, 32, 1),
+                                          (1, 3, 192, 3, 0), (4096, 40000, 256, 16, 0), (9000, 20000, 193, 8, 2)])
+def test_knn_wide_matches_materialised(cuda, Q, R, D, k, pad):
+    """D > 128, queries streamed with the references: the materialised path's bits
+    (last K panels of 1 to 64 elements, pitched rows, one query, several waves, the
+    half-length lists and the pilot chunk)."""
+    q, r = datagen.point_cloud(Q, R, D, seed=Q + D, dup_frac=0.05)
+    qb = torch.zeros((Q, D + pad), dtype=torch.float32, device=cuda)
+    rb = torch.zeros((R, D + pad), dtype=torch.float32, device=cuda)
+    qb[:, pad:] = torch.from_numpy(q).to(cuda)
+    rb[:, pad:] = torch.from_numpy(r).to(cuda)
+    d1, i1 = s2.knn(qb[:, pad:], rb[:, pad:], k)
+    d2, i2 = s2.knn(qb[:, pad:], rb[:, pad:], k, mode="materialised")
+    assert torch.equal(i1, i2)
+    assert torch.equal(d1.view(torch.int32), d2.view(torch.int32))
+    if Q <= 300:
+        check(q, r, k, d1.cpu().numpy(), i1.cpu().numpy())
+    assert s2.device_status() == 0
+
+
 def test_knn_fused_rejects_wide_points(cuda):
     q = torch.zeros(4, 200, device=cuda)
     with pytest.raises(s2.Simd2Error):
