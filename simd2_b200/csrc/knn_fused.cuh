@@ -413,6 +413,41 @@ __global__ void __launch_bounds__(kKfThreads, 1)
       float thr = fminf(bd[K - 1], prior);
       float lim = fmaxf(thr, blim);
       const uint32_t taddr = tmem + acc * kKfBN + half * 128 + ((uint32_t)(quad * 32) << 16);
+      if (K <= 16 && t == 0 && __any_sync(0xffffffffu, row_ok && prior == inf)) {
+        // A first bound: the largest of the minima of K groups of this half's columns
+        // (K pairs of this list lie at or below it).  Without one the first 32
+        // columns of a list all pass the compare, half of the insertions of a unit
+        // of one tile (a call, us: 64 x 256 x 2, k = 1 37.5 / 33.4, 1000 x 4000 x 16,
+        // k = 8 37.0 / 33.1, 1000 x 4000 x 200, k = 8 61.9 / 55.7; with K = 32 nearly
+        // all would pass still).  A pair inside the band may change: it is no evidence.
+        float g[K];
+#pragma unroll
+        for (int u = 0; u < K; u++) g[u] = inf;
+#pragma unroll 1
+        for (int c = 0; c < 4; c++) {
+          uint32_t r[32];
+          tmem_ld32(taddr + c * 32, r);
+          const float4* nb4 = reinterpret_cast<const float4*>(sN + half * 128 + c * 32);
+#pragma unroll
+          for (int q4 = 0; q4 < 8; q4++) {
+            const float4 nb = nb4[q4];
+            const float n4[4] = {nb.x, nb.y, nb.z, nb.w};
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+              const float v = __fmaf_rn(-2.0f, __uint_as_float(r[q4 * 4 + e]), __fadd_rn(na, n4[e]));
+              g[(q4 * 4 + e) % K] = fminf(g[(q4 * 4 + e) % K], v < blim ? inf : v);
+            }
+          }
+        }
+        float top = g[0];
+#pragma unroll
+        for (int u = 1; u < K; u++) top = fmaxf(top, g[u]);
+        if (top < inf) {  // >= blim >= 0: the next float up, since the compares are strict
+          prior = fminf(prior, __uint_as_float(__float_as_uint(top) + 1));
+          thr = prior;
+          lim = fmaxf(thr, blim);
+        }
+      }
 #pragma unroll 1
       for (int c2 = 0; c2 < 2; c2++) {
         // 64 columns per TMEM round trip (tcgen05.ld .x64, one wait)

@@ -125,6 +125,29 @@ def test_knn_fused_strided_and_unaligned_rows(cuda, D, pad, shift):
     assert s2.device_status() == 0
 
 
+@pytest.mark.parametrize("k", [1, 4, 8, 12, 16])
+@pytest.mark.parametrize("spread", ["equal", "zero", "band", "mixed"])
+def test_knn_first_bound(cuda, k, spread):
+    """The bound a list without one takes from its first tile: every distance equal,
+    every distance zero, every pair inside the cancellation band, and some of each."""
+    g = torch.Generator(device="cpu").manual_seed(k)
+    base = torch.randn((1, 24), generator=g)
+    r = base.repeat(700, 1)
+    q = base.repeat(130, 1)
+    if spread == "equal":
+        q = q + 3.0
+    elif spread == "band":
+        r = r + 0.01 * torch.randn(r.shape, generator=g)
+    elif spread == "mixed":
+        r[::3] = torch.randn(r[::3].shape, generator=g)
+        r[1::7] += 0.01 * torch.randn(r[1::7].shape, generator=g)
+    q, r = q.to(cuda), r.to(cuda)
+    d1, i1 = s2.knn(q, r, k)
+    d2, i2 = s2.knn(q, r, k, mode="materialised")
+    assert torch.equal(i1, i2)
+    assert torch.equal(d1.view(torch.int32), d2.view(torch.int32))
+
+
 @pytest.mark.parametrize("Q,R,D,k,pad", [(300, 1000, 129, 16, 0), (129, 257, 136, 5, 3), (64, 4096, 300, 32, 1),
                                           (1, 3, 192, 3, 0), (4096, 40000, 256, 16, 0), (9000, 20000, 193, 8, 2)])
 def test_knn_wide_matches_materialised(cuda, Q, R, D, k, pad):
