@@ -263,7 +263,9 @@ __global__ void __launch_bounds__(256) transpose_fp4_kernel(const T* __restrict_
                                                             uint8_t* __restrict__ b4, int Kp,
                                                             uint8_t* __restrict__ a4, int Np,
                                                             const uint8_t* __restrict__ chg_row,
-                                                            const uint8_t* __restrict__ chg_col, int BN) {
+                                                            const uint8_t* __restrict__ chg_col, int BN,
+                                                            const int* gate) {
+  if (gate && *gate == 0) return;
   __shared__ __align__(16) uint32_t tile[256 * 32 + 8 * 4];
   const int t = threadIdx.x;
   const int k0 = blockIdx.y * 256, j0 = blockIdx.x * 128;

@@ -20,7 +20,7 @@
 //                    cancellation band (small distance relative to the norms).
 //
 // Persistent: one CTA per SM walks the 128 x 256 tiles of D (grouped raster)
-// with 6 warps:
+// with 10 warps:
 //   warp 0 lane 0  -- TMA producer (2D tiled loads, no multicast, 128-byte
 //                     swizzled rows) over every k-tile of every tile, one ring
 //                     of stages,
@@ -250,6 +250,7 @@ struct TcEpilogue {
   float band;           // recompute when dist < band * (|a|^2 + |b|^2)
   int b_rows;           // 1: B32 holds B transposed ([N][K], e.g. k-NN reference points)
   int* changed;         // or_and closure: set to 1 when any D differs from C
+  const int* gate;      // nullable: the launch does nothing when it is 0 (a closure past its fixed point)
   // Delta steps of the or_and closure (tc_gemm2_kernel only): chg_row[i] /
   // chg_col[j] receive a 1 when an element of 256-row tile row i / 256-column
   // tile column j changed; with need_row / need_col (the previous step's maps)
@@ -606,6 +607,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__ CUtensorMap tmA1,
                    const __grid_constant__ CUtensorMap tmB0, const __grid_constant__ CUtensorMap tmB1, int M, int N,
                    int K, TcEpilogue ep, int tiles_m, int tiles_n, int bn) {
+  if (ep.gate && *ep.gate == 0) return;
   using Cfg = TcCfg<KIND>;
   const int S = tc_stages_of<KIND, BT>(bn);
   const int stage_bytes = tc_stage_of<KIND, BT>(bn);

@@ -8,7 +8,7 @@
 // instead of 128 + 256 (tc_gemm.cuh), a third less shared-memory and L2
 // traffic per MMA.
 //
-// Roles (both CTAs run 6 warps):
+// Roles (both CTAs run 10 warps):
 //   warp 0 lane 0 -- TMA producer of this CTA's halves (no multicast).  The
 //                    transaction bytes of both CTAs complete on the even
 //                    CTA's stage barrier (cp.async.bulk.tensor .cta_group::2),
@@ -116,6 +116,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                     const __grid_constant__ CUtensorMap tmB0, const __grid_constant__ CUtensorMap tmB1,
                     const __grid_constant__ CUtensorMap tmBh, int M, int N, int K, TcEpilogue ep, int tiles_m,
                     int tiles_n) {
+  if (ep.gate && *ep.gate == 0) return;  // both CTAs of a pair
   using Cfg = TcCfg<KIND>;
   constexpr int S = tc2_stages<KIND>();
   constexpr int BN = tc_bn<KIND>();

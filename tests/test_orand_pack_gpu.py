@@ -49,3 +49,30 @@ def test_closure_delta_steps(cuda, n, tail):
     got = x.clone()
     it = s2.closure("or_and", got)
     assert torch.equal(got, want) and it == steps
+
+
+@pytest.mark.parametrize("max_iter", [3, 8, 9, 500])
+@pytest.mark.parametrize("n,ld,shift", [(1, 1, 0), (150, 150, 0), (700, 707, 3), (2100, 2112, 1)])
+def test_closure_in_place_and_chunked(cuda, n, ld, shift, max_iter):
+    """or_and closures squared in place, their steps enqueued in chunks of eight: a
+    chain takes more steps than a chunk holds; the step limit inside, at and past a
+    chunk's end; pitched and unaligned rows, single-SM and SM-pair kernel."""
+    buf = torch.full((n * ld + 16,), 7, dtype=torch.uint8, device=cuda)
+    X = buf[shift:shift + n * ld].view(n, ld)[:, :n]
+    X.zero_()
+    i = torch.arange(n - 1, device=cuda)
+    X[i, i + 1] = 1
+    want, steps, changed = X.float(), 0, True
+    while changed and steps < max_iter:
+        nxt = torch.maximum(want, (want @ want > 0).float())
+        changed = not torch.equal(nxt, want)
+        want, steps = nxt, steps + 1
+    if changed:
+        with pytest.raises(s2.Simd2Error):
+            s2.closure("or_and", X, max_iter=max_iter)
+    else:
+        assert s2.closure("or_and", X, max_iter=max_iter) == steps
+    assert torch.equal(X, want.to(torch.uint8))
+    pad = buf[shift:shift + n * ld].view(n, ld)[:, n:]
+    assert bool((pad == 7).all()) and bool((buf[shift + n * ld:] == 7).all())
+    assert s2.device_status() == 0
