@@ -204,7 +204,19 @@ def run_reference_arm(args):
 # --------------------------------------------------------------------------
 # GPU arm
 # --------------------------------------------------------------------------
-def traffic_from_profile(key="srgemm_simt_kernel min_plus 4096^3"):
+# Dispatch slots (lane-cycles) per (x),(+) pair of the CUDA-core kernels on the sweep's
+# values: on 16-bit codes an add-min takes one, a selection three instructions of two
+# per four pairs; FP32 products (no codes) a packed multiply and a three-operand min,
+# two each for two pairs.
+SLOTS_PER_PAIR = {"min_plus": 1.0, "max_plus": 1.0, "max_min": 1.5, "min_max": 1.5, "max_mul": 2.0, "min_mul": 2.0}
+
+
+def issue_peak_gops(op, sm_max):
+    """Dispatch bound of one CUDA-core semiring, two operations a pair."""
+    return SMS * LANES * sm_max * 1e6 / 1e9 * 2.0 / SLOTS_PER_PAIR[op]
+
+
+def traffic_from_profile(key="srgemm_sk_kernel min_plus 4096^3"):
     """DRAM bytes per launch of a kernel, from the byte counts kept beside the
     ncu summaries (profiles/dram_traffic.json)."""
     try:
@@ -369,12 +381,12 @@ def min_plus_8192(dev, reps=3):
     kms /= max(launches, 1)
     peaks, kind = measured_peaks()
     sm_max = float(peaks.get("sm_max_mhz", 1965.0))
-    peak = SMS * LANES * sm_max * 1e6 / 1e9
+    peak = issue_peak_gops("min_plus", sm_max)
     gops = 2.0 * n ** 3 / kms / 1e6
     del A, B, C, D
     return {"kernel_ms": kms, "call_ms": ev0.elapsed_time(ev1) / reps, "gops": gops, "peak_gops": peak,
-            "frac": gops / peak, "peak_source": f"{SMS} SMs x {LANES} lanes x {sm_max:.0f} MHz ({kind} sm_max_mhz)",
-            "how": f"srgemm_simt_kernel, {reps} launches with C; kernel time from CUDA events on the launching stream"}
+            "frac": gops / peak, "peak_source": f"{SMS} SMs x {LANES} pairs x {sm_max:.0f} MHz ({kind} sm_max_mhz)",
+            "how": f"srgemm_sk_kernel on 16-bit codes, {reps} launches with C; kernel time from CUDA events on the launching stream"}
 
 
 def learned_dispatch_mixed(dev, params, weights_path, count=64):
@@ -923,20 +935,22 @@ def main():
     clocks = clk.summary()
     peaks, peak_kind = measured_peaks()
     sm_max = float(peaks.get("sm_max_mhz", 1965.0))
-    issue_peak_gops = SMS * LANES * sm_max * 1e6 / 1e9  # 2 ops/MAC == 2 lane-instructions/MAC
+    # the six semirings do the same number of pairs: the harmonic mean of their bounds
+    simt_run = [op for op in SLOTS_PER_PAIR if op in args.ops.split(",")] or list(SLOTS_PER_PAIR)
+    simt_peak = len(simt_run) / sum(1.0 / issue_peak_gops(op, sm_max) for op in simt_run)
     simt_ms, simt_n, simt_ops = kt.by_kind["simt"]
     tc_ms, tc_n, tc_ops = kt.by_kind["tensor"]
     achieved = simt_ops / (simt_ms / 1e3) / 1e9 if simt_ms > 0 else None
     traffic = traffic_from_profile()
     # tensor-core family: plus_mul / minus_square issue 3 BF16 MMAs per product term
-    # (hi*hi, hi*lo, lo*hi), or_and one INT8 MMA at twice the BF16 rate; both are
+    # (hi*hi, hi*lo, lo*hi), or_and one FP4 MMA at four times the BF16 rate; both are
     # expressed as BF16-equivalent FLOP/s against the measured cuBLAS BF16 peak.
     tc_equiv = 0.0
     for op in SWEEP_OPS:
         if op in ("plus_mul", "minus_square"):
             tc_equiv += 3 * 2.0 * n ** 3 * args.steps
         elif op == "or_and":
-            tc_equiv += 0.5 * 2.0 * n ** 3 * args.steps
+            tc_equiv += 0.25 * 2.0 * n ** 3 * args.steps
     bf16_peak = float(peaks.get("bf16_tflops", 1590.0))
 
     cpu = None
@@ -972,11 +986,11 @@ def main():
                                               "rel over entries >= the rms, normwise, and max |err| / sum of |terms|; "
                                               "min/max semirings and or_and are bit-exact (tests)"),
             "roofline": {"bound": "cuda_core_issue",
-                         "kernel": "srgemm_simt_kernel (min_plus, max_plus, max_min, max_mul, min_mul, min_max)",
-                         "achieved": achieved, "peak": issue_peak_gops, "unit": "Gop/s",
-                         "frac": achieved / issue_peak_gops if achieved else None, "traffic": traffic,
+                         "kernel": "srgemm_sk_kernel (min_plus, max_plus, max_min, max_mul, min_mul, min_max)",
+                         "achieved": achieved, "peak": simt_peak, "unit": "Gop/s",
+                         "frac": achieved / simt_peak if achieved else None, "traffic": traffic,
                          "peak_source": f"{SMS} SMs x {LANES} lanes x {sm_max:.0f} MHz ({peak_kind} sm_max_mhz); "
-                                        "2 ops per (x),(+) pair = 2 lane-instructions",
+                                        "2 ops per (x),(+) pair; dispatch slots per pair: " + json.dumps(SLOTS_PER_PAIR),
                          "share_of_kernel_time": simt_ms / (simt_ms + tc_ms) if simt_ms + tc_ms > 0 else None,
                          "timed_launches": simt_n},
             "roofline_tensor": {"bound": "tensor", "kernel": "tc_gemm2_kernel on SM pairs (plus_mul, minus_square, or_and)",
