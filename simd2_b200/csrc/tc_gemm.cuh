@@ -312,7 +312,9 @@ __device__ __forceinline__ void tc_or_bits(uint32_t trow, uint32_t* buf, int lan
 // Writes the parked flags | C.  A row's columns go to the warp's lanes in order,
 // four to a lane where D's (and C's) rows allow a word of bytes or an int4 --
 // each instruction then covers 128 columns of one row -- else one to a lane;
-// C is loaded for 4 rows before any of it is used.  (With a lane per row, every
+// C is loaded for 8 rows before any of it is used: the loads' latency bounds a
+// product of short k (3000 x 2500 x 2000 int32 call with C, 4 rows / 8: 55.9 / 52.4 us;
+// a 1000-vertex closure 231 / 213).  (With a lane per row, every
 // store of unaligned rows touched 32 rows: the 3000^3 kernel on bytes 184 us, now 39.)
 template <typename T>
 __device__ __forceinline__ void tc_or_store(const TcEpilogue& ep, int M, int N, int n0, int row0, const uint32_t* buf,
@@ -322,6 +324,7 @@ __device__ __forceinline__ void tc_or_store(const TcEpilogue& ep, int M, int N, 
   const bool epi = ep.do_epilogue != 0;
   const int rows = min(32, M - row0);
   constexpr int kVec = sizeof(T) == 1 ? 4 : 16;  // bytes of 4 elements
+  constexpr int R = 8;  // rows of C in flight
   const bool vec = (n0 + ncols <= N) && ((ep.ldd * (long long)sizeof(T)) % kVec == 0) &&
                    ((reinterpret_cast<uintptr_t>(D) + (size_t)n0 * sizeof(T)) % kVec == 0) &&
                    (!epi || (((ep.ldc * (long long)sizeof(T)) % kVec == 0) &&
@@ -331,13 +334,13 @@ __device__ __forceinline__ void tc_or_store(const TcEpilogue& ep, int M, int N, 
 #pragma unroll 1
     for (int c = lane * 4; c < ncols; c += 128) {
 #pragma unroll 1
-      for (int r0 = 0; r0 < rows; r0 += 4) {
-        V old[4];
+      for (int r0 = 0; r0 < rows; r0 += R) {
+        V old[R];
 #pragma unroll
-        for (int q = 0; q < 4; q++)
+        for (int q = 0; q < R; q++)
           if (epi && r0 + q < rows) old[q] = *reinterpret_cast<const V*>(C + (row0 + r0 + q) * ep.ldc + n0 + c);
 #pragma unroll
-        for (int q = 0; q < 4; q++) {
+        for (int q = 0; q < R; q++) {
           if (r0 + q >= rows) break;
           const uint32_t nib = (buf[(r0 + q) * kOrPitch + (c >> 5)] >> (c & 31)) & 15u;
           V* dst = reinterpret_cast<V*>(D + (row0 + r0 + q) * ep.ldd + n0 + c);
@@ -366,13 +369,13 @@ __device__ __forceinline__ void tc_or_store(const TcEpilogue& ep, int M, int N, 
 #pragma unroll 1
     for (int c = lane; c < ncols && n0 + c < N; c += 32) {
 #pragma unroll 1
-      for (int r0 = 0; r0 < rows; r0 += 4) {
-        T old[4];
+      for (int r0 = 0; r0 < rows; r0 += R) {
+        T old[R];
 #pragma unroll
-        for (int q = 0; q < 4; q++)
+        for (int q = 0; q < R; q++)
           if (epi && r0 + q < rows) old[q] = C[(row0 + r0 + q) * ep.ldc + n0 + c];
 #pragma unroll
-        for (int q = 0; q < 4; q++) {
+        for (int q = 0; q < R; q++) {
           if (r0 + q >= rows) break;
           uint32_t v = (buf[(r0 + q) * kOrPitch + (c >> 5)] >> (c & 31)) & 1u;
           if (epi) {
