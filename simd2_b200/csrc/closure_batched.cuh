@@ -433,7 +433,9 @@ __global__ void __launch_bounds__(kSimtThreads, 1) closure_batched_kernel(BatchA
   // tile claimed ahead runs first, and may end another such graph: two at most)
   __shared__ BatchTask s_own[2];
   __shared__ int s_nown;
-  __shared__ BatchTask s_opened;  // the step this CTA opened (graph -1: none)
+  // The step this CTA opened (graph -1: none).  All threads read it after an
+  // iteration's last barrier, so it is written only past the next one's first.
+  __shared__ BatchTask s_opened;
   __shared__ unsigned s_first;    // its first slot
   BatchCta x;
   x.smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -462,11 +464,12 @@ __global__ void __launch_bounds__(kSimtThreads, 1) closure_batched_kernel(BatchA
       else if (s_nown > 0) s_task = s_own[--s_nown];
       else batch_pop(a, slot, s_task);
       s_next.graph = -1;
-      s_opened.graph = -1;
     }
     __syncthreads();
     const BatchTask task = s_task;
     if (task.graph < 0) break;
+    // every thread has passed the barrier above, so none still publishes the step before
+    if (threadIdx.x == 0) s_opened.graph = -1;
     fence_proxy_async_global();  // the acquire that claimed the task, before its TMA reads
     BatchGraph& G = a.graphs[task.graph];
     const BatchMaps* mp = a.maps + task.graph;

@@ -45,6 +45,32 @@ def test_mixed_sizes(cuda, op):
     check(op, graphs)
 
 
+def test_steps_of_more_tiles_than_threads(cuda):
+    """A step of 576 tiles is published by every warp of the CTA that opens it, in
+    two rounds; beside it steps of 36 tiles (two warps).  A disjoint union of small
+    graphs, so the oracle closes it by parts."""
+    part, parts = 48, 63
+    n = part * parts
+    graphs = [datagen.er_graph(part, 0.06, seed=i) for i in range(parts)]
+    x = np.full((n, n), np.inf, np.float32)
+    want = x.copy()
+    steps = 0
+    for i, g in enumerate(graphs):
+        w, it = oracle.closure("min_plus", g)
+        x[i * part:(i + 1) * part, i * part:(i + 1) * part] = g
+        want[i * part:(i + 1) * part, i * part:(i + 1) * part] = w
+        steps = max(steps, it)
+    mid = datagen.er_graph(700, 0.02, seed=9)
+    want_mid, it_mid = oracle.closure("min_plus", mid)
+    for _ in range(3):
+        mats = [torch.from_numpy(g.copy()).cuda() for g in (x, mid, mid)]
+        assert list(s2.closure_batched("min_plus", mats)) == [steps, it_mid, it_mid]
+        same(mats[0], want)
+        same(mats[1], want_mid)
+        same(mats[2], want_mid)
+    assert s2.device_status() == 0
+
+
 @pytest.mark.parametrize("n", [100, 300])
 def test_outgrows_codes(cuda, n):
     """A path of heavy edges: distances pass 16383 in the second squaring, so the
