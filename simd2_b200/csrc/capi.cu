@@ -2832,6 +2832,8 @@ int simd2_batched_plan_create(simd2_op op, int count, float* const* X, const int
   int nbig = 0;
   long long tasks = 0;
   while (nbig < count && n[order[nbig]] > kBM && count <= kBatchSlotMax && n[order[nbig]] <= 1000 * kBM) nbig++;
+  int nalone = count - nbig;
+  while (nalone > 0 && n[order[nbig + nalone - 1]] == 0) nalone--;
   // room for kBatchSlotSteps steps of every shared graph; when the slots are
   // used up a graph is finished by the CTA that had its last tile
   std::vector<unsigned long long> first;
@@ -2888,6 +2890,7 @@ int simd2_batched_plan_create(simd2_op op, int count, float* const* X, const int
   auto* d_order = reinterpret_cast<int*>(base + o_off);
   A.order = d_order;
   A.nbig = nbig;
+  A.nalone = nalone;
   A.count = count;
   A.state = reinterpret_cast<BatchState*>(base + s_off);
   A.ctl = reinterpret_cast<BatchCtl*>(base + c_off);

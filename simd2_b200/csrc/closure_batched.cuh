@@ -82,8 +82,10 @@ struct BatchCtl {
 struct BatchArgs {
   BatchGraph* graphs;
   const BatchMaps* maps;
-  const int* order;   // nbig graphs shared by tiles, then those that one CTA closes alone
-  int nbig, count;
+  // nbig graphs shared by tiles, then nalone that one CTA closes alone, then the
+  // empty ones, which have no tile and are done once the prep kernel has run
+  const int* order;
+  int nbig, nalone, count;
   BatchState* state;
   BatchCtl* ctl;
   // One slot per tile of every opened step, in the order of opening: the first
@@ -176,9 +178,9 @@ __device__ __forceinline__ void batch_pop(const BatchArgs& a, unsigned& slot, Ba
       const unsigned lost = *(volatile unsigned*)&a.ctl->lost;
       if (slot >= a.cap || (lost && slot >= 0x80000000u - lost)) slot = kNoSlot;  // will never be written
     }
-    if (slot == kNoSlot && *(volatile int*)&a.ctl->alone_next < a.count - a.nbig) {
+    if (slot == kNoSlot && *(volatile int*)&a.ctl->alone_next < a.nalone) {
       const int q = atomicAdd(&a.ctl->alone_next, 1);
-      if (q < a.count - a.nbig) {
+      if (q < a.nalone) {
         t.graph = a.order[a.nbig + q];
         t.n = a.graphs[t.graph].n;
         t.tile = 0;
@@ -599,8 +601,8 @@ __global__ void __launch_bounds__(256) batched_prep_kernel(BatchArgs a) {
   for (int g = blockIdx.y; g < a.count; g += gridDim.y) {
     BatchGraph& G = a.graphs[g];
     if (blockIdx.x == 0 && threadIdx.x == 0) {
-      G.iters = 0;
-      G.changed = 1;
+      G.iters = G.n == 0;  // an empty graph is done in one unchanged step
+      G.changed = G.n != 0;
       G.coded = -1;
     }
     if constexpr (Code16<OP>::kHas) {

@@ -71,6 +71,33 @@ def test_steps_of_more_tiles_than_threads(cuda):
     assert s2.device_status() == 0
 
 
+@pytest.mark.parametrize("op", ["min_plus", "max_min", "max_mul"])
+@pytest.mark.parametrize("sizes", [(0,), (0, 0, 0), (0, 40, 0, 300, 128, 0)])
+def test_empty_graphs(cuda, op, sizes):
+    """A graph without vertices takes one unchanged step and no tile."""
+    graphs = []
+    for i, n in enumerate(sizes):
+        x = datagen.closure_graph("max_min" if op == "max_min" else "min_plus", max(n, 1), 0.1, seed=i)[:n, :n]
+        if op == "max_mul":  # weights in (0, 1], no edge 0
+            x = np.where(np.isinf(x), np.float32(0.0), 1.0 / (1.0 + x)).astype(np.float32)
+        graphs.append(np.ascontiguousarray(x))
+    mats = [torch.from_numpy(g.copy()).cuda() for g in graphs]
+    plan = s2.BatchedClosure(op, mats)
+    for _ in range(2):
+        for g, m in zip(graphs, mats):
+            m.copy_(torch.from_numpy(g))
+        plan.run()
+        torch.cuda.synchronize()
+        its, not_converged = plan.iters()
+        assert not_converged == 0
+        for g, m, it in zip(graphs, mats, its):
+            want, want_it = oracle.closure(op, g) if g.shape[0] else (g, 1)
+            assert it == want_it
+            same(m, want)
+    plan.close()
+    assert s2.device_status() == 0
+
+
 @pytest.mark.parametrize("n", [100, 300])
 def test_outgrows_codes(cuda, n):
     """A path of heavy edges: distances pass 16383 in the second squaring, so the
