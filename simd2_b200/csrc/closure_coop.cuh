@@ -25,6 +25,7 @@ struct CoopCtl {
   unsigned bar;      // arrivals at the grid barrier
   int last_changed;  // 1 + the last step that changed something
   int over_neg;      // 0, or 2^30 - t for the first step t whose result has no code (t = -1: an entry)
+                     // compared with the reader's step: a faster CTA may have raised it for the next one
 };
 
 struct CoopArgs {
@@ -140,7 +141,7 @@ __global__ void __launch_bounds__(kSimtThreads, 1)
   coop_barrier(g.ctl, (unsigned)G, failed);
 
   int outcome = 0, it = 0;
-  if (*(volatile int*)&g.ctl->over_neg) outcome = 3;
+  if (*(volatile int*)&g.ctl->over_neg > 1 << 30) outcome = 3;  // an entry; 2^30 is step 0's
   uint32_t base = 0;  // loads of the steps before
   while (!outcome && !*failed) {
     const int cur = it & 1;

@@ -53,6 +53,26 @@ def test_without_codes(cuda, case):
     same(X, want, case)
 
 
+@pytest.mark.parametrize("op", ["min_plus", "max_plus"])
+@pytest.mark.parametrize("n", [90, 200, 500, 1100])
+def test_first_squaring_outgrows_codes(cuda, op, n):
+    """Sums of two entries already have no code, found by CTAs that leave the grid
+    barrier of the coding pass at different times; on one tile and on many."""
+    x = np.full((n, n), np.inf if op == "min_plus" else -np.inf, np.float32)
+    np.fill_diagonal(x, 0.0)
+    for i in range(0, n - 1, 3):  # paths of three vertices
+        x[i, i + 1] = 9000.0 + i
+        if i + 2 < n:
+            x[i + 1, i + 2] = 8200.0 + i
+    want, steps = oracle.closure(op, x)
+    assert np.isfinite(want).sum() > np.isfinite(x).sum()
+    for _ in range(10):
+        X = torch.from_numpy(x.copy()).cuda()
+        assert s2.closure(op, X) == steps
+        same(X, want, f"{op} {n}")
+    assert s2.device_status() == 0
+
+
 @pytest.mark.parametrize("op", ["min_plus", "max_min"])
 @pytest.mark.parametrize("steps", [1, 2, 3])
 def test_step_limit(cuda, op, steps):
