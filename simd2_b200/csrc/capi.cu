@@ -1416,7 +1416,7 @@ int closure_coop(int op, int n, float* X, long long ldx, int max_iter, int conv,
   HostBlock host;
   if (!host.p) return SIMD2_ERR_ALLOC;
   a.out = static_cast<volatile int*>(host.p);
-  a.out[0] = a.out[1] = 0;
+  a.out[0] = a.out[1] = a.out[2] = 0;
   SIMD2_CUDA_TRY(cudaMemsetAsync(ws + ctl_off, 0, off - ctl_off, stream));
   switch (op) {
     case SIMD2_MIN_PLUS: rc = launch_coop<SIMD2_MIN_PLUS>(m, a, grid, stream); break;
@@ -1428,8 +1428,8 @@ int closure_coop(int op, int n, float* X, long long ldx, int max_iter, int conv,
   if (rc) return rc == SIMD2_ERR_UNSUPPORTED ? SIMD2_OK : rc;  // the launch-per-step path takes over
   SIMD2_CUDA_TRY(cudaStreamSynchronize(stream));
   const int iters = a.out[0], outcome = a.out[1];
+  if (a.out[2] || outcome == 0) return SIMD2_ERR_TIMEOUT;  // a bounded wait ran out in some CTA
   if (outcome == 3) return SIMD2_OK;
-  if (outcome == 0) return SIMD2_ERR_TIMEOUT;  // a bounded wait ran out
   *done = true;
   if (iters_out) *iters_out = iters;
   return outcome == 1 ? SIMD2_OK : SIMD2_ERR_NOT_CONVERGED;

@@ -26,6 +26,7 @@ struct CoopCtl {
   int last_changed;  // 1 + the last step that changed something
   int over_neg;      // 0, or 2^30 - t for the first step t whose result has no code (t = -1: an entry)
                      // compared with the reader's step: a faster CTA may have raised it for the next one
+  int failed;        // set by a CTA in which a bounded wait ran out
 };
 
 struct CoopArgs {
@@ -40,15 +41,21 @@ struct CoopArgs {
   int* counters;      // arrivals per split tile, over all steps
   uint4* part;        // two slots of 64 x 64 codes per CTA
   CoopCtl* ctl;
-  volatile int* out;  // host memory: steps, and 1 converged, 2 not converged, 3 no codes (X untouched)
+  volatile int* out;  // host memory: steps, and 1 converged, 2 not converged, 3 no codes (X untouched); 1 when a CTA failed
 };
 
-// All CTAs of the grid; `target` arrivals in total.
+// All CTAs of the grid; `target` arrivals in total.  A CTA in which a wait ran out
+// has folded or written wrong codes: it says so before it arrives, and every CTA
+// leaves the barrier with *failed set.
 __device__ __forceinline__ void coop_barrier(CoopCtl* ctl, unsigned target, volatile int* failed) {
   fence_proxy_async_global();
   __threadfence();
   __syncthreads();
   if (threadIdx.x == 0) {
+    if (*failed) {
+      atomicExch(&ctl->failed, 1);
+      __threadfence();
+    }
     atomicAdd(&ctl->bar, 1u);
     const uint64_t t0 = globaltimer_ns();
     while ((unsigned)ld_acquire(reinterpret_cast<const int*>(&ctl->bar)) < target) {
@@ -58,6 +65,7 @@ __device__ __forceinline__ void coop_barrier(CoopCtl* ctl, unsigned target, vola
         break;
       }
     }
+    if (*(volatile int*)&ctl->failed) *failed = 1;
   }
   __syncthreads();
   fence_proxy_async_global();
@@ -276,9 +284,12 @@ __global__ void __launch_bounds__(kSimtThreads, 1)
     else if (it >= g.max_iter) outcome = 2;
   }
   if (*failed) {
-    if (threadIdx.x == 0)
+    // this CTA's share of X is not written, whatever the others decided
+    if (threadIdx.x == 0) {
+      g.out[2] = 1;
       for (int s = 0; s < S; s++)
         for (int p = 0; p < 2; p++) mbar_wait(&full[s], p, 1000000ull);
+    }
     return;
   }
   if (outcome != 3) {  // X from its codes

@@ -2,6 +2,9 @@
 bit for bit: sizes around the 64-wide tiles and the split of tiles between CTAs,
 entries and results without a 16-bit code (the launch-per-step path takes over),
 the step limit, the change tests, and rows with a pitch."""
+import os
+import subprocess
+
 import numpy as np
 import pytest
 import torch
@@ -96,3 +99,16 @@ def test_tolerance_change_test(cuda, op):
     X = torch.from_numpy(x.copy()).cuda()
     assert s2.closure(op, X, conv="tol") == steps
     same(X, want)
+
+
+def test_failed_wait_reaches_every_cta(cuda, tmp_path):
+    """A CTA whose bounded wait ran out may not leave the others to finish on its
+    data: after the grid barrier all of them know."""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    exe = tmp_path / "coop_barrier"
+    res = subprocess.run(["nvcc", "-gencode", "arch=compute_100a,code=sm_100a", "-std=c++17", "-O1",
+                          os.path.join(root, "tests", "device", "coop_barrier.cu"), "-o", str(exe)],
+                         capture_output=True, text=True)
+    assert res.returncode == 0, res.stderr
+    res = subprocess.run([str(exe)], capture_output=True, text=True, timeout=120)
+    assert res.returncode == 0, (res.returncode, res.stdout)
