@@ -119,7 +119,8 @@ struct SelectCode16 {
   static constexpr bool kHas = true;
   __device__ static uint32_t encode(float x, bool& bad) {
     const __half h = __float2half_rn(x);
-    bad |= __float_as_uint(__half2float(h)) != __float_as_uint(x);  // NaN included
+    // a NaN whose bits survive the trip (the half 0x7fff) has no code either
+    bad |= __float_as_uint(__half2float(h)) != __float_as_uint(x) || x != x;
     return code(__half_as_ushort(h));
   }
   __device__ static uint32_t code(uint32_t u) { return u ^ ((u & 0x8000u) ? 0x7fffu : 0u); }

@@ -58,3 +58,24 @@ def test_f16_entry_all_opcodes(cuda, op, shape):
             err = np.abs(got.astype(np.float64) - want)
             assert np.all(err <= (4 * 2.0 ** -16 + 2 * k * 2.0 ** -24) * S + 1e-30), (op, shape, epi, err.max())
     assert s2.device_status() == 0
+
+
+@pytest.mark.parametrize("op", ["max_min", "min_max"])
+@pytest.mark.parametrize("half", [True, False])
+@pytest.mark.parametrize("n", [48, 600])
+@pytest.mark.parametrize("bits", [0x7FFF, 0x7E00, 0xFFFF])
+def test_nan_entries(cuda, op, half, n, bits):
+    """(x) and (+) return their other operand for a NaN, whichever kernel the size
+    goes to and whatever the NaN's bits: it has no 16-bit code."""
+    rng = np.random.default_rng(n)
+    a, b = (rng.integers(-50, 50, size=(n, n)).astype(np.float16) for _ in range(2))
+    for x in (a, b):
+        x.view(np.uint16)[rng.random((n, n)) < 0.1] = bits
+    A, B = torch.from_numpy(a).cuda(), torch.from_numpy(b).cuda()
+    got = s2.srgemm_f16(op, A, B) if half else s2.srgemm(op, A.float(), B.float())
+    times, plus = (torch.fmin, torch.fmax) if op == "max_min" else (torch.fmax, torch.fmin)
+    want = torch.full((n, n), -np.inf if op == "max_min" else np.inf)
+    for k in range(n):
+        want = plus(want, times(torch.from_numpy(a[:, k:k + 1]).float(), torch.from_numpy(b[k:k + 1]).float()))
+    assert torch.equal(got.cpu(), want)
+    assert s2.device_status() == 0
