@@ -360,7 +360,8 @@ long long simd2_launch_count(void);
 /* Kernel timing: between begin and end, every main srgemm kernel launch is
  * bracketed by CUDA events on its own stream.  end() waits for them and
  * returns the summed kernel time, the number of timed launches and the
- * algorithmic operation count (2*M*N*K per launch). */
+ * algorithmic operation count (2*M*N*K per launch; a small closure that runs
+ * all its steps in one launch counts 2*n^3 for each). */
 int simd2_profile_begin(void);
 int simd2_profile_end(double* kernel_ms, long long* launches, long long* ops);
 /* After simd2_profile_end: the same totals for one kernel family

@@ -78,6 +78,7 @@ std::vector<std::pair<cudaEvent_t, cudaEvent_t>> g_prof_events;
 std::vector<int> g_prof_kind;        // kernel family of each timed launch
 std::vector<long long> g_prof_opsv;  // algorithmic ops of each timed launch
 size_t g_prof_used = 0;
+unsigned g_prof_session = 0;  // counts simd2_profile_begin
 long long g_prof_ops = 0;
 double g_prof_ms[4] = {};
 long long g_prof_n[4] = {}, g_prof_k_ops[4] = {};
@@ -87,8 +88,14 @@ inline void count_launch() { g_launches.fetch_add(1, std::memory_order_relaxed);
 // Kernel families reported separately by simd2_profile_result.
 enum ProfKind { kProfSimt = 0, kProfTensor = 1, kProfBatched = 2 };
 
+// A timed launch whose operations are known only once it has ended.
+struct ProfLater {
+  size_t slot = 0;
+  unsigned session = 0;  // 0: not timed
+};
+
 // Returns the event pair to bracket a main-kernel launch, or nullptr.
-std::pair<cudaEvent_t, cudaEvent_t>* prof_slot(long long ops, int kind = kProfSimt) {
+std::pair<cudaEvent_t, cudaEvent_t>* prof_slot(long long ops, int kind = kProfSimt, ProfLater* later = nullptr) {
   std::lock_guard<std::mutex> lk(g_prof_mu);
   if (!g_prof_on) return nullptr;
   if (g_prof_used == g_prof_events.size()) {
@@ -101,7 +108,15 @@ std::pair<cudaEvent_t, cudaEvent_t>* prof_slot(long long ops, int kind = kProfSi
   g_prof_ops += ops;
   g_prof_kind[g_prof_used] = kind;
   g_prof_opsv[g_prof_used] = ops;
+  if (later) *later = {g_prof_used, g_prof_session};
   return &g_prof_events[g_prof_used++];
+}
+
+void prof_add_ops(const ProfLater& later, long long ops) {
+  std::lock_guard<std::mutex> lk(g_prof_mu);
+  if (!g_prof_on || later.session != g_prof_session) return;
+  g_prof_ops += ops;
+  g_prof_opsv[later.slot] += ops;
 }
 
 // ---------------------------------------------------------------------------
@@ -1339,7 +1354,7 @@ int closure_gated(int op, int n, float* X, long long ldx, int max_iter, int conv
 constexpr int kCoopMaxN = 1536;
 
 template <int OP>
-int launch_coop(const CUtensorMap (&m)[4], CoopArgs& args, int grid, cudaStream_t stream) {
+int launch_coop(const CUtensorMap (&m)[4], CoopArgs& args, int grid, ProfLater* later, cudaStream_t stream) {
   auto kern = closure_coop_kernel<OP>;
   static bool configured[64] = {};
   int dev = 0;
@@ -1359,7 +1374,10 @@ int launch_coop(const CUtensorMap (&m)[4], CoopArgs& args, int grid, cudaStream_
   attr[0].val.cooperative = 1;
   lc.attrs = attr;
   lc.numAttrs = 1;
+  auto* ev = prof_slot(0, kProfSimt, later);
+  if (ev) cudaEventRecord(ev->first, stream);
   const cudaError_t e = cudaLaunchKernelEx(&lc, kern, m[0], m[1], m[2], m[3], args);
+  if (ev) cudaEventRecord(ev->second, stream);
   if (e == cudaErrorCooperativeLaunchTooLarge) {  // fewer SMs than the device reports
     cudaGetLastError();
     return SIMD2_ERR_UNSUPPORTED;
@@ -1418,11 +1436,12 @@ int closure_coop(int op, int n, float* X, long long ldx, int max_iter, int conv,
   a.out = static_cast<volatile int*>(host.p);
   a.out[0] = a.out[1] = a.out[2] = 0;
   SIMD2_CUDA_TRY(cudaMemsetAsync(ws + ctl_off, 0, off - ctl_off, stream));
+  ProfLater later;
   switch (op) {
-    case SIMD2_MIN_PLUS: rc = launch_coop<SIMD2_MIN_PLUS>(m, a, grid, stream); break;
-    case SIMD2_MAX_PLUS: rc = launch_coop<SIMD2_MAX_PLUS>(m, a, grid, stream); break;
-    case SIMD2_MAX_MIN: rc = launch_coop<SIMD2_MAX_MIN>(m, a, grid, stream); break;
-    case SIMD2_MIN_MAX: rc = launch_coop<SIMD2_MIN_MAX>(m, a, grid, stream); break;
+    case SIMD2_MIN_PLUS: rc = launch_coop<SIMD2_MIN_PLUS>(m, a, grid, &later, stream); break;
+    case SIMD2_MAX_PLUS: rc = launch_coop<SIMD2_MAX_PLUS>(m, a, grid, &later, stream); break;
+    case SIMD2_MAX_MIN: rc = launch_coop<SIMD2_MAX_MIN>(m, a, grid, &later, stream); break;
+    case SIMD2_MIN_MAX: rc = launch_coop<SIMD2_MIN_MAX>(m, a, grid, &later, stream); break;
     default: rc = SIMD2_ERR_UNSUPPORTED;
   }
   if (rc) return rc == SIMD2_ERR_UNSUPPORTED ? SIMD2_OK : rc;  // the launch-per-step path takes over
@@ -1430,6 +1449,7 @@ int closure_coop(int op, int n, float* X, long long ldx, int max_iter, int conv,
   const int iters = a.out[0], outcome = a.out[1];
   if (a.out[2] || outcome == 0) return SIMD2_ERR_TIMEOUT;  // a bounded wait ran out in some CTA
   if (outcome == 3) return SIMD2_OK;
+  prof_add_ops(later, 2LL * n * n * n * iters);
   *done = true;
   if (iters_out) *iters_out = iters;
   return outcome == 1 ? SIMD2_OK : SIMD2_ERR_NOT_CONVERGED;
@@ -2733,6 +2753,7 @@ long long simd2_launch_count(void) { return g_launches.load(); }
 int simd2_profile_begin(void) {
   std::lock_guard<std::mutex> lk(g_prof_mu);
   g_prof_on = true;
+  g_prof_session++;
   g_prof_used = 0;
   g_prof_ops = 0;
   for (int k = 0; k < 4; k++) g_prof_ms[k] = 0.0, g_prof_n[k] = 0, g_prof_k_ops[k] = 0;

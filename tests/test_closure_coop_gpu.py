@@ -112,3 +112,19 @@ def test_failed_wait_reaches_every_cta(cuda, tmp_path):
     assert res.returncode == 0, res.stderr
     res = subprocess.run([str(exe)], capture_output=True, text=True, timeout=120)
     assert res.returncode == 0, (res.returncode, res.stdout)
+
+
+def test_profiled(cuda):
+    """The one launch of a small closure is timed, and counts every step's
+    operations; one that falls back adds its discarded launch's time alone."""
+    n = 300
+    x = graph("min_plus", n, 0.03, 7)
+    with s2.KernelTimer() as t:
+        steps = s2.closure("min_plus", torch.from_numpy(x).cuda())
+    assert steps > 1 and t.launches == 1
+    assert t.ops == 2 * n ** 3 * steps
+    assert t.kernel_ms > 0.0
+    assert t.by_kind["simt"][1:] == (1, t.ops)
+    with s2.KernelTimer() as t:
+        steps = s2.closure("min_plus", torch.from_numpy(x + np.float32(0.25)).cuda())
+    assert t.launches > steps and t.ops >= 2 * n ** 3 * steps
