@@ -154,8 +154,7 @@ int simd2_closure_batched(simd2_op op, int count, float* const* X, const int* n,
  * skip = 1 to drop k-blocks whose A or B block
  * holds only the (x)-annihilator (block occupancy computed per call; applies
  * to min_plus, max_plus, max_min, min_max).  All configurations give the same
- * bits.  No reference counterpart: the autotuner and the learned dispatch
- * use it. */
+ * bits.  No reference counterpart: the autotuner times them. */
 int simd2_srgemm_tuned(simd2_op op, int M, int N, int K,
                        const float* A, int lda, const float* B, int ldb,
                        const float* C, int ldc, float* D, int ldd,
@@ -163,11 +162,13 @@ int simd2_srgemm_tuned(simd2_op op, int M, int N, int K,
 
 typedef enum simd2_dispatch {
   SIMD2_DISPATCH_DENSE = 0,   /* no block skipping: the persistent kernel, which spreads each
-                                 step over the SMs by k-tile units (the plain dense path) */
+                                 step over the SMs by k-tile units (the plain dense path), or
+                                 the split factor installed for n (simd2_set_dense_configs) */
   SIMD2_DISPATCH_FIXED = 1,   /* `fixed_config` every step (8: sparse steps, see below) */
   SIMD2_DISPATCH_LEARNED = 2, /* the MLP cost model picks each step's config, sparse or dense */
   SIMD2_DISPATCH_RULES = 3    /* the hand-written policy: sparse steps under fixed
-                                 thresholds, then `fixed_config` (no MLP) */
+                                 thresholds, then dense steps, skipping blocks if
+                                 `fixed_config` does (no MLP) */
 } simd2_dispatch;
 
 /* simd2_closure with a dispatch policy.  mlp_params: device array of
@@ -184,13 +185,16 @@ typedef enum simd2_dispatch {
  * simd2_spgemm_compute supports, both open with CSR SpGEMM steps while X
  * holds at most n^2/32 entries (a result past that is written densely and
  * ends the opening):
- *   LEARNED runs a sparse step when the MLP predicts it faster than every
- *   dense configuration (steps past n^3/16 products are never sparse);
+ *   LEARNED runs a sparse step when the MLP predicts it faster than a dense
+ *   one without or with block skipping (steps past n^3/16 products are never
+ *   sparse);
  *   RULES runs it when the step forms at most n^3/256 products.
- * The dense steps then follow the MLP's per-step choice (LEARNED) or
- * fixed_config (RULES) for n > 2048, and the DENSE path for
+ * The dense steps of n > 2048 then run on the persistent kernels, skipping
+ * blocks by the MLP's per-step choice (LEARNED) or by fixed_config's skip
+ * flag (RULES; its split factor is not used), and the DENSE path runs for
  * 1024 < n <= 2048.  Once every block of X is occupied no step can skip, and
- * both keep the last split factor without the statistics pass.
+ * both go on without the statistics pass.  step_configs holds what ran: 0 or
+ * 4 for a dense step of the persistent kernels.
  * FIXED with fixed_config 8 runs sparse steps while X holds at most n^2/32
  * entries and a step forms at most n^3/16 products, then the DENSE path: the
  * autotuner records sparse-step times with it. */
@@ -201,13 +205,12 @@ int simd2_closure_ex(simd2_op op, int n, float* X, int ldx, int max_iter, simd2_
 
 /* The plain dense path's split-K factor by size, as the autotuner measured it
  * (no reference counterpart).  Entry i (n_min ascending, config 0..3: split
- * 1 << config, no skip) applies to closures of n_min[i] <= n < n_min[i + 1];
- * below n_min[0] the dense path keeps its rule (the largest split with
- * tiles * split <= SMs, at most 4).  count = 0 clears the table.  Applies to
- * simd2_closure and to SIMD2_DISPATCH_DENSE of simd2_closure_ex in this
- * process; same bits whatever the split.  The factor is what step_configs
- * reports; the persistent kernel that runs these steps spreads each one over
- * the SMs by itself, whatever the factor. */
+ * 1 << config, no skip) applies to closures of n_min[i] <= n < n_min[i + 1].
+ * Where no entry applies, or its config is 0, the persistent kernel spreads
+ * each step over the SMs by itself (small closures: all steps in one launch).
+ * count = 0 clears the table.  Applies to simd2_closure, simd2_closure_bf and
+ * SIMD2_DISPATCH_DENSE of simd2_closure_ex in this process; same bits
+ * whatever the split. */
 int simd2_set_dense_configs(const int* n_min, const int* config, int count);
 
 /* Cost-model MLP (15-32-32-1, ReLU) kernels.  X: [batch][15] features+config,

@@ -231,8 +231,9 @@ def srgemm_tuned(op: str, A: torch.Tensor, B: torch.Tensor, C: torch.Tensor | No
 def set_dense_configs(table) -> None:
     """Install the plain dense path's split-K factor by size: ``table`` is a
     list of (n_min, config) with n_min ascending and config 0..3 (split
-    1 << config), as ``autotune.dense_table`` measures it; [] restores the
-    rule.  Every split gives the same bits."""
+    1 << config; 0 is the persistent kernel, which needs no factor), as
+    ``autotune.dense_table`` measures it; [] clears it, and every size runs on
+    the persistent kernel.  Every split gives the same bits."""
     table = sorted((int(n), int(c)) for n, c in table)
     ns = (ctypes.c_int * max(len(table), 1))(*[n for n, _ in table])
     cs = (ctypes.c_int * max(len(table), 1))(*[c for _, c in table])
@@ -246,11 +247,11 @@ def closure_ex(op: str, X: torch.Tensor, dispatch: str = "dense", config: int = 
     ``dispatch``: "dense" (the plain path), "fixed" (``config`` every step;
     ``SPARSE_CONFIG`` runs CSR SpGEMM steps while X fits the sparse store,
     then the plain path), "learned" (above n = 1024, bitwise change test: the
-    MLP in ``mlp_params`` chooses each step between the dense configurations
-    and, while X is sparse, a CSR SpGEMM step) or "rules" (the hand-written
-    policy: sparse steps under fixed entry and product thresholds, then
-    ``config`` for the dense steps).  Every policy gives the same bits and
-    step count.
+    MLP in ``mlp_params`` chooses each step between a dense one without and
+    with block skipping and, while X is sparse, a CSR SpGEMM step) or "rules"
+    (the hand-written policy: sparse steps under fixed entry and product
+    thresholds, then dense steps, skipping blocks if ``config`` does).  Every
+    policy gives the same bits and step count.
 
     Returns the step count, or with ``record`` a dict with the per-step
     configurations (``SPARSE_CONFIG`` for a sparse step), device times (ms)

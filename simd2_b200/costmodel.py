@@ -7,7 +7,8 @@ step's matrix: its block occupancy, stored entries and the products a sparse
 step would form (``simd2_closure_ex`` computes them on the device).  Training and inference run on the GPU through
 libsimd2's own kernels (``simd2_mlp_forward``, ``simd2_mlp_gradient`` with a
 deterministic batch sum, ``simd2_mlp_adam``); the dispatcher evaluates the
-network inside ``simd2_closure_ex`` (dispatch="learned").
+network inside ``simd2_closure_ex`` (dispatch="learned"), which runs its dense
+steps without a split factor and so weighs configurations 0, 4 and 8.
 """
 from __future__ import annotations
 

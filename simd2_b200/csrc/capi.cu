@@ -1211,22 +1211,16 @@ namespace {
 std::mutex g_dense_mu;
 std::vector<int> g_dense_n, g_dense_split;
 
-// Split-K factor of the dense path: the autotuned table's entry for n when
-// one applies, else the largest power of two (at most 4) with
-// tiles * split <= SM count, so small problems still fill the GPU.
-int dense_split(int n, int sms) {
-  {
-    std::lock_guard<std::mutex> lk(g_dense_mu);
-    int pick = 0;
-    for (size_t i = 0; i < g_dense_n.size(); i++)
-      if (g_dense_n[i] <= n) pick = g_dense_split[i];
-    if (pick) return pick;
-  }
-  const long long tiles = (long long)((n + kBM - 1) / kBM) * ((n + kBN - 1) / kBN);
-  int s = 1;
-  while (s < 4 && tiles * s * 2 <= sms) s *= 2;
-  return s;
+// The factor installed for closures of n vertices; 1 (the persistent kernel, which
+// spreads a step over the SMs by itself) where none is.
+int dense_split(int n) {
+  std::lock_guard<std::mutex> lk(g_dense_mu);
+  int pick = 1;
+  for (size_t i = 0; i < g_dense_n.size(); i++)
+    if (g_dense_n[i] <= n) pick = g_dense_split[i];
+  return pick;
 }
+int split_config(int split) { return split == 1 ? 0 : split == 2 ? 1 : split == 4 ? 2 : 3; }
 
 constexpr int kOrAndSparseMinN = 8192;
 
@@ -1259,10 +1253,10 @@ int closure_sparse_opening_u8(int n, uint8_t* X, long long ldx, int max_iter, in
 // point cost only their launches.  The host reads the chunk's flags once.
 int closure_gated(int op, int n, float* X, long long ldx, int max_iter, int conv, int fixed_cfg, bool fixed,
                   bool can_skip, bool need_occ, const OccPlan& occ, uint8_t* ws, size_t x_off, int* changed,
-                  uint8_t* obase, int* iters_out, int* step_cfg, float* step_ms, int sms, cudaStream_t stream,
+                  uint8_t* obase, int* iters_out, int* step_cfg, float* step_ms, cudaStream_t stream,
                   const float* A0 = nullptr, long long lda0 = 0) {
   int rc = SIMD2_OK;
-  const int auto_split = dense_split(n, sms);
+  const int split = fixed ? config_split(fixed_cfg) : dense_split(n);
   float* bufs[2] = {X, reinterpret_cast<float*>(ws + x_off)};
   const long long lds[2] = {ldx, n};
   SIMD2_CUDA_TRY(cudaMemsetAsync(changed, 0, (size_t)(max_iter + 1) * sizeof(int), stream));
@@ -1288,7 +1282,7 @@ int closure_gated(int op, int n, float* X, long long ldx, int max_iter, int conv
         cudaEventRecord(a, stream);
       }
       SimtConfig cfg;
-      cfg.split = fixed ? config_split(fixed_cfg) : 1;
+      cfg.split = split;
       cfg.skip = fixed && config_skip(fixed_cfg) && can_skip && need_occ;
       if (cfg.skip) {
         // occupancy of a gated-off step is harmless work on an unchanged matrix
@@ -1296,8 +1290,7 @@ int closure_gated(int op, int n, float* X, long long ldx, int max_iter, int conv
         cfg.occA = obase + occ.occA;
         cfg.occB = obase + occ.occB;
       }
-      const int rep_split = fixed ? cfg.split : auto_split;
-      if (step_cfg) step_cfg[t] = (cfg.skip ? 4 : 0) | (rep_split == 1 ? 0 : rep_split == 2 ? 1 : rep_split == 4 ? 2 : 3);
+      if (step_cfg) step_cfg[t] = (cfg.skip ? 4 : 0) | split_config(split);
       // A operand: X_t (repeated squaring) or the fixed adjacency A0 (Bellman-Ford form)
       const float* Aop = A0 ? A0 : cur;
       const long long lda_op = A0 ? lda0 : ldcur;
@@ -1456,20 +1449,23 @@ int closure_coop(int op, int n, float* X, long long ldx, int max_iter, int conv,
 }
 
 // Closure by repeated squaring with a per-step kernel configuration:
-//   dispatch 0 (dense)  : no skip, split-K from the tile count (the plain path);
+//   dispatch 0 (dense)  : no skip (the plain path): the persistent kernel, or the
+//                         split factor installed for n (simd2_set_dense_configs);
 //   dispatch 1 (fixed)  : `fixed_cfg` every step: a dense configuration
 //                         (split = 1 << (cfg & 3), skip = cfg >> 2), or
 //                         kSparseConfig: CSR SpGEMM steps for as long as X fits
 //                         the sparse store (under n^3/16 products), then the
 //                         plain dense steps (used to record sparse-step times);
 //   dispatch 2 (learned): per step, the statistics of X_t -> features -> the
-//                         MLP `mlp_params` predicts the time of every dense
-//                         configuration and, while X_t is sparse, of a CSR
-//                         SpGEMM step; the cheapest one runs;
+//                         MLP `mlp_params` predicts the time of a dense step
+//                         without and with block skipping and, while X_t is
+//                         sparse, of a CSR SpGEMM step; the cheapest one runs;
 //   dispatch 3 (rules)  : the hand-written policy without the MLP: sparse
 //                         steps while X_t holds at most n^2/32 entries and the
-//                         step forms at most n^3/256 products, then `fixed_cfg`
-//                         for every dense step.
+//                         step forms at most n^3/256 products, then dense steps,
+//                         skipping blocks if `fixed_cfg` does.
+// The dense steps of the last two run on the persistent kernels, which spread them
+// over the SMs without a split factor.
 // Every configuration computes the same bits, so the dispatch only moves time.
 // step_cfg / step_ms / step_feat (host arrays of max_iter, max_iter,
 // max_iter * kMlpFeat entries, each optional) record what each step ran, its
@@ -1506,9 +1502,10 @@ int closure_f32_ex(int op, int n, float* X, long long ldx, int max_iter, int con
     step_feat = nullptr;
   }
   // A small closure on codes: one cooperative launch (recorded ones keep a launch
-  // per step, whose times and configurations they ask for).
+  // per step, whose times and configurations they ask for, and so do sizes with an
+  // installed split factor).
   if (dispatch == 0 && n <= kCoopMaxN && has_code16(op) && conv != SIMD2_CONV_APLP && !step_cfg && !step_ms &&
-      !step_feat) {
+      !step_feat && dense_split(n) == 1) {
     bool done = false;
     rc = closure_coop(op, n, X, ldx, max_iter, conv, iters_out, &done, stream);
     if (done || rc) return rc;
@@ -1595,7 +1592,7 @@ int closure_f32_ex(int op, int n, float* X, long long ldx, int max_iter, int con
   if (!per_step) {
     int it2 = 0;
     rc = closure_gated(op, n, X, ldx, max_iter, conv, fixed_cfg, dispatch == 1, can_skip, need_occ, occ, ws, x_off,
-                       reinterpret_cast<int*>(ws + f_off + 256), obase, &it2, step_cfg, step_ms, sms, stream);
+                       reinterpret_cast<int*>(ws + f_off + 256), obase, &it2, step_cfg, step_ms, stream);
     if (iters_out) *iters_out = it0 + it2;
     return rc;
   }
@@ -1615,7 +1612,7 @@ int closure_f32_ex(int op, int n, float* X, long long ldx, int max_iter, int con
     if (r) return r;
     if (dispatch == 2) {
       mlp_choose_kernel<<<1, 32, 0, stream>>>(mlp_params, reinterpret_cast<unsigned long long*>(obase + occ.stats), n,
-                                              occ.tiles_m, occ.tiles_n, occ.ktiles, sms, can_skip ? 1 : 0, 8, 0,
+                                              occ.tiles_m, occ.tiles_n, occ.ktiles, sms, can_skip ? 1 : 0, 1, 0,
                                               decision);
       count_launch();
     }
@@ -1638,8 +1635,12 @@ int closure_f32_ex(int op, int n, float* X, long long ldx, int max_iter, int con
     if (step_ms && want_dec) cudaEventElapsedTime(&occ_ms, ev[2], ev[3]);
     return SIMD2_OK;
   };
-  const int ds = dense_split(n, sms);
-  const int default_cfg = dispatch == 1 || dispatch == 3 ? fixed_cfg : (ds == 1 ? 0 : ds == 2 ? 1 : 2);
+  // The learned and rules loops run their dense steps on the persistent kernels,
+  // with or without block skipping (configurations 0 and 4).
+  const int default_cfg = dispatch == 1   ? fixed_cfg
+                          : dispatch == 3 ? fixed_cfg & 4
+                          : dispatch == 0 ? split_config(dense_split(n))
+                                          : 0;
   float* cur = X;
   long long ldcur = ldx;
   float* nxt = Xn;
@@ -1675,9 +1676,7 @@ int closure_f32_ex(int op, int n, float* X, long long ldx, int max_iter, int con
   }
   while (changed && it < max_iter) {
     SimtConfig cfg;
-    // the persistent kernel spreads a step over the SMs by itself; only a fixed
-    // configuration forces its split factor
-    cfg.split = dispatch == 1 ? config_split(cfg_id) : 1;
+    cfg.split = config_split(cfg_id);
     const bool delta = use_delta && prev_chg && (occ_fresh || occ_full);
     cfg.skip = can_skip && ((config_skip(cfg_id) && occ_on) || delta);
     if (cfg.skip) {
@@ -2355,7 +2354,7 @@ int closure_sparse_opening_t(int op, int n, T* X, long long ldx, int max_iter, c
           pol.obase + o.occA, pol.obase + o.occB, stats);
       stats_from_csr_kernel<<<1, 32, 0, stream>>>(stats, nnz, prod);
       mlp_choose_kernel<<<1, 32, 0, stream>>>(pol.mlp, stats, n, o.tiles_m, o.tiles_n, o.ktiles, pol.sms,
-                                              pol.can_skip, 8, 1, pol.decision);
+                                              pol.can_skip, 1, 1, pol.decision);
       for (int i = 0; i < 4; i++) count_launch();
       SIMD2_CUDA_TRY(cudaGetLastError());
       SIMD2_CUDA_TRY(cudaMemcpyAsync(hst, stats, sizeof(hst), cudaMemcpyDeviceToHost, stream));
@@ -3545,9 +3544,6 @@ extern "C" int simd2_closure_bf(simd2_op op, int n, const float* A0, int lda0, f
   if (n == 0 || max_iter == 0) return SIMD2_OK;
   int rc = check_device();
   if (rc) return rc;
-  int dev = 0, sms = 148;
-  SIMD2_CUDA_TRY(cudaGetDevice(&dev));
-  SIMD2_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   const Plan plan = make_plan(n, n, n, true, true, op);
   const OccPlan occ = make_occ_plan(n, n, n, true);
   const size_t x_off = align_up(plan.total, kAlign);
@@ -3557,7 +3553,7 @@ extern "C" int simd2_closure_bf(simd2_op op, int n, const float* A0, int lda0, f
   if ((rc = get_workspace(stream, total, &p))) return rc;
   uint8_t* ws = static_cast<uint8_t*>(p);
   return closure_gated(op, n, X, ldx, max_iter, conv, 0, false, false, false, occ, ws, x_off,
-                       reinterpret_cast<int*>(ws + f_off), nullptr, iters_out, nullptr, nullptr, sms, stream, A0,
+                       reinterpret_cast<int*>(ws + f_off), nullptr, iters_out, nullptr, nullptr, stream, A0,
                        lda0);
 }
 

@@ -141,8 +141,8 @@ __host__ __device__ inline void mlp_features(int n, int tiles_m, int tiles_n, in
 }
 
 // Picks the configuration with the smallest predicted time for one step:
-// the dense ones allowed by allow_skip / max_split, and the sparse step when
-// allow_sparse.  Thread c evaluates configuration c; out[0] = chosen config
+// the dense ones allowed by allow_skip / max_split (1: the persistent kernels), and
+// the sparse step when allow_sparse.  Thread c evaluates configuration c; out[0] = chosen config
 // (the lowest id among equal predictions), out[1 + c] = prediction for
 // config c (as float bits), c = 0..kSparseConfig.  Launch with 32 threads.
 __global__ void mlp_choose_kernel(const float* __restrict__ P, const unsigned long long* __restrict__ stats, int n,

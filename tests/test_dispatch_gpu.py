@@ -282,6 +282,45 @@ def test_autotuned_dense_configs(cuda):
     assert rd["configs"] == ra["configs"]
 
 
+def test_installed_split_runs(cuda):
+    """A table entry that forces a split factor is obeyed by small closures too: a
+    launch per step instead of one for all."""
+    x = datagen.er_graph(300, 0.05, seed=3)
+    want, steps = oracle.closure("min_plus", x)
+
+    def launches():
+        X = torch.from_numpy(x.copy()).to(cuda)
+        before = s2.launch_count()
+        assert s2.closure("min_plus", X) == steps
+        np.testing.assert_array_equal(bits(X.cpu().numpy()), bits(want))
+        return s2.launch_count() - before
+
+    assert launches() == 1
+    try:
+        s2.set_dense_configs([(200, 2)])
+        assert launches() >= 2 * steps
+        s2.set_dense_configs([(200, 0), (301, 2)])
+        assert launches() == 1
+    finally:
+        s2.set_dense_configs([])
+
+
+def test_recorded_configs_are_those_that_ran(cuda):
+    """Without an installed table dense steps report the persistent kernel, and the
+    learned and rules loops report it with or without block skipping, whatever
+    split factor the rules are given."""
+    import os
+    params = costmodel.load(os.path.join(os.path.dirname(s2.__file__), "costmodel_weights.json"), cuda)
+    small = torch.from_numpy(datagen.er_graph(512, 0.05, seed=1)).to(cuda)
+    assert set(s2.closure_ex("min_plus", small, dispatch="dense", record=True)["configs"]) == {0}
+    g = datagen.rmat_graph_device(4096, 40.0, seed=77, device=cuda)
+    untrained = torch.randn(costmodel.param_count(), generator=torch.Generator().manual_seed(5)).to(cuda)
+    for kw in ({"dispatch": "rules", "config": s2.config_id(2, True)}, {"dispatch": "rules", "config": 2},
+               {"dispatch": "learned", "mlp_params": params}, {"dispatch": "learned", "mlp_params": untrained}):
+        ran = s2.closure_ex("min_plus", g.clone(), record=True, **kw)["configs"]
+        assert set(ran) <= {0, 4, s2.SPARSE_CONFIG}, (kw["dispatch"], ran)
+
+
 @pytest.mark.parametrize("case", ["min_plus_rmat", "max_plus_dag"])
 def test_delta_steps_identical(cuda, case):
     """The rules and learned loops of a min_plus / max_plus closure skip, from
