@@ -2874,10 +2874,12 @@ int simd2_batched_plan_create(simd2_op op, int count, float* const* X, const int
   take(sizeof(unsigned long long) * std::max(cap, 1u));
   p->cleared_bytes = sl_off - s_off;
   p->slot_bytes = (cap - first.size()) * sizeof(unsigned long long);
-  struct Sizes { size_t x, p, xc, pc; };
+  // The codes lie in the FP32 buffers, which a graph uses only after it has left its
+  // codes for good (its preparation reads the caller's matrix): 16 bytes an element.
+  // Kh <= 2 Kp, so they fit.
+  struct Sizes { size_t x, p; };
   auto sizes = [&](const BatchGraph& G) {
-    return Sizes{(size_t)G.Mp * G.Kp * 4, (size_t)G.Kp * G.Np * 4, codes ? (size_t)G.Mp * G.Kh * 2 : 0,
-                 codes ? (size_t)G.Kh * G.Np * 2 : 0};
+    return Sizes{(size_t)G.Mp * G.Kp * 4, (size_t)G.Kp * G.Np * 4};
   };
   std::vector<size_t> buf_off(count);
   for (int g = 0; g < count; g++) {
@@ -2892,7 +2894,7 @@ int simd2_batched_plan_create(simd2_op op, int count, float* const* X, const int
     G.ldu = ldx[g];
     tasks += (long long)(G.Mp / kBM) * (G.Np / kBN);
     const Sizes z = sizes(G);
-    buf_off[g] = take(2 * (z.x + z.p + z.xc + z.pc));
+    buf_off[g] = take(2 * (z.x + z.p));
   }
   void* mem = nullptr;
   if (cudaMalloc(&mem, std::max(off, (size_t)kAlign)) != cudaSuccess) {
@@ -2938,8 +2940,8 @@ int simd2_batched_plan_create(simd2_op op, int count, float* const* X, const int
         rc = make_map_f32(&hmaps[g].b[q], G.P[q], G.Kp / 2, 2LL * G.Np, 2LL * G.Np, 2 * kBN, kBK / 2,
                           CU_TENSOR_MAP_SWIZZLE_NONE, false);
       if (!codes || rc != SIMD2_OK) continue;
-      G.Xc[q] = reinterpret_cast<uint16_t*>(b + 2 * (z.x + z.p) + q * z.xc);
-      G.Pc[q] = reinterpret_cast<uint32_t*>(b + 2 * (z.x + z.p + z.xc) + q * z.pc);
+      G.Xc[q] = reinterpret_cast<uint16_t*>(G.X[q]);
+      G.Pc[q] = reinterpret_cast<uint32_t*>(G.P[q]);
       rc = make_map_2d(&hmaps[g].ac[q], CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, G.Xc[q], G.Mp, G.Kh, G.Kh, kSkBK16, kBM,
                        CU_TENSOR_MAP_SWIZZLE_128B);
       if (rc == SIMD2_OK)

@@ -37,8 +37,10 @@ struct BatchGraph {
   int Np;       // columns padded to a multiple of 128 (B role)
   float* X[2];     // [Mp][Kp], ping-pong
   float* P[2];     // [Kp/2][2*Np] interleaved, ping-pong
-  uint16_t* Xc[2];  // [Mp][Kh] codes, ping-pong (null: the semiring has none)
-  uint32_t* Pc[2];  // [Kh/2][Np] words (code of X[2p][j], code of X[2p+1][j]), ping-pong
+  // Codes, ping-pong, in the memory of X and P (null: the semiring has none): a
+  // graph is on codes or, after kPrep32 has written X and P anew, on FP32.
+  uint16_t* Xc[2];  // [Mp][Kh]
+  uint32_t* Pc[2];  // [Kh/2][Np] words (code of X[2p][j], code of X[2p+1][j])
   float* user;  // caller's matrix (result is copied back here)
   long long ldu;
   int iters;    // out: steps run (including the final unchanged one)

@@ -112,6 +112,20 @@ def test_outgrows_codes(cuda, n):
     check("min_plus", [chain, datagen.er_graph(n, 0.1, seed=3), big, frac, datagen.er_graph(40, 0.1, seed=4)])
 
 
+@pytest.mark.parametrize("op", ["min_plus", "max_min", "max_mul"])
+def test_plan_memory(cuda, op):
+    """Both operand layouts of X, twice: 16 bytes an element, codes or not."""
+    n = 8192
+    X = torch.zeros((n, n), device=cuda)
+    s2.closure_batched(op, [torch.ones((130, 130), device=cuda)], max_iter=1)  # kernels loaded
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    plan = s2.BatchedClosure(op, [X])
+    used = before - torch.cuda.mem_get_info()[0]
+    plan.close()
+    assert used <= 16.25 * n * n
+
+
 def test_more_steps_than_entries(cuda):
     """Longest paths around a cycle never settle: every step changes X, past the
     codes' range and past the steps the entry list has room for."""
