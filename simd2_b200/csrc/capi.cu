@@ -537,10 +537,10 @@ int compute_step_stats(int op, int n, const float* X, long long ldx, uint8_t* ba
   return SIMD2_OK;
 }
 
-template <int OP, int TILE>
+template <int OP, int TILE, bool FP32>
 int launch_sk_tile(const CUtensorMap& a16, const CUtensorMap& b16, const CUtensorMap& a32, const CUtensorMap& b32,
                    const SkArgs& args, int grid, const EpilogueArgs& ep, cudaStream_t stream) {
-  auto kern = srgemm_sk_kernel<OP, TILE>;
+  auto kern = srgemm_sk_kernel<OP, TILE, FP32>;
   static bool configured[64] = {};
   int dev = 0;
   SIMD2_CUDA_TRY(cudaGetDevice(&dev));
@@ -549,11 +549,8 @@ int launch_sk_tile(const CUtensorMap& a16, const CUtensorMap& b16, const CUtenso
     SIMD2_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SkCfg<TILE>::kSmem));
     configured[dev] = true;
   }
-  auto* ev = prof_slot(2LL * args.M * args.N * args.K);
-  if (ev) cudaEventRecord(ev->first, stream);
   kern<<<grid, kSimtThreads, SkCfg<TILE>::kSmem, stream>>>(a16, b16, a32, b32, args, ep);
   count_launch();
-  if (ev) cudaEventRecord(ev->second, stream);
   SIMD2_CUDA_TRY(cudaGetLastError());
   return SIMD2_OK;
 }
@@ -579,6 +576,10 @@ int launch_sk_skip(const CUtensorMap& a16, const CUtensorMap& b16, const CUtenso
   SIMD2_CUDA_TRY(cudaGetLastError());
   return SIMD2_OK;
 }
+
+// 64-wide k-tiles a CTA (4.5 us each on codes) from which a product that may be coded
+// gets a launch for its codes and one for FP32 (see srgemm_sk_kernel).
+constexpr int kSkPairUnits = 16;
 
 // One product on srgemm_sk_kernel (with cfg.skip or change maps to write, on
 // srgemm_sk_skip_kernel): the operand preparation, then the kernel.
@@ -654,8 +655,23 @@ int launch_sk(int M, int N, int K, const T* A, long long lda, const T* B, long l
   ga.counters = pa.counters;
   ga.part = split ? reinterpret_cast<float*>(ws + plan.part_off) : nullptr;
   const int grid = split ? sh.grid : (int)std::min<long long>(tiles, device_sms());
-  return t == 128 ? launch_sk_tile<OP, 128>(a16, b16, a32, b32, ga, grid, ep, stream)
-                  : launch_sk_tile<OP, 64>(a16, b16, a32, b32, ga, grid, ep, stream);
+  auto* ev = prof_slot(2LL * M * N * K);  // a pair of launches is timed as one
+  if (ev) cudaEventRecord(ev->first, stream);
+  rc = SIMD2_OK;
+  bool fp32 = true;
+  if constexpr (has_code16(OP)) {
+    if (plan.code16) {
+      ga.pair = t == 128 && tiles * (plan.Kh / kSkBK16) >= kSkPairUnits * (long long)device_sms();
+      rc = t == 128 ? launch_sk_tile<OP, 128, false>(a16, b16, a32, b32, ga, grid, ep, stream)
+                    : launch_sk_tile<OP, 64, false>(a16, b16, a32, b32, ga, grid, ep, stream);
+      fp32 = ga.pair != 0;
+    }
+  }
+  if (!rc && fp32)
+    rc = t == 128 ? launch_sk_tile<OP, 128, true>(a16, b16, a32, b32, ga, grid, ep, stream)
+                  : launch_sk_tile<OP, 64, true>(a16, b16, a32, b32, ga, grid, ep, stream);
+  if (ev) cudaEventRecord(ev->second, stream);
+  return rc;
 }
 
 // Whether srgemm_small_kernel is the faster one, by the time (us) both take: its

@@ -214,7 +214,8 @@ __global__ void __launch_bounds__(256) sk_prep_kernel(SkPrepArgs<T> g) {
     if (g.A16) {
       const int groups = g.Kh >> 3;
       const long long total = (long long)g.M * groups;
-      for (long long t = tid; t < total; t += step) {
+      // a thread that met an entry without a code leaves its other codes out
+      for (long long t = tid; t < total && !bad; t += step) {
         const int i = (int)(t / groups);
         const int k0 = (int)(t - (long long)i * groups) * 8;
         const int left = g.K - k0;
@@ -264,7 +265,7 @@ __global__ void __launch_bounds__(256) sk_prep_kernel(SkPrepArgs<T> g) {
         o[1] = make_float4(x[0][2], x[1][2], x[0][3], x[1][3]);
       }
       if constexpr (k16) {
-        if (g.B16) {
+        if (g.B16 && !bad) {
           uint32_t w[4];
 #pragma unroll
           for (int e = 0; e < 4; e++) {
@@ -324,6 +325,7 @@ struct SkArgs {
   int nnotes;
   int* counters;          // arrivals per split tile
   float* part;            // partial tiles: two slots of TILE x TILE floats per CTA (null: no tile is split)
+  int pair;               // the FP32 kernel follows: this one takes codes only
 };
 
 // One k-tile of a warp's register tile on 16-bit codes: chunk q of an A row
@@ -662,7 +664,12 @@ __device__ __forceinline__ void sk_run(const CUtensorMap* tmA, const CUtensorMap
   }
 }
 
-template <int OP, int TILE>
+// FP32: on FP32 operands only; else the notes decide on the device.  One kernel with
+// both inner loops runs the FP32 one 6 % slower than a kernel of its own (min_plus
+// 4096^3 on fractions 4254 us, 3987 apart), and a second launch costs 2 us: large
+// products get both (g.pair), of which one returns at once, and a plan without codes
+// the FP32 kernel alone.
+template <int OP, int TILE, bool FP32>
 __global__ void __launch_bounds__(kSimtThreads, 1)
     srgemm_sk_kernel(const __grid_constant__ CUtensorMap a16, const __grid_constant__ CUtensorMap b16,
                      const __grid_constant__ CUtensorMap a32, const __grid_constant__ CUtensorMap b32, SkArgs g,
@@ -687,9 +694,15 @@ __global__ void __launch_bounds__(kSimtThreads, 1)
     int bad = g.notes == nullptr;
     if (g.notes)
       for (int i = threadIdx.x; i < g.nnotes; i += kSimtThreads) bad |= (int)g.notes[i];
-    if (!__syncthreads_or(bad)) {
-      sk_run<OP, TILE, true>(&a16, &b16, g, ep, smem, full, empty, red, &s_failed, &s_last);
-      return;
+    const bool coded = !__syncthreads_or(bad);
+    if constexpr (FP32) {
+      if (coded) return;
+    } else {
+      if (coded) {
+        sk_run<OP, TILE, true>(&a16, &b16, g, ep, smem, full, empty, red, &s_failed, &s_last);
+        return;
+      }
+      if (g.pair) return;
     }
   } else {
     __syncthreads();

@@ -106,3 +106,22 @@ def test_small_products(cuda, op, shape):
         ah, bh = (x.astype(np.float16) for x in (a, b))
         got = s2.srgemm_f16(op, place(ah, torch.float16), place(bh, torch.float16))
         same(got.cpu().numpy(), oracle.srgemm(op, ah.astype(np.float32), bh.astype(np.float32)), f"{op} {shape} f16")
+
+
+@pytest.mark.parametrize("op", CODED)
+@pytest.mark.parametrize("shape", [(1500, 1540, 960), (1500, 1540, 1030), (1153, 1409, 1285)])
+def test_pair_of_launches(cuda, op, shape):
+    """Sizes on either side of the line from which a product gets a launch for its
+    codes and one for FP32: coded operands, fractions, and one entry without a code
+    in the last row; a pair is timed as one launch."""
+    m, n, k = shape
+    a, b, c = datagen.semiring_operands(op, m, n, k, seed=m + k)
+    same(call(op, a, b, c), oracle.srgemm(op, a, b, c, do_epilogue=True, threads=8), f"{op} {shape}")
+    a2 = a + np.float32(0.3)
+    same(call(op, a2, b), oracle.srgemm(op, a2, b, threads=8), f"{op} {shape} fractions")
+    b[k - 1, n - 1] = 0.3
+    with s2.KernelTimer() as t:
+        got = call(op, a, b)
+    same(got, oracle.srgemm(op, a, b, threads=8), f"{op} {shape} one fraction")
+    assert (t.launches, t.ops) == (1, 2 * m * n * k)
+    assert s2.device_status() == 0
