@@ -289,7 +289,11 @@ struct SkShape {
 //
 // Split.  With at least as many tiles as SMs, every CTA takes the same number
 // of whole tiles and the rest is split evenly by units, so no wave is partly
-// empty (2048^3: 256 tiles on 148 SMs, 381 us in two waves, 283 split).  With
+// empty (2048^3: 256 tiles on 148 SMs, 381 us in two waves, 283 split) -- unless that
+// saves a CTA fewer than 1.5 k-tiles, about what its parts' way through global memory
+// costs (split / whole tiles, us: min_plus 2000 x 2000 x 128 42.8 / 36.9, 2300 x 2300 x
+// 128, which saves 1.6, 47.2 / 49.2; max_mul 2560 x 2560 x 64 53.4 / 47.1, 2000 x 2000 x
+// 256, which saves 2.2, 86.0 / 88.1).  With
 // fewer tiles, an equal number of CTAs per tile where that occupies at least
 // three quarters of the SMs -- few contributors per tile keep the fold short
 // (512^3 on 64 x 64 tiles: 2 CTAs per tile 17.6 us, an even split of all units
@@ -308,6 +312,7 @@ SkShape sk_shape(int M, int N, int K, bool code16) {
   if (tiles >= sms) {
     p.grid = sms;
     p.whole = (int)(tiles / sms - (tiles % sms ? 1 : 0));
+    if (2 * (sms - tiles % sms) * kt < 3 * sms) p.whole = (int)((tiles + sms - 1) / sms);
     return p;
   }
   const long long fold_max = std::max(1LL, (long long)std::sqrt(4.0 * (double)kt));

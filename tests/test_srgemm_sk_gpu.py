@@ -125,3 +125,16 @@ def test_pair_of_launches(cuda, op, shape):
     same(got, oracle.srgemm(op, a, b, threads=8), f"{op} {shape} one fraction")
     assert (t.launches, t.ops) == (1, 2 * m * n * k)
     assert s2.device_status() == 0
+
+
+@pytest.mark.parametrize("op", ["min_plus", "max_mul"])
+@pytest.mark.parametrize("shape", [(1990, 2000, 64), (1990, 2000, 100), (2000, 2000, 130), (1600, 1601, 96), (2100, 1500, 48)])
+def test_more_tiles_than_sms(cuda, op, shape):
+    """Products of few k-tiles on either side of the line from which the last tiles
+    are split, coded and not."""
+    m, n, k = shape
+    a, b, c = datagen.semiring_operands(op, m, n, k, seed=m + k)
+    same(call(op, a, b, c), oracle.srgemm(op, a, b, c, do_epilogue=True, threads=8), f"{op} {shape}")
+    a2 = (a * np.float32(1.3)).astype(np.float32)
+    same(call(op, a2, b), oracle.srgemm(op, a2, b, threads=8), f"{op} {shape} fractions")
+    assert s2.device_status() == 0
