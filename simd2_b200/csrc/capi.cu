@@ -335,10 +335,13 @@ struct Plan {
   size_t total;
 };
 
+// An op without codes: a plan made for it has none.
+constexpr int kNoCodes = SIMD2_MAX_MUL;
+
 // full: the parts srgemm_sk_kernel needs to split tiles between CTAs and, for
 // an op with 16-bit codes, the coded operands; without it the kernel runs
 // whole tiles on FP32 operands from B' (and packed A) alone.
-Plan make_plan(int M, int N, int K, bool pack_a, bool full = false, int op = SIMD2_MAX_MUL) {
+Plan make_plan(int M, int N, int K, bool pack_a, bool full = false, int op = kNoCodes) {
   Plan p{};
   p.Kp = round_up(std::max(K, 1), kBK);
   p.Np = round_up(std::max(N, 1), kBN);
@@ -585,6 +588,10 @@ int launch_sk_skip(const CUtensorMap& a16, const CUtensorMap& b16, const CUtenso
 // 64-wide k-tiles a CTA (4.5 us each on codes) from which a product that may be coded
 // gets a launch for its codes and one for FP32 (see srgemm_sk_kernel).
 constexpr int kSkPairUnits = 16;
+// A closure's step: those enqueued past the fixed point pay for the second launch too
+// (min_plus on codes, one launch / two: n = 1600 1086 / 1142 us, 2048 1830 / 1868), and
+// only from about 2800 vertices on is FP32 in the shared kernel slower than it was.
+constexpr int kSkPairStepUnits = 128;
 
 // One product on srgemm_sk_kernel (with cfg.skip or change maps to write, on
 // srgemm_sk_skip_kernel): the operand preparation, then the kernel.
@@ -666,7 +673,8 @@ int launch_sk(int M, int N, int K, const T* A, long long lda, const T* B, long l
   bool fp32 = true;
   if constexpr (has_code16(OP)) {
     if (plan.code16) {
-      ga.pair = t == 128 && tiles * (plan.Kh / kSkBK16) >= kSkPairUnits * (long long)device_sms();
+      const long long line = ep.changed ? kSkPairStepUnits : kSkPairUnits;
+      ga.pair = t == 128 && tiles * (plan.Kh / kSkBK16) >= line * device_sms();
       rc = t == 128 ? launch_sk_tile<OP, 128, false>(a16, b16, a32, b32, ga, grid, ep, stream)
                     : launch_sk_tile<OP, 64, false>(a16, b16, a32, b32, ga, grid, ep, stream);
       fp32 = ga.pair != 0;
@@ -1271,11 +1279,12 @@ int closure_sparse_opening_u8(int n, uint8_t* X, long long ldx, int max_iter, in
 // Closure steps enqueued in chunks without a host round trip per step.
 // changed[t] is written by step t; every kernel of step t+1 reads changed[t]
 // as its gate and does nothing when it is 0, so steps enqueued past the fixed
-// point cost only their launches.  The host reads the chunk's flags once.
+// point cost only their launches.  The host reads the chunk's flags once.  codes =
+// false: an entry was seen to have none, so none are made.
 int closure_gated(int op, int n, float* X, long long ldx, int max_iter, int conv, int fixed_cfg, bool fixed,
                   bool can_skip, bool need_occ, const OccPlan& occ, uint8_t* ws, size_t x_off, int* changed,
                   uint8_t* obase, int* iters_out, int* step_cfg, float* step_ms, cudaStream_t stream,
-                  const float* A0 = nullptr, long long lda0 = 0) {
+                  const float* A0 = nullptr, long long lda0 = 0, bool codes = true) {
   int rc = SIMD2_OK;
   const int split = fixed ? config_split(fixed_cfg) : dense_split(n);
   float* bufs[2] = {X, reinterpret_cast<float*>(ws + x_off)};
@@ -1316,7 +1325,7 @@ int closure_gated(int op, int n, float* X, long long ldx, int max_iter, int conv
       const float* Aop = A0 ? A0 : cur;
       const long long lda_op = A0 ? lda0 : ldcur;
       const bool pk = !a_tma_ok(Aop, lda_op);
-      const Plan pl = make_plan(n, n, n, pk, true, op);
+      const Plan pl = make_plan(n, n, n, pk, true, codes ? op : kNoCodes);
       EpilogueArgs ep = make_epilogue(cur, ldcur, nxt, ldnxt, 1, changed + t, conv);
       ep.gate = gate;
       if ((rc = srgemm_core(op, n, n, n, Aop, lda_op, cur, ldcur, ep, ws, pl, pk, stream, cfg))) break;
@@ -1365,6 +1374,11 @@ int closure_gated(int op, int n, float* X, long long ldx, int max_iter, int conv
 // time of a whole call, a launch per step / one (us; min_plus, max_min, 5 to 7
 // steps): n = 32 158 / 63, 512 213 / 94, 228 / 123, 1024 403 / 274, 553 / 431, 1500
 // 780 / 690, 1400 / 1374; at 2000 the launched steps' larger tiles win (2957 / 3070).
+// What a failed attempt costs a closure that has to go on with a launch per step: an
+// entry without a code is found by the coding pass, 25 to 35 us in all (min_plus on
+// fractions, before there was an attempt / now, n = 600 366 / 401 us, 1000 1112 / 1166,
+// 1536 3154 / 3234); a result without one costs the steps up to it as well (weights up
+// to 16000, n = 600 285 / 341, 1000 617 / 704).
 constexpr int kCoopMaxN = 1536;
 
 template <int OP>
@@ -1401,11 +1415,13 @@ int launch_coop(const CUtensorMap (&m)[4], CoopArgs& args, int grid, ProfLater* 
   return SIMD2_OK;
 }
 
-// The whole closure as one cooperative launch on 16-bit codes.  *done = false:
-// an entry or a result has no code; X is as it was.
+// The whole closure as one cooperative launch on 16-bit codes.  *done = false: X is
+// as it was, and *codes = false if an entry was found to have no code (where it was a
+// result, most steps still run on codes: their operands are smaller than their results).
 int closure_coop(int op, int n, float* X, long long ldx, int max_iter, int conv, int* iters_out, bool* done,
-                 cudaStream_t stream) {
+                 bool* codes, cudaStream_t stream) {
   *done = false;
+  *codes = true;
   const int tiles = (n + 63) / 64, Kh = round_up(n, kSkBK16), Np = round_up(n, kBN), rows = tiles * 64;
   const int sms = device_sms();
   // CTAs and whole tiles as for a product on 64 x 64 tiles
@@ -1462,7 +1478,10 @@ int closure_coop(int op, int n, float* X, long long ldx, int max_iter, int conv,
   SIMD2_CUDA_TRY(cudaStreamSynchronize(stream));
   const int iters = a.out[0], outcome = a.out[1];
   if (a.out[2] || outcome == 0) return SIMD2_ERR_TIMEOUT;  // a bounded wait ran out in some CTA
-  if (outcome == 3) return SIMD2_OK;
+  if (outcome >= 3) {
+    *codes = outcome == 3;
+    return SIMD2_OK;
+  }
   prof_add_ops(later, 2LL * n * n * n * iters);
   *done = true;
   if (iters_out) *iters_out = iters;
@@ -1525,10 +1544,11 @@ int closure_f32_ex(int op, int n, float* X, long long ldx, int max_iter, int con
   // A small closure on codes: one cooperative launch (recorded ones keep a launch
   // per step, whose times and configurations they ask for, and so do sizes with an
   // installed split factor).
+  bool codes = true;
   if (dispatch == 0 && n <= kCoopMaxN && has_code16(op) && conv != SIMD2_CONV_APLP && !step_cfg && !step_ms &&
       !step_feat && dense_split(n) == 1) {
     bool done = false;
-    rc = closure_coop(op, n, X, ldx, max_iter, conv, iters_out, &done, stream);
+    rc = closure_coop(op, n, X, ldx, max_iter, conv, iters_out, &done, &codes, stream);
     if (done || rc) return rc;
   }
   const bool can_skip = skip_supported(op) && (n + kBK - 1) / kBK <= kMaxSkipKtiles;
@@ -1613,7 +1633,8 @@ int closure_f32_ex(int op, int n, float* X, long long ldx, int max_iter, int con
   if (!per_step) {
     int it2 = 0;
     rc = closure_gated(op, n, X, ldx, max_iter, conv, fixed_cfg, dispatch == 1, can_skip, need_occ, occ, ws, x_off,
-                       reinterpret_cast<int*>(ws + f_off + 256), obase, &it2, step_cfg, step_ms, stream);
+                       reinterpret_cast<int*>(ws + f_off + 256), obase, &it2, step_cfg, step_ms, stream, nullptr,
+                       0, codes);
     if (iters_out) *iters_out = it0 + it2;
     return rc;
   }

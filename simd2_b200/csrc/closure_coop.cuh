@@ -41,7 +41,8 @@ struct CoopArgs {
   int* counters;      // arrivals per split tile, over all steps
   uint4* part;        // two slots of 64 x 64 codes per CTA
   CoopCtl* ctl;
-  volatile int* out;  // host memory: steps, and 1 converged, 2 not converged, 3 no codes (X untouched); 1 when a CTA failed
+  volatile int* out;  // host memory: steps; 1 converged, 2 not converged, 3 / 4 a result / an entry without a code
+                      // (X untouched); 1 when a CTA failed
 };
 
 // All CTAs of the grid; `target` arrivals in total.  A CTA in which a wait ran out
@@ -149,7 +150,7 @@ __global__ void __launch_bounds__(kSimtThreads, 1)
   coop_barrier(g.ctl, (unsigned)G, failed);
 
   int outcome = 0, it = 0;
-  if (*(volatile int*)&g.ctl->over_neg > 1 << 30) outcome = 3;  // an entry; 2^30 is step 0's
+  if (*(volatile int*)&g.ctl->over_neg > 1 << 30) outcome = 4;  // an entry; 2^30 is step 0's
   uint32_t base = 0;  // loads of the steps before
   while (!outcome && !*failed) {
     const int cur = it & 1;
@@ -292,7 +293,7 @@ __global__ void __launch_bounds__(kSimtThreads, 1)
     }
     return;
   }
-  if (outcome != 3) {  // X from its codes
+  if (outcome < 3) {  // X from its codes
     const uint16_t* R = it & 1 ? g.Xc[1] : g.Xc[0];
     const bool vec = (g.ldx % 4 == 0) && (reinterpret_cast<uintptr_t>(g.X) % 16 == 0);
     const int quads = (n + 3) >> 2;

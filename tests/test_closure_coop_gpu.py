@@ -56,6 +56,19 @@ def test_without_codes(cuda, case):
     same(X, want, case)
 
 
+@pytest.mark.parametrize("op", ["min_plus", "max_min"])
+@pytest.mark.parametrize("n", [130, 700])
+def test_entry_without_code_goes_on_in_fp32(cuda, op, n):
+    """One fraction, then all fractions; on either side of the tile sizes."""
+    x = graph(op, n, 8.0 / n, n)
+    for x in (np.where(np.arange(n * n).reshape(n, n) == 2, np.float32(0.3), x), x + np.float32(0.3)):
+        want, steps = oracle.closure(op, x)
+        X = torch.from_numpy(x.copy()).cuda()
+        assert s2.closure(op, X) == steps
+        same(X, want, f"{op} {n}")
+    assert s2.device_status() == 0
+
+
 @pytest.mark.parametrize("op", ["min_plus", "max_plus"])
 @pytest.mark.parametrize("n", [90, 200, 500, 1100])
 def test_first_squaring_outgrows_codes(cuda, op, n):
