@@ -67,10 +67,9 @@ enum BatchKind { kStep16 = 1, kPrep32 = 2, kStep32 = 3 };
 
 // Cleared before every run.
 struct BatchState {
-  int bad;      // an entry has no code (set by the prep kernel)
-  int done;     // tiles of the open step finished
-  int changed;  // the open step changed something
-  int over;     // a result of the open step has no code
+  int bad;       // an entry has no code (set by the prep kernel)
+  int done;      // tiles of the open step finished
+  int flags[2];  // the open step changed something; a result of it has no code
 };
 struct BatchCtl {
   unsigned next;             // slots claimed (8-byte aligned pair with `open`)
@@ -144,6 +143,11 @@ __device__ __forceinline__ bool batch_claim(const BatchArgs& a, unsigned& t) {
   return true;
 }
 
+// What a graph begins with: without codes it was prepared in FP32 before the launch.
+__device__ __forceinline__ int batch_first_kind(const BatchArgs& a, int graph) {
+  return !a.use_codes ? kStep32 : __ldcg(&a.state[graph].bad) ? kPrep32 : kStep16;
+}
+
 // The task of claimed slot t, if it is written; one thread.
 __device__ __forceinline__ bool batch_task_of(const BatchArgs& a, unsigned t, BatchTask& k) {
   if (t >= a.cap) return false;
@@ -153,7 +157,7 @@ __device__ __forceinline__ bool batch_task_of(const BatchArgs& a, unsigned t, Ba
   k.tile = (int)(v >> 20 & (kBatchSlotMax - 1));
   k.step = (int)(v >> 40 & 1023);
   k.kind = (int)(v >> 50 & 3);
-  if (k.kind == 0) k.kind = a.use_codes && !__ldcg(&a.state[k.graph].bad) ? kStep16 : kPrep32;
+  if (k.kind == 0) k.kind = batch_first_kind(a, k.graph);
   k.n = __ldg(&a.graphs[k.graph].n);
   k.pre = 0;
   k.alone = 0;
@@ -186,7 +190,7 @@ __device__ __forceinline__ void batch_pop(const BatchArgs& a, unsigned& slot, Ba
         t.graph = a.order[a.nbig + q];
         t.n = a.graphs[t.graph].n;
         t.tile = 0;
-        t.kind = a.use_codes && !__ldcg(&a.state[t.graph].bad) ? kStep16 : kPrep32;
+        t.kind = batch_first_kind(a, t.graph);
         t.step = 0;
         t.pre = 0;
         t.alone = 1;
@@ -243,6 +247,22 @@ __device__ __forceinline__ void batch_issue(const BatchCta& x, uint32_t j, const
   tma_load_2d(sa + Cfg::kTileBytes, I16 ? &mp->bc[cur] : &mp->b[cur], &x.full[s], I16 ? n0 : 2 * n0, i * (BK / 2));
 }
 
+// One FP32 k-tile of the first `groups` of a tile's eight 16-row groups.
+template <int OP>
+__device__ __forceinline__ void batch_rows32(int groups, float (&acc)[8][4], const uint8_t* As, const uint8_t* Bs,
+                                             int ty, int tx, int cbase, int nq) {
+  switch (groups) {
+    case 1: sk_ktile32<OP, 128, false, 1>(acc, As, Bs, ty, tx, cbase, 0, nq); break;
+    case 2: sk_ktile32<OP, 128, false, 2>(acc, As, Bs, ty, tx, cbase, 0, nq); break;
+    case 3: sk_ktile32<OP, 128, false, 3>(acc, As, Bs, ty, tx, cbase, 0, nq); break;
+    case 4: sk_ktile32<OP, 128, false, 4>(acc, As, Bs, ty, tx, cbase, 0, nq); break;
+    case 5: sk_ktile32<OP, 128, false, 5>(acc, As, Bs, ty, tx, cbase, 0, nq); break;
+    case 6: sk_ktile32<OP, 128, false, 6>(acc, As, Bs, ty, tx, cbase, 0, nq); break;
+    case 7: sk_ktile32<OP, 128, false, 7>(acc, As, Bs, ty, tx, cbase, 0, nq); break;
+    default: sk_ktile32<OP, 128, false>(acc, As, Bs, ty, tx, cbase, 0, nq); break;
+  }
+}
+
 // One tile of step `step`: X[nxt] (+)= on both layouts.  `pre` loads are already
 // on their way; before_last() runs on every thread before the last k-tile,
 // before_epilogue() after it.
@@ -272,9 +292,10 @@ __device__ __forceinline__ void batch_tile(const BatchArgs& a, BatchCta& x, cons
       if constexpr (I16) acc[i][c] = Code16<OP>::kIdent;
       else acc[i][c] = Mac<OP>::identity();
     }
-  // What lies past the graph is not computed: 16-row groups by halves of the
-  // register tile, and the warps of the upper column half.
-  const int rows = n - m0 <= 32 ? 2 : n - m0 <= 64 ? 4 : 8;
+  // What lies past the graph is not computed: 16-row groups (on codes by halves of
+  // the register tile), and the warps of the upper column half.
+  const int groups = min(8, (n - m0 + 15) >> 4);
+  const int rows = groups <= 2 ? 2 : groups <= 4 ? 4 : 8;
   const bool idle = n0 + cbase >= n;
   for (int i = 0; i < units; i++) {
     const uint32_t j = x.base + i;
@@ -293,10 +314,8 @@ __device__ __forceinline__ void batch_tile(const BatchArgs& a, BatchCta& x, cons
         else if (rows == 4) sk_ktile16<OP, 128, false, 4>(acc, As, Bs, ty, tx, cbase, 0, min(nq, 8));
         else sk_ktile16<OP, 128, false, 2>(acc, As, Bs, ty, tx, cbase, 0, min(nq, 8));
       } else {
-        if (rows == 8 && nq >= 8) sk_ktile32<OP, 128, true>(acc, As, Bs, ty, tx, cbase, 0, 8);
-        else if (rows == 8) sk_ktile32<OP, 128, false>(acc, As, Bs, ty, tx, cbase, 0, nq);
-        else if (rows == 4) sk_ktile32<OP, 128, false, 4>(acc, As, Bs, ty, tx, cbase, 0, min(nq, 8));
-        else sk_ktile32<OP, 128, false, 2>(acc, As, Bs, ty, tx, cbase, 0, min(nq, 8));
+        if (groups == 8 && nq >= 8) sk_ktile32<OP, 128, true>(acc, As, Bs, ty, tx, cbase, 0, 8);
+        else batch_rows32<OP>(groups, acc, As, Bs, ty, tx, cbase, min(nq, 8));
       }
     }
     __syncwarp();
@@ -405,26 +424,60 @@ __device__ __forceinline__ void batch_tile(const BatchArgs& a, BatchCta& x, cons
   }
 }
 
-// One tile of the FP32 preparation: X[0] and P[0] from the caller's matrix with
-// NaN padding, and the padding of X[1] and P[1] (steps write the rest).
-__device__ __forceinline__ void batch_prep_tile(const BatchGraph& G, int tile) {
-  const int n = G.n, tm = batch_tiles_1d(n);
-  const int m0 = (tile % tm) * 128, n0 = (tile / tm) * 128;
-  const float nanv = __int_as_float(0x7fc00000);
-  for (int t = threadIdx.x; t < 128 * 128; t += kSimtThreads) {
-    const int r = m0 + (t >> 7), c = n0 + (t & 127);
-    const bool in = r < n && c < n;
-    const float v = in ? G.user[(long long)r * G.ldu + c] : nanv;
-    if (c < G.Kp) {
-      G.X[0][(long long)r * G.Kp + c] = v;
-      if (!in) G.X[1][(long long)r * G.Kp + c] = nanv;
-    }
-    if (r < G.Kp) {
-      const long long o = (long long)(r >> 1) * (2LL * G.Np) + 2 * c + (r & 1);
-      G.P[0][o] = v;
-      if (!in) G.P[1][o] = nanv;
+// 2 rows x 4 columns of a caller's matrix (from row 2 p, column c0), `fill` past it.
+__device__ __forceinline__ void batch_load2x4(const BatchGraph& G, int p, int c0, bool vec, float fill,
+                                              float (&v)[2][4]) {
+#pragma unroll
+  for (int r = 0; r < 2; r++) {
+    const int row = 2 * p + r;
+    const float* src = G.user + (long long)row * G.ldu + c0;
+    if (vec && row < G.n && c0 + 4 <= G.n) {
+      load4(src, v[r]);
+    } else {
+#pragma unroll
+      for (int e = 0; e < 4; e++) v[r][e] = row < G.n && c0 + e < G.n ? src[e] : fill;
     }
   }
+}
+__device__ __forceinline__ bool batch_vec4(const BatchGraph& G) {
+  return (G.ldu % 4 == 0) && (reinterpret_cast<uintptr_t>(G.user) % 16 == 0);
+}
+
+// The FP32 preparation of row pairs [p0, p1) and columns [c0, c1) (multiples of 4,
+// below Kp), `thread` of `threads`: X[0] and P[0] from the caller's matrix, NaN in
+// the k past it, and those of X[1] and P[1] (steps write the rest).  Rows of A and
+// columns of B past the graph only reach outputs that are never stored.
+__device__ __forceinline__ void batch_prep32(const BatchGraph& G, int p0, int p1, int c0, int c1, int thread,
+                                             int threads) {
+  const bool vec = batch_vec4(G);
+  const int n = G.n, quads = (c1 - c0) >> 2, items = max(0, p1 - p0) * max(0, quads);
+  for (int t = thread; t < items; t += threads) {
+    const int p = p0 + t / quads, c = c0 + (t % quads) * 4;
+    float v[2][4];
+    batch_load2x4(G, p, c, vec, __int_as_float(0x7fc00000), v);
+#pragma unroll
+    for (int r = 0; r < 2; r++) {
+      const long long o = (long long)(2 * p + r) * G.Kp + c;
+      const float4 w = make_float4(v[r][0], v[r][1], v[r][2], v[r][3]);
+      *reinterpret_cast<float4*>(G.X[0] + o) = w;
+      if (c + 4 > n) *reinterpret_cast<float4*>(G.X[1] + o) = w;
+    }
+    const long long o = (long long)p * (2LL * G.Np) + 2 * c;
+    const float4 w0 = make_float4(v[0][0], v[1][0], v[0][1], v[1][1]);
+    const float4 w1 = make_float4(v[0][2], v[1][2], v[0][3], v[1][3]);
+    *reinterpret_cast<float4*>(G.P[0] + o) = w0;
+    *reinterpret_cast<float4*>(G.P[0] + o + 4) = w1;
+    if (2 * p + 1 >= n) {
+      *reinterpret_cast<float4*>(G.P[1] + o) = w0;
+      *reinterpret_cast<float4*>(G.P[1] + o + 4) = w1;
+    }
+  }
+}
+
+// One tile of it, for a graph that leaves its codes.
+__device__ __forceinline__ void batch_prep_tile(const BatchGraph& G, int tile) {
+  const int tm = batch_tiles_1d(G.n), m0 = (tile % tm) * 128, n0 = (tile / tm) * 128;
+  batch_prep32(G, m0 >> 1, min(m0 + 128, G.Kp) >> 1, n0, min(n0 + 128, G.Kp), threadIdx.x, kSimtThreads);
 }
 
 template <int OP>
@@ -441,6 +494,7 @@ __global__ void __launch_bounds__(kSimtThreads, 1) closure_batched_kernel(BatchA
   // iteration's last barrier, so it is written only past the next one's first.
   __shared__ BatchTask s_opened;
   __shared__ unsigned s_first;    // its first slot
+  __shared__ int s_flags[2];      // BatchState::flags of the graph this CTA runs alone
   BatchCta x;
   x.smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   x.full = reinterpret_cast<uint64_t*>(x.smem + Cfg::kStages * Cfg::kStage + Cfg::kRedBytes);
@@ -459,6 +513,7 @@ __global__ void __launch_bounds__(kSimtThreads, 1) closure_batched_kernel(BatchA
     s_task.alone = 0;
     s_opened.graph = -1;
     s_nown = 0;
+    s_flags[0] = s_flags[1] = 0;
   }
   __syncthreads();
   while (true) {
@@ -525,10 +580,14 @@ __global__ void __launch_bounds__(kSimtThreads, 1) closure_batched_kernel(BatchA
         batch_tile<OP, false>(a, x, G, mp, task.n, task.step, task.tile, task.pre, changed, over, claim_early,
                               look_ahead);
     }
-    if (__any_sync(0xffffffffu, changed) && (threadIdx.x & 31) == 0) atomicOr(&st->changed, 1);
-    if (__any_sync(0xffffffffu, over) && (threadIdx.x & 31) == 0) atomicOr(&st->over, 1);
+    // The outcome of a graph that this CTA runs alone stays in shared memory, and its
+    // writes only have to be ordered for this CTA (the flags in global memory and the
+    // wider fence cost a step of a small graph about 3 us).
+    int* flags = task.alone ? s_flags : st->flags;
+    if (__any_sync(0xffffffffu, changed) && (threadIdx.x & 31) == 0) atomicOr(&flags[0], 1);
+    if (__any_sync(0xffffffffu, over) && (threadIdx.x & 31) == 0) atomicOr(&flags[1], 1);
     fence_proxy_async_global();  // this tile's generic writes, before any TMA read of them
-    __threadfence();
+    if (!task.alone) __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) {
       const int tiles = batch_tiles_1d(task.n) * batch_tiles_1d(task.n);
@@ -537,8 +596,8 @@ __global__ void __launch_bounds__(kSimtThreads, 1) closure_batched_kernel(BatchA
         if (task.alone && s_next.graph < 0) s_task.tile++;  // a preparation tile
       } else {
         // the step's last tile: decide and open what follows
-        __threadfence();
-        const int ch = *(volatile int*)&st->changed, ov = *(volatile int*)&st->over;
+        if (!task.alone) __threadfence();
+        const int ch = *(volatile int*)&flags[0], ov = *(volatile int*)&flags[1];
         int kind = task.kind, step = task.step + 1;
         bool closed = false;
         if (kind == kPrep32) {
@@ -550,7 +609,8 @@ __global__ void __launch_bounds__(kSimtThreads, 1) closure_batched_kernel(BatchA
         } else {
           closed = !ch || step >= a.max_iter;
         }
-        st->done = st->changed = st->over = 0;
+        flags[0] = flags[1] = 0;
+        if (!task.alone) st->done = 0;
         if (closed) {
           G.iters = step;
           G.changed = ch;
@@ -607,31 +667,27 @@ __global__ void __launch_bounds__(256) batched_prep_kernel(BatchArgs a) {
       G.changed = G.n != 0;
       G.coded = -1;
     }
+    if (!a.use_codes) {
+      batch_prep32(G, 0, G.Kp >> 1, 0, G.Kp, blockIdx.x * 256 + threadIdx.x, gridDim.x * 256);
+      continue;
+    }
     if constexpr (Code16<OP>::kHas) {
-      if (!a.use_codes) continue;
       const int n = G.n, Kh = G.Kh, Np = G.Np;
       const int quads = Np >> 2;
       const long long total = (long long)(Kh >> 1) * quads;
-      const bool vec = (G.ldu % 4 == 0) && (reinterpret_cast<uintptr_t>(G.user) % 16 == 0);
+      const bool vec = batch_vec4(G);
       bool bad = false;
       for (long long t = blockIdx.x * 256LL + threadIdx.x; t < total; t += gridDim.x * 256LL) {
         const int p = (int)(t / quads), c0 = (int)(t - (long long)p * quads) * 4;
         uint32_t c[2][4];
+        float v[2][4];
+        batch_load2x4(G, p, c0, vec, 0.f, v);
 #pragma unroll
         for (int r = 0; r < 2; r++) {
           const int row = 2 * p + r;
-          const float* src = G.user + (long long)row * G.ldu + c0;
-          float v[4];
-          if (vec && row < n && c0 + 4 <= n) {
-            const float4 u = __ldg(reinterpret_cast<const float4*>(src));
-            v[0] = u.x, v[1] = u.y, v[2] = u.z, v[3] = u.w;
-          } else {
-#pragma unroll
-            for (int e = 0; e < 4; e++) v[e] = row < n && c0 + e < n ? src[e] : 0.f;
-          }
 #pragma unroll
           for (int e = 0; e < 4; e++)
-            c[r][e] = row < n && c0 + e < n ? Code16<OP>::encode(v[e], bad) : Code16<OP>::kPad;
+            c[r][e] = row < n && c0 + e < n ? Code16<OP>::encode(v[r][e], bad) : Code16<OP>::kPad;
           if (c0 < Kh) {
             const uint2 w = make_uint2(c[r][0] | c[r][1] << 16, c[r][2] | c[r][3] << 16);
             *reinterpret_cast<uint2*>(G.Xc[0] + (long long)row * Kh + c0) = w;
