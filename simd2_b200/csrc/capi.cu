@@ -1189,11 +1189,15 @@ int srgemm_f32_ws(int op, int M, int N, int K, const float* A, long long lda, co
   }
   const bool pack_a = !a_tma_ok(A, lda);
   // a caller's workspace holds the base plan only
-  const Plan plan = make_plan(M, N, K, pack_a, ws_or_null == nullptr, op);
+  Plan plan = make_plan(M, N, K, pack_a, ws_or_null == nullptr, op);
   uint8_t* ws = ws_or_null;
   if (!ws) {
     void* p = nullptr;
     int rc = get_workspace(stream, plan.total, &p);
+    if (rc == SIMD2_ERR_ALLOC && plan.code16) {  // no room for the codes beside the FP32 copies
+      plan = make_plan(M, N, K, pack_a, true, kNoCodes);
+      rc = get_workspace(stream, plan.total, &p);
+    }
     if (rc) return rc;
     ws = static_cast<uint8_t*>(p);
   }
@@ -1557,12 +1561,7 @@ int closure_f32_ex(int op, int n, float* X, long long ldx, int max_iter, int con
   const bool need_occ = dispatch == 2 || step_feat != nullptr || (fixed_skip && can_skip);
   // Workspace: [srgemm plan][Xnew n x n][flag + decision][occupancy]
   const bool pack_a = !a_tma_ok(X, ldx) || (n % 4 != 0);
-  const Plan plan = make_plan(n, n, n, pack_a, true, op);
   const OccPlan occ = make_occ_plan(n, n, n, true);
-  const size_t x_off = align_up(plan.total, kAlign);
-  const size_t f_off = x_off + align_up((size_t)n * n * 4, kAlign);
-  // flag word + learned decision (256 bytes), then one change flag per step
-  const size_t o_off = f_off + align_up(256 + (size_t)(max_iter + 1) * sizeof(int), kAlign);
   // Delta steps (see srgemm_simt_kernel, SKIP): the learned and rules loops of
   // a min_plus / max_plus closure with the exact change test keep, per step,
   // which 32 x 32 blocks changed, in two ping-pong pairs of maps laid out as
@@ -1572,10 +1571,20 @@ int closure_f32_ex(int op, int n, float* X, long long ldx, int max_iter, int con
                          (dispatch == 2 || dispatch == 3) && step_feat == nullptr;
   const size_t cmA = align_up((size_t)occ.tiles_m * occ.ktiles, kAlign);
   const size_t cmB = align_up((size_t)occ.ktiles * occ.tiles_n, kAlign);
-  const size_t c_off = o_off + (need_occ ? align_up(occ.total, kAlign) : 0);
-  const size_t total = c_off + (use_delta ? 2 * (cmA + cmB) : 0);
+  size_t x_off, f_off, o_off, c_off;
   void* p = nullptr;
-  if ((rc = get_workspace(stream, total, &p))) return rc;
+  while (true) {
+    const Plan plan = make_plan(n, n, n, pack_a, true, codes ? op : kNoCodes);
+    x_off = align_up(plan.total, kAlign);
+    f_off = x_off + align_up((size_t)n * n * 4, kAlign);
+    // flag word + learned decision (256 bytes), then one change flag per step
+    o_off = f_off + align_up(256 + (size_t)(max_iter + 1) * sizeof(int), kAlign);
+    c_off = o_off + (need_occ ? align_up(occ.total, kAlign) : 0);
+    rc = get_workspace(stream, c_off + (use_delta ? 2 * (cmA + cmB) : 0), &p);
+    if (rc != SIMD2_ERR_ALLOC || !plan.code16) break;
+    codes = false;  // no room for them
+  }
+  if (rc) return rc;
   uint8_t* ws = static_cast<uint8_t*>(p);
   float* Xn = reinterpret_cast<float*>(ws + x_off);
   int* flag = reinterpret_cast<int*>(ws + f_off);
@@ -1733,7 +1742,7 @@ int closure_f32_ex(int op, int n, float* X, long long ldx, int max_iter, int con
     }
     if (step_ms) cudaEventRecord(ev[0], stream);
     const bool pk = !a_tma_ok(cur, ldcur);
-    const Plan pl = make_plan(n, n, n, pk, true, op);
+    const Plan pl = make_plan(n, n, n, pk, true, codes ? op : kNoCodes);
     EpilogueArgs ep = make_epilogue(cur, ldcur, nxt, ldnxt, 1, flag, conv);
     if (use_delta) {
       if (cudaMemsetAsync(chg[par][0], 0, cmA + cmB, stream) != cudaSuccess) {
@@ -3069,12 +3078,18 @@ int simd2_srgemm_tuned(simd2_op op, int M, int N, int K, const float* A, int lda
   if ((rc = check_device())) return rc;
   if (K == 0) return srgemm_k0(op, M, N, C, ldc, D, ldd, do_epilogue, stream);
   const bool pack_a = !a_tma_ok(A, lda);
-  const Plan plan = make_plan(M, N, K, pack_a, true, op);
+  Plan plan = make_plan(M, N, K, pack_a, true, op);
   const bool skip = config_skip(config) && skip_supported(op) && (K + kBK - 1) / kBK <= kMaxSkipKtiles;
   const OccPlan occ = make_occ_plan(M, N, K, false);
-  const size_t o_off = align_up(plan.total, kAlign);
+  size_t o_off = align_up(plan.total, kAlign);
   void* p = nullptr;
-  if ((rc = get_workspace(stream, o_off + (skip ? occ.total : 0), &p))) return rc;
+  rc = get_workspace(stream, o_off + (skip ? occ.total : 0), &p);
+  if (rc == SIMD2_ERR_ALLOC && plan.code16) {  // no room for the codes
+    plan = make_plan(M, N, K, pack_a, true, kNoCodes);
+    o_off = align_up(plan.total, kAlign);
+    rc = get_workspace(stream, o_off + (skip ? occ.total : 0), &p);
+  }
+  if (rc) return rc;
   uint8_t* ws = static_cast<uint8_t*>(p);
   SimtConfig cfg;
   cfg.split = config_split(config);
@@ -3588,17 +3603,23 @@ extern "C" int simd2_closure_bf(simd2_op op, int n, const float* A0, int lda0, f
   if (n == 0 || max_iter == 0) return SIMD2_OK;
   int rc = check_device();
   if (rc) return rc;
-  const Plan plan = make_plan(n, n, n, true, true, op);
   const OccPlan occ = make_occ_plan(n, n, n, true);
-  const size_t x_off = align_up(plan.total, kAlign);
-  const size_t f_off = x_off + align_up((size_t)n * n * 4, kAlign);
-  const size_t total = f_off + align_up((size_t)(max_iter + 1) * sizeof(int), kAlign);
+  size_t x_off, f_off;
   void* p = nullptr;
-  if ((rc = get_workspace(stream, total, &p))) return rc;
+  bool codes = true;
+  while (true) {
+    const Plan plan = make_plan(n, n, n, true, true, codes ? op : kNoCodes);
+    x_off = align_up(plan.total, kAlign);
+    f_off = x_off + align_up((size_t)n * n * 4, kAlign);
+    rc = get_workspace(stream, f_off + align_up((size_t)(max_iter + 1) * sizeof(int), kAlign), &p);
+    if (rc != SIMD2_ERR_ALLOC || !plan.code16) break;
+    codes = false;  // no room for them
+  }
+  if (rc) return rc;
   uint8_t* ws = static_cast<uint8_t*>(p);
   return closure_gated(op, n, X, ldx, max_iter, conv, 0, false, false, false, occ, ws, x_off,
                        reinterpret_cast<int*>(ws + f_off), nullptr, iters_out, nullptr, nullptr, stream, A0,
-                       lda0);
+                       lda0, codes);
 }
 
 // ---------------------------------------------------------------------------
