@@ -1444,6 +1444,8 @@ int closure_coop(int op, int n, float* X, long long ldx, int max_iter, int conv,
   void* w = nullptr;
   int rc = get_workspace(stream, off, &w);
   if (rc) return rc;
+  HostBlock host;
+  if (!host.p) return SIMD2_OK;  // no page-locked memory to be had: the launch-per-step path needs none
   uint8_t* ws = static_cast<uint8_t*>(w);
   CoopArgs a{};
   a.X = X;
@@ -1465,8 +1467,6 @@ int closure_coop(int op, int n, float* X, long long ldx, int max_iter, int conv,
   a.part = reinterpret_cast<uint4*>(ws + part_off);
   a.ctl = reinterpret_cast<CoopCtl*>(ws + ctl_off);
   a.counters = reinterpret_cast<int*>(ws + cnt_off);
-  HostBlock host;
-  if (!host.p) return SIMD2_ERR_ALLOC;
   a.out = static_cast<volatile int*>(host.p);
   a.out[0] = a.out[1] = a.out[2] = 0;
   SIMD2_CUDA_TRY(cudaMemsetAsync(ws + ctl_off, 0, off - ctl_off, stream));
