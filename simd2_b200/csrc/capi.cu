@@ -749,7 +749,7 @@ int srgemm_core(int op, int M, int N, int K, const float* A, long long lda, cons
   if (cfg.split == 1) return launch_sk_op<float>(op, M, N, K, A, lda, B, ldb, ep, ws, plan, pack_a, c1, stream);
   const float pad = pad_value(op);
   float* Bp = reinterpret_cast<float*>(ws + plan.bp_off);
-  interleave_pairs_kernel<float, 0><<<grid_for((long long)plan.Kp / 2 * plan.Np / 4), 256, 0, stream>>>(
+  interleave_pairs_kernel<<<grid_for((long long)plan.Kp / 2 * plan.Np / 4), 256, 0, stream>>>(
       B, ldb, K, N, Bp, plan.Kp, plan.Np, pad, ep.gate);
   count_launch();
   SIMD2_CUDA_TRY(cudaGetLastError());
@@ -757,8 +757,7 @@ int srgemm_core(int op, int M, int N, int K, const float* A, long long lda, cons
   long long a_pitch = lda;
   if (pack_a) {
     float* Ap = reinterpret_cast<float*>(ws + plan.ap_off);
-    pack_rows_kernel<float, 0><<<grid_for((long long)M * plan.Kp), 256, 0, stream>>>(A, lda, M, K, Ap, plan.Kp, pad,
-                                                                                    ep.gate);
+    pack_rows_kernel<<<grid_for((long long)M * plan.Kp), 256, 0, stream>>>(A, lda, M, K, Ap, plan.Kp, pad, ep.gate);
     count_launch();
     SIMD2_CUDA_TRY(cudaGetLastError());
     a_base = Ap;
@@ -2050,14 +2049,13 @@ int simd2_closure_pred(simd2_op op, int n, float* X, int ldx, int32_t* P, int ld
     // interleaved, and A = X itself when its rows suit TMA (else a packed copy)
     transpose_f32_kernel<<<dim3((n + 31) / 32, (n + 31) / 32), dim3(32, 8), 0, stream>>>(n, Xc, ldc, XT, n);
     count_launch();
-    interleave_pairs_kernel<float, 0><<<grid_for((long long)Kp / 2 * Np / 4), 256, 0, stream>>>(Xc, ldc, n, n, Bp, Kp,
-                                                                                               Np, pad);
+    interleave_pairs_kernel<<<grid_for((long long)Kp / 2 * Np / 4), 256, 0, stream>>>(Xc, ldc, n, n, Bp, Kp, Np, pad);
     count_launch();
     const bool pack_a = !a_tma_ok(Xc, ldc) || (n % 4 != 0);
     const float* a_base = Xc;
     long long a_pitch = ldc;
     if (pack_a) {
-      pack_rows_kernel<float, 0><<<grid_for((long long)n * Kp), 256, 0, stream>>>(Xc, ldc, n, n, Ap, Kp, pad);
+      pack_rows_kernel<<<grid_for((long long)n * Kp), 256, 0, stream>>>(Xc, ldc, n, n, Ap, Kp, pad);
       count_launch();
       a_base = Ap;
       a_pitch = Kp;

@@ -12,23 +12,15 @@ namespace simd2 {
 // B'[p][2j+e] = B[2p+e][j] for 2p+e < K and j < N, else `pad`.
 // B' has Kp/2 rows of 2*Np floats (Kp, Np are the padded sizes); a float4 of
 // B' is (B[2p][j], B[2p+1][j], B[2p][j+1], B[2p+1][j+1]).
-template <typename T, int MODE>
-__device__ __forceinline__ float load_operand(const T* p) {
-  if constexpr (MODE == 1) return (*p != T(0)) ? 1.0f : 0.0f;  // boolean (or_and as max_min on {0,1})
-  else return static_cast<float>(*p);
-}
-
-// A thread fills 4 columns (two float4 stores); float B with 16-byte aligned
-// rows is read with one float4 load per k row where the 4 columns are in range.
-template <typename T, int MODE>
-__global__ void interleave_pairs_kernel(const T* __restrict__ B, long long ldb, int K, int N,
+// A thread fills 4 columns (two float4 stores); B with 16-byte aligned rows is
+// read with one float4 load per k row where the 4 columns are in range.
+__global__ void interleave_pairs_kernel(const float* __restrict__ B, long long ldb, int K, int N,
                                         float* __restrict__ Bp, int Kp, int Np, float pad,
                                         const int* gate = nullptr) {
   if (gate && *gate == 0) return;
   const long long quads = Np / 4;
   const long long total = (long long)(Kp / 2) * quads;
-  constexpr bool kFloat = std::is_same<T, float>::value && MODE == 0;
-  const bool vec = kFloat && (ldb % 4 == 0) && (reinterpret_cast<uintptr_t>(B) % 16 == 0);
+  const bool vec = (ldb % 4 == 0) && (reinterpret_cast<uintptr_t>(B) % 16 == 0);
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
        t += (long long)gridDim.x * blockDim.x) {
     const int p = (int)(t / quads);
@@ -37,16 +29,13 @@ __global__ void interleave_pairs_kernel(const T* __restrict__ B, long long ldb, 
 #pragma unroll
     for (int r = 0; r < 2; r++) {
       const int k = 2 * p + r;
-      if constexpr (kFloat) {
-        if (vec && k < K && j + 4 <= N) {
-          const float4 u = __ldg(reinterpret_cast<const float4*>(reinterpret_cast<const float*>(B) + (long long)k * ldb + j));
-          x[r][0] = u.x, x[r][1] = u.y, x[r][2] = u.z, x[r][3] = u.w;
-          continue;
-        }
+      if (vec && k < K && j + 4 <= N) {
+        const float4 u = __ldg(reinterpret_cast<const float4*>(B + (long long)k * ldb + j));
+        x[r][0] = u.x, x[r][1] = u.y, x[r][2] = u.z, x[r][3] = u.w;
+        continue;
       }
 #pragma unroll
-      for (int e = 0; e < 4; e++)
-        x[r][e] = (k < K && j + e < N) ? load_operand<T, MODE>(B + (long long)k * ldb + j + e) : pad;
+      for (int e = 0; e < 4; e++) x[r][e] = (k < K && j + e < N) ? B[(long long)k * ldb + j + e] : pad;
     }
     float4* o = reinterpret_cast<float4*>(Bp) + 2 * t;
     o[0] = make_float4(x[0][0], x[1][0], x[0][1], x[1][1]);
@@ -55,10 +44,8 @@ __global__ void interleave_pairs_kernel(const T* __restrict__ B, long long ldb, 
 }
 
 // Dense copy of A into an [M][Kp] float panel (row pitch Kp), padding k >= K
-// with `pad`.  Used when A's rows are not 16-byte aligned for TMA, or when A
-// must be converted (or_and inputs).
-template <typename T, int MODE>
-__global__ void pack_rows_kernel(const T* __restrict__ A, long long lda, int M, int K, float* __restrict__ Ap,
+// with `pad`, for an A whose rows are not 16-byte aligned for TMA.
+__global__ void pack_rows_kernel(const float* __restrict__ A, long long lda, int M, int K, float* __restrict__ Ap,
                                  int Kp, float pad, const int* gate = nullptr) {
   if (gate && *gate == 0) return;
   const long long total = (long long)M * Kp;
@@ -66,7 +53,7 @@ __global__ void pack_rows_kernel(const T* __restrict__ A, long long lda, int M, 
        t += (long long)gridDim.x * blockDim.x) {
     const int i = (int)(t / Kp);
     const int k = (int)(t - (long long)i * Kp);
-    Ap[t] = k < K ? load_operand<T, MODE>(A + (long long)i * lda + k) : pad;
+    Ap[t] = k < K ? A[(long long)i * lda + k] : pad;
   }
 }
 

@@ -23,9 +23,8 @@
 //   * The epilogue applies (+) C, writes D with coalesced 8-byte stores and,
 //     for the closure, sets one change flag per warp (warp vote + atomicOr).
 //
-// Out-of-range k is filled with NaN for the min/max semirings (TMA OOB fill
-// for A, explicit padding for B'): a NaN product is dropped by min/max, so the
-// tail adds nothing.  The summing semirings use zero fill.
+// Out-of-range k is filled with NaN (TMA OOB fill for A, explicit padding for
+// B'): a NaN product is dropped by min/max, so the tail adds nothing.
 #pragma once
 #include "common.cuh"
 
@@ -54,25 +53,6 @@ struct Mac {
   }
   __device__ static float identity() { return Semiring<OP>::identity(); }
   __device__ static float add(float acc, float p) { return Semiring<OP>::add(acc, p); }
-};
-
-// plus_mul on CUDA cores (reference-precision FP32 path).
-template <>
-struct Mac<SIMD2_PLUS_MUL> {
-  __device__ static float mac2(float acc, float2 a, float2 b) { return fmaf(a.y, b.y, fmaf(a.x, b.x, acc)); }
-  __device__ static float identity() { return 0.0f; }
-  __device__ static float add(float acc, float p) { return __fadd_rn(acc, p); }
-};
-
-// minus_square on CUDA cores: sum_k (a-b)^2.
-template <>
-struct Mac<SIMD2_MINUS_SQUARE> {
-  __device__ static float mac2(float acc, float2 a, float2 b) {
-    const float2 d = __fadd2_rn(a, make_float2(-b.x, -b.y));
-    return fmaf(d.y, d.y, fmaf(d.x, d.x, acc));
-  }
-  __device__ static float identity() { return 0.0f; }
-  __device__ static float add(float acc, float p) { return __fadd_rn(acc, p); }
 };
 
 struct EpilogueArgs {
