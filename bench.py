@@ -734,7 +734,7 @@ def main():
 
     if args.workload == "orand":
         # one or_and reachability closure per rank (independent replicas), the
-        # configuration-4 graph: CSR steps while X is sparse, then INT8 delta steps
+        # configuration-4 graph: CSR steps while X is sparse, then FP4 delta steps
         n = args.rowpanel_n
         rng = np.random.default_rng(44)
         m = 2 * n

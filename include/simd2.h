@@ -126,12 +126,13 @@ int simd2_closure_orand_u8(int n, uint8_t* X, int ldx, int max_iter,
                            int* iters_out, cudaStream_t stream);
 
 /* Batched closure: `count` independent n[g] x n[g] matrices X[g] (device
- * pointers, row pitch ldx[g]) closed in place in ONE persistent kernel launch,
- * each graph by one CTA until its own fixed point (per-graph convergence,
- * bit-exact per graph, same iteration counts as simd2_closure).  Six min/max
+ * pointers, row pitch ldx[g]) closed in place in ONE persistent kernel launch
+ * that hands the tiles of all graphs out to the SMs, each graph until its own
+ * fixed point (per-graph convergence, bit-exact per graph, same iteration
+ * counts as simd2_closure; n[g] = 0 is one unchanged step).  Six min/max
  * semirings.  X, n and ldx are host arrays.
- *   plan_create  allocates the plan's device memory and uploads descriptors
- *                (synchronous);
+ *   plan_create  allocates the plan's device memory (about 16 bytes an element)
+ *                and uploads descriptors (synchronous);
  *   plan_run     launches prep + persistent closure + copy-back on `stream`
  *                and nothing else (no allocation, no host sync), so it can be
  *                captured in a CUDA graph and replayed;
@@ -253,9 +254,10 @@ int simd2_knn_ex(const float* query, int Q, int ldq, const float* ref, int R, in
                  float* out_dist, int32_t* out_idx, int ldo, int mode, cudaStream_t stream);
 
 /* srgemm with FP16 A and B (row-major, __half*), FP32 C and D: the entry
- * behind tensor_srgemm (kernel/tensor_srgemm.cuh:197-218).  The halves are
- * widened to FP32 exactly and the FP32 engine runs; or_and treats any
- * nonzero as true and writes 0/1.  (The reference's FP16 emulation kernel
+ * behind tensor_srgemm (kernel/tensor_srgemm.cuh:197-218).  plus_mul
+ * and minus_square multiply the halves on the tensor cores with FP32 sums,
+ * or_and treats any nonzero as true and writes 0/1, and the min/max semirings
+ * compute as on the halves widened to FP32.  (The reference's FP16 emulation kernel
  * rounds each product to FP16 and starts the max semirings from 0; this
  * entry keeps FP32 products and the true identities.) */
 int simd2_srgemm_f16(simd2_op op, int M, int N, int K, const void* A, int lda, const void* B, int ldb,

@@ -179,7 +179,8 @@ def srgemm_f16(op: str, A: torch.Tensor, B: torch.Tensor, C: torch.Tensor | None
                D: torch.Tensor | None = None, stream=None) -> torch.Tensor:
     """srgemm with float16 A and B and float32 C / D: the entry behind the
     reference's ``tensor_srgemm`` (kernel/tensor_srgemm.cuh:197-218).  The
-    halves are widened exactly; or_and reads any nonzero as true and writes 0/1."""
+    sums multiply the halves with FP32 accumulation, the min/max semirings
+    compute as on the halves widened; or_and reads any nonzero as true and writes 0/1."""
     M, K = A.shape
     K2, N = B.shape
     if K != K2:

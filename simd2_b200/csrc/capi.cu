@@ -1561,7 +1561,7 @@ int closure_f32_ex(int op, int n, float* X, long long ldx, int max_iter, int con
   // Workspace: [srgemm plan][Xnew n x n][flag + decision][occupancy]
   const bool pack_a = !a_tma_ok(X, ldx) || (n % 4 != 0);
   const OccPlan occ = make_occ_plan(n, n, n, true);
-  // Delta steps (see srgemm_simt_kernel, SKIP): the learned and rules loops of
+  // Delta steps (see srgemm_sk_skip_kernel): the learned and rules loops of
   // a min_plus / max_plus closure with the exact change test keep, per step,
   // which 32 x 32 blocks changed, in two ping-pong pairs of maps laid out as
   // the occupancy maps.  Recording runs (autotuner timings per configuration)
@@ -1700,8 +1700,8 @@ int closure_f32_ex(int op, int n, float* X, long long ldx, int max_iter, int con
   int cfg_id = default_cfg;
   // Closure steps only fill X in: once every (tile, k-tile) block triple is
   // occupied, no later step can skip anything, so the learned and rules loops
-  // stop the statistics pass and keep the split factor of the last choice
-  // without skipping (feature recording keeps the pass).
+  // stop the statistics pass and go on without skipping (feature recording
+  // keeps the pass).
   const unsigned long long all_triples = (unsigned long long)occ.tiles_m * occ.tiles_n * occ.ktiles;
   bool occ_on = need_occ;
   // occ_fresh: the occupancy maps hold this step's input; occ_full: every

@@ -16,8 +16,8 @@
 //                     a 4-deep ring of 32 KiB stages,
 //   warp 1 lane 0  -- MMA issuer, which also fetches each tile's reference norms
 //                     into shared memory (from L2 the selection warps waited for
-//                     them 32 columns at a time: 16384 x 65536 x 128, k = 16, 731 us
-//                     a call for 719): per reference tile q.r ~ qh.rh + qh.rl + ql.rh
+//                     them 32 columns at a time; within a call's spread at 16384 x
+//                     65536 x 128): per reference tile q.r ~ qh.rh + qh.rl + ql.rh
 //                     (tcgen05.mma kind::f16, M=128, N=256, FP32 accumulate)
 //                     into one of two TMEM accumulators (2 x 256 columns), so
 //                     the MMAs of tile t+1 run while tile t is selected,
@@ -35,7 +35,6 @@
 // earlier chunk of the same queries); everything else costs an FADD, an FFMA
 // and a compare.
 //
-// Each unit writes, per query, two sorted lists of k (one per column half);
 // WIDE (D > 128): the query panels no longer fit beside the ring, so they come
 // through it as well, one stage (hi and lo, 16 KiB each) before the two of the
 // reference panel, again for every tile: 96 KiB a K panel for its 1536 cycles of
@@ -43,6 +42,7 @@
 // block and this way (us): 2000 x 20000 x 300, k = 20, 652 / 183; 16384 x 65536 x
 // 136, k = 8, 4916 / 1025; 1000 x 4000 x 200, k = 8, 77 / 69.
 //
+// Each unit writes, per query, two sorted lists of k (one per column half);
 // knn_merge_kernel merges the 2 x chunks lists of a query by (distance,
 // index) and writes the k results with their square roots.  Ties keep the
 // lower reference index first, the order of apps/pld/emulation/knncuda.cu:

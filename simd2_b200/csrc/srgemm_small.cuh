@@ -4,9 +4,9 @@
 // and B as they lie: no operand preparation, no tensor maps, several CTAs on an
 // SM.  A thread holds 2 x 2 outputs and folds two k at a time (Mac<OP>::mac2, the
 // same operations as srgemm_sk.cuh on FP32, so the same bits).  What bounds such a
-// call is the launch and the latency of the first loads: 100^3 takes 5.3 us here
-// and 11.4 as prep + persistent kernel, 256^3 7.6 and 14.3; from about 450^3 on the
-// larger register tiles and the 16-bit codes win.
+// call is the launch and the latency of the first loads: 100^3 takes 4.3 us here
+// and 13.0 as prep + persistent kernel, 384^3 9.6 and 15.0; from about 450^3 on the
+// larger register tiles and the 16-bit codes win (see small_product in capi.cu).
 #pragma once
 #include "srgemm_sk.cuh"
 
