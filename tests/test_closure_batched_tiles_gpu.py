@@ -112,6 +112,33 @@ def test_outgrows_codes(cuda, n):
     check("min_plus", [chain, datagen.er_graph(n, 0.1, seed=3), big, frac, datagen.er_graph(40, 0.1, seed=4)])
 
 
+@pytest.mark.parametrize("n", [45, 113, 300])
+def test_runs_of_one_plan_take_turns(cuda, n):
+    """Codes and FP32 operands share their memory: one plan run on graphs that stay
+    on codes, that outgrow them, that have none, and on codes again."""
+    coded = datagen.er_graph(n, 0.1, seed=n)
+    heavy = np.full((n, n), np.inf, np.float32)
+    np.fill_diagonal(heavy, 0.0)
+    heavy[np.arange(n - 1), np.arange(1, n)] = 6000.0
+    frac = coded + np.float32(0.25)
+    first, second = torch.empty((n, n), device=cuda), torch.empty((n, n), device=cuda)
+    plan = s2.BatchedClosure("min_plus", [first, second])
+    graphs = {id(g): (g,) + oracle.closure("min_plus", g) for g in (coded, heavy, frac)}
+    for a, b in ((coded, frac), (heavy, coded), (frac, heavy), (coded, coded), (heavy, frac)):
+        first.copy_(torch.from_numpy(a))
+        second.copy_(torch.from_numpy(b))
+        plan.run()
+        torch.cuda.synchronize()
+        its, not_converged = plan.iters()
+        assert not_converged == 0
+        for m, g, it in ((first, a, its[0]), (second, b, its[1])):
+            _, want, steps = graphs[id(g)]
+            assert it == steps
+            same(m, want)
+    plan.close()
+    assert s2.device_status() == 0
+
+
 @pytest.mark.parametrize("op", ["min_plus", "max_min", "max_mul"])
 def test_plan_memory(cuda, op):
     """Both operand layouts of X, twice: 16 bytes an element, codes or not."""
