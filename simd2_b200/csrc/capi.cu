@@ -1547,8 +1547,8 @@ int closure_f32_ex(int op, int n, float* X, long long ldx, int max_iter, int con
   // A small closure on codes: one cooperative launch (recorded ones keep a launch
   // per step, whose times and configurations they ask for, and so do sizes with an
   // installed split factor).
-  bool codes = true;
-  if (dispatch == 0 && n <= kCoopMaxN && has_code16(op) && conv != SIMD2_CONV_APLP && !step_cfg && !step_ms &&
+  bool codes = conv != SIMD2_CONV_APLP;  // its change test writes -FLT_MAX, which has no code
+  if (dispatch == 0 && n <= kCoopMaxN && has_code16(op) && codes && !step_cfg && !step_ms &&
       !step_feat && dense_split(n) == 1) {
     bool done = false;
     rc = closure_coop(op, n, X, ldx, max_iter, conv, iters_out, &done, &codes, stream);
@@ -3604,7 +3604,7 @@ extern "C" int simd2_closure_bf(simd2_op op, int n, const float* A0, int lda0, f
   const OccPlan occ = make_occ_plan(n, n, n, true);
   size_t x_off, f_off;
   void* p = nullptr;
-  bool codes = true;
+  bool codes = conv != SIMD2_CONV_APLP;
   while (true) {
     const Plan plan = make_plan(n, n, n, true, true, codes ? op : kNoCodes);
     x_off = align_up(plan.total, kAlign);
