@@ -12,8 +12,8 @@
 // CTA, so the waits end; they are bounded all the same.  With one CTA per graph,
 // the largest graph's chain of steps set the time of a batch whose other graphs
 // left SMs idle long before: 512 graphs of up to 1024 vertices, min_plus,
-// 54-59 ms, now 10.5 ms (on codes); 4096 such graphs, 148 ms, now 89 ms.  The
-// arithmetic is 7 of the 10.5 ms; the rest is about 9 us a tile for the
+// 54-59 ms, now 10.3 ms (on codes); 4096 such graphs, 148 ms, now 87 ms.  The
+// arithmetic is 7 of the 10.3 ms; the rest is about 9 us a tile for the
 // epilogue, the fences and the claim, against 18 us of arithmetic for a tile of
 // a 256-vertex graph and 73 us of a 1024-vertex one.
 //
