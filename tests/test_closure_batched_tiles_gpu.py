@@ -139,6 +139,25 @@ def test_runs_of_one_plan_take_turns(cuda, n):
     assert s2.device_status() == 0
 
 
+@pytest.mark.parametrize("op", ["max_plus", "max_min"])
+def test_aplp_change_test(cuda, op):
+    """The change test that writes -FLT_MAX keeps a plan on FP32 from the start."""
+    graphs = []
+    for n in (45, 130, 300):
+        x = datagen.closure_graph("max_min", n, 6.0 / n, seed=n)
+        x = np.where(np.isinf(x), np.float32(-3.4028234663852886e38), x).astype(np.float32)
+        if op == "max_plus":  # a DAG, so longest paths exist
+            x = np.where(np.triu(np.ones((n, n), bool), 1), x, np.float32(-3.4028234663852886e38)).astype(np.float32)
+        graphs.append(x)
+    mats = [torch.from_numpy(g.copy()).cuda() for g in graphs]
+    its = s2.closure_batched(op, mats, conv="aplp")
+    for g, m, it in zip(graphs, mats, its):
+        want, steps = oracle.closure(op, g, tol_mode=2)
+        assert it == steps
+        same(m, want)
+    assert s2.device_status() == 0
+
+
 @pytest.mark.parametrize("op", ["min_plus", "max_min", "max_mul"])
 def test_plan_memory(cuda, op):
     """Both operand layouts of X, twice: 16 bytes an element, codes or not."""
